@@ -78,7 +78,7 @@ struct ItemCtx {
     const double *eorb, *dintc1, *dintx1, *t1v1, *dintc2, *dintx2, *t1v2;
     double *out, *out1;  // energy slots of the item's pair (and of the second pair of a packed item)
     double eaijk;
-    int ncor, nocc, nvir, b0, c0, diag, nV, nch, state;  // state: 1 work, 0 malformed, -1 end
+    int ncor, nocc, nvir, b0, c0, diag, same, nch, state;  // same: i == k; state: 1 work, 0 malformed, -1 end
     int packed, b1;      // packed edge item: pairs (b0, c0) and (b1, c0); b1 < 0 when the second is absent
     // split item (the one-triple system of a split launch): 1 | half << 1 | pair << 2, else 0; this half
     // runs chunks half, half + 2, ...  One int keeps the context at 128 bytes: at 160 bytes (the split
@@ -131,6 +131,18 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long *b, unsigned pa
     unsigned ok;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(saddr(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+// Whether the phase with the given parity has completed, without waiting.
+__device__ __forceinline__ bool mbar_test_wait(unsigned long long *b, unsigned parity)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(ok)
         : "r"(saddr(b)), "r"(parity)
         : "memory");
@@ -203,7 +215,7 @@ __device__ __forceinline__ int kmajor_off(int kk, int x)
 struct FragOffsets {
     int kA0, kA1, kA2, kA3;  // K-major A fragment: (2t, r), (2t, r+8), (2t+1, r), (2t+1, r+8)
     int kB0, kB1;            // K-major B fragment: (2t, c), (2t+1, c)
-    int xA0, xA1;            // X-major A fragment: rows r, r+8 at contraction 2t (128-bit)
+    int xA0;                 // X-major A fragment: rows r and (1024 bytes on) r+8 at contraction 2t (128-bit)
     int xB;                  // X-major B fragment: column c at contraction 2t (128-bit)
     __device__ __forceinline__ FragOffsets(int rx0, int cx0, int g, int t)
     {
@@ -215,7 +227,6 @@ struct FragOffsets {
         kB0 = kmajor_off(2 * t, c);
         kB1 = kmajor_off(2 * t + 1, c);
         xA0 = r * 128 + ((t ^ (r & 7)) << 4);
-        xA1 = (r + 8) * 128 + ((t ^ ((r + 8) & 7)) << 4);
         xB = c * 128 + ((t ^ (c & 7)) << 4);
     }
     __device__ __forceinline__ static double ld(const char *p, int off) { return *reinterpret_cast<const double *>(p + off); }
@@ -234,7 +245,7 @@ struct FragOffsets {
     }
     __device__ __forceinline__ void ldA_X(double (&a)[4], const char *P, int kx) const
     {
-        const double2 lo = ld2(P, xA0 ^ kx), hi = ld2(P, xA1 ^ kx);
+        const double2 lo = ld2(P, xA0 ^ kx), hi = ld2(P, (xA0 ^ kx) + 1024);
         a[0] = lo.x;
         a[2] = lo.y;
         a[1] = hi.x;
@@ -271,74 +282,270 @@ __device__ __forceinline__ void ld_b16_X(const FragOffsets &fo, double (&b)[4], 
     fo.ldB_X(*reinterpret_cast<double(*)[2]>(&b[2]), P, 64);
 }
 
-// One family's products of a packed edge item in one stage slot (layout at PK_*): this warp's
-// sub-block of pair pp, f_x(b,c) = A_x(b,.) B_x(.,c) and f_x(c,b) through the operand-swapped MMA,
-// exactly as the normal items compute them from their o = 0 / o = 1 panels.
-template <int KS, int FAM>
-__device__ __forceinline__ void packed_family(const FragOffsets &fo, const char *st, int pp, bool ph1, int kval,
-                                              double (&f)[8][4], double (&gT)[8][4])
+// ------------------------------------------------------------------------------------------------
+// products of one chunk
+// ------------------------------------------------------------------------------------------------
+// Fragments of one group of four m16n8k8: two A operands, two B operands.
+struct Group {
+    double a0[4], a1[4], b0[2], b1[2];
+};
+
+// Byte offsets of the panels that one family's groups read: the two A operands (K-major), B_1 (K-major, in the
+// occupied phase X-major) and B_3 (X-major) of the products at (b, c) (o = 0) and of the transposes (o = 1).
+struct Panels {
+    int a0[2], a1[2], b0[2], b1[2];
+};
+
+// Ordinary items: panel 2 q + o of the family's eight holds operand q (A_J, A_K, B_1, B_3) of orientation o.
+template <int FAM> __device__ __forceinline__ constexpr Panels item_panels()
+{
+    constexpr int P = FAM * 8 * PANEL_BYTES, S = PANEL_BYTES;
+    return {{P, P + 5 * S}, {P + 2 * S, P + 7 * S}, {P + 4 * S, P + S}, {P + 6 * S, P + 3 * S}};
+}
+
+// Packed edge items (layout at PK_*): pair pp of the two that share the slot.
+__device__ __forceinline__ Panels packed_panels(int pp)
+{
+    constexpr int S = PANEL_BYTES;
+    return {{(PK_A + pp) * S, (PK_B1B + pp) * S},
+            {(PK_A + 2 + pp) * S, (PK_B3B + pp) * S},
+            {PK_B1E * S, PK_AE * S},
+            {PK_B3E * S, (PK_AE + 1) * S}};
+}
+
+// Group O of k-step ks.  O = 0: A_J, A_K rows and B_1, B_3 columns; f1 = A_J B_1, f2 = A_K B_1, f3 = A_J B_3,
+// f4 = A_K B_3 at (b, c).  O = 1: the transposes f_x(c,b) = sum_d B_x(d,b) A_x(c,d): a0, a1 = B_1, B_3 and
+// b0, b1 = A_J, A_K of the C side.  PH1: the occupied phase, where B_1 is X-major.
+template <bool PH1, int O>
+__device__ __forceinline__ void load_group(const FragOffsets &fo, const char *st, const Panels &pn, int ks, Group &g)
+{
+    const int kk = ks * 1024, kx = ks * 64;  // K-major: 8 rows further; X-major: 64 bytes into each row
+    if (O == 0) {
+        fo.ldA_K(g.a0, st + pn.a0[0] + kk);
+        fo.ldA_K(g.a1, st + pn.a1[0] + kk);
+        fo.ldB_X(g.b1, st + pn.b1[0], kx);
+        if (!PH1)
+            fo.ldB_K(g.b0, st + pn.b0[0] + kk);
+        else
+            fo.ldB_X(g.b0, st + pn.b0[0], kx);
+    } else {
+        fo.ldB_K(g.b0, st + pn.b0[1] + kk);
+        fo.ldB_K(g.b1, st + pn.b1[1] + kk);
+        fo.ldA_X(g.a1, st + pn.a1[1], kx);
+        if (!PH1)
+            fo.ldA_K(g.a0, st + pn.a0[1] + kk);
+        else
+            fo.ldA_X(g.a0, st + pn.a0[1], kx);
+    }
+}
+
+template <int FAM, int O>
+__device__ __forceinline__ void mma_group(const Group &g, double (&f)[8][4], double (&gT)[8][4])
 {
     constexpr int x0 = FAM * 4;
-    const char *AJ = st + (PK_A + pp) * PANEL_BYTES, *AK = st + (PK_A + 2 + pp) * PANEL_BYTES;
-    const char *B1 = st + PK_B1E * PANEL_BYTES, *B3 = st + PK_B3E * PANEL_BYTES;
-    const char *AJE = st + PK_AE * PANEL_BYTES, *AKE = st + (PK_AE + 1) * PANEL_BYTES;
-    const char *B1B = st + (PK_B1B + pp) * PANEL_BYTES, *B3B = st + (PK_B3B + pp) * PANEL_BYTES;
-    if (KS == 16 && kval > 8) {
-        double aJ[8], aK[8], b1[4], b3[4];
-        ld_a16_K(fo, aJ, AJ);
-        ld_a16_K(fo, aK, AK);
-        ld_b16_X(fo, b3, B3);
-        if (!ph1)
-            ld_b16_K(fo, b1, B1);
-        else
-            ld_b16_X(fo, b1, B1);
-        dmma_16x8x16(f[x0 + 0], aJ, b1);
-        dmma_16x8x16(f[x0 + 1], aK, b1);
-        dmma_16x8x16(f[x0 + 2], aJ, b3);
-        dmma_16x8x16(f[x0 + 3], aK, b3);
-        double a1[8], a3[8], bJ[4], bK[4];
-        ld_b16_K(fo, bJ, AJE);
-        ld_b16_K(fo, bK, AKE);
-        ld_a16_X(fo, a3, B3B);
-        if (!ph1)
-            ld_a16_K(fo, a1, B1B);
-        else
-            ld_a16_X(fo, a1, B1B);
-        dmma_16x8x16(gT[x0 + 0], a1, bJ);
-        dmma_16x8x16(gT[x0 + 1], a1, bK);
-        dmma_16x8x16(gT[x0 + 2], a3, bJ);
-        dmma_16x8x16(gT[x0 + 3], a3, bK);
+    if (O == 0) {
+        dmma_16x8x8(f[x0 + 0], g.a0, g.b0);
+        dmma_16x8x8(f[x0 + 1], g.a1, g.b0);
+        dmma_16x8x8(f[x0 + 2], g.a0, g.b1);
+        dmma_16x8x8(f[x0 + 3], g.a1, g.b1);
     } else {
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-            if (ks == 1 && kval <= 8) break;
-            const int kk = ks * 1024, kx = ks * 64;
-            double aJ[4], aK[4], b1[2], b3[2];
-            fo.ldA_K(aJ, AJ + kk);
-            fo.ldA_K(aK, AK + kk);
-            fo.ldB_X(b3, B3, kx);
-            if (!ph1)
-                fo.ldB_K(b1, B1 + kk);
-            else
-                fo.ldB_X(b1, B1, kx);
-            dmma_16x8x8(f[x0 + 0], aJ, b1);
-            dmma_16x8x8(f[x0 + 1], aK, b1);
-            dmma_16x8x8(f[x0 + 2], aJ, b3);
-            dmma_16x8x8(f[x0 + 3], aK, b3);
-            double a1[4], a3[4], bJ[2], bK[2];
-            fo.ldB_K(bJ, AJE + kk);
-            fo.ldB_K(bK, AKE + kk);
-            fo.ldA_X(a3, B3B, kx);
-            if (!ph1)
-                fo.ldA_K(a1, B1B + kk);
-            else
-                fo.ldA_X(a1, B1B, kx);
-            dmma_16x8x8(gT[x0 + 0], a1, bJ);
-            dmma_16x8x8(gT[x0 + 1], a1, bK);
-            dmma_16x8x8(gT[x0 + 2], a3, bJ);
-            dmma_16x8x8(gT[x0 + 3], a3, bK);
+        dmma_16x8x8(gT[x0 + 0], g.a0, g.b0);
+        dmma_16x8x8(gT[x0 + 1], g.a0, g.b1);
+        dmma_16x8x8(gT[x0 + 2], g.a1, g.b0);
+        dmma_16x8x8(gT[x0 + 3], g.a1, g.b1);
+    }
+}
+
+// The same four products over both k-steps of a chunk with m16n8k16 (ordinary items).
+template <bool PH1, int FAM, int O>
+__device__ __forceinline__ void group16(const FragOffsets &fo, const char *st, double (&f)[8][4], double (&gT)[8][4])
+{
+    constexpr int x0 = FAM * 4;
+    constexpr Panels pn = item_panels<FAM>();
+    double a0[8], a1[8], b0[4], b1[4];
+    if (O == 0) {
+        ld_a16_K(fo, a0, st + pn.a0[0]);
+        ld_a16_K(fo, a1, st + pn.a1[0]);
+        ld_b16_X(fo, b1, st + pn.b1[0]);
+        if (!PH1)
+            ld_b16_K(fo, b0, st + pn.b0[0]);
+        else
+            ld_b16_X(fo, b0, st + pn.b0[0]);
+        dmma_16x8x16(f[x0 + 0], a0, b0);
+        dmma_16x8x16(f[x0 + 1], a1, b0);
+        dmma_16x8x16(f[x0 + 2], a0, b1);
+        dmma_16x8x16(f[x0 + 3], a1, b1);
+    } else {
+        ld_b16_K(fo, b0, st + pn.b0[1]);
+        ld_b16_K(fo, b1, st + pn.b1[1]);
+        ld_a16_X(fo, a1, st + pn.a1[1]);
+        if (!PH1)
+            ld_a16_K(fo, a0, st + pn.a0[1]);
+        else
+            ld_a16_X(fo, a0, st + pn.a0[1]);
+        dmma_16x8x16(gT[x0 + 0], a0, b0);
+        dmma_16x8x16(gT[x0 + 1], a0, b1);
+        dmma_16x8x16(gT[x0 + 2], a1, b0);
+        dmma_16x8x16(gT[x0 + 3], a1, b1);
+    }
+}
+
+// A consumer warp's place in the stage ring.
+struct RingPos {
+    int stage;
+    unsigned phase;
+    bool ready;  // the stage's full barrier is known to have completed
+    __device__ __forceinline__ void next()
+    {
+        if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
         }
     }
+};
+
+// What a consumer warp's chunk loops need besides the accumulators.
+struct Pipe {
+    const char *stages;
+    unsigned long long *full, *empty;
+    int *status;
+    int lane;
+    __device__ __forceinline__ bool wait(const RingPos &rp) const
+    {
+        return rp.ready || mbar_wait(&full[rp.stage], rp.phase, status);
+    }
+    // releases the stage and looks at the next one without waiting for it
+    __device__ __forceinline__ void release(RingPos &rp) const
+    {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[rp.stage]);
+        rp.next();
+        rp.ready = mbar_test_wait(&full[rp.stage], rp.phase);
+    }
+};
+
+// Products of family FAM with the k8 steps of a chunk, except (TAIL) the last group's MMAs, whose fragments are
+// left in `tail`: the caller releases the stage and looks at the next one in between, so neither the barrier
+// nor the first fragment loads of the next chunk leave the tensor pipe idle.  NKS: k8 steps of the chunk (1
+// when the second lies entirely in the zero padding).  A diagonal pair (DIAG) gets f(c,b) from the other warps
+// at the end of the item.
+template <int NKS, bool PH1, bool DIAG, int FAM, bool TAIL>
+__device__ __forceinline__ void family_products(const FragOffsets &fo, const char *st, const Panels &pn,
+                                                double (&f)[8][4], double (&gT)[8][4], Group &tail)
+{
+    Group g;
+#pragma unroll
+    for (int ks = 0; ks < NKS; ++ks) {
+        const bool last = TAIL && ks == NKS - 1;
+        if (DIAG && last) {
+            load_group<PH1, 0>(fo, st, pn, ks, tail);
+            return;
+        }
+        load_group<PH1, 0>(fo, st, pn, ks, g);
+        mma_group<FAM, 0>(g, f, gT);
+        if (DIAG) continue;
+        if (last) {
+            load_group<PH1, 1>(fo, st, pn, ks, tail);
+            return;
+        }
+        load_group<PH1, 1>(fo, st, pn, ks, g);
+        mma_group<FAM, 1>(g, f, gT);
+    }
+}
+
+// n chunks of one kind of an ordinary item.  Everything that differs between chunks (phase, diagonal pair,
+// number of k-steps, SAME: i == k, where the t family equals the n family and is not computed) is a template
+// parameter, so that a chunk is straight-line code and the fragment loads of one group are scheduled over the
+// MMAs of the group before.  With the same choices as branches between the groups, and generic instead of
+// shared-memory loads, the MMA loop ran at 76 % of the FP64 tensor pipe's rate (measured without epilogue).
+template <int KS, int NKS, bool PH1, bool DIAG, bool SAME>
+__device__ __forceinline__ bool run_chunks(int n, const FragOffsets &fo, const Pipe &pp, RingPos &rp, double (&f)[8][4],
+                                           double (&gT)[8][4])
+{
+    constexpr bool K16 = KS == 16 && NKS == 2;
+    constexpr int LAST = SAME ? 0 : 1;
+#pragma unroll 1
+    for (; n > 0; --n) {
+        if (!pp.wait(rp)) return false;
+        const char *st = pp.stages + (size_t)rp.stage * STAGE_BYTES;
+        Group tail;
+        if (K16) {
+            group16<PH1, 0, 0>(fo, st, f, gT);
+            if (!DIAG) group16<PH1, 0, 1>(fo, st, f, gT);
+            if (!SAME) group16<PH1, 1, 0>(fo, st, f, gT);
+            if (!SAME && !DIAG) group16<PH1, 1, 1>(fo, st, f, gT);
+        } else {
+            if (!SAME) family_products<NKS, PH1, DIAG, 0, false>(fo, st, item_panels<0>(), f, gT, tail);
+            family_products<NKS, PH1, DIAG, LAST, true>(fo, st, item_panels<LAST>(), f, gT, tail);
+        }
+        pp.release(rp);
+        if (!K16) mma_group<LAST, DIAG ? 0 : 1>(tail, f, gT);
+    }
+    return true;
+}
+
+// n chunks of a packed edge item: one stage slot per (chunk, family), m16n8k8 in both kernels (the packed path's
+// extra fragment registers would push the k16 kernel's MMA warps past their register budget).
+template <int NKS, bool PH1, bool SAME>
+__device__ __forceinline__ bool run_packed(int n, const FragOffsets &fo, const Panels &pn, const Pipe &pp, RingPos &rp,
+                                           double (&f)[8][4], double (&gT)[8][4])
+{
+#pragma unroll 1
+    for (; n > 0; --n) {
+        Group tail;
+        if (!pp.wait(rp)) return false;
+        family_products<NKS, PH1, false, 0, true>(fo, pp.stages + (size_t)rp.stage * STAGE_BYTES, pn, f, gT, tail);
+        pp.release(rp);
+        mma_group<0, 1>(tail, f, gT);
+        if (SAME) continue;
+        if (!pp.wait(rp)) return false;
+        family_products<NKS, PH1, false, 1, true>(fo, pp.stages + (size_t)rp.stage * STAGE_BYTES, pn, f, gT, tail);
+        pp.release(rp);
+        mma_group<1, 1>(tail, f, gT);
+    }
+    return true;
+}
+
+// Chunk indices lo <= ch < hi with the item's parity (split items take every second chunk).
+__device__ __forceinline__ int count_chunks(int lo, int hi, int first, int step)
+{
+    if (step == 1) return hi - lo;
+    const int c0 = lo + ((lo ^ first) & 1);
+    return c0 < hi ? (hi - c0 + 1) >> 1 : 0;
+}
+
+// The item's chunks by kind: full and one-k-step chunks of the virtual phase, then of the occupied one (the last
+// chunk of a phase runs one k-step when the second lies entirely in the zero padding).
+struct ChunkCounts {
+    int v2, v1, o2, o1;
+    __device__ __forceinline__ ChunkCounts(int nvir, int nocc, int first, int step)
+    {
+        const int nV = (nvir + DK - 1) / DK, nO = (nocc + DK - 1) / DK;
+        v1 = nvir - (nV - 1) * DK <= 8 ? count_chunks(nV - 1, nV, first, step) : 0;
+        o1 = nocc - (nO - 1) * DK <= 8 ? count_chunks(nV + nO - 1, nV + nO, first, step) : 0;
+        v2 = count_chunks(0, nV, first, step) - v1;
+        o2 = count_chunks(nV, nV + nO, first, step) - o1;
+    }
+};
+
+template <int KS, bool DIAG, bool SAME>
+__device__ __forceinline__ bool run_item(const ChunkCounts &n, const FragOffsets &fo, const Pipe &pp, RingPos &rp,
+                                         double (&f)[8][4], double (&gT)[8][4])
+{
+    return run_chunks<KS, 2, false, DIAG, SAME>(n.v2, fo, pp, rp, f, gT) &&
+           run_chunks<KS, 1, false, DIAG, SAME>(n.v1, fo, pp, rp, f, gT) &&
+           run_chunks<KS, 2, true, DIAG, SAME>(n.o2, fo, pp, rp, f, gT) &&
+           run_chunks<KS, 1, true, DIAG, SAME>(n.o1, fo, pp, rp, f, gT);
+}
+
+template <bool SAME>
+__device__ __forceinline__ bool run_packed_item(const ChunkCounts &n, const FragOffsets &fo, const Panels &pn,
+                                                const Pipe &pp, RingPos &rp, double (&f)[8][4], double (&gT)[8][4])
+{
+    return run_packed<2, false, SAME>(n.v2, fo, pn, pp, rp, f, gT) &&
+           run_packed<1, false, SAME>(n.v1, fo, pn, pp, rp, f, gT) &&
+           run_packed<2, true, SAME>(n.o2, fo, pn, pp, rp, f, gT) &&
+           run_packed<1, true, SAME>(n.o1, fo, pn, pp, rp, f, gT);
 }
 
 // Brings the 128-byte lines of the energy vectors the item's epilogue will read into L1 (lanes 0..27:
@@ -364,32 +571,39 @@ __device__ __forceinline__ void prefetch_epilogue(const ItemCtx &cx, int lane)
 // ------------------------------------------------------------------------------------------------
 // energies of one warp's sub-block, in registers (as fused.cu)
 // ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ TengyIdx load_idx(const ItemCtx &cx, int x)
+{
+    return {__ldg(cx.t1v1 + x), __ldg(cx.t1v2 + x), __ldg(cx.dintx1 + x), __ldg(cx.dintx2 + x), __ldg(cx.dintc1 + x),
+            __ldg(cx.dintc2 + x)};
+}
+
+// DIAG: the pair's own mirror block is a block of the same tile (another warp, or this one, adds its terms).
+template <bool DIAG>
 __device__ __forceinline__ void warp_epilogue(const ItemCtx &cx, const double (&f)[8][4], const double (&gT)[8][4],
                                               int rb0, int cb0, int g, int t, int lane, double *out)
 {
     TengySums su = {0.0, 0.0, 0.0, 0.0};
-    const int V = cx.nvir, voff = cx.ncor + cx.nocc;
+    const int V = cx.nvir;
+    const double *ev = cx.eorb + cx.ncor + cx.nocc;
     const double eaijk = cx.eaijk;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int b = rb0 + perm8(g) + ((e & 2) ? 8 : 0);
-        const int c = cb0 + perm8(2 * t + (e & 1));
-        if (b < V && c < V) {
+    for (int h = 0; h < 2; ++h) {
+        const int b = rb0 + perm8(g) + 8 * h;
+        if (b >= V) continue;
+        const TengyIdx vb = load_idx(cx, b);
+        const double eb = __ldg(ev + b);
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const int e = 2 * h + w, c = cb0 + perm8(2 * t + w);
+            if (c >= V) continue;
             double fbc[8], fcb[8];
 #pragma unroll
             for (int x = 0; x < 8; ++x) {
                 fbc[x] = f[x][e];
                 fcb[x] = gT[x][e];
             }
-            const double eb = __ldg(cx.eorb + voff + b), ec = __ldg(cx.eorb + voff + c);
             // omp/ccsd_tengy_c99.c:65 denominator; e_b + e_c == e_c + e_b, so (b,c) and (c,b) share it
-            const double denom = -1.0 / (eb + ec + eaijk);
-            // term at (b,c): :91-111 forms
-            tengy_term_factored(fbc, fcb, denom, __ldg(cx.t1v1 + b), __ldg(cx.t1v2 + b), __ldg(cx.dintx1 + c),
-                                __ldg(cx.dintx2 + c), __ldg(cx.dintc1 + c), __ldg(cx.dintc2 + c), su);
-            if (!cx.diag)  // term at (c,b) of the mirrored tile
-                tengy_term_factored(fcb, fbc, denom, __ldg(cx.t1v1 + c), __ldg(cx.t1v2 + c), __ldg(cx.dintx1 + b),
-                                    __ldg(cx.dintx2 + b), __ldg(cx.dintc1 + b), __ldg(cx.dintc2 + b), su);
+            tengy_pair<!DIAG>(fbc, fcb, -1.0 / (eb + __ldg(ev + c) + eaijk), vb, load_idx(cx, c), su);
         }
     }
     su.e4i = warp_sum(su.e4i);
@@ -488,6 +702,8 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
         }
         const int nV = (V + DK - 1) / DK, nO = (O + DK - 1) / DK;
         const bool diag = (B == C);
+        // i == k: both families read the same blocks (a staged one-triple system holds them twice and may not)
+        const bool same = i == k && !one;
         if (lane == 0) {
             cx.eorb = S.eorb;
             const size_t ao = (size_t)ai * zO;  // the a block of the a-dependent vectors
@@ -512,7 +728,7 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
             cx.b0 = B0;
             cx.c0 = C0;
             cx.diag = diag;
-            cx.nV = nV;
+            cx.same = same;
             cx.split_tag = (SPLIT && S.split) ? 1 | hpart << 1 | (int)own << 2 : 0;
             cx.nch = (SPLIT && S.split) ? (nV + nO - hpart + 1) / 2 : nV + nO;
             cx.state = 1;
@@ -544,7 +760,7 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
             tb = tb >= 0 ? tb * T : -1;
             const int pch0 = (SPLIT && S.split) ? hpart : 0, pstep = (SPLIT && S.split) ? 2 : 1;
             const int nsl = 2 * ((SPLIT && S.split) ? (nV + nO - hpart + 1) / 2 : nV + nO);
-            for (int sl = 0; sl < nsl; ++sl) {
+            for (int sl = 0; sl < nsl; sl += same ? 2 : 1) {
                 if (!mbar_wait(&empty[stage], phase ^ 1, status)) return;
                 const int fam = sl & 1, ch = pch0 + (sl >> 1) * pstep;
                 const bool ph1 = ch >= nV;
@@ -597,8 +813,8 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
         const int cb = o ? B0 : C0;                      // B columns: C for (B,C), B for (C,B)
         const int half = slot & 1;                       // second 16-row box of a K-major panel
         const int pnl = fam * 8 + (slot < 2 ? 0 : slot < 4 ? 2 : slot < 6 ? 4 : 6) + o;
-        const bool mine = lane < 28 && (!diag || o == 0);
-        const unsigned bytes = (diag ? NPANEL / 2 : NPANEL) * PANEL_BYTES;
+        const bool mine = lane < 28 && (!diag || o == 0) && (!same || fam == 0);
+        const unsigned bytes = ((NPANEL * PANEL_BYTES) >> (diag ? 1 : 0)) >> (same ? 1 : 0);
         for (int ch = (SPLIT && S.split) ? hpart : 0; ch < nV + nO; ch += (SPLIT && S.split) ? 2 : 1) {
             if (!mbar_wait(&empty[stage], phase ^ 1, status)) return;
             if (lane == 0) mbar_arrive_expect_tx(&full[stage], bytes);
@@ -678,6 +894,28 @@ __device__ __forceinline__ bool split_combine(const trpdrv_dev_system *__restric
     return true;
 }
 
+// Releases the n stage slots of an item whose sub-block of this warp lies entirely in the padding.
+__device__ __forceinline__ bool skip_slots(int n, const Pipe &pp, RingPos &rp)
+{
+    for (; n > 0; --n) {
+        if (!pp.wait(rp)) return false;
+        pp.release(rp);
+    }
+    return true;
+}
+
+// i == k: the t family's operands are the n family's, so its products are the same numbers.
+__device__ __forceinline__ void copy_families(double (&f)[8][4], double (&gT)[8][4])
+{
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            f[4 + x][e] = f[x][e];
+            gT[4 + x][e] = gT[x][e];
+        }
+}
+
 // ------------------------------------------------------------------------------------------------
 template <int KS, bool SPLIT>
 __global__ void __launch_bounds__(NTHREAD, 1)
@@ -690,7 +928,9 @@ fused_tma_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long 
     __shared__ double xbuf[2 * XBUF];                       // diagonal-pair transpose exchange
     __shared__ __align__(8) unsigned long long xbar[1];
     __shared__ int split_flag[1];
-    char *stages = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    // aligned by an offset, not by integer arithmetic on the pointer: the compiler then still knows that the
+    // fragment reads are shared-memory loads (32-bit addresses)
+    char *stages = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
@@ -717,10 +957,12 @@ fused_tma_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long 
     const FragOffsets fo(rx0, cx0, g, t);
 
     double f[8][4], gT[8][4];
-    int stage = 0;
-    unsigned phase = 0, xphase = 0;
+    const Pipe pipe = {stages, full, empty, status, lane};
+    RingPos rp = {0, 0u, false};
+    unsigned xphase = 0;
     for (long long n = 0;; ++n) {
-        if (!mbar_wait(&full[stage], phase, status)) return;
+        if (!pipe.wait(rp)) return;
+        rp.ready = true;
         const ItemCtx &cx = ring[n % RING];
         const int state = cx.state;
         if (state < 0) return;
@@ -729,58 +971,40 @@ fused_tma_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long 
                 double *o = cx.out + warp * 4;
                 o[0] = o[1] = o[2] = o[3] = 0.0;
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[stage]);
-            if (++stage == STAGES) {
-                stage = 0;
-                phase ^= 1;
-            }
+            pipe.release(rp);
             continue;
         }
 #pragma unroll
         for (int x = 0; x < 8; ++x)
 #pragma unroll
             for (int e = 0; e < 4; ++e) f[x][e] = gT[x][e] = 0.0;
+        const int first = SPLIT ? (cx.split_tag >> 1) & 1 : 0, step = SPLIT ? (cx.split_tag & 1) + 1 : 1;
+        const ChunkCounts nc(cx.nvir, cx.nocc, first, step);
+        const bool same = cx.same != 0;
+        prefetch_epilogue(cx, lane);
         if (cx.packed) {
             // two edge pairs (b0, c0) and (b1, c0): warp w takes pair w >> 2, sub-block w & 3 of it; each
             // (chunk, family) has its own stage slot
-            const int pp = warp >> 2, sub = warp & 3, prs = sub >> 1, pcs = sub & 1;
-            const FragOffsets fp(prs * 16, pcs * 8, g, t);
-            const int pb0 = pp ? cx.b1 : cx.b0;
-            const bool pactive = pb0 >= 0 && cx.c0 + pcs * 8 < cx.nvir;
-            const int nsl = 2 * cx.nch, pnV = cx.nV;
-            // per-item values in registers: every field read after a wait would be reloaded from the ring
-            const int inocc = cx.nocc, invir = cx.nvir;
-            const int ich0 = SPLIT ? (cx.split_tag >> 1) & 1 : 0, istep = SPLIT ? (cx.split_tag & 1) + 1 : 1;
-            for (int sl = 0; sl < nsl; ++sl) {
-                if (sl > 0 && !mbar_wait(&full[stage], phase, status)) return;
-                const char *st = stages + (size_t)stage * STAGE_BYTES;
-                const int ch = ich0 + (sl >> 1) * istep;
-                const bool ph1 = ch >= pnV;
-                const int kval = ph1 ? inocc - (ch - pnV) * DK : invir - ch * DK;
-                if (pactive) {
-                    // m16n8k8 here in both kernels: the packed path's extra fragment registers would
-                    // push the k16 kernel's MMA warps past their register budget
-                    if (sl & 1)
-                        packed_family<8, 1>(fp, st, pp, ph1, kval, f, gT);
-                    else
-                        packed_family<8, 0>(fp, st, pp, ph1, kval, f, gT);
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&empty[stage]);
-                if (++stage == STAGES) {
-                    stage = 0;
-                    phase ^= 1;
-                }
+            const int pair = warp >> 2, sub = warp & 3, prs = sub >> 1, pcs = sub & 1;
+            const int pb0 = pair ? cx.b1 : cx.b0;
+            if (pb0 >= 0 && cx.c0 + pcs * 8 < cx.nvir) {
+                const FragOffsets fp(prs * 16, pcs * 8, g, t);
+                const Panels pn = packed_panels(pair);
+                if (!(same ? run_packed_item<true>(nc, fp, pn, pipe, rp, f, gT)
+                           : run_packed_item<false>(nc, fp, pn, pipe, rp, f, gT)))
+                    return;
+            } else if (!skip_slots(same ? cx.nch : 2 * cx.nch, pipe, rp)) {
+                return;
             }
             if (SPLIT && (cx.split_tag & 1)) {
                 int fin = 0;
                 if (!split_combine(sys, cx, f, gT, warp, lane, xbar, xphase, split_flag, status, fin)) return;
                 if (!fin) continue;
             }
+            if (same) copy_families(f, gT);
             if (pb0 >= 0) {  // this pair's slots: the 4 sub-blocks' sums, zeros in the other 4
-                double *out = pp ? cx.out1 : cx.out;
-                warp_epilogue(cx, f, gT, pb0 + prs * 16, cx.c0 + pcs * 8, g, t, lane, out + sub * 4);
+                double *out = pair ? cx.out1 : cx.out;
+                warp_epilogue<false>(cx, f, gT, pb0 + prs * 16, cx.c0 + pcs * 8, g, t, lane, out + sub * 4);
                 if (lane == 0) {
                     double *z = out + (sub + 4) * 4;
                     z[0] = z[1] = z[2] = z[3] = 0.0;
@@ -788,103 +1012,18 @@ fused_tma_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long 
             }
             continue;
         }
-        const int nch = cx.nch, nV = cx.nV;
-        // per-item values in registers: every field read after a wait would be reloaded from the ring
-        const int inocc = cx.nocc, invir = cx.nvir;
-        const int ich0 = SPLIT ? (cx.split_tag >> 1) & 1 : 0, istep = SPLIT ? (cx.split_tag & 1) + 1 : 1;
-        const bool active = (cx.b0 + rx0 < cx.nvir) && (cx.c0 + cx0 < cx.nvir);
         const bool diag = cx.diag != 0;
-        const int pf = nch > 3 ? nch - 3 : 0;
-        for (int c = 0; c < nch; ++c) {
-            const int ch = ich0 + c * istep;
-            if (c > 0 && !mbar_wait(&full[stage], phase, status)) return;
-            const char *st = stages + (size_t)stage * STAGE_BYTES;
-            const bool ph1 = ch >= nV;
-            // the second k-step of a chunk is skipped when it lies entirely in the zero padding
-            const int kval = ph1 ? inocc - (ch - nV) * DK : invir - ch * DK;
-            if (c == pf) prefetch_epilogue(cx, lane);
-            if (KS == 16 && active && kval > 8) {
-                // one m16n8k16 per product: the fragments of both k-steps of the chunk side by side
-#pragma unroll
-                for (int fam = 0; fam < 2; ++fam) {
-                    const char *P = st + fam * 8 * PANEL_BYTES;   // o = 0 panels
-                    const char *Q = P + PANEL_BYTES;             // o = 1 panels
-                    const int x0 = fam * 4;
-                    double aJ[8], aK[8], b1[4], b3[4];
-                    ld_a16_K(fo, aJ, P + 0 * PANEL_BYTES);
-                    ld_a16_K(fo, aK, P + 2 * PANEL_BYTES);
-                    ld_b16_X(fo, b3, P + 6 * PANEL_BYTES);
-                    if (!ph1)
-                        ld_b16_K(fo, b1, P + 4 * PANEL_BYTES);
-                    else
-                        ld_b16_X(fo, b1, P + 4 * PANEL_BYTES);
-                    dmma_16x8x16(f[x0 + 0], aJ, b1);
-                    dmma_16x8x16(f[x0 + 1], aK, b1);
-                    dmma_16x8x16(f[x0 + 2], aJ, b3);
-                    dmma_16x8x16(f[x0 + 3], aK, b3);
-                    if (!diag) {
-                        double a1[8], a3[8], bJ[4], bK[4];
-                        ld_b16_K(fo, bJ, Q + 0 * PANEL_BYTES);
-                        ld_b16_K(fo, bK, Q + 2 * PANEL_BYTES);
-                        ld_a16_X(fo, a3, Q + 6 * PANEL_BYTES);
-                        if (!ph1)
-                            ld_a16_K(fo, a1, Q + 4 * PANEL_BYTES);
-                        else
-                            ld_a16_X(fo, a1, Q + 4 * PANEL_BYTES);
-                        dmma_16x8x16(gT[x0 + 0], a1, bJ);
-                        dmma_16x8x16(gT[x0 + 1], a1, bK);
-                        dmma_16x8x16(gT[x0 + 2], a3, bJ);
-                        dmma_16x8x16(gT[x0 + 3], a3, bK);
-                    }
-                }
-            } else if (active) {
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-                for (int fam = 0; fam < 2; ++fam) {
-                    if (ks == 1 && kval <= 8) break;
-                    const char *P = st + fam * 8 * PANEL_BYTES + ks * 1024;    // o = 0 panels (K-major k-step)
-                    const char *Q = P + PANEL_BYTES;               // o = 1 panels (C side)
-                    const char *PX = st + fam * 8 * PANEL_BYTES;   // X-major bases
-                    const char *QX = PX + PANEL_BYTES;
-                    const int kx = ks * 64;
-                    const int x0 = fam * 4;
-                    double aJ[4], aK[4], b1[2], b3[2];
-                    fo.ldA_K(aJ, P + 0 * PANEL_BYTES);
-                    fo.ldA_K(aK, P + 2 * PANEL_BYTES);
-                    fo.ldB_X(b3, PX + 6 * PANEL_BYTES, kx);
-                    if (!ph1)
-                        fo.ldB_K(b1, P + 4 * PANEL_BYTES);
-                    else
-                        fo.ldB_X(b1, PX + 4 * PANEL_BYTES, kx);
-                    // f1 = A_J B_1, f2 = A_K B_1, f3 = A_J B_3, f4 = A_K B_3
-                    dmma_16x8x8(f[x0 + 0], aJ, b1);
-                    dmma_16x8x8(f[x0 + 1], aK, b1);
-                    dmma_16x8x8(f[x0 + 2], aJ, b3);
-                    dmma_16x8x8(f[x0 + 3], aK, b3);
-                    if (!diag) {  // a diagonal pair gets f(c,b) from the other warps instead (below)
-                        double a1[4], a3[4], bJ[2], bK[2];
-                        fo.ldB_K(bJ, Q + 0 * PANEL_BYTES);
-                        fo.ldB_K(bK, Q + 2 * PANEL_BYTES);
-                        fo.ldA_X(a3, QX + 6 * PANEL_BYTES, kx);
-                        if (!ph1)
-                            fo.ldA_K(a1, Q + 4 * PANEL_BYTES);
-                        else
-                            fo.ldA_X(a1, QX + 4 * PANEL_BYTES, kx);
-                        // transposes: f_x(c,b) = sum_d B_x(d,b) A_x(c,d)
-                        dmma_16x8x8(gT[x0 + 0], a1, bJ);
-                        dmma_16x8x8(gT[x0 + 1], a1, bK);
-                        dmma_16x8x8(gT[x0 + 2], a3, bJ);
-                        dmma_16x8x8(gT[x0 + 3], a3, bK);
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[stage]);
-            if (++stage == STAGES) {
-                stage = 0;
-                phase ^= 1;
-            }
+        if (cx.b0 + rx0 < cx.nvir && cx.c0 + cx0 < cx.nvir) {
+            bool ok;
+            if (!same)
+                ok = diag ? run_item<KS, true, false>(nc, fo, pipe, rp, f, gT)
+                          : run_item<KS, false, false>(nc, fo, pipe, rp, f, gT);
+            else
+                ok = diag ? run_item<KS, true, true>(nc, fo, pipe, rp, f, gT)
+                          : run_item<KS, false, true>(nc, fo, pipe, rp, f, gT);
+            if (!ok) return;
+        } else if (!skip_slots(cx.nch, pipe, rp)) {  // only padding
+            return;
         }
         if (SPLIT && (cx.split_tag & 1)) {  // the second half to arrive adds the first's partial sums and finishes
             int fin = 0;
@@ -897,6 +1036,7 @@ fused_tma_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long 
             // separated by a consumer-only mbarrier (bounded wait; no CTA-wide barrier).
 #pragma unroll
             for (int x = 0; x < 8; ++x) {
+                if (x == 4 && same) break;
                 double *xb = xbuf + (x & 1) * XBUF;
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
@@ -910,7 +1050,11 @@ fused_tma_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long 
                     gT[x][e] = xb[(cx0 + perm8(2 * t + (e & 1))) * (T + 1) + rx0 + perm8(g) + ((e & 2) ? 8 : 0)];
             }
         }
-        warp_epilogue(cx, f, gT, cx.b0 + rx0, cx.c0 + cx0, g, t, lane, cx.out + warp * 4);
+        if (same) copy_families(f, gT);
+        if (diag)
+            warp_epilogue<true>(cx, f, gT, cx.b0 + rx0, cx.c0 + cx0, g, t, lane, cx.out + warp * 4);
+        else
+            warp_epilogue<false>(cx, f, gT, cx.b0 + rx0, cx.c0 + cx0, g, t, lane, cx.out + warp * 4);
     }
 }
 
