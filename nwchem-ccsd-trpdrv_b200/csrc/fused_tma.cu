@@ -48,25 +48,22 @@ constexpr int DK = 16;          // contraction indices per stage (two m16n8k8 st
 constexpr int STAGES = 3;
 constexpr int NCW = TRPDRV_FUSED_SLOTS;  // consumer warps (8) = two warpgroups
 constexpr int NTHREAD = (NCW + 4) * 32;  // + one producer warpgroup (one thread issues)
-// Register split by setmaxnreg: launched at 65536 / 384 = 168 per thread; the producer warpgroup
-// drops and the two consumer warpgroups rise, within 384 * 168 = 64512: the m16n8k16 kernel's MMA
-// warps take 224 (producer 56: 2*128*224 + 128*56 = 64512), the m16n8k8 kernel's 216 (producer 64),
-// the splits under which neither kernel's MMA loop spills.
-constexpr int REG_LAUNCH = 168;
-template <int KS> struct Regs {
-    static constexpr int CONSUMER = KS == 16 ? 224 : 216, PRODUCER = KS == 16 ? 56 : 64;
-    static_assert(2 * 128 * CONSUMER + 128 * PRODUCER <= NTHREAD * REG_LAUNCH, "register split exceeds the launch");
-};
+// Register split by setmaxnreg: launched at 65536 / 384 = 168 per thread; the producer warpgroup drops to 88 and
+// the two consumer warpgroups rise to 208 (2*128*208 + 128*88 = 384*168): at this split the MMA loops do not
+// spill and the producers least (-Xptxas -v; 216 / 64 and 200 / 96 both spill more).
+constexpr int REG_LAUNCH = 168, REG_CONSUMER = 208, REG_PRODUCER = 88;
+static_assert(2 * 128 * REG_CONSUMER + 128 * REG_PRODUCER <= NTHREAD * REG_LAUNCH, "register split exceeds the launch");
 constexpr int PANEL_BYTES = 4096;
 constexpr int NPANEL = 16;
 constexpr int STAGE_BYTES = NPANEL * PANEL_BYTES;
 constexpr int RING = 16;
+constexpr int TICKETS = 8;  // work tickets in flight between the producer warps (>= STAGES + 2)
 constexpr int XBUF = T * (T + 1);  // one padded 32x32 f tile
 constexpr int KBOX = PANEL_BYTES / 2;  // one 16-row K-major box
 constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_BYTES + 1024;  // + alignment slack
 constexpr unsigned long long WAIT_LIMIT_NS = 4000000000ull;       // 4 s: far above any legitimate wait
 
-static_assert(RING >= STAGES + 2, "context ring too small");
+static_assert(RING >= STAGES + 2 && TICKETS >= STAGES + 2, "context or ticket ring too small");
 
 enum { M_J = 0, M_K, M_NT, M_NX, M_T2K, M_T2X, M_JOV, M_KOV, NMAP };
 
@@ -186,6 +183,12 @@ __global__ void bounded_wait_selftest_kernel(unsigned long long limit_ns, int *s
     const bool completed = mbar_wait_for(&bar, 0u, status, limit_ns);
     *elapsed_ns = globaltimer() - t0;
     if (completed) atomicOr(status, 4);  // a phase nothing arrived on reported complete
+}
+
+// One arrival on the barrier once every cp.async of this thread has landed.
+__device__ __forceinline__ void cp_async_arrive(unsigned long long *b)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(saddr(b)) : "memory");
 }
 
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, unsigned long long *bar, int x, int y,
@@ -339,20 +342,32 @@ __device__ __forceinline__ void load_group(const FragOffsets &fo, const char *st
     }
 }
 
-template <int FAM, int O>
+// m16n8k8, or (KS = 4) the two m16n8k4 it consists of: its fragments hold the contraction indices 2t and 2t + 1.
+template <int KS>
+__device__ __forceinline__ void mma8(double (&d)[4], const double (&a)[4], const double (&b)[2])
+{
+    if (KS == 4) {
+        dmma_16x8x4(d, a[0], a[1], b[0]);
+        dmma_16x8x4(d, a[2], a[3], b[1]);
+    } else {
+        dmma_16x8x8(d, a, b);
+    }
+}
+
+template <int KS, int FAM, int O>
 __device__ __forceinline__ void mma_group(const Group &g, double (&f)[8][4], double (&gT)[8][4])
 {
     constexpr int x0 = FAM * 4;
     if (O == 0) {
-        dmma_16x8x8(f[x0 + 0], g.a0, g.b0);
-        dmma_16x8x8(f[x0 + 1], g.a1, g.b0);
-        dmma_16x8x8(f[x0 + 2], g.a0, g.b1);
-        dmma_16x8x8(f[x0 + 3], g.a1, g.b1);
+        mma8<KS>(f[x0 + 0], g.a0, g.b0);
+        mma8<KS>(f[x0 + 1], g.a1, g.b0);
+        mma8<KS>(f[x0 + 2], g.a0, g.b1);
+        mma8<KS>(f[x0 + 3], g.a1, g.b1);
     } else {
-        dmma_16x8x8(gT[x0 + 0], g.a0, g.b0);
-        dmma_16x8x8(gT[x0 + 1], g.a0, g.b1);
-        dmma_16x8x8(gT[x0 + 2], g.a1, g.b0);
-        dmma_16x8x8(gT[x0 + 3], g.a1, g.b1);
+        mma8<KS>(gT[x0 + 0], g.a0, g.b0);
+        mma8<KS>(gT[x0 + 1], g.a0, g.b1);
+        mma8<KS>(gT[x0 + 2], g.a1, g.b0);
+        mma8<KS>(gT[x0 + 3], g.a1, g.b1);
     }
 }
 
@@ -429,7 +444,7 @@ struct Pipe {
 // nor the first fragment loads of the next chunk leave the tensor pipe idle.  NKS: k8 steps of the chunk (1
 // when the second lies entirely in the zero padding).  A diagonal pair (DIAG) gets f(c,b) from the other warps
 // at the end of the item.
-template <int NKS, bool PH1, bool DIAG, int FAM, bool TAIL>
+template <int KS, int NKS, bool PH1, bool DIAG, int FAM, bool TAIL>
 __device__ __forceinline__ void family_products(const FragOffsets &fo, const char *st, const Panels &pn,
                                                 double (&f)[8][4], double (&gT)[8][4], Group &tail)
 {
@@ -442,14 +457,14 @@ __device__ __forceinline__ void family_products(const FragOffsets &fo, const cha
             return;
         }
         load_group<PH1, 0>(fo, st, pn, ks, g);
-        mma_group<FAM, 0>(g, f, gT);
+        mma_group<KS, FAM, 0>(g, f, gT);
         if (DIAG) continue;
         if (last) {
             load_group<PH1, 1>(fo, st, pn, ks, tail);
             return;
         }
         load_group<PH1, 1>(fo, st, pn, ks, g);
-        mma_group<FAM, 1>(g, f, gT);
+        mma_group<KS, FAM, 1>(g, f, gT);
     }
 }
 
@@ -475,18 +490,18 @@ __device__ __forceinline__ bool run_chunks(int n, const FragOffsets &fo, const P
             if (!SAME) group16<PH1, 1, 0>(fo, st, f, gT);
             if (!SAME && !DIAG) group16<PH1, 1, 1>(fo, st, f, gT);
         } else {
-            if (!SAME) family_products<NKS, PH1, DIAG, 0, false>(fo, st, item_panels<0>(), f, gT, tail);
-            family_products<NKS, PH1, DIAG, LAST, true>(fo, st, item_panels<LAST>(), f, gT, tail);
+            if (!SAME) family_products<KS, NKS, PH1, DIAG, 0, false>(fo, st, item_panels<0>(), f, gT, tail);
+            family_products<KS, NKS, PH1, DIAG, LAST, true>(fo, st, item_panels<LAST>(), f, gT, tail);
         }
         pp.release(rp);
-        if (!K16) mma_group<LAST, DIAG ? 0 : 1>(tail, f, gT);
+        if (!K16) mma_group<KS, LAST, DIAG ? 0 : 1>(tail, f, gT);
     }
     return true;
 }
 
 // n chunks of a packed edge item: one stage slot per (chunk, family), m16n8k8 in both kernels (the packed path's
 // extra fragment registers would push the k16 kernel's MMA warps past their register budget).
-template <int NKS, bool PH1, bool SAME>
+template <int KS, int NKS, bool PH1, bool SAME>
 __device__ __forceinline__ bool run_packed(int n, const FragOffsets &fo, const Panels &pn, const Pipe &pp, RingPos &rp,
                                            double (&f)[8][4], double (&gT)[8][4])
 {
@@ -494,14 +509,14 @@ __device__ __forceinline__ bool run_packed(int n, const FragOffsets &fo, const P
     for (; n > 0; --n) {
         Group tail;
         if (!pp.wait(rp)) return false;
-        family_products<NKS, PH1, false, 0, true>(fo, pp.stages + (size_t)rp.stage * STAGE_BYTES, pn, f, gT, tail);
+        family_products<KS, NKS, PH1, false, 0, true>(fo, pp.stages + (size_t)rp.stage * STAGE_BYTES, pn, f, gT, tail);
         pp.release(rp);
-        mma_group<0, 1>(tail, f, gT);
+        mma_group<KS, 0, 1>(tail, f, gT);
         if (SAME) continue;
         if (!pp.wait(rp)) return false;
-        family_products<NKS, PH1, false, 1, true>(fo, pp.stages + (size_t)rp.stage * STAGE_BYTES, pn, f, gT, tail);
+        family_products<KS, NKS, PH1, false, 1, true>(fo, pp.stages + (size_t)rp.stage * STAGE_BYTES, pn, f, gT, tail);
         pp.release(rp);
-        mma_group<1, 1>(tail, f, gT);
+        mma_group<KS, 1, 1>(tail, f, gT);
     }
     return true;
 }
@@ -538,14 +553,14 @@ __device__ __forceinline__ bool run_item(const ChunkCounts &n, const FragOffsets
            run_chunks<KS, 1, true, DIAG, SAME>(n.o1, fo, pp, rp, f, gT);
 }
 
-template <bool SAME>
+template <int KS, bool SAME>
 __device__ __forceinline__ bool run_packed_item(const ChunkCounts &n, const FragOffsets &fo, const Panels &pn,
                                                 const Pipe &pp, RingPos &rp, double (&f)[8][4], double (&gT)[8][4])
 {
-    return run_packed<2, false, SAME>(n.v2, fo, pn, pp, rp, f, gT) &&
-           run_packed<1, false, SAME>(n.v1, fo, pn, pp, rp, f, gT) &&
-           run_packed<2, true, SAME>(n.o2, fo, pn, pp, rp, f, gT) &&
-           run_packed<1, true, SAME>(n.o1, fo, pn, pp, rp, f, gT);
+    return run_packed<KS, 2, false, SAME>(n.v2, fo, pn, pp, rp, f, gT) &&
+           run_packed<KS, 1, false, SAME>(n.v1, fo, pn, pp, rp, f, gT) &&
+           run_packed<KS, 2, true, SAME>(n.o2, fo, pn, pp, rp, f, gT) &&
+           run_packed<KS, 1, true, SAME>(n.o1, fo, pn, pp, rp, f, gT);
 }
 
 // Brings the 128-byte lines of the energy vectors the item's epilogue will read into L1 (lanes 0..27:
@@ -619,228 +634,367 @@ __device__ __forceinline__ void warp_epilogue(const ItemCtx &cx, const double (&
 }
 
 // ------------------------------------------------------------------------------------------------
-// producer warp: tickets and item contexts (lane 0), TMA loads (one box per lane)
+// producer warps: tickets and item contexts (warp 0, lane 0), operand staging (all four)
 // ------------------------------------------------------------------------------------------------
+// Operand kinds of one family: A_J, A_K (K-major), B_1 (K-major in the virtual phase, X-major in the occupied
+// one), B_3 (X-major).
+enum { OP_AJ = 0, OP_AK, OP_B1, OP_B3 };
+
+__device__ __forceinline__ bool op_kmajor(int kind, bool virt) { return kind < OP_B1 || (kind == OP_B1 && virt); }
+
+// A work item, decoded from its ticket.  Every producer warp decodes it for itself.
+struct Item {
+    const trpdrv_dev_system *S;
+    long long own;  // index of the item's energy slots
+    int s, B, C, i, j, k, ai;
+    int za0, za1, zb0, zb1;  // blocks of the A and B operands per family (n, t): A: i / k slot, B: [j][k] / [j][i]
+    int zO;            // occupied slots per a block of J and K
+    int first, step;   // chunks first, first + step, ... (split items take every second chunk)
+    bool in_range, ok, pack, skip, same, diag;
+    __device__ __forceinline__ int za(int fam) const { return fam ? za1 : za0; }
+    __device__ __forceinline__ int zb(int fam) const { return fam ? zb1 : zb0; }
+};
+
 // SPLIT: the instantiation that also runs split systems (two work items per pair); without it the
 // producer and consumer loops carry no split logic at all.
 template <bool SPLIT>
+__device__ __forceinline__ Item decode_item(const trpdrv_dev_system *__restrict__ sys, int nsys, long long item)
+{
+    Item it;
+    int s = 0;
+    while (s + 1 < nsys && item >= sys[s + 1].item_begin) ++s;
+    const trpdrv_dev_system &S = sys[s];
+    it.S = &S;
+    it.s = s;
+    // a split system has two work items (halves of the contraction) per pair
+    const bool split = SPLIT && S.split;
+    it.first = split ? (int)((item - S.item_begin) & 1) : 0;
+    it.step = split ? 2 : 1;
+    const long long local = split ? (item - S.item_begin) >> 1 : item - S.item_begin;
+    const long long qpos = local / S.npairs;  // processing position over the system's records
+    const int p = (int)(local - qpos * S.npairs);
+    // a index (records are [a][triple], fewer than 2^31: the host checks); no division for a single a
+    const long long ai = (S.nt > 0 && qpos >= S.nt) ? (long long)((unsigned)qpos / (unsigned)S.nt) : 0;
+    const long long tpos = qpos - ai * S.nt;
+    const long long tt = (S.order && local >= 0 && qpos < S.ntriples) ? (long long)S.order[tpos] : tpos;
+    it.own = (ai * S.nt + tt) * S.npairs + p;  // energies go to the record's own items
+    int B = 0, rem = p;
+    while (B < S.nb && rem >= S.nb - B) {
+        rem -= S.nb - B;
+        ++B;
+    }
+    const int C = B + rem, O = S.nocc;
+    it.B = B;
+    it.C = C;
+    it.ai = (int)ai;
+    it.diag = B == C;
+    // edge pairs (B, E) with B odd are computed by the packed item of B - 1
+    it.pack = S.pack_edge && C == S.nb - 1 && B < C;
+    it.skip = it.pack && (B & 1);
+    it.in_range = local >= 0 && qpos < S.ntriples && tt >= 0 && tt < S.nt && ai < S.n_a;
+    const int packed = it.in_range ? S.triples[tt] : 0;
+    it.i = packed & 1023;
+    it.j = (packed >> 10) & 1023;
+    it.k = (packed >> 20) & 1023;
+    // occupied slots of the i, j and k roles in the tensors (a one-triple system holds two slots)
+    const int one = S.one_triple;
+    const int zi = one ? 0 : it.i, zj = one ? 0 : it.j, zk = one ? 1 : it.k;
+    it.zO = one ? 2 : O;
+    it.za0 = zi;
+    it.za1 = zk;
+    it.zb0 = zj * it.zO + zk;
+    it.zb1 = zj * it.zO + zi;
+    it.ok = it.in_range && B < S.nb && C < S.nb && it.i < O && it.j < O && it.k < O && (one || it.k <= it.i) &&
+            (!one || ai == 0);
+    // i == k: both families read the same blocks (a staged one-triple system holds them twice and may not)
+    it.same = it.i == it.k && !one;
+    return it;
+}
+
+template <bool SPLIT>
+__device__ __forceinline__ void write_ctx(ItemCtx &cx, const Item &it)
+{
+    const trpdrv_dev_system &S = *it.S;
+    const int O = S.nocc, V = S.nvir, nV = (V + DK - 1) / DK, nO = (O + DK - 1) / DK;
+    cx.eorb = S.eorb;
+    const size_t vi = ((size_t)it.ai * it.zO + it.za0) * V, vk = ((size_t)it.ai * it.zO + it.za1) * V;
+    cx.dintc1 = S.dintc + vi;
+    cx.dintx1 = S.dintx + vi;
+    cx.t1v1 = S.t1v + vi;
+    cx.dintc2 = S.dintc + vk;
+    cx.dintx2 = S.dintx + vk;
+    cx.t1v2 = S.t1v + vk;
+    cx.out = S.partial + (size_t)it.own * NCW * 4;
+    // the second pair (B2, E) of a packed item: its own slots, at its triangular pair index
+    // (B2 = B + 1: nb - B - 1 pairs further)
+    const bool two = it.pack && it.B + 1 < it.C;
+    cx.out1 = cx.out + (two ? (S.nb - it.B - 1) * NCW * 4 : 0);
+    cx.packed = it.pack;
+    cx.b1 = two ? (it.B + 1) * T : -1;
+    // omp/ccsd_trpdrv_omp_cbody.c:126 (a is 1-based, i/j/k here 0-based)
+    cx.eaijk = S.eorb[S.a - 1 + it.ai] - (S.eorb[S.ncor + it.i] + S.eorb[S.ncor + it.j] + S.eorb[S.ncor + it.k]);
+    cx.ncor = S.ncor;
+    cx.nocc = O;
+    cx.nvir = V;
+    cx.b0 = it.B * T;
+    cx.c0 = it.C * T;
+    cx.diag = it.diag;
+    cx.same = it.same;
+    cx.split_tag = (SPLIT && S.split) ? 1 | it.first << 1 | (int)it.own << 2 : 0;
+    cx.nch = it.step == 2 ? (nV + nO - it.first + 1) / 2 : nV + nO;
+    cx.state = 1;
+}
+
+// The panels of producer warp pw: for an ordinary item the four operands of group (family pw >> 1, orientation
+// pw & 1); for a packed item operand kind pw of the three tiles B, B + 1, E.  Spread over one warp per scheduler,
+// the staging takes few issue slots from any one scheduler's MMA warps (with one warp issuing every TMA box,
+// its scheduler's MMA warps ran 3 % behind the others).
+struct Role {
+    int npanel, fam, o;
+    bool idle;
+    __device__ __forceinline__ Role(const Item &it, int pw)
+    {
+        npanel = it.pack ? 3 : 4;
+        fam = it.pack ? 0 : pw >> 1;
+        o = it.pack ? 0 : pw & 1;
+        idle = !it.pack && ((it.diag && o == 1) || (it.same && fam == 1));
+    }
+};
+
+// Panel q of the role: its operand kind, the first virtual index of its tile (-1: absent) and its place.
+__device__ __forceinline__ void role_panel(const Item &it, const Role &r, int pw, int q, int &kind, int &tile, int &off)
+{
+    if (!it.pack) {
+        kind = q;
+        // A rows: B for (B,C), C for (C,B); B columns: C for (B,C), B for (C,B)
+        tile = ((q < OP_B1) == (r.o == 0) ? it.B : it.C) * T;
+        off = (r.fam * 8 + 2 * q + r.o) * PANEL_BYTES;
+    } else {
+        kind = pw;
+        tile = q == 2 ? it.C * T : q == 0 ? it.B * T : it.B + 1 < it.C ? (it.B + 1) * T : -1;
+        const int base = pw < OP_B1 ? (q < 2 ? PK_A + 2 * pw : PK_AE + pw) : pw == OP_B1 ? (q < 2 ? PK_B1B : PK_B1E)
+                                                                                        : (q < 2 ? PK_B3B : PK_B3E);
+        off = (base + (q < 2 ? q : 0)) * PANEL_BYTES;
+    }
+}
+
+// TMA staging: one box per lane (ordinary items: 7 per warp, packed ones: 5).
+struct TmaStage {
+    const Maps *maps;
+    const CUtensorMap *mv, *mo;  // this lane's box in the virtual / occupied phase
+    int kind, tile, half, off, zav;
+    bool act_v, act_o;
+    unsigned bytes_v, bytes_o;
+
+    __device__ __forceinline__ void begin(const Item &it, const Role &r, int pw, int lane)
+    {
+        // K-major panels are two 16-row boxes, X-major ones a single box; the E tile of a packed item has at
+        // most 16 valid rows
+        const int q = lane >> 1;
+        half = lane & 1;
+        const bool mine = !r.idle && q < r.npanel;
+        role_panel(it, r, pw, mine ? q : 0, kind, tile, off);
+        off += half * KBOX;
+        const bool box = mine && tile >= 0;
+        const bool second = half == 1, e_tile = it.pack && q == 2;
+        act_v = box && (!second || (op_kmajor(kind, true) && !e_tile));
+        act_o = box && (!second || (op_kmajor(kind, false) && !e_tile));
+        bytes_v = __reduce_add_sync(0xffffffffu, act_v ? (op_kmajor(kind, true) ? KBOX : PANEL_BYTES) : 0);
+        bytes_o = __reduce_add_sync(0xffffffffu, act_o ? (op_kmajor(kind, false) ? KBOX : PANEL_BYTES) : 0);
+        const CUtensorMap *mp = maps->m[it.s];
+        mv = &mp[kind == OP_AJ ? M_J : kind == OP_AK ? M_K : kind == OP_B1 ? M_T2K : M_T2X];
+        mo = &mp[kind == OP_AJ ? M_NT : kind == OP_AK ? M_NX : kind == OP_B1 ? M_KOV : M_JOV];
+        zav = it.ai * it.zO;  // J and K carry the a index, -T and -X do not
+    }
+
+    __device__ __forceinline__ void slot(const Item &it, const Role &, int, char *st, unsigned long long *full,
+                                         bool virt, int kk0, int fam, int lane)
+    {
+        const unsigned bytes = virt ? bytes_v : bytes_o;
+        if (lane == 0) {
+            if (bytes)
+                mbar_arrive_expect_tx(full, bytes);
+            else
+                mbar_arrive(full);
+        }
+        __syncwarp();
+        if (virt ? act_v : act_o) {
+            const bool km = op_kmajor(kind, virt);
+            const int row = tile + 16 * half;
+            const int z = kind < OP_B1 ? it.za(fam) + (virt ? zav : 0) : it.zb(fam);
+            tma_load_3d(st + off, virt ? mv : mo, full, km ? row : kk0, km ? kk0 : tile, z);
+        }
+    }
+    static constexpr unsigned FULL_COUNT = 4;  // one arrival (with its byte count) per producer warp
+    __device__ __forceinline__ static void marker(unsigned long long *full, int, int lane)
+    {
+        if (lane == 0) mbar_arrive(full);
+    }
+};
+
+// cp.async staging, into the same swizzled panels: any sizes and alignments (VEC = 1: 8-byte copies; VEC = 2:
+// 16-byte copies, even row pitches and 16-byte aligned tensors) and any number of systems.  A pad element at the
+// end of an odd row (VEC = 2) must be zero: in an X-major panel it stands at a contraction index.
+template <int VEC>
+struct CpStage {
+    static constexpr unsigned FULL_COUNT = 129;  // every producer thread's copies, and the item context's writer
+
+    __device__ __forceinline__ void begin(const Item &, const Role &, int, int) {}
+
+    // One K-major panel: rows src[0 .. rows) of contraction indices 0 .. klim - 1 (ld apart), zeros elsewhere.
+    __device__ __forceinline__ static void panel_k(char *dst, const double *src, int ld, int rows, int klim, int lane)
+    {
+        constexpr int KSTEP = VEC;  // 32 lanes cover 32 * VEC rows: VEC contraction indices per pass
+        const int x = (lane * VEC) & 31, k0 = VEC == 2 ? lane >> 4 : 0;
+        const bool row_ok = x < rows;
+        const double *q = src + (row_ok ? x : 0) + (size_t)k0 * ld;
+        char *d = dst + (x >> 4) * KBOX + ((x & 1) << 3);
+        const int c = (x & 15) >> 1;
+#pragma unroll 4
+        for (int kk = k0; kk < DK; kk += KSTEP, q += (size_t)KSTEP * ld) {
+            const bool ok = row_ok && kk < klim;
+            char *w = d + kk * 128 + ((c ^ (kk & 7)) << 4);
+            if (VEC == 2)
+                cp_async_16(w, ok ? q : src, ok);
+            else
+                cp_async_8(w, ok ? q : src, ok);
+        }
+    }
+
+    // One X-major panel: columns src + c ld, c < rows, of contraction indices 0 .. klim - 1 (contiguous).
+    __device__ __forceinline__ static void panel_x(char *dst, const double *src, int ld, int rows, int klim, int lane)
+    {
+        constexpr int PER = DK / VEC, CSTEP = 32 / PER;  // copies per row, rows per pass
+        const int dd = (lane & (PER - 1)) * VEC, r0 = lane / PER;
+        const bool k_ok = dd < klim;
+        const double *q = src + (k_ok ? dd : 0) + (size_t)r0 * ld;
+#pragma unroll 4
+        for (int r = r0; r < T; r += CSTEP, q += (size_t)CSTEP * ld) {
+            const bool ok = k_ok && r < rows;
+            char *w = dst + r * 128 + (((dd >> 1) ^ (r & 7)) << 4) + ((dd & 1) << 3);
+            if (VEC == 2)
+                cp_async_16(w, ok ? q : src, ok);
+            else
+                cp_async_8(w, ok ? q : src, ok);
+        }
+    }
+
+    __device__ __forceinline__ void slot(const Item &it, const Role &r, int pw, char *st, unsigned long long *full,
+                                         bool virt, int kk0, int fam, int lane)
+    {
+        const trpdrv_dev_system &S = *it.S;
+        const int V = S.nvir, O = S.nocc, klim = (virt ? V : O) - kk0;
+        const int ldv = S.ldv ? S.ldv : V, ldo = S.ldo ? S.ldo : O;
+        if (!r.idle) {
+#pragma unroll 1
+            for (int q = 0; q < r.npanel; ++q) {
+                int kind, tile, off;
+                role_panel(it, r, pw, q, kind, tile, off);
+                if (tile < 0) continue;
+                // block of the operand's matrix
+                const double *m;
+                if (virt)
+                    m = (kind == OP_AJ ? S.jvv : kind == OP_AK ? S.kvv : S.t2) +
+                        (size_t)(kind < OP_B1 ? it.ai * it.zO + it.za(fam) : it.zb(fam)) * ldv * V;
+                else if (kind < OP_B1)
+                    m = (kind == OP_AJ ? S.ntov : S.nxov) + (size_t)it.za(fam) * ldv * O;
+                else
+                    m = (kind == OP_B1 ? S.kov : S.jov) + (size_t)it.zb(fam) * ldo * V;
+                const int ld = virt || kind < OP_B1 ? ldv : ldo;
+                if (op_kmajor(kind, virt))
+                    panel_k(st + off, m + tile + (size_t)kk0 * ld, ld, V - tile, klim, lane);
+                else
+                    panel_x(st + off, m + kk0 + (size_t)tile * ld, ld, V - tile, klim, lane);
+            }
+        }
+        cp_async_arrive(full);
+        if (pw == 0 && lane == 0) mbar_arrive(full);
+    }
+    __device__ __forceinline__ static void marker(unsigned long long *full, int pw, int lane)
+    {
+        cp_async_arrive(full);
+        if (pw == 0 && lane == 0) mbar_arrive(full);
+    }
+};
+
+template <bool SPLIT, class Stage>
 __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ sys, int nsys, long long total,
-                                         unsigned long long *counter, int *status, const Maps &maps, char *stages,
-                                         unsigned long long *full, unsigned long long *empty, ItemCtx *ring, int lane)
+                                         unsigned long long *counter, int *status, Stage &sg, char *stages,
+                                         unsigned long long *full, unsigned long long *empty, ItemCtx *ring,
+                                         long long *tickets, unsigned long long *tbar, int pw, int lane)
 {
     const unsigned FULL = 0xffffffffu;
-    // this lane's box within a chunk: group = family*2 + orientation, slot 0..6 (lanes 28..31 idle)
-    const int grp = lane / 7, slot = lane - 7 * grp;
-    const int fam = grp >> 1, o = grp & 1;
     int stage = 0;
     unsigned phase = 0;  // parity of the current pass over the stages
     long long next = 0;
-    if (lane == 0) next = (long long)atomicAdd(counter, 1ULL);
-    next = __shfl_sync(FULL, next, 0);
-    for (long long n = 0;;) {
-        const long long item = next;
-        if (item < total) {  // ticket for the following item, early
-            if (lane == 0) next = (long long)atomicAdd(counter, 1ULL);
-            next = __shfl_sync(FULL, next, 0);
+    if (pw == 0) {
+        if (lane == 0) next = (long long)atomicAdd(counter, 1ULL);
+        next = __shfl_sync(FULL, next, 0);
+    }
+    for (long long n = 0;; ++n) {
+        // warp 0 draws the tickets; the others read them from a ring (warp 0 is at most STAGES slots ahead: a stage
+        // is released only after all four warps have filled it, and every ticket in the ring has a slot)
+        const int tq = (int)(n % TICKETS);
+        long long item;
+        Item it;
+        if (pw == 0) {
+            for (;;) {
+                item = next;
+                if (item >= total) break;
+                if (lane == 0) next = (long long)atomicAdd(counter, 1ULL);  // the following ticket, early
+                next = __shfl_sync(FULL, next, 0);
+                it = decode_item<SPLIT>(sys, nsys, item);
+                if (!it.skip) break;
+            }
+            if (lane == 0) {
+                tickets[tq] = item;
+                mbar_arrive(&tbar[tq]);
+            }
+        } else {
+            if (!mbar_wait(&tbar[tq], (unsigned)((n / TICKETS) & 1), status)) return;
+            item = tickets[tq];
+            if (item < total) it = decode_item<SPLIT>(sys, nsys, item);
         }
         ItemCtx &cx = ring[n % RING];
-        if (item >= total) {
-            if (mbar_wait(&empty[stage], phase ^ 1, status) && lane == 0) {
-                cx.state = -1;
-                mbar_arrive(&full[stage]);
-            }
-            return;
-        }
-        int s = 0;
-        while (s + 1 < nsys && item >= sys[s + 1].item_begin) ++s;
-        const trpdrv_dev_system &S = sys[s];
-        // a split system has two work items (halves of the contraction) per pair
-        const int hpart = (SPLIT && S.split) ? (int)((item - S.item_begin) & 1) : 0;
-        const long long local = (SPLIT && S.split) ? (item - S.item_begin) >> 1 : item - S.item_begin;
-        const long long qpos = local / S.npairs;  // processing position over the system's records
-        const int p = (int)(local - qpos * S.npairs);
-        // a index (records are [a][triple], fewer than 2^31: the host checks); no division for a single a
-        const long long ai = (S.nt > 0 && qpos >= S.nt) ? (long long)((unsigned)qpos / (unsigned)S.nt) : 0;
-        const long long tpos = qpos - ai * S.nt;
-        const long long tt = (S.order && local >= 0 && qpos < S.ntriples) ? (long long)S.order[tpos] : tpos;
-        const long long own = (ai * S.nt + tt) * S.npairs + p;  // energies go to the record's own items
-        int B = 0, rem = p;
-        while (B < S.nb && rem >= S.nb - B) {
-            rem -= S.nb - B;
-            ++B;
-        }
-        const int C = B + rem;
-        // edge pairs (B, E) with B odd are computed by the packed item of B - 1
-        const bool pack = S.pack_edge && C == S.nb - 1 && B < C;
-        if (pack && (B & 1)) continue;
-        const int O = S.nocc, V = S.nvir;
-        const bool in_range = local >= 0 && qpos < S.ntriples && tt >= 0 && tt < S.nt && ai < S.n_a;
-        const int packed = in_range ? S.triples[tt] : 0;
-        const int i = packed & 1023, j = (packed >> 10) & 1023, k = (packed >> 20) & 1023;
-        // occupied slots of the i, j and k roles in the tensors (a one-triple system holds two slots)
-        const int one = S.one_triple;
-        const int zi = one ? 0 : i, zj = one ? 0 : j, zk = one ? 1 : k, zO = one ? 2 : O;
-        const bool ok = in_range && B < S.nb && C < S.nb && i < O && j < O && k < O && (one || k <= i) &&
-                        (!one || ai == 0) && s < TRPDRV_TMA_MAX_SYSTEMS;
-        const int B0 = B * T, C0 = C * T;
-        if (!ok) {
+        if (item >= total || !it.ok) {
             if (!mbar_wait(&empty[stage], phase ^ 1, status)) return;
-            if (lane == 0) {
-                atomicOr(status, 1);
-                cx.state = 0;
-                cx.packed = 0;
-                cx.out = in_range ? S.partial + (size_t)own * NCW * 4 : nullptr;
+            if (pw == 0 && lane == 0) {
                 cx.nch = 0;
-                mbar_arrive(&full[stage]);
+                cx.packed = 0;
+                if (item >= total) {
+                    cx.state = -1;
+                } else {
+                    atomicOr(status, 1);
+                    cx.state = 0;
+                    cx.out = it.in_range ? it.S->partial + (size_t)it.own * NCW * 4 : nullptr;
+                }
             }
+            Stage::marker(&full[stage], pw, lane);
+            if (item >= total) return;
             if (++stage == STAGES) {
                 stage = 0;
                 phase ^= 1;
             }
-            ++n;
             continue;
         }
-        const int nV = (V + DK - 1) / DK, nO = (O + DK - 1) / DK;
-        const bool diag = (B == C);
-        // i == k: both families read the same blocks (a staged one-triple system holds them twice and may not)
-        const bool same = i == k && !one;
-        if (lane == 0) {
-            cx.eorb = S.eorb;
-            const size_t ao = (size_t)ai * zO;  // the a block of the a-dependent vectors
-            cx.dintc1 = S.dintc + (ao + zi) * V;
-            cx.dintx1 = S.dintx + (ao + zi) * V;
-            cx.t1v1 = S.t1v + (ao + zi) * V;
-            cx.dintc2 = S.dintc + (ao + zk) * V;
-            cx.dintx2 = S.dintx + (ao + zk) * V;
-            cx.t1v2 = S.t1v + (ao + zk) * V;
-            cx.out = S.partial + (size_t)own * NCW * 4;
-            // the second pair (B2, E) of a packed item: its own slots, at its triangular pair index
-            // (B2 = B + 1: nb - B - 1 pairs further)
-            const bool two = pack && B + 1 < C;
-            cx.out1 = cx.out + (two ? (S.nb - B - 1) * NCW * 4 : 0);
-            cx.packed = pack;
-            cx.b1 = two ? (B + 1) * T : -1;
-            // omp/ccsd_trpdrv_omp_cbody.c:126 (a is 1-based, i/j/k here 0-based)
-            cx.eaijk = S.eorb[S.a - 1 + ai] - (S.eorb[S.ncor + i] + S.eorb[S.ncor + j] + S.eorb[S.ncor + k]);
-            cx.ncor = S.ncor;
-            cx.nocc = O;
-            cx.nvir = V;
-            cx.b0 = B0;
-            cx.c0 = C0;
-            cx.diag = diag;
-            cx.same = same;
-            cx.split_tag = (SPLIT && S.split) ? 1 | hpart << 1 | (int)own << 2 : 0;
-            cx.nch = (SPLIT && S.split) ? (nV + nO - hpart + 1) / 2 : nV + nO;
-            cx.state = 1;
-        }
-
-        const CUtensorMap *mp = maps.m[s];
-        if (pack) {
-            // one stage slot per (chunk, family); lanes 0..17 each own at most one box of the layout at
-            // PK_*: kind 0 / 1 = J / K-role A rows (K-major), 2 = B_1 columns, 3 = B_3 columns (X-major)
-            const int E = C, B2 = B + 1 < C ? B + 1 : -1;
-            int kind = 3, tb = -1, half = 0, off = 0;
-            if (lane < 8) {
-                const int pnl = lane >> 1;
-                kind = pnl >> 1;
-                tb = (pnl & 1) ? B2 : B;
-                half = lane & 1;
-                off = (PK_A + pnl) * PANEL_BYTES + half * KBOX;
-            } else if (lane < 12) {
-                kind = lane == 8 ? 2 : lane == 9 ? 3 : lane - 10;
-                tb = E;
-                off = (lane == 8 ? PK_B1E : lane == 9 ? PK_B3E : PK_AE + lane - 10) * PANEL_BYTES;
-            } else if (lane < 18) {
-                const int pp = lane < 16 ? (lane - 12) >> 1 : lane - 16;
-                kind = lane < 16 ? 2 : 3;
-                tb = pp ? B2 : B;
-                half = lane < 16 ? (lane & 1) : 0;
-                off = (lane < 16 ? PK_B1B + pp : PK_B3B + pp) * PANEL_BYTES + half * KBOX;
-            }
-            tb = tb >= 0 ? tb * T : -1;
-            const int pch0 = (SPLIT && S.split) ? hpart : 0, pstep = (SPLIT && S.split) ? 2 : 1;
-            const int nsl = 2 * ((SPLIT && S.split) ? (nV + nO - hpart + 1) / 2 : nV + nO);
-            for (int sl = 0; sl < nsl; sl += same ? 2 : 1) {
+        if (pw == 0 && lane == 0) write_ctx<SPLIT>(cx, it);
+        const Role role(it, pw);
+        sg.begin(it, role, pw, lane);
+        const int nV = (it.S->nvir + DK - 1) / DK, nch = nV + (it.S->nocc + DK - 1) / DK;
+        // packed items: one slot per (chunk, family)
+        const int f0 = it.pack ? 0 : role.fam, f1 = it.pack ? (it.same ? 1 : 2) : role.fam + 1;
+        for (int ch = it.first; ch < nch; ch += it.step) {
+            const bool virt = ch < nV;
+            const int kk0 = (virt ? ch : ch - nV) * DK;
+            for (int f = f0; f < f1; ++f) {
                 if (!mbar_wait(&empty[stage], phase ^ 1, status)) return;
-                const int fam = sl & 1, ch = pch0 + (sl >> 1) * pstep;
-                const bool ph1 = ch >= nV;
-                const int kk0 = (ph1 ? ch - nV : ch) * DK;
-                const int za = fam ? zk : zi;
-                const int zb = fam ? zj * zO + zi : zj * zO + zk;
-                const CUtensorMap *m = nullptr;
-                int x = kk0, y = tb, z = zb;
-                unsigned bytes = 0;
-                if (tb >= 0) {
-                    if (kind < 2) {  // A rows: J / K (virtual), -T / -X (occupied)
-                        m = &mp[ph1 ? (kind ? M_NX : M_NT) : (kind ? M_K : M_J)];
-                        x = tb + 16 * half;
-                        y = kk0;
-                        z = ph1 ? za : za + (int)ai * zO;
-                        bytes = KBOX;
-                    } else if (kind == 2) {  // B_1 columns: T(c,d) K-major boxes, or one K(m,c) X-major box
-                        if (!ph1) {
-                            m = &mp[M_T2K];
-                            x = tb + 16 * half;
-                            y = kk0;
-                            bytes = KBOX;
-                        } else if (half == 0) {
-                            m = &mp[M_KOV];
-                            bytes = PANEL_BYTES;
-                        }
-                    } else {  // B_3 columns: T(d,c) / J(m,c), X-major
-                        m = &mp[ph1 ? M_JOV : M_T2X];
-                        bytes = PANEL_BYTES;
-                    }
-                }
-                const unsigned total = __reduce_add_sync(FULL, bytes);
-                if (lane == 0) mbar_arrive_expect_tx(&full[stage], total);
-                __syncwarp();
-                if (m) tma_load_3d(stages + (size_t)stage * STAGE_BYTES + off, m, &full[stage], x, y, z);
+                sg.slot(it, role, pw, stages + (size_t)stage * STAGE_BYTES, &full[stage], virt, kk0, f, lane);
                 if (++stage == STAGES) {
                     stage = 0;
                     phase ^= 1;
                 }
             }
-            ++n;
-            continue;
         }
-
-        // per-lane box: A_J (slots 0,1), A_K (2,3) rows; B_1 (4,5) and B_3 (6) columns
-        const int za = fam ? zk : zi;                    // A operands: Jia/Kia (n), Jka/Kka (t)
-        const int zaj = za + (int)ai * zO;               // J/K carry the a index, -T/-X do not
-        const int zb = fam ? zj * zO + zi : zj * zO + zk;  // B operands: Tkj/Kkj/Jkj (n), Tij/Kij/Jij (t)
-        const int ra = o ? C0 : B0;                      // A rows: B for (B,C), C for (C,B)
-        const int cb = o ? B0 : C0;                      // B columns: C for (B,C), B for (C,B)
-        const int half = slot & 1;                       // second 16-row box of a K-major panel
-        const int pnl = fam * 8 + (slot < 2 ? 0 : slot < 4 ? 2 : slot < 6 ? 4 : 6) + o;
-        const bool mine = lane < 28 && (!diag || o == 0) && (!same || fam == 0);
-        const unsigned bytes = ((NPANEL * PANEL_BYTES) >> (diag ? 1 : 0)) >> (same ? 1 : 0);
-        for (int ch = (SPLIT && S.split) ? hpart : 0; ch < nV + nO; ch += (SPLIT && S.split) ? 2 : 1) {
-            if (!mbar_wait(&empty[stage], phase ^ 1, status)) return;
-            if (lane == 0) mbar_arrive_expect_tx(&full[stage], bytes);
-            __syncwarp();
-            const bool ph1 = ch >= nV;
-            const int kk0 = (ph1 ? ch - nV : ch) * DK;
-            char *dst = stages + (size_t)stage * STAGE_BYTES + pnl * PANEL_BYTES;
-            if (mine) {
-                if (slot < 4) {  // A rows, K-major (J/K in the virtual phase, -T/-X in the occupied one)
-                    const CUtensorMap *m = &mp[slot < 2 ? (ph1 ? M_NT : M_J) : (ph1 ? M_NX : M_K)];
-                    tma_load_3d(dst + half * KBOX, m, &full[stage], ra + 16 * half, kk0, ph1 ? za : zaj);
-                } else if (slot < 6) {  // B_1 columns: T(c,d) K-major, or K(m,c) X-major (one box)
-                    if (!ph1)
-                        tma_load_3d(dst + half * KBOX, &mp[M_T2K], &full[stage], cb + 16 * half, kk0, zb);
-                    else if (!half)
-                        tma_load_3d(dst, &mp[M_KOV], &full[stage], kk0, cb, zb);
-                } else {  // B_3 columns: T(d,c) / J(m,c), X-major
-                    tma_load_3d(dst, &mp[ph1 ? M_JOV : M_T2X], &full[stage], kk0, cb, zb);
-                }
-            }
-            if (++stage == STAGES) {
-                stage = 0;
-                phase ^= 1;
-            }
-        }
-        ++n;
     }
 }
 
@@ -917,14 +1071,26 @@ __device__ __forceinline__ void copy_families(double (&f)[8][4], double (&gT)[8]
 }
 
 // ------------------------------------------------------------------------------------------------
-template <int KS, bool SPLIT>
+// The tensor maps travel as a kernel parameter of the TMA instantiations only.
+template <int STG> struct StageParam {
+    Maps maps;
+};
+struct NoParam {
+    int unused;
+};
+template <> struct StageParam<1> : NoParam {};
+template <> struct StageParam<2> : NoParam {};
+
+// STG: operand staging, 0 = TMA, 1 / 2 = cp.async with 8 / 16-byte copies.  KS: FP64 MMA shape.
+template <int KS, bool SPLIT, int STG>
 __global__ void __launch_bounds__(NTHREAD, 1)
-fused_tma_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long total, unsigned long long *counter,
-                 int *status, const __grid_constant__ Maps maps)
+fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long total, unsigned long long *counter,
+             int *status, const __grid_constant__ StageParam<STG> param)
 {
     extern __shared__ char smem_raw[];
-    __shared__ __align__(8) unsigned long long full[STAGES], empty[STAGES];
+    __shared__ __align__(8) unsigned long long full[STAGES], empty[STAGES], tbar[TICKETS];
     __shared__ ItemCtx ring[RING];
+    __shared__ long long tickets[TICKETS];
     __shared__ double xbuf[2 * XBUF];                       // diagonal-pair transpose exchange
     __shared__ __align__(8) unsigned long long xbar[1];
     __shared__ int split_flag[1];
@@ -935,20 +1101,31 @@ fused_tma_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&full[s], 1);
+            mbar_init(&full[s], STG ? CpStage<1>::FULL_COUNT : TmaStage::FULL_COUNT);
             mbar_init(&empty[s], NCW);
         }
+        for (int q = 0; q < TICKETS; ++q) mbar_init(&tbar[q], 1);
         mbar_init(xbar, NCW);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
 
-    if (warp >= NCW) {  // producer warpgroup: its first warp issues everything
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<KS>::PRODUCER));
-        if (warp == NCW) producer<SPLIT>(sys, nsys, total, counter, status, maps, stages, full, empty, ring, lane);
+    if (warp >= NCW) {  // producer warpgroup
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REG_PRODUCER));
+        if constexpr (STG == 0) {
+            TmaStage sg;
+            sg.maps = &param.maps;
+            producer<SPLIT>(sys, nsys, total, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
+                            lane);
+        } else {
+            CpStage<STG> sg;
+            producer<SPLIT>(sys, nsys, total, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
+                            lane);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        }
         return;
     }
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<KS>::CONSUMER));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REG_CONSUMER));
 
     const int g = lane >> 2, t = lane & 3;
     // sub-block: rows (b) rs*16.., columns (c) cs*8..; warps w and w+4 share a scheduler and differ in both
@@ -990,8 +1167,8 @@ fused_tma_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long 
             if (pb0 >= 0 && cx.c0 + pcs * 8 < cx.nvir) {
                 const FragOffsets fp(prs * 16, pcs * 8, g, t);
                 const Panels pn = packed_panels(pair);
-                if (!(same ? run_packed_item<true>(nc, fp, pn, pipe, rp, f, gT)
-                           : run_packed_item<false>(nc, fp, pn, pipe, rp, f, gT)))
+                if (!(same ? run_packed_item<KS, true>(nc, fp, pn, pipe, rp, f, gT)
+                           : run_packed_item<KS, false>(nc, fp, pn, pipe, rp, f, gT)))
                     return;
             } else if (!skip_slots(same ? cx.nch : 2 * cx.nch, pipe, rp)) {
                 return;
@@ -1097,7 +1274,7 @@ static int make_map(CUtensorMap *m, const double *base, unsigned long long d0, u
 
 using namespace trpdrv;
 
-extern "C" size_t trpdrv_tma_maps_bytes(void) { return sizeof(tma::Maps); }
+extern "C" size_t trpdrv_tma_maps_bytes(void) { return sizeof(tma::StageParam<0>); }
 
 // Registers per thread the kernel is launched with (read back at init).  The setmaxnreg split is
 // only valid when this equals REG_LAUNCH: with fewer, the consumers' increase could never be met.
@@ -1155,28 +1332,45 @@ extern "C" int trpdrv_tma_prepare(const trpdrv_dev_system *h_sys, int nsys, void
     return 0;
 }
 
+template <int KS, bool SPLIT, int STG>
+static int launch_kernel(const trpdrv_dev_system *d_sys, int nsys, int64_t total, unsigned long long *counter,
+                         int *status, int grid, const tma::StageParam<STG> &param, void *stream)
+{
+    tma::fused_kernel<KS, SPLIT, STG><<<grid, tma::NTHREAD, tma::SMEM_BYTES, (cudaStream_t)stream>>>(
+        d_sys, nsys, total, counter, status, param);
+    return (int)cudaGetLastError();
+}
+
 extern "C" int trpdrv_launch_fused_tma(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items,
                                        unsigned long long *counter, int *status, int grid, const void *maps,
                                        int mma_k, int split, void *stream)
 {
     if (grid <= 0 || total_items <= 0) return 0;
     if (g_launch_regs != tma::REG_LAUNCH) return (int)cudaErrorInvalidConfiguration;
-    const tma::Maps &m = *static_cast<const tma::Maps *>(maps);
-    cudaStream_t st = (cudaStream_t)stream;
+    if (nsys > TRPDRV_TMA_MAX_SYSTEMS) return (int)cudaErrorInvalidValue;
+    const tma::StageParam<0> &m = *static_cast<const tma::StageParam<0> *>(maps);
     if (split && mma_k == 8)
-        tma::fused_tma_kernel<8, true><<<grid, tma::NTHREAD, tma::SMEM_BYTES, st>>>(d_sys, nsys, total_items,
-                                                                                   counter, status, m);
-    else if (split)
-        return (int)cudaErrorInvalidValue;
-    else if (mma_k == 16)
-        tma::fused_tma_kernel<16, false><<<grid, tma::NTHREAD, tma::SMEM_BYTES, st>>>(d_sys, nsys, total_items,
-                                                                                     counter, status, m);
-    else if (mma_k == 8)
-        tma::fused_tma_kernel<8, false><<<grid, tma::NTHREAD, tma::SMEM_BYTES, st>>>(d_sys, nsys, total_items,
-                                                                                    counter, status, m);
-    else
-        return (int)cudaErrorInvalidValue;
-    return (int)cudaGetLastError();
+        return launch_kernel<8, true, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
+    if (!split && mma_k == 16)
+        return launch_kernel<16, false, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
+    if (!split && mma_k == 8)
+        return launch_kernel<8, false, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
+    return (int)cudaErrorInvalidValue;
+}
+
+extern "C" int trpdrv_launch_fused(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items,
+                                   unsigned long long *counter, int *status, int grid, int vec2, int mma_k,
+                                   void *stream)
+{
+    if (grid <= 0 || total_items <= 0) return 0;
+    if (g_launch_regs != tma::REG_LAUNCH) return (int)cudaErrorInvalidConfiguration;
+    const tma::StageParam<1> p1 = {};
+    const tma::StageParam<2> p2 = {};
+    if (mma_k == 4)
+        return vec2 ? launch_kernel<4, false, 2>(d_sys, nsys, total_items, counter, status, grid, p2, stream)
+                    : launch_kernel<4, false, 1>(d_sys, nsys, total_items, counter, status, grid, p1, stream);
+    return vec2 ? launch_kernel<8, false, 2>(d_sys, nsys, total_items, counter, status, grid, p2, stream)
+                : launch_kernel<8, false, 1>(d_sys, nsys, total_items, counter, status, grid, p1, stream);
 }
 
 extern "C" int trpdrv_launch_wait_selftest(unsigned long long limit_ns, int *status, unsigned long long *elapsed_ns,
@@ -1188,17 +1382,27 @@ extern "C" int trpdrv_launch_wait_selftest(unsigned long long limit_ns, int *sta
 
 // Every instantiation must be launched with REG_LAUNCH registers per thread (the setmaxnreg split
 // assumes it); g_launch_regs holds the common value, or 0 when they differ.
+template <int KS, bool SPLIT, int STG>
+static cudaError_t init_kernel(int *regs)
+{
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, tma::fused_kernel<KS, SPLIT, STG>);
+    if (e != cudaSuccess) return e;
+    *regs = *regs < 0 || *regs == a.numRegs ? a.numRegs : 0;
+    return cudaFuncSetAttribute(tma::fused_kernel<KS, SPLIT, STG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)tma::SMEM_BYTES);
+}
+
 extern "C" int trpdrv_fused_tma_init(void)
 {
-    cudaFuncAttributes a[3];
-    cudaError_t e = cudaFuncGetAttributes(&a[0], tma::fused_tma_kernel<8, false>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a[1], tma::fused_tma_kernel<16, false>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a[2], tma::fused_tma_kernel<8, true>);
-    if (e != cudaSuccess) return (int)e;
-    g_launch_regs = a[0].numRegs == a[1].numRegs && a[0].numRegs == a[2].numRegs ? a[0].numRegs : 0;
-    const cudaFuncAttribute dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    e = cudaFuncSetAttribute(tma::fused_tma_kernel<8, false>, dyn, (int)tma::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(tma::fused_tma_kernel<16, false>, dyn, (int)tma::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(tma::fused_tma_kernel<8, true>, dyn, (int)tma::SMEM_BYTES);
+    int regs = -1;
+    cudaError_t e = init_kernel<8, false, 0>(&regs);
+    if (e == cudaSuccess) e = init_kernel<16, false, 0>(&regs);
+    if (e == cudaSuccess) e = init_kernel<8, true, 0>(&regs);
+    if (e == cudaSuccess) e = init_kernel<8, false, 1>(&regs);
+    if (e == cudaSuccess) e = init_kernel<8, false, 2>(&regs);
+    if (e == cudaSuccess) e = init_kernel<4, false, 1>(&regs);
+    if (e == cudaSuccess) e = init_kernel<4, false, 2>(&regs);
+    if (e == cudaSuccess) g_launch_regs = regs;
     return (int)e;
 }

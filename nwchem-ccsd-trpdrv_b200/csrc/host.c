@@ -18,7 +18,6 @@
 #include <sys/file.h>
 #include <unistd.h>
 
-int trpdrv_fused_init(void);
 int trpdrv_plain_init(void);
 
 /* ------------------------------------------------------------------------------------------ */
@@ -119,8 +118,7 @@ static int ensure_device(int device, int *out_dev, int *out_nsm)
     pthread_mutex_lock(&g_init_mu);
     int rc = 0;
     if (!g_init_done[dev]) {
-        rc = trpdrv_fused_init();
-        if (!rc) rc = trpdrv_fused_tma_init();
+        rc = trpdrv_fused_tma_init();
         if (!rc) rc = trpdrv_plain_init();
         if (!rc) rc = trpdrv_oz_init();
         if (!rc) g_init_done[dev] = 1;
@@ -175,7 +173,9 @@ typedef struct sysbuf {
     trpdrv_system shape;
     const double *t[TRPDRV_T_COUNT]; /* device tensors in use (owned or bound) */
     double *own[TRPDRV_T_COUNT];     /* owned device copies made by upload */
-    double *ntov, *nxov;             /* -tov, -xov */
+    double *ntov, *nxov;             /* -tov, -xov (rows of ldv doubles when padded) */
+    double *pad[TRPDRV_T_COUNT];     /* fused, cp.async staging: t2, jvv, kvv, jov, kov with rows padded to an even
+                                        length, refilled by every execution from the bound tensors */
     int32_t *d_triples, *h_triples;
     int32_t *d_order;                /* fused/emulated processing order (trpdrv_processing_order) */
     int32_t *h_order;                /* its host copy (chunks of trpdrv_plan_upload_execute) */
@@ -190,6 +190,7 @@ typedef struct sysbuf {
 
 struct trpdrv_plan {
     int nsys, device, nsm, grid, grid_tma, vec2, bound;
+    int padded;         /* FUSED: the cp.async staging reads row-padded copies (sysbuf.pad) */
     trpdrv_options opt;
     cudaStream_t stream;
     sysbuf *s;
@@ -251,6 +252,8 @@ static void plan_free(trpdrv_plan *p)
             sysbuf *b = &p->s[q];
             for (int w = 0; w < TRPDRV_T_COUNT; ++w)
                 if (b->own[w]) cudaFree(b->own[w]);
+            for (int w = 0; w < TRPDRV_T_COUNT; ++w)
+                if (b->pad[w]) cudaFree(b->pad[w]);
             if (b->ntov) cudaFree(b->ntov);
             if (b->nxov) cudaFree(b->nxov);
             if (b->d_triples) cudaFree(b->d_triples);
@@ -365,7 +368,6 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
                 CUDA_TRY(cudaMemset(b->partial, 0, pb));
             }
         }
-        const size_t ov = (size_t)nocc * nocc * nvir;
         if (o->mode == TRPDRV_MODE_EMULATED) {
             trpdrv_oz_system *z = &b->oz;
             z->nocc = nocc;
@@ -381,8 +383,9 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
             b->oz_maps = aligned_alloc(64, (trpdrv_oz_maps_bytes() + 63) & ~(size_t)63);
             if (!b->oz_maps) return fail(TRPDRV_ERR_NOMEM, "host allocation failed");
         }
-        CUDA_TRY(cudaMalloc((void **)&b->ntov, sizeof(double) * ov));
-        CUDA_TRY(cudaMalloc((void **)&b->nxov, sizeof(double) * ov));
+        const size_t ovp = (size_t)nocc * nocc * (size_t)(nvir + (nvir & 1)); /* room for padded rows */
+        CUDA_TRY(cudaMalloc((void **)&b->ntov, sizeof(double) * ovp));
+        CUDA_TRY(cudaMalloc((void **)&b->nxov, sizeof(double) * ovp));
 
         trpdrv_dev_system *d = &p->h_dev[q];
         d->ncor = shape[q].ncor;
@@ -430,11 +433,7 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
     }
 
     int per_sm = o->ctas_per_sm;
-    if (per_sm <= 0) {
-        int occ = 1;
-        if (trpdrv_fused_max_ctas_per_sm(&occ) != 0 || occ < 1) occ = 1;
-        per_sm = occ;
-    }
+    if (per_sm <= 0) per_sm = 1; /* the fused kernel's stages fill an SM's shared memory */
     int64_t grid = (int64_t)per_sm * p->nsm;
     if (grid > p->total_items) grid = p->total_items;
     p->grid = (int)(grid > 0 ? grid : 0);
@@ -509,23 +508,156 @@ int trpdrv_plan_create(trpdrv_plan **plan, const trpdrv_system *shape, int nsys,
     return TRPDRV_OK;
 }
 
+/* Doubles per row and rows of tensor w of system b as the kernels read it (t2, jvv, kvv: rows of nvir; jov,
+ * kov: rows of nocc). */
+static int tensor_rows(const sysbuf *b, int w, long long *rows)
+{
+    const long long O = b->shape.nocc, V = b->shape.nvir;
+    switch (w) {
+    case TRPDRV_T_T2: *rows = O * O * V; return (int)V;
+    case TRPDRV_T_JVV:
+    case TRPDRV_T_KVV: *rows = b->n_a * O * V; return (int)V;
+    case TRPDRV_T_JOV:
+    case TRPDRV_T_KOV: *rows = O * O * V; return (int)O;
+    default: *rows = 0; return 0;
+    }
+}
+
+static int row_pitch(int width) { return width + (width & 1); }
+
+/* Fused plans that cannot copy 16 bytes at a time from the bound tensors (an odd nvir or nocc, or an
+ * unaligned pointer) and do not use TMA: the tensors concerned get copies with rows padded to an even length
+ * (zero pads), which every execution refills.  Copying each input once costs little beside the kernel, which
+ * reads a block of T2 for every triple: (13, 151) runs 4.2 ms with 8-byte copies from the bound tensors.
+ * Without the memory for the copies the kernel reads the bound tensors with 8-byte copies. */
+static int plan_pad(trpdrv_plan *p, int tma_ok)
+{
+    p->padded = 0;
+    for (int q = 0; q < p->nsys; ++q) p->h_dev[q].ldv = p->h_dev[q].ldo = 0;
+    if (p->opt.mode != TRPDRV_MODE_FUSED || p->vec2 || tma_ok) return TRPDRV_OK;
+    int ok = 1;
+    for (int q = 0; q < p->nsys && ok; ++q) {
+        sysbuf *b = &p->s[q];
+        for (int w = 0; w < TRPDRV_T_COUNT && ok; ++w) {
+            long long rows;
+            const int width = tensor_rows(b, w, &rows);
+            if (!width || rows == 0 || (!(width & 1) && !(((uintptr_t)b->t[w]) & 15u)) || b->pad[w]) continue;
+            if (cudaMalloc((void **)&b->pad[w], sizeof(double) * (size_t)rows * row_pitch(width)) != cudaSuccess) {
+                b->pad[w] = NULL;
+                cudaGetLastError();
+                ok = 0;
+            }
+        }
+    }
+    if (!ok) {
+        for (int q = 0; q < p->nsys; ++q)
+            for (int w = 0; w < TRPDRV_T_COUNT; ++w) {
+                if (p->s[q].pad[w]) cudaFree(p->s[q].pad[w]);
+                p->s[q].pad[w] = NULL;
+            }
+        return TRPDRV_OK;
+    }
+    p->padded = 1;
+    return TRPDRV_OK;
+}
+
+/* Whether tensor w of system q is read through its padded copy. */
+static int reads_pad(const trpdrv_plan *p, int q, int w)
+{
+    long long rows;
+    const sysbuf *b = &p->s[q];
+    const int width = tensor_rows(b, w, &rows);
+    return p->padded && width && b->pad[w] && ((width & 1) || (((uintptr_t)b->t[w]) & 15u));
+}
+
+static const double *fused_tensor(const trpdrv_plan *p, int q, int w)
+{
+    return reads_pad(p, q, w) ? p->s[q].pad[w] : p->s[q].t[w];
+}
+
+/* Refills padded copies of system q from its tensors: those every j reads (want_all), and blocks
+ * jlo <= j < jhi of the others. */
+static int pad_refill(trpdrv_plan *p, int q, int want_all, int jlo, int jhi, cudaStream_t st, int64_t *launches)
+{
+    if (!p->padded || p->use_tma) return TRPDRV_OK;
+    const sysbuf *b = &p->s[q];
+    trpdrv_pack_list L;
+    memset(&L, 0, sizeof L);
+    for (int w = 0; w < TRPDRV_T_COUNT; ++w) {
+        if (!reads_pad(p, q, w)) continue;
+        const int byj = w == TRPDRV_T_T2 || w == TRPDRV_T_JOV || w == TRPDRV_T_KOV;
+        if (byj ? jlo >= jhi : !want_all) continue;
+        long long rows, first = 0;
+        const int width = tensor_rows(b, w, &rows);
+        if (byj) {
+            const long long per_j = (long long)b->shape.nocc * b->shape.nvir;
+            first = jlo * per_j;
+            rows = (jhi - jlo) * per_j;
+        }
+        L.seg[L.n].src = b->t[w] + first * width;
+        L.seg[L.n].dst = b->pad[w] + first * row_pitch(width);
+        L.seg[L.n].rows = rows;
+        L.seg[L.n].width = width;
+        L.seg[L.n].pitch = row_pitch(width);
+        ++L.n;
+    }
+    if (!L.n) return TRPDRV_OK;
+    LAUNCH_TRY(trpdrv_launch_pack_rows(&L, st));
+    if (launches) ++*launches;
+    return TRPDRV_OK;
+}
+
 static int plan_publish(trpdrv_plan *p)
 {
+    /* TMA reads the bound tensors themselves */
+    for (int q = 0; q < p->nsys; ++q) {
+        p->h_dev[q].t2 = p->s[q].t[TRPDRV_T_T2];
+        p->h_dev[q].jvv = p->s[q].t[TRPDRV_T_JVV];
+        p->h_dev[q].kvv = p->s[q].t[TRPDRV_T_KVV];
+        p->h_dev[q].jov = p->s[q].t[TRPDRV_T_JOV];
+        p->h_dev[q].kov = p->s[q].t[TRPDRV_T_KOV];
+    }
+    const int want = p->opt.staging;
+    const int tma_ok = p->opt.mode == TRPDRV_MODE_FUSED && want != 1 && trpdrv_tma_supported(p->h_dev, p->nsys);
+    if (p->opt.mode == TRPDRV_MODE_FUSED && want == 2 && !tma_ok)
+        return fail(TRPDRV_ERR_UNSUPPORTED, "TMA staging needs even nvir and nocc, 16-byte aligned tensors "
+                                            "and at most %d systems", TRPDRV_TMA_MAX_SYSTEMS);
+    TRY(plan_pad(p, tma_ok));
     for (int q = 0; q < p->nsys; ++q) {
         sysbuf *b = &p->s[q];
         trpdrv_dev_system *d = &p->h_dev[q];
         d->eorb = b->t[TRPDRV_T_EORB];
-        d->t2 = b->t[TRPDRV_T_T2];
-        d->jvv = b->t[TRPDRV_T_JVV];
-        d->kvv = b->t[TRPDRV_T_KVV];
-        d->jov = b->t[TRPDRV_T_JOV];
-        d->kov = b->t[TRPDRV_T_KOV];
+        d->t2 = fused_tensor(p, q, TRPDRV_T_T2);
+        d->jvv = fused_tensor(p, q, TRPDRV_T_JVV);
+        d->kvv = fused_tensor(p, q, TRPDRV_T_KVV);
+        d->jov = fused_tensor(p, q, TRPDRV_T_JOV);
+        d->kov = fused_tensor(p, q, TRPDRV_T_KOV);
         d->dintc = b->t[TRPDRV_T_DINTC];
         d->dintx = b->t[TRPDRV_T_DINTX];
         d->t1v = b->t[TRPDRV_T_T1V];
-        const size_t ov = (size_t)b->shape.nocc * b->shape.nocc * b->shape.nvir;
-        LAUNCH_TRY(trpdrv_launch_negate(b->t[TRPDRV_T_TOV], b->ntov, ov, p->stream));
-        LAUNCH_TRY(trpdrv_launch_negate(b->t[TRPDRV_T_XOV], b->nxov, ov, p->stream));
+        const int O = b->shape.nocc, V = b->shape.nvir;
+        if (p->padded) { /* one pitch per dimension: even sizes keep theirs */
+            d->ldv = row_pitch(V);
+            d->ldo = row_pitch(O);
+        }
+        trpdrv_pack_list N;
+        memset(&N, 0, sizeof N);
+        if (p->padded) {
+            N.n = 2;
+            for (int x = 0; x < 2; ++x) {
+                N.seg[x].src = b->t[x ? TRPDRV_T_XOV : TRPDRV_T_TOV];
+                N.seg[x].dst = x ? b->nxov : b->ntov;
+                N.seg[x].rows = (long long)O * O;
+                N.seg[x].width = V;
+                N.seg[x].pitch = row_pitch(V);
+                N.seg[x].neg = 1;
+            }
+            LAUNCH_TRY(trpdrv_launch_pack_rows(&N, p->stream));
+        } else {
+            const size_t ov = (size_t)O * O * V;
+            LAUNCH_TRY(trpdrv_launch_negate(b->t[TRPDRV_T_TOV], b->ntov, ov, p->stream));
+            LAUNCH_TRY(trpdrv_launch_negate(b->t[TRPDRV_T_XOV], b->nxov, ov, p->stream));
+        }
     }
     if (p->opt.mode == TRPDRV_MODE_EMULATED) {
         for (int q = 0; q < p->nsys; ++q) {
@@ -541,12 +673,7 @@ static int plan_publish(trpdrv_plan *p)
         p->graph_ready = 0;
     }
     if (p->opt.mode == TRPDRV_MODE_FUSED) {
-        const int want = p->opt.staging;
-        const int tma_ok = want != 1 && trpdrv_tma_supported(p->h_dev, p->nsys);
         const int ok = tma_ok && p->tuned_staging != 1;
-        if (want == 2 && !tma_ok)
-            return fail(TRPDRV_ERR_UNSUPPORTED, "TMA staging needs even nvir and nocc, 16-byte aligned tensors "
-                                                "and at most %d systems", TRPDRV_TMA_MAX_SYSTEMS);
         if (tma_ok) { /* maps whenever TMA is possible, so that the autotuner can time it */
             if (!p->tma_maps) {
                 p->tma_maps = aligned_alloc(64, (trpdrv_tma_maps_bytes() + 63) & ~(size_t)63);
@@ -638,12 +765,14 @@ static int enqueue_fused(trpdrv_plan *p, cudaStream_t st, int capturing)
     CUDA_TRY(cudaMemsetAsync(p->d_tot, 0, sizeof(double) * 4 * (size_t)p->nsys, st));
     CUDA_TRY(cudaEventRecordWithFlags(p->ev0, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
     if (p->total_items > 0) {
+        for (int q = 0; q < p->nsys; ++q)
+            if (p->h_dev[q].ntriples > 0) TRY(pad_refill(p, q, 1, 0, p->s[q].shape.nocc, st, &launches));
         if (p->use_tma)
             LAUNCH_TRY(trpdrv_launch_fused_tma(p->d_dev, p->nsys, p->total_items, p->d_counter, p->d_status,
                                                p->grid_tma, p->tma_maps, p->tma_mma_k, 0, st));
         else
             LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, p->total_items, p->d_counter, p->d_status, p->grid,
-                                           p->vec2, p->opt.mma_k, st));
+                                           p->vec2 || p->padded, p->opt.mma_k, st));
         ++launches;
     }
     CUDA_TRY(cudaEventRecordWithFlags(p->ev1, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
@@ -1007,7 +1136,7 @@ int trpdrv_plan_upload_execute(trpdrv_plan *p, const trpdrv_system *host, int ch
     int maxo = 1;
     for (int q = 0; q < p->nsys; ++q)
         if (p->s[q].shape.nocc > maxo) maxo = p->s[q].shape.nocc;
-    if (rc == TRPDRV_OK && !(have = (unsigned char *)malloc((size_t)maxo)))
+    if (rc == TRPDRV_OK && !(have = (unsigned char *)malloc(2 * (size_t)maxo)))
         rc = fail(TRPDRV_ERR_NOMEM, "host allocation failed");
 #define STEP(call)                          \
     do {                                    \
@@ -1053,13 +1182,21 @@ int trpdrv_plan_upload_execute(trpdrv_plan *p, const trpdrv_system *host, int ch
     int prev_q = -1;
     for (int c = 0; c < nsp && rc == TRPDRV_OK; ++c) {
         if (sp[c].q != prev_q) {
-            memset(have, 0, (size_t)maxo);
+            memset(have, 0, 2 * (size_t)maxo);
             prev_q = sp[c].q;
+            STEP(pad_refill(p, sp[c].q, 1, 0, 0, p->stream, &launches));
         }
         if (sp[c].p0 >= 0) {
+            unsigned char *padded = have + maxo; /* j blocks already in the padded copies */
             STEP(span_copies(p, host, &sp[c], have));
             STEP_CUDA(cudaEventRecord(p->chunk_ev[c], p->copy_stream));
             STEP_CUDA(cudaStreamWaitEvent(p->stream, p->chunk_ev[c], 0));
+            for (int lo = 0; lo < p->s[sp[c].q].shape.nocc;) {
+                int hi = lo;
+                while (hi < p->s[sp[c].q].shape.nocc && have[hi] && !padded[hi]) padded[hi++] = 1;
+                if (hi > lo) STEP(pad_refill(p, sp[c].q, 0, lo, hi, p->stream, &launches));
+                lo = hi > lo ? hi : lo + 1;
+            }
         }
         const int64_t n = sp[c].end - sp[c].first;
         const int cap = p->use_tma ? p->grid_tma : p->grid;
@@ -1068,7 +1205,7 @@ int trpdrv_plan_upload_execute(trpdrv_plan *p, const trpdrv_system *host, int ch
         int e = p->use_tma ? trpdrv_launch_fused_tma(p->d_dev, p->nsys, sp[c].end, p->d_chunk_first + c, p->d_status,
                                                      grid, p->tma_maps, p->tma_mma_k, 0, p->stream)
                            : trpdrv_launch_fused(p->d_dev, p->nsys, sp[c].end, p->d_chunk_first + c, p->d_status,
-                                                 grid, p->vec2, p->opt.mma_k, p->stream);
+                                                 grid, p->vec2 || p->padded, p->opt.mma_k, p->stream);
         if (e) rc = fail(TRPDRV_ERR_CUDA, "fused launch of span %d: %s", c, cudaGetErrorString((cudaError_t)e));
         ++launches;
     }
@@ -1287,7 +1424,7 @@ static int tune_usable(const trpdrv_plan *p, const trpdrv_tune_candidate *c)
     return c->batch >= 1 && c->batch <= p->fbuf_batch;
 }
 
-/* the TMA kernel's edge tile shape on every system (host mirror and device copy of the descriptors) */
+/* the fused kernel's edge tile shape on every system (host mirror and device copy of the descriptors) */
 static int tune_set_edge_pack(trpdrv_plan *p, int pack)
 {
     int changed = 0;
@@ -1308,7 +1445,7 @@ static void tune_apply(trpdrv_plan *p, const trpdrv_tune_candidate *c)
         p->use_tma = c->staging == 2;
         p->tuned_staging = c->staging; /* a later upload/bind keeps it where TMA remains possible */
         if (c->staging == 2) p->tma_mma_k = c->mma_k;
-        if (c->staging == 2) tune_set_edge_pack(p, c->edge_pack);
+        tune_set_edge_pack(p, c->edge_pack);
         if (c->staging == 1) {
             p->opt.mma_k = c->mma_k;
             p->opt.ctas_per_sm = c->ctas_per_sm;
@@ -1348,6 +1485,7 @@ static int tune_time(trpdrv_plan *p, const trpdrv_tune_candidate *c, double *est
         if (d->ntriples <= 0) continue;
         float ms = 0.0f;
         if (p->opt.mode == TRPDRV_MODE_FUSED) {
+            TRY(pad_refill(p, q, 1, 0, p->s[q].shape.nocc, st, NULL));
             const int64_t items = d->ntriples * d->npairs;
             int64_t sample = items / 8;
             if (sample < (int64_t)p->nsm * 64) sample = (int64_t)p->nsm * 64;
@@ -1355,7 +1493,7 @@ static int tune_time(trpdrv_plan *p, const trpdrv_tune_candidate *c, double *est
             const unsigned long long first = (unsigned long long)d->item_begin;
             int grid = c->staging == 2 ? p->nsm : c->ctas_per_sm * p->nsm;
             if (grid > sample) grid = (int)sample;
-            if (c->staging == 2) TRY(tune_set_edge_pack(p, c->edge_pack));
+            TRY(tune_set_edge_pack(p, c->edge_pack));
             float best = 0.0f;
             for (int rep = 0; rep < TUNE_REPS; ++rep) {
                 CUDA_TRY(cudaMemcpyAsync(p->d_counter, &first, sizeof first, cudaMemcpyHostToDevice, st));
@@ -1366,7 +1504,7 @@ static int tune_time(trpdrv_plan *p, const trpdrv_tune_candidate *c, double *est
                                                        p->d_status, grid, p->tma_maps, c->mma_k, 0, st));
                 else
                     LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, d->item_begin + sample, p->d_counter,
-                                                   p->d_status, grid, p->vec2, c->mma_k, st));
+                                                   p->d_status, grid, p->vec2 || p->padded, c->mma_k, st));
                 CUDA_TRY(cudaEventRecord(p->ev1, st));
                 TRY(tune_elapsed(p, &ms));
                 if (rep == 0 || ms < best) best = ms;
@@ -1559,11 +1697,9 @@ int trpdrv_plan_autotune(trpdrv_plan *p, trpdrv_tune_result *result)
     trpdrv_tune_candidate *c = r->cand;
     int n = 0;
     if (p->opt.mode == TRPDRV_MODE_FUSED) {
-        int occ = 1;
-        if (trpdrv_fused_max_ctas_per_sm(&occ) != 0 || occ < 1) occ = 1;
+        int packable = 0;
+        for (int q = 0; q < p->nsys; ++q) packable |= trpdrv_tma_pack_edge(p->s[q].shape.nvir);
         if (p->opt.staging != 1 && trpdrv_tma_supported(p->h_dev, p->nsys) && p->tma_maps) {
-            int packable = 0;
-            for (int q = 0; q < p->nsys; ++q) packable |= trpdrv_tma_pack_edge(p->s[q].shape.nvir);
             c[n++] = (trpdrv_tune_candidate){2, 8, 1, 0, packable, 0.0};
             c[n++] = (trpdrv_tune_candidate){2, 16, 1, 0, packable, 0.0};
             if (packable) {
@@ -1572,9 +1708,8 @@ int trpdrv_plan_autotune(trpdrv_plan *p, trpdrv_tune_result *result)
             }
         }
         if (p->opt.staging != 2) {
-            c[n++] = (trpdrv_tune_candidate){1, 8, occ, 0, 0, 0.0};
-            c[n++] = (trpdrv_tune_candidate){1, 4, occ, 0, 0, 0.0};
-            if (occ > 1 && n < 8) c[n++] = (trpdrv_tune_candidate){1, 8, 1, 0, 0, 0.0};
+            c[n++] = (trpdrv_tune_candidate){1, 8, 1, 0, packable, 0.0};
+            c[n++] = (trpdrv_tune_candidate){1, 4, 1, 0, packable, 0.0};
         }
     } else {
         static const int batches[4] = {8, 16, 32, 64};

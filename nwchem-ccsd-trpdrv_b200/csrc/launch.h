@@ -45,6 +45,9 @@ typedef struct trpdrv_dev_system {
                             adds the other's and runs the energy epilogue */
     double *split_scratch;
     unsigned *split_count;  /* one per item, zero at launch; left at zero */
+    int ldv, ldo;        /* cp.async staging: leading dimension of the rows of nvir (t2, jvv, kvv, ntov, nxov) and of
+                            nocc (jov, kov) doubles; 0 = nvir / nocc (packed, as callers hold them).  The
+                            plans pad odd rows to the next even length (trpdrv_launch_pack_rows). */
     int pack_edge;       /* 1: the last tile holds 1..16 valid virtual indices and the TMA kernel runs the
                             edge pairs (B, E), (B + 1, E) (B even) as one packed work item; the item of
                             (B + 1, E) is then skipped (its energy slots are written by the packed one) */
@@ -56,25 +59,22 @@ typedef struct trpdrv_dev_system {
     double *rec;            /* [ntriples][4] per triple */
 } trpdrv_dev_system;
 
-/* Fused persistent kernel: grid CTAs pull (triple, tile pair) items from *counter (must be 0 at
- * launch) and write per-item energies.  vec2 = 1 requires even nvir and nocc for every system;
- * mma_k selects the FP64 MMA shape m16n8k4 (4) or m16n8k8 (8). */
+/* Fused persistent kernel (fused_tma.cu): grid CTAs (one per SM) pull (triple, tile pair) items from
+ * *counter (must be 0 at launch) and write per-item energies.  *status bit 0: malformed queue entry; bit 1: a
+ * pipeline wait ran out.  Two stagings of the operands feed the same MMA loop:
+ *   trpdrv_launch_fused: cp.async; any sizes, any number of systems.  vec2 = 1 (16-byte copies) requires
+ *     even nvir and nocc and 16-byte aligned tensors for every system; mma_k selects the FP64 MMA shape
+ *     m16n8k4 (4) or m16n8k8 (8).
+ *   trpdrv_launch_fused_tma: TMA; even nvir and nocc, 16-byte aligned tensors and at most
+ *     TRPDRV_TMA_MAX_SYSTEMS systems (trpdrv_tma_supported); mma_k 8 or 16.  trpdrv_tma_prepare encodes the
+ *     tensor maps of every system into a host blob of trpdrv_tma_maps_bytes() bytes (64-byte aligned)
+ *     that each launch passes by value. */
 int trpdrv_launch_fused(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items,
                         unsigned long long *counter, int *status, int grid, int vec2, int mma_k,
                         void *stream);
-size_t trpdrv_fused_smem_bytes(void);
-int trpdrv_fused_threads(void);
-int trpdrv_fused_max_ctas_per_sm(int *n);
-int trpdrv_fused_init(void);
-
-/* The same fused computation with TMA-staged panels and mbarrier pipelines (fused_tma.cu).  Needs
- * even nvir and nocc, 16-byte aligned tensors and at most TRPDRV_TMA_MAX_SYSTEMS systems
- * (trpdrv_tma_supported).  trpdrv_tma_prepare encodes the tensor maps of every system into a
- * host blob of trpdrv_tma_maps_bytes() bytes (64-byte aligned) that each launch passes by value.
- * One CTA per SM.  *status bit 0: malformed queue entry; bit 1: a pipeline wait ran out. */
 #define TRPDRV_TMA_MAX_SYSTEMS 8
 int trpdrv_tma_supported(const trpdrv_dev_system *h_sys, int nsys);
-/* 1 if the TMA kernel packs the edge pairs of a system with this nvir (see pack_edge). */
+/* 1 if the fused kernel packs the edge pairs of a system with this nvir (see pack_edge). */
 int trpdrv_tma_pack_edge(int nvir);
 size_t trpdrv_tma_maps_bytes(void);
 int trpdrv_tma_prepare(const trpdrv_dev_system *h_sys, int nsys, void *maps_out);
@@ -136,6 +136,20 @@ int trpdrv_launch_system_reduce(const double *rec, const int32_t *triples, int64
 
 /* dst[i] = -src[i]. */
 int trpdrv_launch_negate(const double *src, double *dst, size_t n, void *stream);
+
+/* Rows copied to an even pitch: dst[r * pitch + c] = src[r * width + c] (negated where neg), zeros for
+ * c >= width, for every segment s < n and r < rows, in one launch.  pitch even, dst 16-byte aligned. */
+#define TRPDRV_PACK_LIST_MAX 8
+typedef struct trpdrv_pack_list {
+    int n;
+    struct {
+        const double *src;
+        double *dst;
+        long long rows;
+        int width, pitch, neg;
+    } seg[TRPDRV_PACK_LIST_MAX];
+} trpdrv_pack_list;
+int trpdrv_launch_pack_rows(const trpdrv_pack_list *list, void *stream);
 
 /* Device-to-device copies dst[s][0..len[s]) = src[s][..] (negated where neg[s]) for s < n, in one launch. */
 #define TRPDRV_COPY_LIST_MAX 24

@@ -6,6 +6,7 @@
 //                        omp/ccsd_trpdrv_omp_cbody.c:133-142), as a double-double (hi, lo) pair,
 //                        built with error-free TwoSum in a fixed order.
 //  negate_kernel:        dst = -src (the occupied A operands are stored negated).
+//  pack_rows_kernel:     rows of odd length copied to an even pitch (operands of the cp.async staging).
 //  gather_kernel:        a list of device-to-device copies in one launch (the drop-in entry points'
 //                        registered inputs, gathered into their staging layout).
 
@@ -124,9 +125,43 @@ __global__ void gather_kernel(const trpdrv_copy_list L)
     }
 }
 
+// One row of the grid per segment; a block copies whole rows, two destination elements per thread and step.
+// HBM-bound (reads width, writes pitch doubles a row).
+constexpr int PACK_PAIRS = 2048;  // destination pairs per block and pass
+__global__ void pack_rows_kernel(const trpdrv_pack_list L)
+{
+    const auto &g = L.seg[blockIdx.y];
+    const int ppr = g.pitch >> 1, rpb = ppr < PACK_PAIRS ? PACK_PAIRS / ppr : 1;
+    const double sg = g.neg ? -1.0 : 1.0;
+    for (long long row0 = (long long)blockIdx.x * rpb; row0 < g.rows; row0 += (long long)gridDim.x * rpb) {
+        const int nr = g.rows - row0 < rpb ? (int)(g.rows - row0) : rpb;
+        const double *src = g.src + row0 * g.width;
+        double2 *dst = reinterpret_cast<double2 *>(g.dst + row0 * g.pitch);
+        for (int e = threadIdx.x; e < nr * ppr; e += blockDim.x) {
+            const int r = e / ppr, c = 2 * (e - r * ppr);
+            const double *s = src + (long long)r * g.width + c;
+            dst[e] = make_double2(sg * __ldg(s), c + 1 < g.width ? sg * __ldg(s + 1) : 0.0);
+        }
+    }
+}
+
 }  // namespace trpdrv
 
 using namespace trpdrv;
+
+extern "C" int trpdrv_launch_pack_rows(const trpdrv_pack_list *list, void *stream)
+{
+    if (!list || list->n <= 0) return 0;
+    if (list->n > TRPDRV_PACK_LIST_MAX) return (int)cudaErrorInvalidValue;
+    long long most = 1;
+    for (int s = 0; s < list->n; ++s) {
+        const long long b = (list->seg[s].rows * (list->seg[s].pitch / 2) + PACK_PAIRS - 1) / PACK_PAIRS;
+        if (b > most) most = b;
+    }
+    pack_rows_kernel<<<dim3((unsigned)(most < 2048 ? most : 2048), (unsigned)list->n), 256, 0,
+                       (cudaStream_t)stream>>>(*list);
+    return (int)cudaGetLastError();
+}
 
 extern "C" int trpdrv_launch_gather(const trpdrv_copy_list *list, void *stream)
 {
