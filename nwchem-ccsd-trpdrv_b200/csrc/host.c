@@ -199,7 +199,7 @@ struct trpdrv_plan {
     int *d_status;
     double *d_tot;
     int64_t total_items;
-    double *d_f, *d_bpart;
+    double *d_f, *d_bpart; /* plain form: f and energy partials of one batch of triples */
     unsigned *d_tcount;
     cudaGraph_t graph;
     cudaGraphExec_t gexec;
@@ -298,6 +298,13 @@ static void plan_free(trpdrv_plan *p)
     free(p);
 }
 
+/* Triples per launch of a plain plan's system. */
+static int64_t plain_batch(const sysbuf *b)
+{
+    const int64_t n = trpdrv_plain_batch(b->shape.nvir);
+    return b->ntriples < n ? (b->ntriples > 0 ? b->ntriples : 1) : n;
+}
+
 static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
 {
     const trpdrv_options *o = &p->opt;
@@ -309,7 +316,7 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
     if (!p->s || !p->h_dev) return fail(TRPDRV_ERR_NOMEM, "host allocation failed");
 
     int64_t item = 0;
-    int maxv = 0, maxpairs = 0;
+    int maxv = 0;
     int even = 1;
     for (int q = 0; q < p->nsys; ++q) {
         sysbuf *b = &p->s[q];
@@ -319,7 +326,6 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
         b->nb = (nvir + TRPDRV_TILE - 1) / TRPDRV_TILE;
         b->npairs = b->nb * (b->nb + 1) / 2;
         if (nvir > maxv) maxv = nvir;
-        if (b->npairs > maxpairs) maxpairs = b->npairs;
 
         /* the reference driver's order, then this rank's contiguous share (uniform cost per system) */
         const int64_t n = trpdrv_shard_triples(nocc, o->nkpass, o->rank, o->world, NULL);
@@ -426,10 +432,17 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
         }
     }
     if (o->mode == TRPDRV_MODE_PLAIN) {
-        CUDA_TRY(cudaMalloc((void **)&p->d_f, sizeof(double) * 8 * (size_t)maxv * maxv));
-        CUDA_TRY(cudaMalloc((void **)&p->d_bpart, sizeof(double) * 4 * (size_t)maxpairs));
-        CUDA_TRY(cudaMalloc((void **)&p->d_tcount, sizeof(unsigned)));
-        CUDA_TRY(cudaMemset(p->d_tcount, 0, sizeof(unsigned)));
+        size_t nf = 1, nbp = 1, nct = 1; /* one batch of the largest system */
+        for (int q = 0; q < p->nsys; ++q) {
+            const size_t V = (size_t)shape[q].nvir, n = (size_t)plain_batch(&p->s[q]);
+            if (n * 8 * V * V > nf) nf = n * 8 * V * V;
+            if (n * 4 * (size_t)trpdrv_tengy_pairs((int)V) > nbp) nbp = n * 4 * (size_t)trpdrv_tengy_pairs((int)V);
+            if (n > nct) nct = n;
+        }
+        CUDA_TRY(cudaMalloc((void **)&p->d_f, sizeof(double) * nf));
+        CUDA_TRY(cudaMalloc((void **)&p->d_bpart, sizeof(double) * nbp));
+        CUDA_TRY(cudaMalloc((void **)&p->d_tcount, sizeof(unsigned) * nct));
+        CUDA_TRY(cudaMemset(p->d_tcount, 0, sizeof(unsigned) * nct));
     }
 
     int per_sm = o->ctas_per_sm;
@@ -881,62 +894,10 @@ static int enqueue_plain(trpdrv_plan *p, cudaStream_t st)
     CUDA_TRY(cudaEventRecord(p->ev0, st));
     for (int q = 0; q < p->nsys; ++q) {
         const sysbuf *b = &p->s[q];
-        const int O = b->shape.nocc, V = b->shape.nvir;
-        const size_t lnvv = (size_t)V * V, lnov = (size_t)O * V;
-        trpdrv_plain_args ga;
-        trpdrv_tengy_args ta;
-        memset(&ga, 0, sizeof ga);
-        memset(&ta, 0, sizeof ta);
-        ga.nocc = O;
-        ga.nvir = V;
-        ga.f = p->d_f;
-        ta.ncor = b->shape.ncor;
-        ta.nocc = O;
-        ta.nvir = V;
-        ta.use_eaijk = 0;
-        ta.a = b->shape.a;
-        ta.f = p->d_f;
-        ta.eorb = b->t[TRPDRV_T_EORB];
-        ta.block_partial = p->d_bpart;
-        ta.counter = p->d_tcount;
-        for (int64_t r = 0; r < b->ntriples; ++r) {
-            const int64_t ai = r / b->nt, t = r - ai * b->nt; /* records are [a][triple] */
-            const int pk = b->h_triples[t];
-            const int i = pk & 1023, j = (pk >> 10) & 1023, k = (pk >> 20) & 1023; /* 0-based */
-            const size_t jo = (size_t)j * O, ao = (size_t)ai * O;
-            const double *jia = b->t[TRPDRV_T_JVV] + (ao + i) * lnvv, *kia = b->t[TRPDRV_T_KVV] + (ao + i) * lnvv;
-            const double *jka = b->t[TRPDRV_T_JVV] + (ao + k) * lnvv, *kka = b->t[TRPDRV_T_KVV] + (ao + k) * lnvv;
-            const double *tij = b->t[TRPDRV_T_T2] + (jo + i) * lnvv, *tkj = b->t[TRPDRV_T_T2] + (jo + k) * lnvv;
-            const double *ntia = b->ntov + i * lnov, *nxia = b->nxov + i * lnov;
-            const double *ntka = b->ntov + k * lnov, *nxka = b->nxov + k * lnov;
-            const double *jij = b->t[TRPDRV_T_JOV] + (jo + i) * lnov, *kij = b->t[TRPDRV_T_KOV] + (jo + i) * lnov;
-            const double *jkj = b->t[TRPDRV_T_JOV] + (jo + k) * lnov, *kkj = b->t[TRPDRV_T_KOV] + (jo + k) * lnov;
-            /* f1n f2n f3n f4n f1t f2t f3t f4t: omp/ccsd_trpdrv_omp_cbody.c:70-117 */
-            const double *a1[8] = {jia, kia, jia, kia, jka, kka, jka, kka};
-            const double *b1[8] = {tkj, tkj, tkj, tkj, tij, tij, tij, tij};
-            const int nt[8] = {1, 1, 0, 0, 1, 1, 0, 0};
-            const double *a2[8] = {ntia, nxia, ntia, nxia, ntka, nxka, ntka, nxka};
-            const double *b2[8] = {kkj, kkj, jkj, jkj, kij, kij, jij, jij};
-            for (int x = 0; x < 8; ++x) {
-                ga.a1[x] = a1[x];
-                ga.b1[x] = b1[x];
-                ga.b1_nt[x] = nt[x];
-                ga.a2[x] = a2[x];
-                ga.b2[x] = b2[x];
-            }
-            LAUNCH_TRY(trpdrv_launch_plain_gemm(&ga, p->vec2, st));
-            ta.a = b->shape.a + (int)ai;
-            ta.i = i + 1;
-            ta.j = j + 1;
-            ta.k = k + 1;
-            ta.dintc1 = b->t[TRPDRV_T_DINTC] + (ao + i) * V;
-            ta.dintx1 = b->t[TRPDRV_T_DINTX] + (ao + i) * V;
-            ta.t1v1 = b->t[TRPDRV_T_T1V] + (ao + i) * V;
-            ta.dintc2 = b->t[TRPDRV_T_DINTC] + (ao + k) * V;
-            ta.dintx2 = b->t[TRPDRV_T_DINTX] + (ao + k) * V;
-            ta.t1v2 = b->t[TRPDRV_T_T1V] + (ao + k) * V;
-            ta.out4 = b->rec + 4 * r;
-            LAUNCH_TRY(trpdrv_launch_tengy(&ta, st));
+        const int64_t batch = plain_batch(b);
+        for (int64_t r = 0; r < b->ntriples; r += batch) {
+            const int n = (int)(b->ntriples - r < batch ? b->ntriples - r : batch);
+            LAUNCH_TRY(trpdrv_launch_plain_batch(&p->h_dev[q], r, n, p->d_f, p->d_bpart, p->d_tcount, p->vec2, r > 0, st));
             launches += 2;
         }
     }
@@ -1778,7 +1739,6 @@ static struct dropin_state {
     size_t cap_vv, cap_ov, cap_v, cap_bf, cap_pairs;
     double *vv[DI_NVV];
     double *ov[DO_NOV];
-    double *nov[4];
     double *vec[6];
     double *eorb, *f, *bpart, *out4;
     unsigned *tcount;
@@ -1829,7 +1789,6 @@ static void di_release(void)
     reg_release();
     for (int q = 0; q < DI_NVV; ++q) cudaFree(g_di.vv[q]);
     for (int q = 0; q < DO_NOV; ++q) cudaFree(g_di.ov[q]);
-    for (int q = 0; q < 4; ++q) cudaFree(g_di.nov[q]);
     for (int q = 0; q < 6; ++q) cudaFree(g_di.vec[q]);
     cudaFree(g_di.eorb);
     cudaFree(g_di.f);
@@ -1975,8 +1934,7 @@ static int di_reserve(int nocc, int nvir, int nbf)
         CUDA_TRY(cudaSetDevice(g_di.device));
     }
     const size_t vv = (size_t)nvir * nvir, ov = (size_t)nocc * nvir, v = (size_t)nvir, bf = (size_t)nbf;
-    const int nb = (nvir + TRPDRV_TILE - 1) / TRPDRV_TILE;
-    const size_t pairs = (size_t)nb * (nb + 1) / 2;
+    const size_t pairs = (size_t)trpdrv_tengy_pairs(nvir);
     if (vv > g_di.cap_vv) {
         for (int q = 0; q < DI_NVV; ++q) DI_GROW(g_di.vv[q], vv);
         DI_GROW(g_di.f, 8 * vv);
@@ -1984,7 +1942,6 @@ static int di_reserve(int nocc, int nvir, int nbf)
     }
     if (ov > g_di.cap_ov) {
         for (int q = 0; q < DO_NOV; ++q) DI_GROW(g_di.ov[q], ov);
-        for (int q = 0; q < 4; ++q) DI_GROW(g_di.nov[q], ov);
         g_di.cap_ov = ov;
     }
     if (v > g_di.cap_v) {
@@ -2382,20 +2339,19 @@ static int body_impl(double *f1n, double *f1t, double *f2n, double *f2t, double 
     const double *vecs[6] = {dintc1, dintx1, t1v1, dintc2, dintx2, t1v2};
     for (int q = 0; q < 6; ++q) TRY(h2d(&dvec[q], g_di.vec[q], vecs[q], (size_t)nvir));
     TRY(h2d(&deorb, g_di.eorb, eorb, (size_t)nbf));
-    for (int q = 0; q < 4; ++q) LAUNCH_TRY(trpdrv_launch_negate(dov[q], g_di.nov[q], lnov, g_di.stream));
 
     trpdrv_plain_args ga;
     memset(&ga, 0, sizeof ga);
     ga.nocc = nocc;
     ga.nvir = nvir;
+    ga.neg2 = 1; /* the reference's alpha = -1 GEMMs */
     ga.f = g_di.f;
     const double *const *V = dv;
-    double *const *N = g_di.nov;
     const double *const *Ob = dov;
     const double *a1[8] = {V[DI_JIA], V[DI_KIA], V[DI_JIA], V[DI_KIA], V[DI_JKA], V[DI_KKA], V[DI_JKA], V[DI_KKA]};
     const double *b1[8] = {V[DI_TKJ], V[DI_TKJ], V[DI_TKJ], V[DI_TKJ], V[DI_TIJ], V[DI_TIJ], V[DI_TIJ], V[DI_TIJ]};
     const int nt[8] = {1, 1, 0, 0, 1, 1, 0, 0};
-    const double *a2[8] = {N[0], N[1], N[0], N[1], N[2], N[3], N[2], N[3]};
+    const double *a2[8] = {Ob[DO_TIA], Ob[DO_XIA], Ob[DO_TIA], Ob[DO_XIA], Ob[DO_TKA], Ob[DO_XKA], Ob[DO_TKA], Ob[DO_XKA]};
     const double *b2[8] = {Ob[DO_KKJ], Ob[DO_KKJ], Ob[DO_JKJ], Ob[DO_JKJ], Ob[DO_KIJ], Ob[DO_KIJ], Ob[DO_JIJ], Ob[DO_JIJ]};
     for (int x = 0; x < 8; ++x) {
         ga.a1[x] = a1[x];
@@ -2404,7 +2360,9 @@ static int body_impl(double *f1n, double *f1t, double *f2n, double *f2t, double 
         ga.a2[x] = a2[x];
         ga.b2[x] = b2[x];
     }
-    const int vec2 = !(nvir & 1) && !(nocc & 1);
+    int vec2 = !(nvir & 1) && !(nocc & 1);
+    for (int x = 0; x < 8; ++x) /* slices of registered arrays may start anywhere */
+        if (((uintptr_t)ga.a1[x] | (uintptr_t)ga.b1[x] | (uintptr_t)ga.a2[x] | (uintptr_t)ga.b2[x]) & 15u) vec2 = 0;
     LAUNCH_TRY(trpdrv_launch_plain_gemm(&ga, vec2, g_di.stream));
 
     /* omp/ccsd_trpdrv_omp_cbody.c:122-126 */

@@ -162,20 +162,25 @@ typedef struct trpdrv_copy_list {
 } trpdrv_copy_list;
 int trpdrv_launch_gather(const trpdrv_copy_list *list, void *stream);
 
-/* Plain per-triple path: one grouped launch computes the eight f = A1*op(B1) + A2*B2 into
- * f[8][nvir][nvir] (order f1n f2n f3n f4n f1t f2t f3t f4t); b1_nt[x] = 1 if B1 is used transposed. */
+/* Plain path.  Single triple: one grouped launch computes the eight f = A1*op(B1) + A2*B2 (neg2: - A2*B2) into
+ * f[8][nvir][nvir] (order f1n f2n f3n f4n f1t f2t f3t f4t); b1_nt[x] = 1 if B1 is used transposed.  counter, if
+ * not NULL, is zeroed for the trpdrv_launch_tengy that follows on the stream. */
 typedef struct trpdrv_plain_args {
-    int nocc, nvir;
+    int nocc, nvir, neg2;
     const double *a1[8], *b1[8], *a2[8], *b2[8];
     int b1_nt[8];
     double *f;
+    unsigned *counter;
 } trpdrv_plain_args;
 int trpdrv_launch_plain_gemm(const trpdrv_plain_args *args, int vec2, void *stream);
 
+/* Tile pairs trpdrv_launch_tengy sums one by one (the length of block_partial in fours). */
+int64_t trpdrv_tengy_pairs(int nvir);
 /* Standalone tengy over f[8][nvir][nvir] on the device.  eaijk is taken from `eaijk` when
  * use_eaijk != 0, else computed on the device from eorb and the 1-based a, i, j, k.  Writes
- * out4[0..3] = emp4i, emp5i, emp4k, emp5k.  block_partial needs 4*npairs doubles, counter one
- * zeroed unsigned int (it is left at zero again). */
+ * out4[0..3] = emp4i, emp5i, emp4k, emp5k.  block_partial needs 4*trpdrv_tengy_pairs(nvir) doubles, counter
+ * one zeroed unsigned int (it is left at zero again).  Launched as a programmatic dependent of the launch
+ * before it on the stream, which must be what writes f (or no kernel). */
 typedef struct trpdrv_tengy_args {
     int ncor, nocc, nvir;
     int use_eaijk;
@@ -188,8 +193,14 @@ typedef struct trpdrv_tengy_args {
     double *out4;
 } trpdrv_tengy_args;
 int trpdrv_launch_tengy(const trpdrv_tengy_args *args, void *stream);
-size_t trpdrv_tengy_smem_bytes(void);
 
+/* Records pos0 .. pos0 + n - 1 of a plan's system: f into f[n][8][nvir][nvir], then the energies into
+ * h_sys->rec.  block_partial: n * 4 * trpdrv_tengy_pairs(nvir) doubles; counter: n zeros (left at zero).
+ * trpdrv_plain_batch: the batch plans use for this nvir.  vec2 as for the fused kernel.  chained: the launch
+ * before it on the stream is the same system's previous batch, whose energies this one's products may overlap. */
+int trpdrv_plain_batch(int nvir);
+int trpdrv_launch_plain_batch(const trpdrv_dev_system *h_sys, int64_t pos0, int n, double *f, double *block_partial,
+                              unsigned *counter, int vec2, int chained, void *stream);
 
 /* Sets the dynamic shared memory limits of every kernel (call once per device). */
 int trpdrv_kernels_init(void);

@@ -10,7 +10,7 @@
 // one statically sized device array that the CUDA module reserves when it loads:
 //
 //   * at most TRPDRV_NOALLOC_MAX_NVIR virtual and TRPDRV_NOALLOC_MAX_NOCC occupied orbitals;
-//   * every GPU that loads the library keeps the array (about 4.7 MB) until the process exits;
+//   * every GPU that loads the library keeps the array (about 4.2 MB) until the process exits;
 //   * all calls on a device share it, so calls that overlap on the GPU (different streams, or
 //     different host threads) race on it and produce garbage: serialise them;
 //   * the first call on each device looks up the array's device address (cudaGetSymbolAddress)
@@ -34,14 +34,13 @@ namespace {
 
 constexpr int MAXV = TRPDRV_NOALLOC_MAX_NVIR;
 constexpr int MAXO = TRPDRV_NOALLOC_MAX_NOCC;
-constexpr int MAXNB = (MAXV + TRPDRV_TILE - 1) / TRPDRV_TILE;
+constexpr int MAXNB = (MAXV + 15) / 16;  // the energy kernel's 16-wide tiles
 constexpr int MAXPAIRS = MAXNB * (MAXNB + 1) / 2;
 
-// scratch layout (doubles): [counter block][tengy partials][4 negated occupied operands][8 f tiles]
+// scratch layout (doubles): [counter block][tengy partials][8 f tiles]
 constexpr size_t OFF_COUNTER = 0;                                  // one unsigned int, 256-byte block
 constexpr size_t OFF_PARTIAL = 32;                                 // 4 * MAXPAIRS doubles
-constexpr size_t OFF_NEG = OFF_PARTIAL + ((4 * MAXPAIRS + 31) / 32) * 32;
-constexpr size_t OFF_F = OFF_NEG + 4 * (size_t)MAXV * MAXO;
+constexpr size_t OFF_F = OFF_PARTIAL + ((4 * MAXPAIRS + 31) / 32) * 32;
 constexpr size_t SCRATCH_DOUBLES = OFF_F + 8 * (size_t)MAXV * MAXV;
 
 static __device__ __align__(256) double g_noalloc_scratch[SCRATCH_DOUBLES];
@@ -123,29 +122,22 @@ extern "C" int trpdrv_body_device_noalloc(const trpdrv_body_device_args *a, void
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned int *counter = reinterpret_cast<unsigned int *>(scratch + OFF_COUNTER);
     double *partial = scratch + OFF_PARTIAL;
-    double *neg = scratch + OFF_NEG;
     double *f = scratch + OFF_F;
-    const size_t lnov = (size_t)O * V;
 
-    // the last CTA of the reduction must see a zero counter, whatever a previous call left behind
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
-    if (e != cudaSuccess) return fail(TRPDRV_ERR_CUDA, "trpdrv_body_device_noalloc: clearing the counter failed");
-    // -tia, -xia, -tka, -xka (the reference's alpha = -1 GEMMs, omp/ccsd_trpdrv_omp_cbody.c:73-116)
-    const double *occ[4] = {a->tia, a->xia, a->tka, a->xka};
-    for (int q = 0; q < 4; ++q)
-        if (trpdrv_launch_negate(occ[q], neg + q * lnov, lnov, st) != 0)
-            return fail(TRPDRV_ERR_CUDA, "trpdrv_body_device_noalloc: launch failed");
-
+    // two launches: the GEMM subtracts its occupied products (the reference's alpha = -1 GEMMs,
+    // omp/ccsd_trpdrv_omp_cbody.c:73-116) and zeroes the counter that the reduction's last CTA needs to see at
+    // zero, whatever a previous call left behind
     trpdrv_plain_args ga = {};
     ga.nocc = O;
     ga.nvir = V;
+    ga.neg2 = 1;
     ga.f = f;
-    const double *nt_i = neg, *nx_i = neg + lnov, *nt_k = neg + 2 * lnov, *nx_k = neg + 3 * lnov;
+    ga.counter = counter;
     // f1n f2n f3n f4n f1t f2t f3t f4t: omp/ccsd_trpdrv_omp_cbody.c:70-117
     const double *a1[8] = {a->jia, a->kia, a->jia, a->kia, a->jka, a->kka, a->jka, a->kka};
     const double *b1[8] = {a->tkj, a->tkj, a->tkj, a->tkj, a->tij, a->tij, a->tij, a->tij};
     const int nt[8] = {1, 1, 0, 0, 1, 1, 0, 0};
-    const double *a2[8] = {nt_i, nx_i, nt_i, nx_i, nt_k, nx_k, nt_k, nx_k};
+    const double *a2[8] = {a->tia, a->xia, a->tia, a->xia, a->tka, a->xka, a->tka, a->xka};
     const double *b2[8] = {a->kkj, a->kkj, a->jkj, a->jkj, a->kij, a->kij, a->jij, a->jij};
     int vec2 = !(V & 1) && !(O & 1);
     for (int x = 0; x < 8; ++x) {
