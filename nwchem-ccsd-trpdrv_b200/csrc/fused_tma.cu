@@ -58,7 +58,6 @@ constexpr int NPANEL = 16;
 constexpr int STAGE_BYTES = NPANEL * PANEL_BYTES;
 constexpr int RING = 16;
 constexpr int TICKETS = 8;  // work tickets in flight between the producer warps (>= STAGES + 2)
-constexpr int XBUF = T * (T + 1);  // one padded 32x32 f tile
 constexpr int KBOX = PANEL_BYTES / 2;  // one 16-row K-major box
 constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_BYTES + 1024;  // + alignment slack
 constexpr unsigned long long WAIT_LIMIT_NS = 4000000000ull;       // 4 s: far above any legitimate wait
@@ -600,7 +599,6 @@ __device__ __forceinline__ void warp_epilogue(const ItemCtx &cx, const double (&
     TengySums su = {0.0, 0.0, 0.0, 0.0};
     const int V = cx.nvir;
     const double *ev = cx.eorb + cx.ncor + cx.nocc;
-    const double eaijk = cx.eaijk;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int b = rb0 + perm8(g) + 8 * h;
@@ -618,7 +616,7 @@ __device__ __forceinline__ void warp_epilogue(const ItemCtx &cx, const double (&
                 fcb[x] = gT[x][e];
             }
             // omp/ccsd_tengy_c99.c:65 denominator; e_b + e_c == e_c + e_b, so (b,c) and (c,b) share it
-            tengy_pair<!DIAG>(fbc, fcb, -1.0 / (eb + __ldg(ev + c) + eaijk), vb, load_idx(cx, c), su);
+            tengy_pair<!DIAG>(fbc, fcb, -1.0 / (eb + __ldg(ev + c) + cx.eaijk), vb, load_idx(cx, c), su);
         }
     }
     su.e4i = warp_sum(su.e4i);
@@ -995,6 +993,14 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
                 }
             }
         }
+        if (it.diag) {  // a slot for the consumers' exchange
+            if (!mbar_wait(&empty[stage], phase ^ 1, status)) return;
+            Stage::marker(&full[stage], pw, lane);
+            if (++stage == STAGES) {
+                stage = 0;
+                phase ^= 1;
+            }
+        }
     }
 }
 
@@ -1058,6 +1064,10 @@ __device__ __forceinline__ bool skip_slots(int n, const Pipe &pp, RingPos &rp)
     return true;
 }
 
+// Place of (row, col) in a 32x32 exchange tile: the half-warp's four rows {0,6,1,7} or {2,4,3,5} (mod 8) and four
+// columns, and the same with the roles swapped, fall in 16 different bank pairs.
+__device__ __forceinline__ int xch_off(int row, int col) { return row * T + (col ^ ((row & 3) << 2)); }
+
 // i == k: the t family's operands are the n family's, so its products are the same numbers.
 __device__ __forceinline__ void copy_families(double (&f)[8][4], double (&gT)[8][4])
 {
@@ -1091,8 +1101,7 @@ fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long tota
     __shared__ __align__(8) unsigned long long full[STAGES], empty[STAGES], tbar[TICKETS];
     __shared__ ItemCtx ring[RING];
     __shared__ long long tickets[TICKETS];
-    __shared__ double xbuf[2 * XBUF];                       // diagonal-pair transpose exchange
-    __shared__ __align__(8) unsigned long long xbar[1];
+    __shared__ __align__(8) unsigned long long xbar[1];     // diagonal-pair exchange, split items
     __shared__ int split_flag[1];
     // aligned by an offset, not by integer arithmetic on the pointer: the compiler then still knows that the
     // fragment reads are shared-memory loads (32-bit addresses)
@@ -1205,27 +1214,42 @@ fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long tota
         if (SPLIT && (cx.split_tag & 1)) {  // the second half to arrive adds the first's partial sums and finishes
             int fin = 0;
             if (!split_combine(sys, cx, f, gT, warp, lane, xbar, xphase, split_flag, status, fin)) return;
-            if (!fin) continue;
+            if (!fin) {
+                if (diag && !skip_slots(1, pipe, rp)) return;  // the exchange slot
+                continue;
+            }
         }
         if (diag) {
-            // f(c,b) of a diagonal pair is f at the mirrored position of the same 32x32 block, held
-            // by another warp: exchange one f at a time through two alternating shared buffers,
-            // separated by a consumer-only mbarrier (bounded wait; no CTA-wide barrier).
+            // f(c,b) of a diagonal pair is f at the mirrored position of the same 32x32 block, held by another
+            // warp.  The item has one more stage slot, which the producers leave empty: all tiles (8 KB each, rows
+            // of 256 bytes with the columns XORed so that neither the writes nor the mirrored reads conflict)
+            // are exchanged through it with one consumer-only mbarrier (bounded wait; no CTA-wide barrier).
+            if (!pipe.wait(rp)) return;
+            double *xt = reinterpret_cast<double *>(stages + (size_t)rp.stage * STAGE_BYTES);
 #pragma unroll
             for (int x = 0; x < 8; ++x) {
                 if (x == 4 && same) break;
-                double *xb = xbuf + (x & 1) * XBUF;
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    xb[(rx0 + perm8(g) + ((e & 2) ? 8 : 0)) * (T + 1) + cx0 + perm8(2 * t + (e & 1))] = f[x][e];
-                __syncwarp();
-                if (lane == 0) mbar_arrive(xbar);
-                if (!mbar_wait(xbar, xphase, status)) return;
-                xphase ^= 1;
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    gT[x][e] = xb[(cx0 + perm8(2 * t + (e & 1))) * (T + 1) + rx0 + perm8(g) + ((e & 2) ? 8 : 0)];
+                for (int e = 0; e < 4; ++e) {
+                    const int row = rx0 + perm8(g) + ((e & 2) ? 8 : 0), col = cx0 + perm8(2 * t + (e & 1));
+                    xt[x * T * T + xch_off(row, col)] = f[x][e];
+                }
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(xbar);
+            if (!mbar_wait(xbar, xphase, status)) return;
+            xphase ^= 1;
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+                if (x == 4 && same) break;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int row = rx0 + perm8(g) + ((e & 2) ? 8 : 0), col = cx0 + perm8(2 * t + (e & 1));
+                    gT[x][e] = xt[x * T * T + xch_off(col, row)];
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the slot's next TMA writes
+            pipe.release(rp);
         }
         if (same) copy_families(f, gT);
         if (diag)
