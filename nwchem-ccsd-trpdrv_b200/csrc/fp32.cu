@@ -4,14 +4,14 @@
 // because its entry points keep the reference's names with float arguments
 // (gpu-omp/test.c:24-62).  It exists to compare with that variant's numbers, not for speed:
 //
-//  * sgemm_group_kernel: the eight f = A1 op(B1) - A2 B2 of one triple in IEEE FP32 (FFMA, no TF32),
-//    64 x 64 output tiles, 16-index contraction chunks staged in shared memory, 4 x 4 outputs per
-//    thread;
-//  * tengy_f32_kernel: the (b,c) sum of the reference's float energy forms over 32 x 32 tile pairs
-//    (the denominator formed as the reference forms it: -1.0 / (float sum), a double division
-//    rounded to float), float partial sums per tile pair, then one block sums the pairs in a fixed
-//    order.
+//  * sgemm_group_kernel: the eight f = A1 op(B1) - A2 B2 of one triple in IEEE FP32 (FFMA, no TF32), 64 x 64 or
+//    (few tiles) 32 x 32 outputs per CTA, 16-index contraction chunks staged by cp.async three deep, 4 x 4
+//    outputs per thread;
+//  * tengy_f32_kernel: the (b,c) sum of the reference's float energy forms over 16 x 16 tile pairs (the denominator
+//    formed as the reference forms it: -1.0 / (float sum), a double division rounded to float), float partial
+//    sums per tile pair, which the last CTA sums in a fixed order and writes to pinned host memory.
 //
+// A call is bound by the host: its slices are compared with a pinned mirror and sent in one or two pieces (stage.h).
 // All arithmetic of the energies is float, like the reference's (its emp4i..emp5k are float).
 
 #include <cuda_runtime.h>
@@ -20,104 +20,154 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "stage.h"
 #include "trpdrv_fp32.h"
 
 namespace trpdrv {
 namespace f32 {
 
-constexpr int BT = 64;   // output tile edge
-constexpr int KB = 16;   // contraction chunk
-constexpr int TT = 32;   // tengy tile edge
-constexpr int NT = 256;  // threads per CTA
+constexpr int KB = 16;     // contraction chunk
+constexpr int STAGES = 3;
+constexpr int TT = 16;     // tengy tile edge
+constexpr int NT = TT * TT;
 
 struct GemmArgs {
-    int nocc, nvir;
+    int nocc, nvir, ldv, ldo;  // ldv, ldo: row lengths of nvir and nocc floats, multiples of 4 (zero pads)
     const float *a1[8], *b1[8], *a2[8], *b2[8];
-    int b1_t[8];  // 1: B1 enters transposed (B1'(d, c) = B1[c + d nvir])
+    int b1_t[8];  // 1: B1 enters transposed (B1'(d, c) = B1[c + d ldv])
     float *f;     // [8][nvir][nvir]
+    unsigned *counter;  // zeroed for the energy kernel that follows
 };
 
-// f_x(b, c) = sum_d A1(b, d) B1'(d, c) - sum_m A2(b, m) B2(m, c), column-major like the reference.
-__global__ void __launch_bounds__(NT) sgemm_group_kernel(const GemmArgs P)
+__device__ __forceinline__ void cp16(float *smem, const float *gmem, bool ok)
 {
-    __shared__ float As[KB][BT + 4], Bs[KB][BT + 4];
-    const int x = blockIdx.z, V = P.nvir, O = P.nocc;
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    const int n = ok ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
+}
+
+// Threads of a CTA of BT x BT outputs, and one stage: A K-major [KB][BT + 4]; B K-major the same or X-major
+// [BT][KB + 4] (pitch 20: eight columns' float4 fall in eight different 16-byte bank groups).
+template <int BT> struct Tile {
+    static constexpr int THREADS = (BT / 4) * (BT / 4);
+    static constexpr int PK = BT + 4, PX = KB + 4;
+    static constexpr int APANEL = KB * PK, BPANEL = APANEL > BT * PX ? APANEL : BT * PX;
+    static constexpr int STAGE = APANEL + BPANEL;
+};
+
+// f_x(b, c) = sum_d A1(b, d) B1'(d, c) - sum_m A2(b, m) B2(m, c), column-major like the reference; each output one
+// FFMA chain in the order d, then m.
+template <int BT>
+__global__ void __launch_bounds__(Tile<BT>::THREADS) sgemm_group_kernel(const __grid_constant__ GemmArgs P)
+{
+    using L = Tile<BT>;
+    constexpr int W = BT / 4;  // threads along a tile edge
+    __shared__ __align__(16) float sm[STAGES][L::STAGE];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if ((blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) *P.counter = 0u;
+    const int x = blockIdx.z, V = P.nvir, O = P.nocc, tid = threadIdx.x;
     const int b0 = blockIdx.x * BT, c0 = blockIdx.y * BT;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
+    const int tx = tid % W, ty = tid / W;
     const float *A1 = P.a1[x], *B1 = P.b1[x], *A2 = P.a2[x], *B2 = P.b2[x];
-    const int bt = P.b1_t[x];
-    for (int phase = 0; phase < 2; ++phase) {
-        const int K = phase ? O : V;
-        for (int k0 = 0; k0 < K; k0 += KB) {
-            for (int e = threadIdx.x; e < KB * BT; e += NT) {
-                // A tile: rows b contiguous in memory
-                const int bb = e % BT, kk = e / BT, b = b0 + bb, k = k0 + kk;
-                float av = 0.0f;
-                if (b < V && k < K) av = phase ? -A2[b + (size_t)k * V] : A1[b + (size_t)k * V];
-                As[kk][bb] = av;
-                // B tile: contiguous along c when B1 enters transposed, else along the contraction
-                int cc, kb;
-                if (!phase && bt) {
-                    cc = e % BT;
-                    kb = e / BT;
-                } else {
-                    kb = e % KB;
-                    cc = e / KB;
-                }
-                const int c = c0 + cc, k2 = k0 + kb;
-                float bv = 0.0f;
-                if (c < V && k2 < K)
-                    bv = phase ? B2[k2 + (size_t)c * O] : (bt ? B1[c + (size_t)k2 * V] : B1[k2 + (size_t)c * V]);
-                Bs[kb][cc] = bv;
+    const int bt = P.b1_t[x], nV = (V + KB - 1) / KB, nch = nV + (O + KB - 1) / KB;
+
+    auto load = [&](int ch) {
+        if (ch < nch) {
+            const bool occ = ch >= nV;
+            const int k0 = (occ ? ch - nV : ch) * KB, K = occ ? O : V;
+            float *As = sm[ch % STAGES], *Bs = As + L::APANEL;
+            const float *A = occ ? A2 : A1, *B = occ ? B2 : B1;
+            for (int e = tid; e < KB * W; e += L::THREADS) {  // rows b contiguous
+                const int k = e / W, r = (e % W) * 4;
+                const bool ok = b0 + r < P.ldv && k0 + k < K;
+                cp16(As + k * L::PK + r, ok ? A + (b0 + r) + (size_t)(k0 + k) * P.ldv : A, ok);
             }
-            __syncthreads();
-#pragma unroll
-            for (int kk = 0; kk < KB; ++kk) {
-                float a[4], b[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    a[u] = As[kk][ty + 16 * u];
-                    b[u] = Bs[kk][tx + 16 * u];
+            if (!occ && bt) {
+                for (int e = tid; e < KB * W; e += L::THREADS) {
+                    const int k = e / W, c = (e % W) * 4;
+                    const bool ok = c0 + c < P.ldv && k0 + k < K;
+                    cp16(Bs + k * L::PK + c, ok ? B + (c0 + c) + (size_t)(k0 + k) * P.ldv : B, ok);
                 }
+            } else {  // contraction contiguous; a row's pad holds zeros
+                const int ld = occ ? P.ldo : P.ldv;
+                for (int e = tid; e < BT * (KB / 4); e += L::THREADS) {
+                    const int c = e / (KB / 4), k = (e % (KB / 4)) * 4;
+                    const bool ok = c0 + c < V && k0 + k < ld;
+                    cp16(Bs + c * L::PX + k, ok ? B + (k0 + k) + (size_t)(c0 + c) * ld : B, ok);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+
+    float acc[4][4] = {};
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) load(s);
+    for (int ch = 0; ch < nch; ++ch) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
+        __syncthreads();
+        load(ch + STAGES - 1);
+        const float *As = sm[ch % STAGES], *Bs = As + L::APANEL;
+        const bool occ = ch >= nV;
+        const float sg = occ ? -1.0f : 1.0f;
+        const bool bk = !occ && bt;
+#pragma unroll
+        for (int k4 = 0; k4 < KB / 4; ++k4) {
+            float bv[4][4];  // [kk][w]
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const int c = tx + W * w;
+                if (bk) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) bv[q][w] = Bs[(4 * k4 + q) * L::PK + c];
+                } else {
+                    const float4 v = *reinterpret_cast<const float4 *>(Bs + c * L::PX + 4 * k4);
+                    bv[0][w] = v.x;
+                    bv[1][w] = v.y;
+                    bv[2][w] = v.z;
+                    bv[3][w] = v.w;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 a = *reinterpret_cast<const float4 *>(As + (4 * k4 + q) * L::PK + 4 * ty);
+                const float av[4] = {sg * a.x, sg * a.y, sg * a.z, sg * a.w};
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) acc[u][w] = fmaf(a[u], b[w], acc[u][w]);
+                    for (int w = 0; w < 4; ++w) acc[u][w] = fmaf(av[u], bv[q][w], acc[u][w]);
             }
-            __syncthreads();
         }
     }
+    asm volatile("cp.async.wait_group 0;\n" ::);
     float *F = P.f + (size_t)x * V * V;
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-            const int b = b0 + ty + 16 * u, c = c0 + tx + 16 * w;
+            const int b = b0 + 4 * ty + u, c = c0 + tx + W * w;
             if (b < V && c < V) F[b + (size_t)c * V] = acc[u][w];
         }
 }
 
 struct TengyArgs {
-    int ncor, nocc, nvir, nb;
+    int ncor, nocc, nvir;
     float eaijk;
     const float *f;  // f1n f2n f3n f4n f1t f2t f3t f4t
     const float *eorb, *dintc1, *dintx1, *t1v1, *dintc2, *dintx2, *t1v2;
     float *pair;     // [npairs][4]
+    unsigned *counter;
+    float *out;      // emp4i, emp5i, emp4k, emp5k
 };
 
 // the reference's float forms at one (b, c): gpu-omp/ccsd_trpdrv_omp_cbody.c:176-217
-__device__ __forceinline__ void term(const TengyArgs &P, int b, int c, float (&s)[4])
+__device__ __forceinline__ void term(const TengyArgs &P, const float (&bc)[8], const float (&cb)[8], float denom, int b,
+                                     int c, float (&s)[4])
 {
-    const int V = P.nvir;
-    const size_t vv = (size_t)V * V, bc = b + (size_t)c * V, cb = c + (size_t)b * V;
-    const float *f = P.f;
-    const float e_b = P.eorb[P.ncor + P.nocc + b], e_c = P.eorb[P.ncor + P.nocc + c];
-    const float denom = (float)(-1.0 / (double)(e_b + e_c + P.eaijk));
-    const float n1bc = f[bc], n2bc = f[vv + bc], n3bc = f[2 * vv + bc], n4bc = f[3 * vv + bc];
-    const float t1bc = f[4 * vv + bc], t2bc = f[5 * vv + bc], t3bc = f[6 * vv + bc], t4bc = f[7 * vv + bc];
-    const float n1cb = f[cb], n2cb = f[vv + cb], n3cb = f[2 * vv + cb], n4cb = f[3 * vv + cb];
-    const float t1cb = f[4 * vv + cb], t2cb = f[5 * vv + cb], t3cb = f[6 * vv + cb], t4cb = f[7 * vv + cb];
+    const float n1bc = bc[0], n2bc = bc[1], n3bc = bc[2], n4bc = bc[3];
+    const float t1bc = bc[4], t2bc = bc[5], t3bc = bc[6], t4bc = bc[7];
+    const float n1cb = cb[0], n2cb = cb[1], n3cb = cb[2], n4cb = cb[3];
+    const float t1cb = cb[4], t2cb = cb[5], t3cb = cb[6], t4cb = cb[7];
     s[0] += denom * (t1bc + n1cb + t2cb + n3bc + n4cb) * (t1bc - t2bc * 2 - t3bc * 2 + t4bc)
           - denom * (n1bc + t1cb + n2cb + n3cb) * (t1bc * 2 - t2bc - t3bc + t4bc * 2)
           + denom * 3 * (n1bc * (n1bc + n3cb + t4cb * 2) + n2bc * t2cb + n3bc * t4bc);
@@ -134,24 +184,9 @@ __device__ __forceinline__ void term(const TengyArgs &P, int b, int c, float (&s
           + denom * t1v2b * dc2c * (t1bc + t4bc + n1cb - (t2bc + t3bc + n2cb) * 2);
 }
 
-// one CTA per 32 x 32 tile pair (B <= C); the pair's sums over (b, c) in B x C and, for B < C, C x B
-__global__ void __launch_bounds__(NT) tengy_f32_kernel(const TengyArgs P)
+// The CTA's sums of the four values, in thread q < 4's s[0] (a fixed order).
+__device__ __forceinline__ float block_sum(const float (&s)[4], float (&red)[4][NT / 32])
 {
-    __shared__ float red[4][NT / 32];
-    int B = 0, rem = blockIdx.x;
-    while (rem >= P.nb - B) {
-        rem -= P.nb - B;
-        ++B;
-    }
-    const int C = B + rem, V = P.nvir;
-    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int e = threadIdx.x; e < TT * TT; e += NT) {
-        const int b = B * TT + (e & 31), c = C * TT + (e >> 5);
-        if (b < V && c < V) {
-            term(P, b, c, s);
-            if (B != C) term(P, c, b, s);
-        }
-    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -161,35 +196,80 @@ __global__ void __launch_bounds__(NT) tengy_f32_kernel(const TengyArgs P)
         if (lane == 0) red[q][warp] = v;
     }
     __syncthreads();
-    if (threadIdx.x < 4) {
-        float v = 0.0f;
+    float v = 0.0f;
+    if (threadIdx.x < 4)
         for (int w = 0; w < NT / 32; ++w) v += red[threadIdx.x][w];
-        P.pair[4 * blockIdx.x + threadIdx.x] = v;
-    }
+    __syncthreads();
+    return v;
 }
 
-// the tile pairs' sums in a fixed order: out[0..3] = emp4i, emp5i, emp4k, emp5k
-__global__ void pair_sum_kernel(const float *pair, int npairs, float *out)
+// one CTA per 16 x 16 tile pair (B <= C), one thread per (b, c): the terms of (b, c) and, for B < C, of (c, b); the
+// mirrored tile's values cross through shared memory, so every load is coalesced
+__global__ void __launch_bounds__(NT) tengy_f32_kernel(const __grid_constant__ TengyArgs P)
 {
-    if (threadIdx.x < 4) {
-        float v = 0.0f;
-        for (int p = 0; p < npairs; ++p) v += pair[4 * p + threadIdx.x];
-        out[threadIdx.x] = v;
+    __shared__ float xch[8][TT][TT + 1];
+    __shared__ float red[4][NT / 32];
+    __shared__ int last;
+    const int V = P.nvir, nb = (V + TT - 1) / TT, tid = threadIdx.x;
+    int B = 0, rem = blockIdx.x;
+    while (rem >= nb - B) {
+        rem -= nb - B;
+        ++B;
     }
+    const int C = B + rem, r = tid & (TT - 1), q = tid / TT;
+    const int b = B * TT + r, c = C * TT + q, cr = C * TT + r, bq = B * TT + q;
+    const size_t vv = (size_t)V * V;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // f and the counter come from the launch before
+    float fbc[8], fcb[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        fbc[x] = b < V && c < V ? __ldcg(P.f + x * vv + b + (size_t)c * V) : 0.0f;
+        fcb[x] = cr < V && bq < V ? __ldcg(P.f + x * vv + cr + (size_t)bq * V) : 0.0f;
+    }
+#pragma unroll
+    for (int x = 0; x < 8; ++x) xch[x][q][r] = fcb[x];
+    __syncthreads();
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (b < V && c < V) {
+#pragma unroll
+        for (int x = 0; x < 8; ++x) fcb[x] = xch[x][r][q];
+        const float denom = (float)(-1.0 / (double)(P.eorb[P.ncor + P.nocc + b] + P.eorb[P.ncor + P.nocc + c] + P.eaijk));
+        term(P, fbc, fcb, denom, b, c, s);
+        if (B != C) term(P, fcb, fbc, denom, c, b, s);
+    }
+    const float v = block_sum(s, red);
+    if (tid < 4) P.pair[4 * (size_t)blockIdx.x + tid] = v;
+    if (tid < 4) __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(P.counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (unsigned p = tid; p < gridDim.x; p += NT)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) t[u] += __ldcg(P.pair + 4 * (size_t)p + u);
+    const float o = block_sum(t, red);
+    if (tid < 4) P.out[tid] = o;
+    if (tid == 0) *P.counter = 0u;
 }
 
 // ------------------------------------------------------------------------------------------------
 // host state: one device, one stream, buffers grown to the largest shape seen
 // ------------------------------------------------------------------------------------------------
-enum { S_TIJ, S_TKJ, S_JIA, S_JKA, S_KIA, S_KKA, S_NVV };
-enum { O_TIA, O_TKA, O_XIA, O_XKA, O_JIJ, O_JKJ, O_KIJ, O_KKJ, O_NOV };
+// Staging layout as in the double-precision library (host.c): I = tij jia kia tia xia jij kij, K = the same blocks of
+// the k role, then dintc1 dintx1 t1v1 dintc2 dintx2 t1v2 eorb.  Rows are padded to multiples of 4 floats.
+enum { DS_I = 0, DS_K = 7, DS_VEC = 14, DS_N = 21 };
+enum { DS_T = 0, DS_J, DS_KV, DS_TO, DS_XO, DS_JO, DS_KO };
+constexpr size_t SEGMENT = (size_t)512 << 10;
 
 struct State {
-    int ready;
+    int ready, ncor, nocc, nvir;
     cudaStream_t st;
-    size_t cap_vv, cap_ov, cap_v, cap_bf, cap_pairs;
-    float *vv[S_NVV], *ov[O_NOV], *vec[6], *eorb, *f, *pair, *out;
-    float *h_out;  // pinned, 4 floats
+    size_t off[DS_N + 1], cap_stage, cap_f, cap_pair, cap_vec;
+    float *d_stage, *h_stage, *f, *pair, *vec;
+    unsigned *counter;
+    float *h_out;  // pinned, 4 floats: the energy kernel writes it
 };
 State g;
 pthread_mutex_t g_mu = PTHREAD_MUTEX_INITIALIZER;
@@ -223,7 +303,9 @@ int grow(float **p, size_t *cap, size_t want)
     return 0;
 }
 
-int reserve(int nocc, int nvir, int nbf)
+int pitch4(int n) { return (n + 3) & ~3; }
+
+int reserve(int nvir, int nbf)
 {
     if (!g.ready) {
         int dev = 0, major = 0;
@@ -231,47 +313,52 @@ int reserve(int nocc, int nvir, int nbf)
         F32_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
         if (major != 10) return fail(4, "the current device is not sm_100");
         F32_TRY(cudaStreamCreateWithFlags(&g.st, cudaStreamNonBlocking));
-        F32_TRY(cudaMalloc((void **)&g.out, sizeof(float) * 4));
+        F32_TRY(cudaMalloc((void **)&g.counter, sizeof(unsigned)));
+        F32_TRY(cudaMemset(g.counter, 0, sizeof(unsigned)));
         F32_TRY(cudaMallocHost((void **)&g.h_out, sizeof(float) * 4));
         g.ready = 1;
     }
-    const size_t vv = (size_t)nvir * nvir, ov = (size_t)nocc * nvir, v = (size_t)nvir;
-    const int nb = (nvir + TT - 1) / TT;
-    const size_t pairs = (size_t)nb * (nb + 1) / 2;
-    if (vv > g.cap_vv) {
-        size_t c = 0;
-        for (int q = 0; q < S_NVV; ++q) {
-            c = 0;
-            if (g.vv[q]) cudaFree(g.vv[q]);
-            g.vv[q] = nullptr;
-            if (grow(&g.vv[q], &c, vv)) return t_status;
-        }
-        c = 0;
-        if (g.f) cudaFree(g.f);
-        g.f = nullptr;
-        if (grow(&g.f, &c, 8 * vv)) return t_status;
-        g.cap_vv = vv;
+    const size_t vv = (size_t)nvir * nvir, nb = (size_t)(nvir + TT - 1) / TT;
+    if (int rc = grow(&g.f, &g.cap_f, 8 * vv)) return rc;
+    if (int rc = grow(&g.pair, &g.cap_pair, 4 * (nb * (nb + 1) / 2))) return rc;
+    return grow(&g.vec, &g.cap_vec, 6 * (size_t)nvir + (size_t)nbf);
+}
+
+// Lays the staging block out for this shape and clears it (the pads must be zero, and mirror and device equal).
+int layout(int ncor, int nocc, int nvir)
+{
+    if (g.cap_stage && g.ncor == ncor && g.nocc == nocc && g.nvir == nvir) return 0;
+    g.nvir = 0;  // no valid layout until the end
+    const size_t V = (size_t)nvir, O = (size_t)nocc, ldv = (size_t)pitch4(nvir), ldo = (size_t)pitch4(nocc);
+    const size_t role[7] = {ldv * V, ldv * V, ldv * V, ldv * O, ldv * O, ldo * V, ldo * V};
+    size_t o = 0;
+    for (int q = 0; q < DS_N; ++q) {
+        g.off[q] = o;
+        const size_t n = q < DS_VEC ? role[q % 7] : q < DS_N - 1 ? V : (size_t)(ncor + nocc + nvir);
+        o += (n + 31) & ~(size_t)31;
     }
-    if (ov > g.cap_ov) {
-        for (int q = 0; q < O_NOV; ++q) {
-            size_t c = 0;
-            if (g.ov[q]) cudaFree(g.ov[q]);
-            g.ov[q] = nullptr;
-            if (grow(&g.ov[q], &c, ov)) return t_status;
-        }
-        g.cap_ov = ov;
+    F32_TRY(cudaStreamSynchronize(g.st));  // no transfer of a failed call still reads the mirror
+    if (o > g.cap_stage) {
+        if (g.d_stage) cudaFree(g.d_stage);
+        if (g.h_stage) cudaFreeHost(g.h_stage);
+        g.d_stage = g.h_stage = nullptr;
+        g.cap_stage = 0;
+        F32_TRY(cudaMalloc((void **)&g.d_stage, sizeof(float) * o));
+        F32_TRY(cudaMallocHost((void **)&g.h_stage, sizeof(float) * o));
+        g.cap_stage = o;
     }
-    if (v > g.cap_v) {
-        for (int q = 0; q < 6; ++q) {
-            size_t c = 0;
-            if (g.vec[q]) cudaFree(g.vec[q]);
-            g.vec[q] = nullptr;
-            if (grow(&g.vec[q], &c, v)) return t_status;
-        }
-        g.cap_v = v;
-    }
-    if (grow(&g.eorb, &g.cap_bf, (size_t)nbf)) return t_status;
-    if (grow(&g.pair, &g.cap_pairs, 4 * pairs)) return t_status;
+    memset(g.h_stage, 0, sizeof(float) * o);
+    F32_TRY(cudaMemsetAsync(g.d_stage, 0, sizeof(float) * o, g.st));
+    g.ncor = ncor;
+    g.nocc = nocc;
+    g.nvir = nvir;
+    return 0;
+}
+
+int send(void *, char *lo, char *hi)
+{
+    const size_t a = (size_t)(lo - (char *)g.h_stage), n = (size_t)(hi - lo);
+    F32_TRY(cudaMemcpyAsync((char *)g.d_stage + a, (char *)g.h_stage + a, n, cudaMemcpyHostToDevice, g.st));
     return 0;
 }
 
@@ -281,16 +368,15 @@ int h2d(float *dst, const float *src, size_t n)
     return 0;
 }
 
-int launch_tengy(int ncor, int nocc, int nvir, float eaijk, const float *f, const float *const *vec,
-                 const float *eorb, float *out4)
+// The energies of the f at g.f; a programmatic dependent of the launch before it on the stream.
+int launch_tengy(int ncor, int nocc, int nvir, float eaijk, const float *const *vec, const float *eorb, float *out4)
 {
     TengyArgs T;
     T.ncor = ncor;
     T.nocc = nocc;
     T.nvir = nvir;
-    T.nb = (nvir + TT - 1) / TT;
     T.eaijk = eaijk;
-    T.f = f;
+    T.f = g.f;
     T.eorb = eorb;
     T.dintc1 = vec[0];
     T.dintx1 = vec[1];
@@ -299,11 +385,19 @@ int launch_tengy(int ncor, int nocc, int nvir, float eaijk, const float *f, cons
     T.dintx2 = vec[4];
     T.t1v2 = vec[5];
     T.pair = g.pair;
-    const int npairs = T.nb * (T.nb + 1) / 2;
-    tengy_f32_kernel<<<npairs, NT, 0, g.st>>>(T);
-    pair_sum_kernel<<<1, 32, 0, g.st>>>(g.pair, npairs, g.out);
-    F32_TRY(cudaGetLastError());
-    F32_TRY(cudaMemcpyAsync(g.h_out, g.out, sizeof(float) * 4, cudaMemcpyDeviceToHost, g.st));
+    T.counter = g.counter;
+    T.out = g.h_out;
+    const unsigned nb = (unsigned)(nvir + TT - 1) / TT;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nb * (nb + 1) / 2);
+    cfg.blockDim = dim3(NT);
+    cfg.stream = g.st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    F32_TRY(cudaLaunchKernelEx(&cfg, tengy_f32_kernel, T));
     F32_TRY(cudaStreamSynchronize(g.st));
     for (int q = 0; q < 4; ++q) out4[q] = g.h_out[q];
     return 0;
@@ -332,48 +426,64 @@ int body(float *f1n, float *f1t, float *f2n, float *f2t, float *f3n, float *f3t,
     const int write_f = wf && strcmp(wf, "1") == 0;
     if (write_f && (!f1n || !f1t || !f2n || !f2t || !f3n || !f3t || !f4n || !f4t))
         return fail(1, "TRPDRV_WRITE_F=1 with a NULL f array");
-    if (int rc = reserve(nocc, nvir, nbf)) return rc;
-    const size_t vv = (size_t)nvir * nvir, ov = (size_t)nocc * nvir;
+    if (int rc = reserve(nvir, nbf)) return rc;
+    if (int rc = layout(ncor, nocc, nvir)) return rc;
+    const size_t V = (size_t)nvir, O = (size_t)nocc, vv = V * V, ov = O * V;
     const size_t kv = (size_t)(k - klo) * vv, ko = (size_t)(k - klo) * ov;
     // the reference's offsets of the k-chunk slices (gpu-omp/ccsd_trpdrv_omp_cbody.c:64-70)
-    const float *svv[S_NVV] = {tij, tkj + kv, jia, jka + kv, kia, kka + kv};
-    const float *sov[O_NOV] = {tia, tka + ko, xia, xka + ko, jij, jkj + ko, kij, kkj + ko};
-    const float *svec[6] = {dintc1, dintx1, t1v1, dintc2, dintx2, t1v2};
-    for (int q = 0; q < S_NVV; ++q)
-        if (int rc = h2d(g.vv[q], svv[q], vv)) return rc;
-    for (int q = 0; q < O_NOV; ++q)
-        if (int rc = h2d(g.ov[q], sov[q], ov)) return rc;
-    for (int q = 0; q < 6; ++q)
-        if (int rc = h2d(g.vec[q], svec[q], (size_t)nvir)) return rc;
-    if (int rc = h2d(g.eorb, eorb, (size_t)nbf)) return rc;
+    const float *in[DS_N] = {tij, jia, kia, tia, xia, jij, kij, tkj + kv, jka + kv, kka + kv, tka + ko, xka + ko,
+                             jkj + ko, kkj + ko, dintc1, dintx1, t1v1, dintc2, dintx2, t1v2, eorb};
+    const float *dev[DS_N];
+    stage_piece pc[DS_N];
+    for (int q = 0; q < DS_N; ++q) {
+        const int b = q % 7, is_vec = q >= DS_VEC;
+        const size_t width = is_vec ? (q < DS_N - 1 ? V : (size_t)nbf) : b < DS_JO ? V : O;
+        const size_t rows = is_vec ? 1 : b < DS_TO || b >= DS_JO ? V : O;
+        const size_t pitch = is_vec ? width : (size_t)pitch4((int)width);
+        const bool flat = pitch == width;
+        dev[q] = g.d_stage + g.off[q];
+        pc[q].dst = (char *)(g.h_stage + g.off[q]);
+        pc[q].src = (const char *)in[q];
+        pc[q].rows = flat ? 1 : rows;
+        pc[q].width = sizeof(float) * (flat ? rows * width : width);
+        pc[q].pitch = sizeof(float) * (flat ? rows * width : pitch);
+    }
+    const int threads = stage_threads();
+    int rc = stage_send(pc + DS_K, DS_N - DS_K, threads, SEGMENT, send, nullptr);
+    if (!rc) rc = stage_send(pc, DS_K, threads, SEGMENT, send, nullptr);
+    if (rc) {
+        g.nvir = 0;  // mirror and device may differ now
+        return rc;
+    }
 
     // f1n f2n f3n f4n f1t f2t f3t f4t: gpu-omp/ccsd_trpdrv_omp_cbody.c:72-167
     GemmArgs G;
     G.nocc = nocc;
     G.nvir = nvir;
+    G.ldv = pitch4(nvir);
+    G.ldo = pitch4(nocc);
     G.f = g.f;
-    float *const *V = g.vv, *const *Ob = g.ov;
-    const float *a1[8] = {V[S_JIA], V[S_KIA], V[S_JIA], V[S_KIA], V[S_JKA], V[S_KKA], V[S_JKA], V[S_KKA]};
-    const float *b1[8] = {V[S_TKJ], V[S_TKJ], V[S_TKJ], V[S_TKJ], V[S_TIJ], V[S_TIJ], V[S_TIJ], V[S_TIJ]};
-    const int bt[8] = {1, 1, 0, 0, 1, 1, 0, 0};
-    const float *a2[8] = {Ob[O_TIA], Ob[O_XIA], Ob[O_TIA], Ob[O_XIA], Ob[O_TKA], Ob[O_XKA], Ob[O_TKA], Ob[O_XKA]};
-    const float *b2[8] = {Ob[O_KKJ], Ob[O_KKJ], Ob[O_JKJ], Ob[O_JKJ], Ob[O_KIJ], Ob[O_KIJ], Ob[O_JIJ], Ob[O_JIJ]};
+    G.counter = g.counter;
     for (int x = 0; x < 8; ++x) {
-        G.a1[x] = a1[x];
-        G.b1[x] = b1[x];
-        G.b1_t[x] = bt[x];
-        G.a2[x] = a2[x];
-        G.b2[x] = b2[x];
+        const int A = x < 4 ? DS_I : DS_K, B = x < 4 ? DS_K : DS_I, two = (x >> 1) & 1;
+        G.a1[x] = dev[A + (x & 1 ? DS_KV : DS_J)];
+        G.b1[x] = dev[B + DS_T];
+        G.b1_t[x] = !two;
+        G.a2[x] = dev[A + (x & 1 ? DS_XO : DS_TO)];
+        G.b2[x] = dev[B + (two ? DS_JO : DS_KO)];
     }
-    const dim3 grid((nvir + BT - 1) / BT, (nvir + BT - 1) / BT, 8);
-    sgemm_group_kernel<<<grid, NT, 0, g.st>>>(G);
+    // 64-wide tiles once they fill the chip
+    const unsigned n64 = (unsigned)(nvir + 63) / 64, n32 = (unsigned)(nvir + 31) / 32;
+    if (n64 * n64 * 8 >= 148)
+        sgemm_group_kernel<64><<<dim3(n64, n64, 8), Tile<64>::THREADS, 0, g.st>>>(G);
+    else
+        sgemm_group_kernel<32><<<dim3(n32, n32, 8), Tile<32>::THREADS, 0, g.st>>>(G);
     F32_TRY(cudaGetLastError());
 
     // gpu-omp/ccsd_trpdrv_omp_cbody.c:62
     const float eaijk = eorb[a - 1] - (eorb[ncor + i - 1] + eorb[ncor + j - 1] + eorb[ncor + k - 1]);
-    const float *dvec[6] = {g.vec[0], g.vec[1], g.vec[2], g.vec[3], g.vec[4], g.vec[5]};
     float r[4];
-    if (int rc = launch_tengy(ncor, nocc, nvir, eaijk, g.f, dvec, g.eorb, r)) return rc;
+    if (int rc2 = launch_tengy(ncor, nocc, nvir, eaijk, dev + DS_VEC, dev[DS_N - 1], r)) return rc2;
     if (write_f) {
         float *outs[8] = {f1n, f2n, f3n, f4n, f1t, f2t, f3t, f4t};
         for (int x = 0; x < 8; ++x)
@@ -401,18 +511,21 @@ int tengy(const float *const *f8, const float *const *vec, const float *eorb, fl
         if (!vec[q]) return fail(1, "NULL vector");
     if (!eorb || nocc < 1 || nvir < 1 || ncor < 0 || nvir > 16384) return fail(1, "bad tengy arguments");
     const int nbf = ncor + nocc + nvir;
-    if (int rc = reserve(nocc, nvir, nbf)) return rc;
+    if (int rc = reserve(nvir, nbf)) return rc;
     const size_t vv = (size_t)nvir * nvir;
     // device order f1n f2n f3n f4n f1t f2t f3t f4t from the argument order f1n f1t f2n f2t ...
     for (int x = 0; x < 4; ++x) {
         if (int rc = h2d(g.f + (size_t)x * vv, f8[2 * x], vv)) return rc;
         if (int rc = h2d(g.f + (size_t)(4 + x) * vv, f8[2 * x + 1], vv)) return rc;
     }
-    for (int q = 0; q < 6; ++q)
-        if (int rc = h2d(g.vec[q], vec[q], (size_t)nvir)) return rc;
-    if (int rc = h2d(g.eorb, eorb, (size_t)nbf)) return rc;
-    const float *dvec[6] = {g.vec[0], g.vec[1], g.vec[2], g.vec[3], g.vec[4], g.vec[5]};
-    return launch_tengy(ncor, nocc, nvir, eaijk, g.f, dvec, g.eorb, out4);
+    const float *dvec[6];
+    for (int q = 0; q < 6; ++q) {
+        dvec[q] = g.vec + (size_t)q * nvir;
+        if (int rc = h2d(g.vec + (size_t)q * nvir, vec[q], (size_t)nvir)) return rc;
+    }
+    float *deorb = g.vec + 6 * (size_t)nvir;
+    if (int rc = h2d(deorb, eorb, (size_t)nbf)) return rc;
+    return launch_tengy(ncor, nocc, nvir, eaijk, dvec, deorb, out4);
 }
 
 void report(int rc, const char *who)

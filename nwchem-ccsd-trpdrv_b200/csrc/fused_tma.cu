@@ -76,13 +76,11 @@ struct ItemCtx {
     double eaijk;
     int ncor, nocc, nvir, b0, c0, diag, same, nch, state;  // same: i == k; state: 1 work, 0 malformed, -1 end
     int packed, b1;      // packed edge item: pairs (b0, c0) and (b1, c0); b1 < 0 when the second is absent
-    // split item (the one-triple system of a split launch): 1 | half << 1 | pair << 2, else 0; this half
-    // runs chunks half, half + 2, ...  One int keeps the context at 128 bytes: at 160 bytes (the split
-    // fields as separate members) the batched kernel measured 6 % slower.
-    int split_tag;
+    int pad;
 };
 
-static_assert(sizeof(ItemCtx) == 128, "the item context is kept at 128 bytes (see split_tag)");
+// at 160 bytes the batched kernel measured 6 % slower
+static_assert(sizeof(ItemCtx) == 128, "the item context is kept at 128 bytes");
 
 // Packed edge items (systems with pack_edge: the last column tile E holds 1..16 valid indices).  The
 // pairs (B, E) and (B + 1, E), B even, run as one item: each family of a chunk gets its own stage
@@ -520,25 +518,17 @@ __device__ __forceinline__ bool run_packed(int n, const FragOffsets &fo, const P
     return true;
 }
 
-// Chunk indices lo <= ch < hi with the item's parity (split items take every second chunk).
-__device__ __forceinline__ int count_chunks(int lo, int hi, int first, int step)
-{
-    if (step == 1) return hi - lo;
-    const int c0 = lo + ((lo ^ first) & 1);
-    return c0 < hi ? (hi - c0 + 1) >> 1 : 0;
-}
-
 // The item's chunks by kind: full and one-k-step chunks of the virtual phase, then of the occupied one (the last
 // chunk of a phase runs one k-step when the second lies entirely in the zero padding).
 struct ChunkCounts {
     int v2, v1, o2, o1;
-    __device__ __forceinline__ ChunkCounts(int nvir, int nocc, int first, int step)
+    __device__ __forceinline__ ChunkCounts(int nvir, int nocc)
     {
         const int nV = (nvir + DK - 1) / DK, nO = (nocc + DK - 1) / DK;
-        v1 = nvir - (nV - 1) * DK <= 8 ? count_chunks(nV - 1, nV, first, step) : 0;
-        o1 = nocc - (nO - 1) * DK <= 8 ? count_chunks(nV + nO - 1, nV + nO, first, step) : 0;
-        v2 = count_chunks(0, nV, first, step) - v1;
-        o2 = count_chunks(nV, nV + nO, first, step) - o1;
+        v1 = nvir - (nV - 1) * DK <= 8;
+        o1 = nocc - (nO - 1) * DK <= 8;
+        v2 = nV - v1;
+        o2 = nO - o1;
     }
 };
 
@@ -646,16 +636,11 @@ struct Item {
     long long own;  // index of the item's energy slots
     int s, B, C, i, j, k, ai;
     int za0, za1, zb0, zb1;  // blocks of the A and B operands per family (n, t): A: i / k slot, B: [j][k] / [j][i]
-    int zO;            // occupied slots per a block of J and K
-    int first, step;   // chunks first, first + step, ... (split items take every second chunk)
     bool in_range, ok, pack, skip, same, diag;
     __device__ __forceinline__ int za(int fam) const { return fam ? za1 : za0; }
     __device__ __forceinline__ int zb(int fam) const { return fam ? zb1 : zb0; }
 };
 
-// SPLIT: the instantiation that also runs split systems (two work items per pair); without it the
-// producer and consumer loops carry no split logic at all.
-template <bool SPLIT>
 __device__ __forceinline__ Item decode_item(const trpdrv_dev_system *__restrict__ sys, int nsys, long long item)
 {
     Item it;
@@ -664,11 +649,7 @@ __device__ __forceinline__ Item decode_item(const trpdrv_dev_system *__restrict_
     const trpdrv_dev_system &S = sys[s];
     it.S = &S;
     it.s = s;
-    // a split system has two work items (halves of the contraction) per pair
-    const bool split = SPLIT && S.split;
-    it.first = split ? (int)((item - S.item_begin) & 1) : 0;
-    it.step = split ? 2 : 1;
-    const long long local = split ? (item - S.item_begin) >> 1 : item - S.item_begin;
+    const long long local = item - S.item_begin;
     const long long qpos = local / S.npairs;  // processing position over the system's records
     const int p = (int)(local - qpos * S.npairs);
     // a index (records are [a][triple], fewer than 2^31: the host checks); no division for a single a
@@ -694,28 +675,21 @@ __device__ __forceinline__ Item decode_item(const trpdrv_dev_system *__restrict_
     it.i = packed & 1023;
     it.j = (packed >> 10) & 1023;
     it.k = (packed >> 20) & 1023;
-    // occupied slots of the i, j and k roles in the tensors (a one-triple system holds two slots)
-    const int one = S.one_triple;
-    const int zi = one ? 0 : it.i, zj = one ? 0 : it.j, zk = one ? 1 : it.k;
-    it.zO = one ? 2 : O;
-    it.za0 = zi;
-    it.za1 = zk;
-    it.zb0 = zj * it.zO + zk;
-    it.zb1 = zj * it.zO + zi;
-    it.ok = it.in_range && B < S.nb && C < S.nb && it.i < O && it.j < O && it.k < O && (one || it.k <= it.i) &&
-            (!one || ai == 0);
-    // i == k: both families read the same blocks (a staged one-triple system holds them twice and may not)
-    it.same = it.i == it.k && !one;
+    it.za0 = it.i;
+    it.za1 = it.k;
+    it.zb0 = it.j * O + it.k;
+    it.zb1 = it.j * O + it.i;
+    it.ok = it.in_range && B < S.nb && C < S.nb && it.i < O && it.j < O && it.k <= it.i;
+    it.same = it.i == it.k;  // both families read the same blocks
     return it;
 }
 
-template <bool SPLIT>
 __device__ __forceinline__ void write_ctx(ItemCtx &cx, const Item &it)
 {
     const trpdrv_dev_system &S = *it.S;
     const int O = S.nocc, V = S.nvir, nV = (V + DK - 1) / DK, nO = (O + DK - 1) / DK;
     cx.eorb = S.eorb;
-    const size_t vi = ((size_t)it.ai * it.zO + it.za0) * V, vk = ((size_t)it.ai * it.zO + it.za1) * V;
+    const size_t vi = ((size_t)it.ai * O + it.za0) * V, vk = ((size_t)it.ai * O + it.za1) * V;
     cx.dintc1 = S.dintc + vi;
     cx.dintx1 = S.dintx + vi;
     cx.t1v1 = S.t1v + vi;
@@ -738,8 +712,7 @@ __device__ __forceinline__ void write_ctx(ItemCtx &cx, const Item &it)
     cx.c0 = it.C * T;
     cx.diag = it.diag;
     cx.same = it.same;
-    cx.split_tag = (SPLIT && S.split) ? 1 | it.first << 1 | (int)it.own << 2 : 0;
-    cx.nch = it.step == 2 ? (nV + nO - it.first + 1) / 2 : nV + nO;
+    cx.nch = nV + nO;
     cx.state = 1;
 }
 
@@ -802,7 +775,7 @@ struct TmaStage {
         const CUtensorMap *mp = maps->m[it.s];
         mv = &mp[kind == OP_AJ ? M_J : kind == OP_AK ? M_K : kind == OP_B1 ? M_T2K : M_T2X];
         mo = &mp[kind == OP_AJ ? M_NT : kind == OP_AK ? M_NX : kind == OP_B1 ? M_KOV : M_JOV];
-        zav = it.ai * it.zO;  // J and K carry the a index, -T and -X do not
+        zav = it.ai * it.S->nocc;  // J and K carry the a index, -T and -X do not
     }
 
     __device__ __forceinline__ void slot(const Item &it, const Role &, int, char *st, unsigned long long *full,
@@ -893,7 +866,7 @@ struct CpStage {
                 const double *m;
                 if (virt)
                     m = (kind == OP_AJ ? S.jvv : kind == OP_AK ? S.kvv : S.t2) +
-                        (size_t)(kind < OP_B1 ? it.ai * it.zO + it.za(fam) : it.zb(fam)) * ldv * V;
+                        (size_t)(kind < OP_B1 ? it.ai * O + it.za(fam) : it.zb(fam)) * ldv * V;
                 else if (kind < OP_B1)
                     m = (kind == OP_AJ ? S.ntov : S.nxov) + (size_t)it.za(fam) * ldv * O;
                 else
@@ -915,7 +888,7 @@ struct CpStage {
     }
 };
 
-template <bool SPLIT, class Stage>
+template <class Stage>
 __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ sys, int nsys, long long total,
                                          unsigned long long *counter, int *status, Stage &sg, char *stages,
                                          unsigned long long *full, unsigned long long *empty, ItemCtx *ring,
@@ -941,7 +914,7 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
                 if (item >= total) break;
                 if (lane == 0) next = (long long)atomicAdd(counter, 1ULL);  // the following ticket, early
                 next = __shfl_sync(FULL, next, 0);
-                it = decode_item<SPLIT>(sys, nsys, item);
+                it = decode_item(sys, nsys, item);
                 if (!it.skip) break;
             }
             if (lane == 0) {
@@ -951,7 +924,7 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
         } else {
             if (!mbar_wait(&tbar[tq], (unsigned)((n / TICKETS) & 1), status)) return;
             item = tickets[tq];
-            if (item < total) it = decode_item<SPLIT>(sys, nsys, item);
+            if (item < total) it = decode_item(sys, nsys, item);
         }
         ItemCtx &cx = ring[n % RING];
         if (item >= total || !it.ok) {
@@ -975,13 +948,13 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
             }
             continue;
         }
-        if (pw == 0 && lane == 0) write_ctx<SPLIT>(cx, it);
+        if (pw == 0 && lane == 0) write_ctx(cx, it);
         const Role role(it, pw);
         sg.begin(it, role, pw, lane);
         const int nV = (it.S->nvir + DK - 1) / DK, nch = nV + (it.S->nocc + DK - 1) / DK;
         // packed items: one slot per (chunk, family)
         const int f0 = it.pack ? 0 : role.fam, f1 = it.pack ? (it.same ? 1 : 2) : role.fam + 1;
-        for (int ch = it.first; ch < nch; ch += it.step) {
+        for (int ch = 0; ch < nch; ++ch) {
             const bool virt = ch < nV;
             const int kk0 = (virt ? ch : ch - nV) * DK;
             for (int f = f0; f < f1; ++f) {
@@ -1005,55 +978,6 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
 }
 
 // ------------------------------------------------------------------------------------------------
-// Split items: both halves write their partial f and f-transposed to scratch (thread-major, so the
-// 256 consumer threads write consecutive addresses), make them visible (fence), and one thread counts
-// the arrival.  The second half to arrive adds the first's partials and finishes the item (fin = 1);
-// the first stops there.  Two rounds of the consumer barrier order the writes before the count and
-// broadcast its result; the counter is reset by the second arrival.  Nothing waits for the other CTA.
-// Returns false when a barrier wait ran out (status set).
-__device__ __forceinline__ bool split_combine(const trpdrv_dev_system *__restrict__ sys, const ItemCtx &cx,
-                                              double (&f)[8][4], double (&gT)[8][4], int warp, int lane,
-                                              unsigned long long *xbar, unsigned &xphase, int *flag, int *status,
-                                              int &fin)
-{
-    const int tc = warp * 32 + lane, half = (cx.split_tag >> 1) & 1;
-    const size_t pair = (size_t)(cx.split_tag >> 2);
-    double *const scr = sys[0].split_scratch + pair * 2 * 64 * 256;  // [2 halves][64][256] of this pair
-    unsigned *const cnt = sys[0].split_count + pair;                 // arrivals of the two halves
-    double *mine = scr + (size_t)(half ? 64 * 256 : 0) + tc;
-#pragma unroll
-    for (int x = 0; x < 8; ++x)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            mine[(x * 4 + e) * 256] = f[x][e];
-            mine[(32 + x * 4 + e) * 256] = gT[x][e];
-        }
-    __threadfence();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(xbar);
-    if (!mbar_wait(xbar, xphase, status)) return false;
-    xphase ^= 1;
-    if (tc == 0) *flag = (int)atomicAdd(cnt, 1u);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(xbar);
-    if (!mbar_wait(xbar, xphase, status)) return false;
-    xphase ^= 1;
-    fin = *flag != 0;
-    if (fin) {
-        __threadfence();
-        const double *other = scr + (size_t)(half ? 0 : 64 * 256) + tc;
-#pragma unroll
-        for (int x = 0; x < 8; ++x)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                f[x][e] += __ldcg(other + (x * 4 + e) * 256);
-                gT[x][e] += __ldcg(other + (32 + x * 4 + e) * 256);
-            }
-        if (tc == 0) *cnt = 0u;
-    }
-    return true;
-}
-
 // Releases the n stage slots of an item whose sub-block of this warp lies entirely in the padding.
 __device__ __forceinline__ bool skip_slots(int n, const Pipe &pp, RingPos &rp)
 {
@@ -1092,7 +1016,7 @@ template <> struct StageParam<1> : NoParam {};
 template <> struct StageParam<2> : NoParam {};
 
 // STG: operand staging, 0 = TMA, 1 / 2 = cp.async with 8 / 16-byte copies.  KS: FP64 MMA shape.
-template <int KS, bool SPLIT, int STG>
+template <int KS, int STG>
 __global__ void __launch_bounds__(NTHREAD, 1)
 fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long total, unsigned long long *counter,
              int *status, const __grid_constant__ StageParam<STG> param)
@@ -1101,8 +1025,7 @@ fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long tota
     __shared__ __align__(8) unsigned long long full[STAGES], empty[STAGES], tbar[TICKETS];
     __shared__ ItemCtx ring[RING];
     __shared__ long long tickets[TICKETS];
-    __shared__ __align__(8) unsigned long long xbar[1];     // diagonal-pair exchange, split items
-    __shared__ int split_flag[1];
+    __shared__ __align__(8) unsigned long long xbar[1];     // diagonal-pair exchange
     // aligned by an offset, not by integer arithmetic on the pointer: the compiler then still knows that the
     // fragment reads are shared-memory loads (32-bit addresses)
     char *stages = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
@@ -1124,11 +1047,11 @@ fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long tota
         if constexpr (STG == 0) {
             TmaStage sg;
             sg.maps = &param.maps;
-            producer<SPLIT>(sys, nsys, total, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
+            producer(sys, nsys, total, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
                             lane);
         } else {
             CpStage<STG> sg;
-            producer<SPLIT>(sys, nsys, total, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
+            producer(sys, nsys, total, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
                             lane);
             asm volatile("cp.async.wait_all;" ::: "memory");
         }
@@ -1164,8 +1087,7 @@ fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long tota
         for (int x = 0; x < 8; ++x)
 #pragma unroll
             for (int e = 0; e < 4; ++e) f[x][e] = gT[x][e] = 0.0;
-        const int first = SPLIT ? (cx.split_tag >> 1) & 1 : 0, step = SPLIT ? (cx.split_tag & 1) + 1 : 1;
-        const ChunkCounts nc(cx.nvir, cx.nocc, first, step);
+        const ChunkCounts nc(cx.nvir, cx.nocc);
         const bool same = cx.same != 0;
         prefetch_epilogue(cx, lane);
         if (cx.packed) {
@@ -1181,11 +1103,6 @@ fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long tota
                     return;
             } else if (!skip_slots(same ? cx.nch : 2 * cx.nch, pipe, rp)) {
                 return;
-            }
-            if (SPLIT && (cx.split_tag & 1)) {
-                int fin = 0;
-                if (!split_combine(sys, cx, f, gT, warp, lane, xbar, xphase, split_flag, status, fin)) return;
-                if (!fin) continue;
             }
             if (same) copy_families(f, gT);
             if (pb0 >= 0) {  // this pair's slots: the 4 sub-blocks' sums, zeros in the other 4
@@ -1210,14 +1127,6 @@ fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long tota
             if (!ok) return;
         } else if (!skip_slots(cx.nch, pipe, rp)) {  // only padding
             return;
-        }
-        if (SPLIT && (cx.split_tag & 1)) {  // the second half to arrive adds the first's partial sums and finishes
-            int fin = 0;
-            if (!split_combine(sys, cx, f, gT, warp, lane, xbar, xphase, split_flag, status, fin)) return;
-            if (!fin) {
-                if (diag && !skip_slots(1, pipe, rp)) return;  // the exchange slot
-                continue;
-            }
         }
         if (diag) {
             // f(c,b) of a diagonal pair is f at the mirrored position of the same 32x32 block, held by another
@@ -1276,14 +1185,13 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 }
 
 // 3-D map over doubles: dims {d0 (contiguous), d1, d2}, box {b0, b1, 1}
-// zstride: distance in doubles between consecutive blocks of the third dimension (0 = d0 * d1, packed)
 static int make_map(CUtensorMap *m, const double *base, unsigned long long d0, unsigned long long d1,
-                    unsigned long long d2, unsigned b0, unsigned b1, bool swizzle, unsigned long long zstride = 0)
+                    unsigned long long d2, unsigned b0, unsigned b1, bool swizzle)
 {
     PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
     if (!fn) return 1;
     const cuuint64_t dims[3] = {d0, d1, d2};
-    const cuuint64_t strides[2] = {d0 * 8ull, (zstride ? zstride : d0 * d1) * 8ull};
+    const cuuint64_t strides[2] = {d0 * 8ull, d0 * d1 * 8ull};
     const cuuint32_t box[3] = {b0, b1, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(base), dims, strides, box, estr,
@@ -1335,50 +1243,43 @@ extern "C" int trpdrv_tma_prepare(const trpdrv_dev_system *h_sys, int nsys, void
     for (int s = 0; s < nsys && s < TRPDRV_TMA_MAX_SYSTEMS; ++s) {
         const trpdrv_dev_system &S = h_sys[s];
         const unsigned long long V = S.nvir, O = S.nocc;
-        // occupied slots along the block dimension: nocc (x nocc for the j-blocked tensors), or the
-        // two slots (one j block) of a one-triple system
-        const unsigned long long X = S.one_triple ? 2 : O, O2 = S.one_triple ? 2 : O * O;
         CUtensorMap *m = M->m[s];
         int e = 0;
-        const unsigned long long OA = X * (unsigned long long)(S.n_a > 0 ? S.n_a : 1);
-        // a one-triple system may place its two slots of every tensor slot_stride doubles apart
-        const unsigned long long zs = S.one_triple ? (unsigned long long)S.slot_stride : 0ull;
-        e |= tma::make_map(&m[tma::M_J], S.jvv, V, V, OA, 16, tma::DK, true, zs);    // [a][i][d][b]
-        e |= tma::make_map(&m[tma::M_K], S.kvv, V, V, OA, 16, tma::DK, true, zs);
-        e |= tma::make_map(&m[tma::M_NT], S.ntov, V, O, X, 16, tma::DK, true, zs);  // [i][m][b]
-        e |= tma::make_map(&m[tma::M_NX], S.nxov, V, O, X, 16, tma::DK, true, zs);
-        e |= tma::make_map(&m[tma::M_T2K], S.t2, V, V, O2, 16, tma::DK, true, zs);  // [jx][d][c]: T(c,d)
-        e |= tma::make_map(&m[tma::M_T2X], S.t2, V, V, O2, tma::DK, 32, true, zs); // [jx][c][d]: T(d,c)
-        e |= tma::make_map(&m[tma::M_JOV], S.jov, O, V, O2, tma::DK, 32, true, zs);  // [jx][c][m]
-        e |= tma::make_map(&m[tma::M_KOV], S.kov, O, V, O2, tma::DK, 32, true, zs);
+        const unsigned long long OA = O * (unsigned long long)(S.n_a > 0 ? S.n_a : 1), O2 = O * O;
+        e |= tma::make_map(&m[tma::M_J], S.jvv, V, V, OA, 16, tma::DK, true);    // [a][i][d][b]
+        e |= tma::make_map(&m[tma::M_K], S.kvv, V, V, OA, 16, tma::DK, true);
+        e |= tma::make_map(&m[tma::M_NT], S.ntov, V, O, O, 16, tma::DK, true);   // [i][m][b]
+        e |= tma::make_map(&m[tma::M_NX], S.nxov, V, O, O, 16, tma::DK, true);
+        e |= tma::make_map(&m[tma::M_T2K], S.t2, V, V, O2, 16, tma::DK, true);   // [jx][d][c]: T(c,d)
+        e |= tma::make_map(&m[tma::M_T2X], S.t2, V, V, O2, tma::DK, 32, true);  // [jx][c][d]: T(d,c)
+        e |= tma::make_map(&m[tma::M_JOV], S.jov, O, V, O2, tma::DK, 32, true);  // [jx][c][m]
+        e |= tma::make_map(&m[tma::M_KOV], S.kov, O, V, O2, tma::DK, 32, true);
         if (e) return e;
     }
     return 0;
 }
 
-template <int KS, bool SPLIT, int STG>
+template <int KS, int STG>
 static int launch_kernel(const trpdrv_dev_system *d_sys, int nsys, int64_t total, unsigned long long *counter,
                          int *status, int grid, const tma::StageParam<STG> &param, void *stream)
 {
-    tma::fused_kernel<KS, SPLIT, STG><<<grid, tma::NTHREAD, tma::SMEM_BYTES, (cudaStream_t)stream>>>(
+    tma::fused_kernel<KS, STG><<<grid, tma::NTHREAD, tma::SMEM_BYTES, (cudaStream_t)stream>>>(
         d_sys, nsys, total, counter, status, param);
     return (int)cudaGetLastError();
 }
 
 extern "C" int trpdrv_launch_fused_tma(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items,
                                        unsigned long long *counter, int *status, int grid, const void *maps,
-                                       int mma_k, int split, void *stream)
+                                       int mma_k, void *stream)
 {
     if (grid <= 0 || total_items <= 0) return 0;
     if (g_launch_regs != tma::REG_LAUNCH) return (int)cudaErrorInvalidConfiguration;
     if (nsys > TRPDRV_TMA_MAX_SYSTEMS) return (int)cudaErrorInvalidValue;
     const tma::StageParam<0> &m = *static_cast<const tma::StageParam<0> *>(maps);
-    if (split && mma_k == 8)
-        return launch_kernel<8, true, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
-    if (!split && mma_k == 16)
-        return launch_kernel<16, false, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
-    if (!split && mma_k == 8)
-        return launch_kernel<8, false, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
+    if (mma_k == 16)
+        return launch_kernel<16, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
+    if (mma_k == 8)
+        return launch_kernel<8, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
     return (int)cudaErrorInvalidValue;
 }
 
@@ -1391,10 +1292,10 @@ extern "C" int trpdrv_launch_fused(const trpdrv_dev_system *d_sys, int nsys, int
     const tma::StageParam<1> p1 = {};
     const tma::StageParam<2> p2 = {};
     if (mma_k == 4)
-        return vec2 ? launch_kernel<4, false, 2>(d_sys, nsys, total_items, counter, status, grid, p2, stream)
-                    : launch_kernel<4, false, 1>(d_sys, nsys, total_items, counter, status, grid, p1, stream);
-    return vec2 ? launch_kernel<8, false, 2>(d_sys, nsys, total_items, counter, status, grid, p2, stream)
-                : launch_kernel<8, false, 1>(d_sys, nsys, total_items, counter, status, grid, p1, stream);
+        return vec2 ? launch_kernel<4, 2>(d_sys, nsys, total_items, counter, status, grid, p2, stream)
+                    : launch_kernel<4, 1>(d_sys, nsys, total_items, counter, status, grid, p1, stream);
+    return vec2 ? launch_kernel<8, 2>(d_sys, nsys, total_items, counter, status, grid, p2, stream)
+                : launch_kernel<8, 1>(d_sys, nsys, total_items, counter, status, grid, p1, stream);
 }
 
 extern "C" int trpdrv_launch_wait_selftest(unsigned long long limit_ns, int *status, unsigned long long *elapsed_ns,
@@ -1406,27 +1307,26 @@ extern "C" int trpdrv_launch_wait_selftest(unsigned long long limit_ns, int *sta
 
 // Every instantiation must be launched with REG_LAUNCH registers per thread (the setmaxnreg split
 // assumes it); g_launch_regs holds the common value, or 0 when they differ.
-template <int KS, bool SPLIT, int STG>
+template <int KS, int STG>
 static cudaError_t init_kernel(int *regs)
 {
     cudaFuncAttributes a;
-    cudaError_t e = cudaFuncGetAttributes(&a, tma::fused_kernel<KS, SPLIT, STG>);
+    cudaError_t e = cudaFuncGetAttributes(&a, tma::fused_kernel<KS, STG>);
     if (e != cudaSuccess) return e;
     *regs = *regs < 0 || *regs == a.numRegs ? a.numRegs : 0;
-    return cudaFuncSetAttribute(tma::fused_kernel<KS, SPLIT, STG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(tma::fused_kernel<KS, STG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)tma::SMEM_BYTES);
 }
 
 extern "C" int trpdrv_fused_tma_init(void)
 {
     int regs = -1;
-    cudaError_t e = init_kernel<8, false, 0>(&regs);
-    if (e == cudaSuccess) e = init_kernel<16, false, 0>(&regs);
-    if (e == cudaSuccess) e = init_kernel<8, true, 0>(&regs);
-    if (e == cudaSuccess) e = init_kernel<8, false, 1>(&regs);
-    if (e == cudaSuccess) e = init_kernel<8, false, 2>(&regs);
-    if (e == cudaSuccess) e = init_kernel<4, false, 1>(&regs);
-    if (e == cudaSuccess) e = init_kernel<4, false, 2>(&regs);
+    cudaError_t e = init_kernel<8, 0>(&regs);
+    if (e == cudaSuccess) e = init_kernel<16, 0>(&regs);
+    if (e == cudaSuccess) e = init_kernel<8, 1>(&regs);
+    if (e == cudaSuccess) e = init_kernel<8, 2>(&regs);
+    if (e == cudaSuccess) e = init_kernel<4, 1>(&regs);
+    if (e == cudaSuccess) e = init_kernel<4, 2>(&regs);
     if (e == cudaSuccess) g_launch_regs = regs;
     return (int)e;
 }

@@ -5,11 +5,11 @@
  */
 #include "trpdrv.h"
 #include "launch.h"
+#include "stage.h"
 
 #include <cuda_runtime_api.h>
 #include <fcntl.h>
 #include <math.h>
-#include <omp.h>
 #include <pthread.h>
 #include <stdarg.h>
 #include <stdio.h>
@@ -782,7 +782,7 @@ static int enqueue_fused(trpdrv_plan *p, cudaStream_t st, int capturing)
             if (p->h_dev[q].ntriples > 0) TRY(pad_refill(p, q, 1, 0, p->s[q].shape.nocc, st, &launches));
         if (p->use_tma)
             LAUNCH_TRY(trpdrv_launch_fused_tma(p->d_dev, p->nsys, p->total_items, p->d_counter, p->d_status,
-                                               p->grid_tma, p->tma_maps, p->tma_mma_k, 0, st));
+                                               p->grid_tma, p->tma_maps, p->tma_mma_k, st));
         else
             LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, p->total_items, p->d_counter, p->d_status, p->grid,
                                            p->vec2 || p->padded, p->opt.mma_k, st));
@@ -1164,7 +1164,7 @@ int trpdrv_plan_upload_execute(trpdrv_plan *p, const trpdrv_system *host, int ch
         const int grid = (int64_t)cap < n ? cap : (int)n;
         if (n <= 0 || rc != TRPDRV_OK) continue;
         int e = p->use_tma ? trpdrv_launch_fused_tma(p->d_dev, p->nsys, sp[c].end, p->d_chunk_first + c, p->d_status,
-                                                     grid, p->tma_maps, p->tma_mma_k, 0, p->stream)
+                                                     grid, p->tma_maps, p->tma_mma_k, p->stream)
                            : trpdrv_launch_fused(p->d_dev, p->nsys, sp[c].end, p->d_chunk_first + c, p->d_status,
                                                  grid, p->vec2 || p->padded, p->opt.mma_k, p->stream);
         if (e) rc = fail(TRPDRV_ERR_CUDA, "fused launch of span %d: %s", c, cudaGetErrorString((cudaError_t)e));
@@ -1462,7 +1462,7 @@ static int tune_time(trpdrv_plan *p, const trpdrv_tune_candidate *c, double *est
                 CUDA_TRY(cudaEventRecord(p->ev0, st));
                 if (c->staging == 2)
                     LAUNCH_TRY(trpdrv_launch_fused_tma(p->d_dev, p->nsys, d->item_begin + sample, p->d_counter,
-                                                       p->d_status, grid, p->tma_maps, c->mma_k, 0, st));
+                                                       p->d_status, grid, p->tma_maps, c->mma_k, st));
                 else
                     LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, d->item_begin + sample, p->d_counter,
                                                    p->d_status, grid, p->vec2 || p->padded, c->mma_k, st));
@@ -1730,19 +1730,30 @@ int trpdrv_run(const trpdrv_system *host, int nsys, const trpdrv_options *opt, d
 /* drop-in entry points                                                                         */
 /* ------------------------------------------------------------------------------------------ */
 
-enum { DI_JIA, DI_KIA, DI_JKA, DI_KKA, DI_TIJ, DI_TKJ, DI_NVV };
-enum { DO_TIA, DO_XIA, DO_TKA, DO_XKA, DO_JIJ, DO_JKJ, DO_KIJ, DO_KKJ, DO_NOV };
+/* One triple's inputs as the drop-in body stages them, on the device and in a pinned host mirror (the two always
+ * hold the same bytes once the transfers of a call have run):
+ *   I    the i-role blocks: tij, jia, kia, tia, xia, jij, kij
+ *   K    the k-role blocks: tkj, jka, kka, tka, xka, jkj, kkj
+ *   VEC  dintc1, dintx1, t1v1, dintc2, dintx2, t1v2, eorb
+ * Rows of odd length are padded to the next even one (zero pads), so that the GEMM copies 16 bytes at a time
+ * whatever the sizes.  K and VEC, which the reference driver's k-inner loop (omp/test.c:160-176) changes from
+ * call to call, are contiguous: a small call sends one piece. */
+enum { DS_I = 0, DS_K = 7, DS_VEC = 14, DS_N = 21 };
+enum { DS_T = 0, DS_J, DS_KV, DS_TO, DS_XO, DS_JO, DS_KO }; /* blocks of a role, after its first slot */
 
 static struct dropin_state {
     int ready, device;
     cudaStream_t stream;
-    size_t cap_vv, cap_ov, cap_v, cap_bf, cap_pairs;
-    double *vv[DI_NVV];
-    double *ov[DO_NOV];
-    double *vec[6];
-    double *eorb, *f, *bpart, *out4;
+    int ncor, nocc, nvir;      /* shape of the staging layout */
+    size_t off[DS_N + 1];      /* its slots' offsets (doubles) */
+    size_t cap_stage;          /* doubles in d_stage / h_stage */
+    double *d_stage, *h_stage;
+    size_t cap_f, cap_part;
+    double *f, *bpart;
+    size_t cap_vec;
+    double *vec;               /* the tengy entry points' vectors */
     unsigned *tcount;
-    double *h_out4; /* pinned */
+    double *h_out4;            /* pinned: the energy kernel writes it directly */
 } g_di;
 static pthread_mutex_t g_di_mu = PTHREAD_MUTEX_INITIALIZER;
 
@@ -1779,21 +1790,16 @@ static const double *reg_lookup(const double *p, size_t n)
     return NULL;
 }
 
-static void dif_release(void);
-
 static void di_release(void)
 {
     if (!g_di.ready) return;
     cudaSetDevice(g_di.device);
-    dif_release();
     reg_release();
-    for (int q = 0; q < DI_NVV; ++q) cudaFree(g_di.vv[q]);
-    for (int q = 0; q < DO_NOV; ++q) cudaFree(g_di.ov[q]);
-    for (int q = 0; q < 6; ++q) cudaFree(g_di.vec[q]);
-    cudaFree(g_di.eorb);
+    cudaFree(g_di.d_stage);
+    cudaFreeHost(g_di.h_stage);
     cudaFree(g_di.f);
     cudaFree(g_di.bpart);
-    cudaFree(g_di.out4);
+    cudaFree(g_di.vec);
     cudaFree(g_di.tcount);
     cudaFreeHost(g_di.h_out4);
     cudaStreamDestroy(g_di.stream);
@@ -1910,16 +1916,21 @@ void trpdrv_finalize(void)
     pthread_mutex_unlock(&g_di_mu);
 }
 
-#define DI_GROW(ptr, count)                                                                         \
+#define DI_GROW(ptr, cap, count)                                                                    \
     do {                                                                                            \
-        if (ptr) cudaFree(ptr);                                                                     \
-        ptr = NULL;                                                                                 \
-        CUDA_TRY(cudaMalloc((void **)&(ptr), sizeof(double) * (count)));                            \
+        if ((size_t)(count) > (cap)) {                                                              \
+            if (ptr) cudaFree(ptr);                                                                 \
+            ptr = NULL;                                                                             \
+            cap = 0;                                                                                \
+            CUDA_TRY(cudaMalloc((void **)&(ptr), sizeof(double) * (count)));                        \
+            cap = (count);                                                                          \
+        }                                                                                           \
     } while (0)
 
-/* Makes the drop-in device buffers at least as large as one triple of (nocc, nvir, nbf) needs. */
+/* Device, stream and the buffers that the energies of one triple of this size need. */
 static int di_reserve(int nocc, int nvir, int nbf)
 {
+    (void)nocc;
     if (!g_di.ready) {
         int dev = 0;
         TRY(ensure_device(-1, &dev, NULL));
@@ -1927,51 +1938,66 @@ static int di_reserve(int nocc, int nvir, int nbf)
         CUDA_TRY(cudaStreamCreateWithFlags(&g_di.stream, cudaStreamNonBlocking));
         CUDA_TRY(cudaMalloc((void **)&g_di.tcount, sizeof(unsigned)));
         CUDA_TRY(cudaMemset(g_di.tcount, 0, sizeof(unsigned)));
-        CUDA_TRY(cudaMalloc((void **)&g_di.out4, sizeof(double) * 4));
         CUDA_TRY(cudaMallocHost((void **)&g_di.h_out4, sizeof(double) * 4));
         g_di.ready = 1;
     } else {
         CUDA_TRY(cudaSetDevice(g_di.device));
     }
-    const size_t vv = (size_t)nvir * nvir, ov = (size_t)nocc * nvir, v = (size_t)nvir, bf = (size_t)nbf;
-    const size_t pairs = (size_t)trpdrv_tengy_pairs(nvir);
-    if (vv > g_di.cap_vv) {
-        for (int q = 0; q < DI_NVV; ++q) DI_GROW(g_di.vv[q], vv);
-        DI_GROW(g_di.f, 8 * vv);
-        g_di.cap_vv = vv;
-    }
-    if (ov > g_di.cap_ov) {
-        for (int q = 0; q < DO_NOV; ++q) DI_GROW(g_di.ov[q], ov);
-        g_di.cap_ov = ov;
-    }
-    if (v > g_di.cap_v) {
-        for (int q = 0; q < 6; ++q) DI_GROW(g_di.vec[q], v);
-        g_di.cap_v = v;
-    }
-    if (bf > g_di.cap_bf) {
-        DI_GROW(g_di.eorb, bf);
-        g_di.cap_bf = bf;
-    }
-    if (pairs > g_di.cap_pairs) {
-        DI_GROW(g_di.bpart, 4 * pairs);
-        g_di.cap_pairs = pairs;
-    }
+    DI_GROW(g_di.f, g_di.cap_f, 8 * (size_t)nvir * nvir);
+    DI_GROW(g_di.bpart, g_di.cap_part, 4 * (size_t)trpdrv_tengy_pairs(nvir));
+    DI_GROW(g_di.vec, g_di.cap_vec, 6 * (size_t)nvir + (size_t)nbf);
     return TRPDRV_OK;
 }
 
-/* Device copy of host [src, src + n): the registered copy when there is one, else a copy into `slot`. */
-static int h2d(const double **out, double *slot, const double *src, size_t n)
+static size_t round32(size_t n) { return (n + 31) & ~(size_t)31; }
+
+/* Lays the staging block out for this shape and clears it (the pads must be zero, and mirror and device equal). */
+static int di_layout(int ncor, int nocc, int nvir)
 {
-    const double *d = reg_lookup(src, n);
-    if (!d) {
-        CUDA_TRY(cudaMemcpyAsync(slot, src, sizeof(double) * n, cudaMemcpyHostToDevice, g_di.stream));
-        d = slot;
+    if (g_di.cap_stage && g_di.ncor == ncor && g_di.nocc == nocc && g_di.nvir == nvir) return TRPDRV_OK;
+    g_di.nvir = 0; /* no valid layout until the end */
+    const size_t V = (size_t)nvir, O = (size_t)nocc, ldv = (size_t)row_pitch(nvir), ldo = (size_t)row_pitch(nocc);
+    const size_t role[7] = {ldv * V, ldv * V, ldv * V, ldv * O, ldv * O, ldo * V, ldo * V};
+    size_t o = 0;
+    for (int q = 0; q < DS_N; ++q) {
+        g_di.off[q] = o;
+        o += round32(q < DS_VEC ? role[q % 7] : q < DS_N - 1 ? V : (size_t)(ncor + nocc + nvir));
     }
-    *out = d;
+    g_di.off[DS_N] = o;
+    if (o > g_di.cap_stage) {
+        if (g_di.d_stage) cudaFree(g_di.d_stage);
+        if (g_di.h_stage) cudaFreeHost(g_di.h_stage);
+        g_di.d_stage = g_di.h_stage = NULL;
+        g_di.cap_stage = 0;
+        CUDA_TRY(cudaMalloc((void **)&g_di.d_stage, sizeof(double) * o));
+        CUDA_TRY(cudaMallocHost((void **)&g_di.h_stage, sizeof(double) * o));
+        g_di.cap_stage = o;
+    }
+    CUDA_TRY(cudaStreamSynchronize(g_di.stream)); /* no transfer of a failed call still reads the mirror */
+    memset(g_di.h_stage, 0, sizeof(double) * o);
+    CUDA_TRY(cudaMemsetAsync(g_di.d_stage, 0, sizeof(double) * o, g_di.stream));
+    g_di.ncor = ncor;
+    g_di.nocc = nocc;
+    g_di.nvir = nvir;
     return TRPDRV_OK;
 }
 
-static int di_tengy_launch(int ncor, int nocc, int nvir, double eaijk, const double *const *vec, const double *eorb)
+/* Enqueues the transfer of the mirror range [lo, hi) (widened to 16 bytes) to the device block. */
+static int di_send(void *ctx, char *lo, char *hi)
+{
+    (void)ctx;
+    const size_t a = ((size_t)(lo - (char *)g_di.h_stage)) & ~(size_t)15;
+    const size_t b = ((size_t)(hi - (char *)g_di.h_stage) + 15) & ~(size_t)15;
+    CUDA_TRY(cudaMemcpyAsync((char *)g_di.d_stage + a, (char *)g_di.h_stage + a, b - a, cudaMemcpyHostToDevice,
+                             g_di.stream));
+    return TRPDRV_OK;
+}
+
+/* Segments of a call's transfer: the comparison of one runs while the one before crosses the bus. */
+#define DI_SEGMENT ((size_t)512 << 10)
+
+/* The energies of the f at g_di.f into g_di.h_out4; waits for them. */
+static int di_tengy(int ncor, int nocc, int nvir, double eaijk, const double *const *vec, const double *eorb)
 {
     trpdrv_tengy_args ta;
     memset(&ta, 0, sizeof ta);
@@ -1990,272 +2016,9 @@ static int di_tengy_launch(int ncor, int nocc, int nvir, double eaijk, const dou
     ta.t1v2 = vec[5];
     ta.block_partial = g_di.bpart;
     ta.counter = g_di.tcount;
-    ta.out4 = g_di.out4;
+    ta.out4 = g_di.h_out4;
     LAUNCH_TRY(trpdrv_launch_tengy(&ta, g_di.stream));
-    CUDA_TRY(cudaMemcpyAsync(g_di.h_out4, g_di.out4, sizeof(double) * 4, cudaMemcpyDeviceToHost, g_di.stream));
     CUDA_TRY(cudaStreamSynchronize(g_di.stream));
-    return TRPDRV_OK;
-}
-
-/* ---- the drop-in body on the fused TMA kernel --------------------------------------------
- * One call stages its triple's inputs into a fixed "one-triple system" (trpdrv_dev_system with
- * one_triple = 1) on the device and its pinned host mirror:
- *   HDR   the system descriptor and the packed triple (512 bytes)
- *   VEC   dintc, dintx, t1v as [2][nvir] (i role, k role), then eorb
- *   I     the i-role blocks: tij, jia, kia, -tia, -xia, jij, kij
- *   K     the k-role blocks: tkj, jka, kka, -tka, -xka, jkj, kkj, at the same offsets RS doubles on
- * so that every TMA-read tensor is [2 slots] with slot stride RS.  Host slices are compared with the
- * mirror block by block and copied (negated where the kernel wants -T / -X) only where they differ;
- * a region goes to the device only when something in it changed (or the device copy is not known to
- * match the mirror): the reference driver's k-inner loop changes only the K region from call to call.
- * Slices inside registered arrays are gathered on the device instead.  One fused launch (one work item
- * per tile pair; f never leaves the SMs) then writes the per-item energy slots, which come back with
- * the kernel's status and are summed on the host in a fixed order. */
-enum { DR_HDR, DR_VEC, DR_I, DR_K, DR_N };
-enum { DT_T2, DT_JVV, DT_KVV, DT_NTOV, DT_NXOV, DT_JOV, DT_KOV, DT_N };
-#define DS_HDR_DOUBLES 64 /* the system descriptor and the packed triple, 512 bytes */
-
-static struct dropin_fused {
-    int ready, ncor, nocc, nvir, nsm, npairs;
-    size_t reg_off[DR_N + 1];  /* region offsets (doubles) in the staging block */
-    size_t toff[DT_N];         /* tensor offsets inside an I / K region */
-    size_t vec_v;              /* nvir */
-    int dev_valid[DR_N];       /* the device copy of the region equals the host mirror */
-    double *d_block, *h_block;
-    trpdrv_dev_system h_sys;
-    double *d_io, *h_io; /* per-item energy slots [npairs][8][4], then the work counter (8 bytes), the status
-                            and the split items' arrival counters, all cleared before every launch */
-    double *d_split;     /* split items: partial f of both halves of every item */
-    void *maps;
-} g_dif;
-
-static void dif_release(void)
-{
-    if (!g_dif.ready) return;
-    cudaFree(g_dif.d_block);
-    cudaFreeHost(g_dif.h_block);
-    cudaFree(g_dif.d_io);
-    cudaFreeHost(g_dif.h_io);
-    cudaFree(g_dif.d_split);
-    free(g_dif.maps);
-    memset(&g_dif, 0, sizeof g_dif);
-}
-
-/* The fused drop-in path needs what the TMA kernel needs: even nvir and nocc (16-byte rows). */
-static int dif_eligible(int nocc, int nvir) { return !(nocc & 1) && !(nvir & 1); }
-
-static size_t round32(size_t n) { return (n + 31) & ~(size_t)31; }
-
-static int dif_prepare(int ncor, int nocc, int nvir)
-{
-    if (g_dif.ready && g_dif.ncor == ncor && g_dif.nocc == nocc && g_dif.nvir == nvir) return TRPDRV_OK;
-    dif_release();
-    const size_t vv = (size_t)nvir * nvir, ov = (size_t)nocc * nvir, v = (size_t)nvir;
-    const size_t tlen[DT_N] = {vv, vv, vv, ov, ov, ov, ov};
-    size_t o = 0;
-    for (int q = 0; q < DT_N; ++q) {
-        g_dif.toff[q] = o;
-        o += round32(tlen[q]);
-    }
-    const size_t rs = o; /* region size = slot stride of every TMA-read tensor */
-    g_dif.reg_off[DR_HDR] = 0;
-    g_dif.reg_off[DR_VEC] = DS_HDR_DOUBLES;
-    g_dif.reg_off[DR_I] = DS_HDR_DOUBLES + round32(6 * v + (size_t)(ncor + nocc + nvir));
-    g_dif.reg_off[DR_K] = g_dif.reg_off[DR_I] + rs;
-    g_dif.reg_off[DR_N] = g_dif.reg_off[DR_K] + rs;
-    g_dif.vec_v = v;
-    const int nb = (nvir + TRPDRV_TILE - 1) / TRPDRV_TILE, npairs = nb * (nb + 1) / 2;
-    int dev = 0, nsm = 0;
-    TRY(ensure_device(g_di.device, &dev, &nsm));
-    const size_t total = g_dif.reg_off[DR_N];
-    CUDA_TRY(cudaMalloc((void **)&g_dif.d_block, sizeof(double) * total));
-    CUDA_TRY(cudaMallocHost((void **)&g_dif.h_block, sizeof(double) * total));
-    const size_t nslot = 4 * TRPDRV_FUSED_SLOTS * (size_t)npairs;
-    CUDA_TRY(cudaMalloc((void **)&g_dif.d_io, sizeof(double) * (nslot + 2 + (size_t)(npairs + 1) / 2)));
-    CUDA_TRY(cudaMallocHost((void **)&g_dif.h_io, sizeof(double) * (nslot + 2)));
-    g_dif.ready = 1; /* from here dif_release frees whatever was allocated */
-    /* every tile pair's contraction runs as two halves on two SMs (one triple has only npairs items) */
-    CUDA_TRY(cudaMalloc((void **)&g_dif.d_split, sizeof(double) * 2 * 64 * 256 * (size_t)npairs));
-    memset(g_dif.h_block, 0, sizeof(double) * total);
-    double *d = g_dif.d_block;
-    const double *I = d + g_dif.reg_off[DR_I], *vec = d + g_dif.reg_off[DR_VEC];
-    trpdrv_dev_system *S = &g_dif.h_sys;
-    memset(S, 0, sizeof *S);
-    S->ncor = ncor;
-    S->nocc = nocc;
-    S->nvir = nvir;
-    S->nb = nb;
-    S->npairs = npairs;
-    S->pack_edge = trpdrv_tma_pack_edge(nvir);
-    S->ntriples = 1;
-    S->nt = 1;
-    S->n_a = 1;
-    S->one_triple = 1;
-    S->split = 1;
-    S->split_scratch = g_dif.d_split;
-    S->split_count = (unsigned *)(g_dif.d_io + nslot + 2);
-    S->slot_stride = (int64_t)rs;
-    S->item_begin = 0;
-    S->t2 = I + g_dif.toff[DT_T2];
-    S->jvv = I + g_dif.toff[DT_JVV];
-    S->kvv = I + g_dif.toff[DT_KVV];
-    S->ntov = I + g_dif.toff[DT_NTOV];
-    S->nxov = I + g_dif.toff[DT_NXOV];
-    S->jov = I + g_dif.toff[DT_JOV];
-    S->kov = I + g_dif.toff[DT_KOV];
-    S->dintc = vec;
-    S->dintx = vec + 2 * v;
-    S->t1v = vec + 4 * v;
-    S->eorb = vec + 6 * v;
-    S->triples = (const int32_t *)d + 2 * (sizeof(trpdrv_dev_system) / 8 + 1);
-    S->order = NULL;
-    S->partial = g_dif.d_io;
-    S->rec = NULL;
-    if (sizeof(trpdrv_dev_system) + 16 > DS_HDR_DOUBLES * sizeof(double))
-        return fail(TRPDRV_ERR_STATE, "drop-in staging header too small");
-    if (!trpdrv_tma_supported(S, 1)) return fail(TRPDRV_ERR_UNSUPPORTED, "TMA staging unavailable");
-    g_dif.maps = aligned_alloc(64, (trpdrv_tma_maps_bytes() + 63) & ~(size_t)63);
-    if (!g_dif.maps) return fail(TRPDRV_ERR_NOMEM, "host allocation failed");
-    const int e = trpdrv_tma_prepare(S, 1, g_dif.maps);
-    if (e) return fail(TRPDRV_ERR_CUDA, "tensor-map encoding failed (%d)", e);
-    g_dif.ncor = ncor;
-    g_dif.nocc = nocc;
-    g_dif.nvir = nvir;
-    g_dif.nsm = nsm;
-    g_dif.npairs = npairs;
-    return TRPDRV_OK;
-}
-
-/* Host threads for the staging copies: TRPDRV_STAGE_THREADS, else up to 16 of OpenMP's. */
-static int stage_threads(void)
-{
-    const char *v = getenv("TRPDRV_STAGE_THREADS");
-    int n = v ? atoi(v) : 0;
-    if (n <= 0) {
-        n = omp_get_max_threads();
-        if (n > 16) n = 16;
-    }
-    return n < 1 ? 1 : n;
-}
-
-/* 64-bit words that may alias the doubles they are read from (bitwise comparison and negation) */
-typedef uint64_t __attribute__((may_alias)) word64;
-
-typedef struct stage_piece {
-    double *dst;
-    const double *src;
-    size_t n;
-    int neg; /* the mirror holds -src */
-} stage_piece;
-
-/* Brings the mirror pieces up to date with their sources (negated where asked), in blocks of 16 KB
- * spread over up to `threads` host threads; a block is written only where it differs bit for bit.
- * Returns 1 if any block was written. */
-static int stage_update(const stage_piece *pc, int npc, int threads)
-{
-    enum { BLK = 2048 };
-    int nblk = 0;
-    for (int q = 0; q < npc; ++q) nblk += (int)((pc[q].n + BLK - 1) / BLK);
-    if (nblk == 0) return 0;
-    if (threads > nblk) threads = nblk;
-    int changed = 0;
-#pragma omp parallel for num_threads(threads) schedule(static) reduction(| : changed) if (threads > 1)
-    for (int b = 0; b < nblk; ++b) {
-        int q = 0, r = b;
-        while (r >= (int)((pc[q].n + BLK - 1) / BLK)) {
-            r -= (int)((pc[q].n + BLK - 1) / BLK);
-            ++q;
-        }
-        const size_t lo = (size_t)r * BLK, n = pc[q].n - lo < BLK ? pc[q].n - lo : BLK;
-        const word64 *src = (const word64 *)(pc[q].src + lo);
-        word64 *dst = (word64 *)(pc[q].dst + lo);
-        const uint64_t flip = pc[q].neg ? 0x8000000000000000ull : 0ull; /* negation = sign bit */
-        uint64_t diff = 0;
-        for (size_t e = 0; e < n; ++e) diff |= dst[e] ^ src[e] ^ flip;
-        if (diff) {
-            for (size_t e = 0; e < n; ++e) dst[e] = src[e] ^ flip;
-            changed = 1;
-        }
-    }
-    return changed;
-}
-
-/* One triple through the fused kernel; rec[4] = emp4i, emp5i, emp4k, emp5k.  in[q], len[q]: the
- * slice, reg[q]: its region (DR_VEC / DR_I / DR_K), off[q]: its offset in the block, neg[q]: stored
- * negated. */
-static int body_fused(int ncor, int nocc, int nvir, int a, int i, int j, int k, int nin, const double *const *in,
-                      const size_t *len, const int *reg, const size_t *off, const int *neg, double *rec)
-{
-    TRY(dif_prepare(ncor, nocc, nvir));
-    cudaStream_t st = g_di.stream;
-    double *h = g_dif.h_block;
-    const int threads = stage_threads();
-    /* header: the system descriptor with this call's a, then the packed triple */
-    trpdrv_dev_system S = g_dif.h_sys;
-    S.a = a;
-    memcpy(h, &S, sizeof S);
-    ((int32_t *)h)[2 * (sizeof(trpdrv_dev_system) / 8 + 1)] = pack_triple(i, j, k);
-
-    trpdrv_copy_list gl;
-    memset(&gl, 0, sizeof gl);
-    int has_dev[DR_N] = {0, 0, 0, 0};
-    stage_piece pc[DR_N][24];
-    int npc[DR_N] = {0, 0, 0, 0};
-    for (int q = 0; q < nin; ++q) {
-        const double *dsrc = reg_lookup(in[q], len[q]);
-        if (dsrc && gl.n < TRPDRV_COPY_LIST_MAX) {
-            gl.src[gl.n] = dsrc;
-            gl.dst[gl.n] = g_dif.d_block + off[q];
-            gl.len[gl.n] = (long long)len[q];
-            gl.neg[gl.n] = neg[q];
-            ++gl.n;
-            has_dev[reg[q]] = 1;
-        } else {
-            stage_piece *p = &pc[reg[q]][npc[reg[q]]++];
-            p->dst = h + off[q];
-            p->src = in[q];
-            p->n = len[q];
-            p->neg = neg[q];
-        }
-    }
-    /* the large regions first, each sent as soon as it is up to date (the copy overlaps the next
-     * region's comparison); then the header and the vectors, always sent */
-    static const int order[2] = {DR_K, DR_I};
-    for (int r = 0; r < 2; ++r) {
-        const int R = order[r];
-        const int changed = stage_update(pc[R], npc[R], threads);
-        if (npc[R] && (changed || !g_dif.dev_valid[R])) {
-            const size_t lo = g_dif.reg_off[R], n = g_dif.reg_off[R + 1] - lo;
-            CUDA_TRY(cudaMemcpyAsync(g_dif.d_block + lo, h + lo, sizeof(double) * n, cudaMemcpyHostToDevice, st));
-        }
-        /* a region that received device slices no longer mirrors the host block */
-        g_dif.dev_valid[R] = npc[R] && !has_dev[R];
-    }
-    stage_update(pc[DR_VEC], npc[DR_VEC], 1);
-    CUDA_TRY(cudaMemcpyAsync(g_dif.d_block, h, sizeof(double) * g_dif.reg_off[DR_I], cudaMemcpyHostToDevice, st));
-    if (gl.n) LAUNCH_TRY(trpdrv_launch_gather(&gl, st));
-    const size_t nslot = 4 * TRPDRV_FUSED_SLOTS * (size_t)g_dif.npairs;
-    CUDA_TRY(cudaMemsetAsync(g_dif.d_io + nslot, 0, sizeof(double) * (2 + (size_t)(g_dif.npairs + 1) / 2), st));
-    const int items = 2 * g_dif.npairs; /* two halves per tile pair */
-    const int grid = items < g_dif.nsm ? items : g_dif.nsm;
-    LAUNCH_TRY(trpdrv_launch_fused_tma((const trpdrv_dev_system *)g_dif.d_block, 1, items,
-                                       (unsigned long long *)(g_dif.d_io + nslot), (int *)(g_dif.d_io + nslot + 1),
-                                       grid, g_dif.maps, 8, 1, st));
-    CUDA_TRY(cudaMemcpyAsync(g_dif.h_io, g_dif.d_io, sizeof(double) * (nslot + 2), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    int status = 0;
-    memcpy(&status, g_dif.h_io + nslot + 1, sizeof status);
-    if (status) return fail(TRPDRV_ERR_DEVICE, "fused kernel reported status %d", status);
-    /* the item slots in a fixed order, compensated (Neumaier) */
-    for (int c = 0; c < 4; ++c) {
-        double sum = 0.0, comp = 0.0;
-        for (size_t q = (size_t)c; q < nslot; q += 4) {
-            const double x = g_dif.h_io[q], t = sum + x;
-            comp += fabs(sum) >= fabs(x) ? (sum - t) + x : (x - t) + sum;
-            sum = t;
-        }
-        rec[c] = sum + comp;
-    }
     return TRPDRV_OK;
 }
 
@@ -2287,58 +2050,42 @@ static int body_impl(double *f1n, double *f1t, double *f2n, double *f2t, double 
         return fail(TRPDRV_ERR_ARG, "TRPDRV_WRITE_F=1 with a NULL f array");
 
     TRY(di_reserve(nocc, nvir, nbf));
-    const size_t lnvv = (size_t)nvir * nvir, lnov = (size_t)nocc * nvir;
+    TRY(di_layout(ncor, nocc, nvir));
+    const size_t lnvv = (size_t)nvir * nvir, lnov = (size_t)nocc * nvir, V = (size_t)nvir, O = (size_t)nocc;
     const size_t vv = (size_t)(k - klo) * lnvv, ov = (size_t)(k - klo) * lnov;
-
-    if (!write_f && dif_eligible(nocc, nvir) && !env_flag("TRPDRV_DROPIN_PATH", "plain")) {
-        TRY(dif_prepare(ncor, nocc, nvir));
-        /* the 21 input slices: region, offset in the staging block, stored negated or not */
-        const size_t v = (size_t)nvir, I = g_dif.reg_off[DR_I], K = g_dif.reg_off[DR_K], VE = g_dif.reg_off[DR_VEC];
-        const size_t *T = g_dif.toff;
-        const double *in[21] = {tij, jia, kia, tia, xia, jij, kij, tkj + vv, jka + vv, kka + vv, tka + ov, xka + ov,
-                                jkj + ov, kkj + ov, dintc1, dintc2, dintx1, dintx2, t1v1, t1v2, eorb};
-        const size_t len[21] = {lnvv, lnvv, lnvv, lnov, lnov, lnov, lnov, lnvv, lnvv, lnvv, lnov, lnov,
-                                lnov, lnov, v, v, v, v, v, v, (size_t)nbf};
-        const int reg[21] = {DR_I, DR_I, DR_I, DR_I, DR_I, DR_I, DR_I, DR_K, DR_K, DR_K, DR_K, DR_K, DR_K, DR_K,
-                             DR_VEC, DR_VEC, DR_VEC, DR_VEC, DR_VEC, DR_VEC, DR_VEC};
-        const size_t off[21] = {I + T[DT_T2], I + T[DT_JVV], I + T[DT_KVV], I + T[DT_NTOV], I + T[DT_NXOV],
-                                I + T[DT_JOV], I + T[DT_KOV], K + T[DT_T2], K + T[DT_JVV], K + T[DT_KVV],
-                                K + T[DT_NTOV], K + T[DT_NXOV], K + T[DT_JOV], K + T[DT_KOV],
-                                VE, VE + v, VE + 2 * v, VE + 3 * v, VE + 4 * v, VE + 5 * v, VE + 6 * v};
-        const int neg[21] = {0, 0, 0, 1, 1, 0, 0, 0, 0, 0, 1, 1, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-        double rec[4] = {0.0, 0.0, 0.0, 0.0};
-        TRY(body_fused(ncor, nocc, nvir, a, i, j, k, 21, in, len, reg, off, neg, rec));
-        /* omp/ccsd_trpdrv_omp_cbody.c:133-142 */
-        double emp4 = *emp4_, emp5 = *emp5_;
-        emp4 += rec[0];
-        emp5 += rec[1];
-        if (i != k) {
-            emp4 += rec[2];
-            emp5 += rec[3];
-        }
-        *emp4_ = emp4;
-        *emp5_ = emp5;
-        return TRPDRV_OK;
+    /* the slices in the order of the staging block; slices of registered arrays are read where they are */
+    const double *in[DS_N] = {tij, jia, kia, tia, xia, jij, kij, tkj + vv, jka + vv, kka + vv, tka + ov, xka + ov,
+                              jkj + ov, kkj + ov, dintc1, dintx1, t1v1, dintc2, dintx2, t1v2, eorb};
+    const double *dev[DS_N];
+    int ld[DS_N];
+    stage_piece pc[DS_N];
+    int npi = 0, npk = 0; /* pieces of I from the front, of K and VEC from DS_K on */
+    for (int q = 0; q < DS_N; ++q) {
+        const int b = q % 7, is_vec = q >= DS_VEC;
+        const size_t width = is_vec ? (q < DS_N - 1 ? V : (size_t)nbf) : b < DS_JO ? V : O;
+        const size_t rows = is_vec ? 1 : b < DS_TO || b >= DS_JO ? V : O;
+        const double *d = reg_lookup(in[q], rows * width);
+        ld[q] = (int)width;
+        dev[q] = d;
+        if (d) continue;
+        dev[q] = g_di.d_stage + g_di.off[q];
+        const size_t pitch = is_vec ? width : (size_t)row_pitch((int)width);
+        ld[q] = (int)pitch;
+        stage_piece *p = q < DS_K ? &pc[npi++] : &pc[DS_K + npk++];
+        const int flat = pitch == width;
+        p->dst = (char *)(g_di.h_stage + g_di.off[q]);
+        p->src = (const char *)in[q];
+        p->rows = flat ? 1 : rows;
+        p->width = sizeof(double) * (flat ? rows * width : width);
+        p->pitch = sizeof(double) * (flat ? rows * width : pitch);
     }
-
-    const double *dv[DI_NVV], *dov[DO_NOV], *dvec[6], *deorb;
-    TRY(h2d(&dv[DI_JIA], g_di.vv[DI_JIA], jia, lnvv));
-    TRY(h2d(&dv[DI_KIA], g_di.vv[DI_KIA], kia, lnvv));
-    TRY(h2d(&dv[DI_JKA], g_di.vv[DI_JKA], jka + vv, lnvv));
-    TRY(h2d(&dv[DI_KKA], g_di.vv[DI_KKA], kka + vv, lnvv));
-    TRY(h2d(&dv[DI_TIJ], g_di.vv[DI_TIJ], tij, lnvv));
-    TRY(h2d(&dv[DI_TKJ], g_di.vv[DI_TKJ], tkj + vv, lnvv));
-    TRY(h2d(&dov[DO_TIA], g_di.ov[DO_TIA], tia, lnov));
-    TRY(h2d(&dov[DO_XIA], g_di.ov[DO_XIA], xia, lnov));
-    TRY(h2d(&dov[DO_TKA], g_di.ov[DO_TKA], tka + ov, lnov));
-    TRY(h2d(&dov[DO_XKA], g_di.ov[DO_XKA], xka + ov, lnov));
-    TRY(h2d(&dov[DO_JIJ], g_di.ov[DO_JIJ], jij, lnov));
-    TRY(h2d(&dov[DO_JKJ], g_di.ov[DO_JKJ], jkj + ov, lnov));
-    TRY(h2d(&dov[DO_KIJ], g_di.ov[DO_KIJ], kij, lnov));
-    TRY(h2d(&dov[DO_KKJ], g_di.ov[DO_KKJ], kkj + ov, lnov));
-    const double *vecs[6] = {dintc1, dintx1, t1v1, dintc2, dintx2, t1v2};
-    for (int q = 0; q < 6; ++q) TRY(h2d(&dvec[q], g_di.vec[q], vecs[q], (size_t)nvir));
-    TRY(h2d(&deorb, g_di.eorb, eorb, (size_t)nbf));
+    const int threads = stage_threads();
+    int rc = stage_send(pc + DS_K, npk, threads, DI_SEGMENT, di_send, NULL);
+    if (!rc) rc = stage_send(pc, npi, threads, DI_SEGMENT, di_send, NULL);
+    if (rc) {
+        g_di.nvir = 0; /* mirror and device may differ now */
+        return rc;
+    }
 
     trpdrv_plain_args ga;
     memset(&ga, 0, sizeof ga);
@@ -2346,28 +2093,29 @@ static int body_impl(double *f1n, double *f1t, double *f2n, double *f2t, double 
     ga.nvir = nvir;
     ga.neg2 = 1; /* the reference's alpha = -1 GEMMs */
     ga.f = g_di.f;
-    const double *const *V = dv;
-    const double *const *Ob = dov;
-    const double *a1[8] = {V[DI_JIA], V[DI_KIA], V[DI_JIA], V[DI_KIA], V[DI_JKA], V[DI_KKA], V[DI_JKA], V[DI_KKA]};
-    const double *b1[8] = {V[DI_TKJ], V[DI_TKJ], V[DI_TKJ], V[DI_TKJ], V[DI_TIJ], V[DI_TIJ], V[DI_TIJ], V[DI_TIJ]};
-    const int nt[8] = {1, 1, 0, 0, 1, 1, 0, 0};
-    const double *a2[8] = {Ob[DO_TIA], Ob[DO_XIA], Ob[DO_TIA], Ob[DO_XIA], Ob[DO_TKA], Ob[DO_XKA], Ob[DO_TKA], Ob[DO_XKA]};
-    const double *b2[8] = {Ob[DO_KKJ], Ob[DO_KKJ], Ob[DO_JKJ], Ob[DO_JKJ], Ob[DO_KIJ], Ob[DO_KIJ], Ob[DO_JIJ], Ob[DO_JIJ]};
-    for (int x = 0; x < 8; ++x) {
-        ga.a1[x] = a1[x];
-        ga.b1[x] = b1[x];
-        ga.b1_nt[x] = nt[x];
-        ga.a2[x] = a2[x];
-        ga.b2[x] = b2[x];
+    ga.counter = g_di.tcount;
+    int vec2 = 1;
+    for (int x = 0; x < 8; ++x) { /* f1n f2n f3n f4n f1t f2t f3t f4t: omp/ccsd_trpdrv_omp_cbody.c:70-117 */
+        const int A = x < 4 ? DS_I : DS_K, B = x < 4 ? DS_K : DS_I, two = (x >> 1) & 1;
+        const int a1 = A + (x & 1 ? DS_KV : DS_J), b1 = B + DS_T, a2 = A + (x & 1 ? DS_XO : DS_TO);
+        const int b2 = B + (two ? DS_JO : DS_KO);
+        ga.a1[x] = dev[a1];
+        ga.b1[x] = dev[b1];
+        ga.a2[x] = dev[a2];
+        ga.b2[x] = dev[b2];
+        ga.lda1[x] = ld[a1];
+        ga.ldb1[x] = ld[b1];
+        ga.lda2[x] = ld[a2];
+        ga.ldb2[x] = ld[b2];
+        ga.b1_nt[x] = !two;
+        if ((ld[a1] | ld[b1] | ld[a2] | ld[b2]) & 1) vec2 = 0;
+        if (((uintptr_t)dev[a1] | (uintptr_t)dev[b1] | (uintptr_t)dev[a2] | (uintptr_t)dev[b2]) & 15u) vec2 = 0;
     }
-    int vec2 = !(nvir & 1) && !(nocc & 1);
-    for (int x = 0; x < 8; ++x) /* slices of registered arrays may start anywhere */
-        if (((uintptr_t)ga.a1[x] | (uintptr_t)ga.b1[x] | (uintptr_t)ga.a2[x] | (uintptr_t)ga.b2[x]) & 15u) vec2 = 0;
     LAUNCH_TRY(trpdrv_launch_plain_gemm(&ga, vec2, g_di.stream));
 
     /* omp/ccsd_trpdrv_omp_cbody.c:122-126 */
     const double eaijk = eorb[a - 1] - (eorb[ncor + i - 1] + eorb[ncor + j - 1] + eorb[ncor + k - 1]);
-    TRY(di_tengy_launch(ncor, nocc, nvir, eaijk, dvec, deorb));
+    TRY(di_tengy(ncor, nocc, nvir, eaijk, dev + DS_VEC, dev[DS_N - 1]));
 
     if (write_f) {
         double *outs[8] = {f1n, f2n, f3n, f4n, f1t, f2t, f3t, f4t};
@@ -2442,11 +2190,17 @@ static int tengy_impl(const double *f1n, const double *f1t, const double *f2n, c
     for (int x = 0; x < 8; ++x)
         CUDA_TRY(cudaMemcpyAsync(g_di.f + (size_t)x * lnvv, fs[x], sizeof(double) * lnvv, cudaMemcpyHostToDevice,
                                  g_di.stream));
-    const double *vecs[6] = {dintc1, dintx1, t1v1, dintc2, dintx2, t1v2};
-    const double *dvec[6], *deorb;
-    for (int q = 0; q < 6; ++q) TRY(h2d(&dvec[q], g_di.vec[q], vecs[q], (size_t)nvir));
-    TRY(h2d(&deorb, g_di.eorb, eorb, (size_t)nbf));
-    TRY(di_tengy_launch(ncor, nocc, nvir, eaijk, dvec, deorb));
+    /* vectors: slices of registered arrays where they are, the others copied */
+    const double *vecs[7] = {dintc1, dintx1, t1v1, dintc2, dintx2, t1v2, eorb}, *dvec[7];
+    for (int q = 0; q < 7; ++q) {
+        const size_t n = q < 6 ? (size_t)nvir : (size_t)nbf;
+        dvec[q] = reg_lookup(vecs[q], n);
+        if (dvec[q]) continue;
+        double *slot = g_di.vec + (size_t)q * nvir;
+        CUDA_TRY(cudaMemcpyAsync(slot, vecs[q], sizeof(double) * n, cudaMemcpyHostToDevice, g_di.stream));
+        dvec[q] = slot;
+    }
+    TRY(di_tengy(ncor, nocc, nvir, eaijk, dvec, dvec[6]));
     *emp4i = g_di.h_out4[0];
     *emp5i = g_di.h_out4[1];
     *emp4k = g_di.h_out4[2];

@@ -31,20 +31,6 @@ typedef struct trpdrv_dev_system {
     int64_t ntriples;    /* records of this system in the plan: n_a * nt */
     int64_t nt;          /* triples per a (this rank's share): the length of `triples` and `order` */
     int n_a;             /* virtual indices a .. a + n_a - 1 swept (1 = the reference driver's single a) */
-    int one_triple;      /* 1: the tensors hold only what one triple (i, j, k) reads, the i-role block at
-                            occupied slot 0 and the k-role block at slot 1 (t2, jov, kov: one j block
-                            of two slots; jvv, kvv, ntov, nxov, dintc, dintx, t1v: two slots), as the
-                            drop-in entry points stage them; `triples` holds that triple (its i, j, k
-                            give eaijk) and n_a is 1.  TMA kernel only. */
-    int64_t slot_stride; /* one_triple: doubles between the i-role and k-role blocks of every TMA-read tensor
-                            (t2, jvv, kvv, ntov, nxov, jov, kov); 0 = the packed [2][block] layout.  The
-                            vectors (dintc, dintx, t1v) stay packed [2][nvir]. */
-    int split;           /* 1 (one_triple systems): every item's contraction runs as two work items (even and
-                            odd chunks, item indices 2 q and 2 q + 1) on two SMs; each writes its partial f to
-                            split_scratch [item][2][64][256] and the second to arrive (split_count[item])
-                            adds the other's and runs the energy epilogue */
-    double *split_scratch;
-    unsigned *split_count;  /* one per item, zero at launch; left at zero */
     int ldv, ldo;        /* cp.async staging: leading dimension of the rows of nvir (t2, jvv, kvv, ntov, nxov) and of
                             nocc (jov, kov) doubles; 0 = nvir / nocc (packed, as callers hold them).  The
                             plans pad odd rows to the next even length (trpdrv_launch_pack_rows). */
@@ -80,7 +66,7 @@ size_t trpdrv_tma_maps_bytes(void);
 int trpdrv_tma_prepare(const trpdrv_dev_system *h_sys, int nsys, void *maps_out);
 int trpdrv_launch_fused_tma(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items,
                             unsigned long long *counter, int *status, int grid, const void *maps,
-                            int mma_k, int split, void *stream);
+                            int mma_k, void *stream);
 int trpdrv_fused_tma_init(void);
 /* One thread waits, with the production bounded wait and the given limit, on an mbarrier that
  * nothing completes: sets bit 1 of *status when the wait gives up (bit 2 if it wrongly completes)
@@ -151,23 +137,13 @@ typedef struct trpdrv_pack_list {
 } trpdrv_pack_list;
 int trpdrv_launch_pack_rows(const trpdrv_pack_list *list, void *stream);
 
-/* Device-to-device copies dst[s][0..len[s]) = src[s][..] (negated where neg[s]) for s < n, in one launch. */
-#define TRPDRV_COPY_LIST_MAX 24
-typedef struct trpdrv_copy_list {
-    int n;
-    const double *src[TRPDRV_COPY_LIST_MAX];
-    double *dst[TRPDRV_COPY_LIST_MAX];
-    long long len[TRPDRV_COPY_LIST_MAX];
-    int neg[TRPDRV_COPY_LIST_MAX];  /* 1: dst = -src */
-} trpdrv_copy_list;
-int trpdrv_launch_gather(const trpdrv_copy_list *list, void *stream);
-
 /* Plain path.  Single triple: one grouped launch computes the eight f = A1*op(B1) + A2*B2 (neg2: - A2*B2) into
  * f[8][nvir][nvir] (order f1n f2n f3n f4n f1t f2t f3t f4t); b1_nt[x] = 1 if B1 is used transposed.  counter, if
  * not NULL, is zeroed for the trpdrv_launch_tengy that follows on the stream. */
 typedef struct trpdrv_plain_args {
     int nocc, nvir, neg2;
     const double *a1[8], *b1[8], *a2[8], *b2[8];
+    int lda1[8], ldb1[8], lda2[8], ldb2[8]; /* even for vec2 */
     int b1_nt[8];
     double *f;
     unsigned *counter;

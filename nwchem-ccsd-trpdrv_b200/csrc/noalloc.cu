@@ -146,6 +146,8 @@ extern "C" int trpdrv_body_device_noalloc(const trpdrv_body_device_args *a, void
         ga.b1_nt[x] = nt[x];
         ga.a2[x] = a2[x];
         ga.b2[x] = b2[x];
+        ga.lda1[x] = ga.ldb1[x] = ga.lda2[x] = V;
+        ga.ldb2[x] = O;
         const double *ops[4] = {a1[x], b1[x], a2[x], b2[x]};
         for (const double *p : ops)
             if (reinterpret_cast<uintptr_t>(p) & 15u) vec2 = 0;  // 16-byte copies need 16-byte alignment

@@ -31,10 +31,10 @@ template <int BM> struct Tile {
     static constexpr int MI = BM / 32, NI = BM / 16;  // m16 and n8 tiles per warp (BM / 2 square)
 };
 
-// Stages in flight: three where several CTAs share an SM; six 32-wide ones for a single triple, whose few CTAs wait
-// for L2 otherwise.
+// Stages in flight: three where the CTAs of a batch share the SMs; four 32-wide ones for a single triple, six CTAs of
+// which fit an SM, so that nvir = 300 (800 tiles) is one wave.
 constexpr int BATCH_STAGES = 3;
-template <int BM> constexpr int one_stages() { return BM == 32 ? 6 : 3; }
+template <int BM> constexpr int one_stages() { return BM == 32 ? 4 : 3; }
 
 // Column that lane group g owns of its 8 (conflict-free X-major reads, see Tile).
 __device__ __forceinline__ int perm8(int g) { return (0x53427160 >> (4 * g)) & 7; }
@@ -170,6 +170,8 @@ __device__ __forceinline__ bool batch_sources(const BatchArgs &B, int n, int x, 
     ph[0].bk = !two;
     ph[1].a = ((x & 1) ? S.nxov : S.ntov) + (size_t)ia * ov;
     ph[1].b = (two ? S.jov : S.kov) + jb * ov;
+    ph[0].lda = ph[0].ldb = ph[1].lda = S.nvir;
+    ph[1].ldb = S.nocc;
     return true;
 }
 
@@ -180,6 +182,10 @@ __device__ __forceinline__ bool one_sources(const trpdrv_plain_args &P, int x, S
     ph[0].bk = P.b1_nt[x];
     ph[1].a = P.a2[x];
     ph[1].b = P.b2[x];
+    ph[0].lda = P.lda1[x];
+    ph[0].ldb = P.ldb1[x];
+    ph[1].lda = P.lda2[x];
+    ph[1].ldb = P.ldb2[x];
     return true;
 }
 
@@ -197,9 +203,8 @@ __device__ __forceinline__ void gemm_body(const trpdrv_plain_args *one, const Ba
 
     Src ph[2];
     if (!(BATCH ? batch_sources(*batch, n, x, ph) : one_sources(*one, x, ph))) return;
-    ph[0].lda = ph[1].lda = ph[0].ldb = nvir;
     ph[0].klim = nvir;
-    ph[1].ldb = ph[1].klim = nocc;
+    ph[1].klim = nocc;
     ph[1].bk = 0;
     const int nV = (nvir + DK - 1) / DK, nO = (nocc + DK - 1) / DK, nch = nV + nO;
     auto load = [&](int ch) {
@@ -265,7 +270,7 @@ __device__ __forceinline__ void gemm_body(const trpdrv_plain_args *one, const Ba
 }
 
 template <int BM, int VEC>
-__global__ void __launch_bounds__(NTHREAD, BM == 64 ? 3 : 5) plain_gemm_kernel(const __grid_constant__ trpdrv_plain_args args)
+__global__ void __launch_bounds__(NTHREAD, BM == 64 ? 3 : 6) plain_gemm_kernel(const __grid_constant__ trpdrv_plain_args args)
 {
     // the dependent tengy launch may start its prologue (it waits for this grid before reading f)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
