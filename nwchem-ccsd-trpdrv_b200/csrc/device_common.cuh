@@ -95,70 +95,20 @@ __device__ __forceinline__ void two_sum(double a, double b, double &s, double &e
 }
 
 // ------------------------------------------------------------------------------------------------
-// The tengy term at one (b,c).  f index order used throughout the library:
+// The tengy terms.  f index order used throughout the library:
 //   0 f1n, 1 f2n, 2 f3n, 3 f4n, 4 f1t, 5 f2t, 6 f3t, 7 f4t
-// bc[x] = f_x(b,c), cb[x] = f_x(c,b).  Arithmetic as omp/ccsd_tengy_c99.c:65-111.
+// bc[x] = f_x(b,c), cb[x] = f_x(c,b).  The four forms of omp/ccsd_tengy_c99.c:91-111 with the denominator
+// denom = -1/(e_b + e_c + eaijk) factored out of each (equal up to floating-point reassociation).
 // ------------------------------------------------------------------------------------------------
 struct TengySums {
     double e4i, e5i, e4k, e5k;
 };
 
-__device__ __forceinline__ void tengy_term(const double (&bc)[8], const double (&cb)[8], double denom,
-                                           double t1v1b, double t1v2b, double dx1c, double dx2c,
-                                           double dc1c, double dc2c, TengySums &s)
-{
-    const double n1bc = bc[0], n2bc = bc[1], n3bc = bc[2], n4bc = bc[3];
-    const double t1bc = bc[4], t2bc = bc[5], t3bc = bc[6], t4bc = bc[7];
-    const double n1cb = cb[0], n2cb = cb[1], n3cb = cb[2], n4cb = cb[3];
-    const double t1cb = cb[4], t2cb = cb[5], t3cb = cb[6], t4cb = cb[7];
-
-    s.e4i += denom * (t1bc + n1cb + t2cb + n3bc + n4cb) * (t1bc - t2bc * 2 - t3bc * 2 + t4bc)
-           - denom * (n1bc + t1cb + n2cb + n3cb) * (t1bc * 2 - t2bc - t3bc + t4bc * 2)
-           + denom * 3 * (n1bc * (n1bc + n3cb + t4cb * 2) + n2bc * t2cb + n3bc * t4bc);
-    s.e4k += denom * (n1bc + t1cb + n2cb + t3bc + t4cb) * (n1bc - n2bc * 2 - n3bc * 2 + n4bc)
-           - denom * (t1bc + n1cb + t2cb + t3cb) * (n1bc * 2 - n2bc - n3bc + n4bc * 2)
-           + denom * 3 * (t1bc * (t1bc + t3cb + n4cb * 2) + t2bc * n2cb + t3bc * n4bc);
-    s.e5i += denom * t1v1b * dx1c * (t1bc + n2bc + n4cb - (t3bc + n4bc + n2cb + n1bc + t2bc + n3cb) * 2
-                                     + (n3bc + t4bc + n1cb) * 4)
-           + denom * t1v1b * dc1c * (n1bc + n4bc + t1cb - (n2bc + n3bc + t2cb) * 2);
-    s.e5k += denom * t1v2b * dx2c * (n1bc + t2bc + t4cb - (n3bc + t4bc + t2cb + t1bc + n2bc + t3cb) * 2
-                                     + (t3bc + n4bc + t1cb) * 4)
-           + denom * t1v2b * dc2c * (t1bc + t4bc + n1cb - (t2bc + t3bc + n2cb) * 2);
-}
-
-// The same four forms with the denominator factored out of each, for callers that already hold
-// denom = -1/(e_b + e_c + eaijk) (shared by the mirrored positions (b,c) and (c,b)).  Equal to
-// tengy_term up to floating-point reassociation.
-__device__ __forceinline__ void tengy_term_factored(const double (&bc)[8], const double (&cb)[8], double denom,
-                                                    double t1v1b, double t1v2b, double dx1c, double dx2c,
-                                                    double dc1c, double dc2c, TengySums &s)
-{
-    const double n1bc = bc[0], n2bc = bc[1], n3bc = bc[2], n4bc = bc[3];
-    const double t1bc = bc[4], t2bc = bc[5], t3bc = bc[6], t4bc = bc[7];
-    const double n1cb = cb[0], n2cb = cb[1], n3cb = cb[2], n4cb = cb[3];
-    const double t1cb = cb[4], t2cb = cb[5], t3cb = cb[6], t4cb = cb[7];
-
-    const double a4i = (t1bc + n1cb + t2cb + n3bc + n4cb) * (t1bc - t2bc * 2 - t3bc * 2 + t4bc)
-                     - (n1bc + t1cb + n2cb + n3cb) * (t1bc * 2 - t2bc - t3bc + t4bc * 2)
-                     + 3 * (n1bc * (n1bc + n3cb + t4cb * 2) + n2bc * t2cb + n3bc * t4bc);
-    const double a4k = (n1bc + t1cb + n2cb + t3bc + t4cb) * (n1bc - n2bc * 2 - n3bc * 2 + n4bc)
-                     - (t1bc + n1cb + t2cb + t3cb) * (n1bc * 2 - n2bc - n3bc + n4bc * 2)
-                     + 3 * (t1bc * (t1bc + t3cb + n4cb * 2) + t2bc * n2cb + t3bc * n4bc);
-    const double f5i = t1bc + n2bc + n4cb - (t3bc + n4bc + n2cb + n1bc + t2bc + n3cb) * 2 + (n3bc + t4bc + n1cb) * 4;
-    const double g5i = n1bc + n4bc + t1cb - (n2bc + n3bc + t2cb) * 2;
-    const double f5k = n1bc + t2bc + t4cb - (n3bc + t4bc + t2cb + t1bc + n2bc + t3cb) * 2 + (t3bc + n4bc + t1cb) * 4;
-    const double g5k = t1bc + t4bc + n1cb - (t2bc + t3bc + n2cb) * 2;
-    s.e4i += denom * a4i;
-    s.e4k += denom * a4k;
-    s.e5i += denom * (t1v1b * (dx1c * f5i + dc1c * g5i));
-    s.e5k += denom * (t1v2b * (dx2c * f5k + dc2c * g5k));
-}
-
 // The terms of a position (b,c) and its mirror (c,b) together (BOTH = false: of (b,c) alone).  They share the
 // denominator, and the sums t2 + t3, t1 + t4, n2 + n3, n1 + n4 of each position enter both positions' forms, so a
-// pair costs about 135 FP64 instructions instead of the 200 of two tengy_term_factored calls (FP64 arithmetic
+// pair costs about 135 FP64 instructions; the forms written out twice cost 200 (FP64 arithmetic
 // is issued at half a warp instruction per clock per scheduler, on the same pipe as the MMAs).  vb, vc: the
-// per-index vectors at b and at c.  Equal to the forms above up to floating-point reassociation.
+// per-index vectors at b and at c.
 struct TengyIdx {
     double t1v1, t1v2, dx1, dx2, dc1, dc2;
 };

@@ -180,6 +180,7 @@ typedef struct sysbuf {
     int32_t *d_order;                /* fused/emulated processing order (trpdrv_processing_order) */
     int32_t *h_order;                /* its host copy (chunks of trpdrv_plan_upload_execute) */
     trpdrv_oz_system oz;             /* emulated form: digit slices and scales (device) */
+    int64_t *oz_job0;                /* emulated form: first entry of oz.jobs of each position */
     void *oz_maps;                   /* emulated form: tensor maps of oz.sa / oz.sb (host blob) */
     int64_t ntriples;                /* records: n_a * nt */
     int64_t nt;                      /* triples per a (this rank's share) */
@@ -263,6 +264,8 @@ static void plan_free(trpdrv_plan *p)
             if (b->oz.sb) cudaFree(b->oz.sb);
             if (b->oz.ea) cudaFree(b->oz.ea);
             if (b->oz.eb) cudaFree(b->oz.eb);
+            if (b->oz.jobs) cudaFree(b->oz.jobs);
+            free(b->oz_job0);
             free(b->oz_maps);
             if (b->partial) cudaFree(b->partial);
             if (b->rec) cudaFree(b->rec);
@@ -386,6 +389,29 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
             CUDA_TRY(cudaMalloc((void **)&z->sb, per * (size_t)nocc * nocc));
             CUDA_TRY(cudaMalloc((void **)&z->ea, sizeof(double) * rows * (size_t)nocc * (size_t)z->n_a));
             CUDA_TRY(cudaMalloc((void **)&z->eb, sizeof(double) * rows * (size_t)nocc * nocc));
+            /* the products of every record position; a position's first job: oz_job0 */
+            const int64_t nr = b->ntriples;
+            int32_t *jobs = (int32_t *)malloc(sizeof(int32_t) * (size_t)(2 * nr + 1));
+            b->oz_job0 = (int64_t *)malloc(sizeof(int64_t) * (size_t)(nr + 1));
+            if (!jobs || !b->oz_job0 || nr > INT32_MAX / 2) {
+                free(jobs);
+                return nr > INT32_MAX / 2 ? fail(TRPDRV_ERR_ARG, "system %d: more than 2^30 (a, triple) records", q)
+                                          : fail(TRPDRV_ERR_NOMEM, "host allocation failed");
+            }
+            int64_t nj = 0;
+            for (int64_t r = 0; r < nr; ++r) {
+                const int64_t t = r % b->nt;
+                const int pk = b->h_triples[b->h_order ? b->h_order[t] : t];
+                b->oz_job0[r] = nj;
+                jobs[nj++] = (int32_t)(r << 1);
+                if ((pk & 1023) != ((pk >> 20) & 1023)) jobs[nj++] = (int32_t)(r << 1 | 1);
+            }
+            b->oz_job0[nr] = nj;
+            cudaError_t je = cudaMalloc((void **)&z->jobs, sizeof(int32_t) * (size_t)(nj + 1));
+            if (je == cudaSuccess)
+                je = cudaMemcpy(z->jobs, jobs, sizeof(int32_t) * (size_t)nj, cudaMemcpyHostToDevice);
+            free(jobs);
+            CUDA_TRY(je);
             b->oz_maps = aligned_alloc(64, (trpdrv_oz_maps_bytes() + 63) & ~(size_t)63);
             if (!b->oz_maps) return fail(TRPDRV_ERR_NOMEM, "host allocation failed");
         }
@@ -423,7 +449,7 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
     CUDA_TRY(cudaMemset(p->d_tot, 0, sizeof(double) * 4 * (size_t)p->nsys));
     if (o->mode == TRPDRV_MODE_EMULATED) {
         p->fbuf_batch = o->batch > TUNE_MAX_BATCH ? o->batch : TUNE_MAX_BATCH;
-        p->fbuf_half = 8 * (size_t)p->fbuf_batch * maxv * maxv;
+        p->fbuf_half = 8 * (size_t)p->fbuf_batch * maxv * trpdrv_oz_ldf(maxv);
         CUDA_TRY(cudaMalloc((void **)&p->d_fbuf, sizeof(double) * 2 * p->fbuf_half));
         CUDA_TRY(cudaStreamCreateWithFlags(&p->aux_stream, cudaStreamNonBlocking));
         for (int h = 0; h < 2; ++h) {
@@ -820,8 +846,10 @@ static int emulated_batches(trpdrv_plan *p, const trpdrv_dev_system *d, const sy
             const int h = (int)(*bi & 1);
             double *fb = p->d_fbuf + (size_t)h * p->fbuf_half;
             if (n > 0 && *bi >= 2) CUDA_TRY(cudaStreamWaitEvent(st, p->ev_tengy[h], 0));  /* separate-launch readers */
-            LAUNCH_TRY(trpdrv_launch_oz_gemm(d, &b->oz, b->oz_maps, pos, n, fb, epos, en, efb, p->d_status, p->nsm,
-                                             st));
+            const int64_t j0 = n > 0 ? b->oz_job0[pos] : 0;
+            const int nj = n > 0 ? (int)(b->oz_job0[pos + n] - j0) : 0;
+            LAUNCH_TRY(trpdrv_launch_oz_gemm(d, &b->oz, b->oz_maps, pos, j0, nj, fb, epos, en, efb, p->d_status,
+                                             p->nsm, st));
             if (launches) *launches += 1;
             if (n == 0) break;
             epos = pos;
@@ -836,7 +864,9 @@ static int emulated_batches(trpdrv_plan *p, const trpdrv_dev_system *d, const sy
         const int h = (int)(*bi & 1);
         double *fb = p->d_fbuf + (size_t)h * p->fbuf_half;
         if (*bi >= 2) CUDA_TRY(cudaStreamWaitEvent(st, p->ev_tengy[h], 0));
-        LAUNCH_TRY(trpdrv_launch_oz_gemm(d, &b->oz, b->oz_maps, pos, n, fb, 0, 0, NULL, p->d_status, p->nsm, st));
+        LAUNCH_TRY(trpdrv_launch_oz_gemm(d, &b->oz, b->oz_maps, pos, b->oz_job0[pos],
+                                         (int)(b->oz_job0[pos + n] - b->oz_job0[pos]), fb, 0, 0, NULL, p->d_status,
+                                         p->nsm, st));
         CUDA_TRY(cudaEventRecord(p->ev_gemm[h], st));
         CUDA_TRY(cudaStreamWaitEvent(p->aux_stream, p->ev_gemm[h], 0));
         LAUNCH_TRY(trpdrv_launch_oz_tengy(d, pos, n, fb, 128, p->d_status, p->aux_stream));

@@ -80,7 +80,7 @@ int trpdrv_launch_wait_selftest(unsigned long long limit_ns, int *status, unsign
  * eb [nocc*nocc][2 nvir].  trpdrv_oz_prepare encodes the two tensor maps into a host blob of
  * trpdrv_oz_maps_bytes() bytes (64-byte aligned).  A batch is npos consecutive positions of the
  * system's processing order starting at pos0: the contraction kernel writes their f into
- * fbuf [npos][8][nvir][nvir] and the tengy kernel writes the sums of each 16-wide tile pair into
+ * fbuf [npos][8][nvir][trpdrv_oz_ldf(nvir)] and the tengy kernel writes the sums of each 16-wide tile pair into
  * one slot of the triple's items in `partial` (the other slots must be zero), for
  * trpdrv_launch_item_reduce.  *status as the fused kernels (bit 0 malformed entry, bit 1 a wait
  * ran out).  The contraction kernel is persistent: grid = CTAs (one per SM). */
@@ -90,24 +90,31 @@ typedef struct trpdrv_oz_system {
     int nocc, nvir, slices, dp, n_a;  /* n_a: a values swept; sa holds n_a * nocc planes */
     signed char *sa, *sb;
     double *ea, *eb;
+    int32_t *jobs;  /* the products of every position in order, position << 1 | group: group 0 (n: SA[i] SB[j,k])
+                       and, unless i == k, group 1 (t: SA[k] SB[j,i]); with i == k group 0 stores both */
 } trpdrv_oz_system;
+/* Doubles between the columns of f in a batch buffer: nvir rounded up to even (16-byte rows for TMA). */
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+static inline int trpdrv_oz_ldf(int nvir) { return nvir + (nvir & 1); }
 int trpdrv_oz_slices_supported(int slices);
 int trpdrv_oz_dp(int nocc, int nvir);
 size_t trpdrv_oz_maps_bytes(void);
 int trpdrv_oz_prepare(const trpdrv_oz_system *oz, void *maps_out);
 int trpdrv_launch_oz_slices(const trpdrv_dev_system *h_sys, const trpdrv_oz_system *oz, void *stream);
-/* Products of positions pos0 .. pos0 + npos - 1 into fbuf; enpos > 0 (requires
+/* Products oz->jobs[job0 .. job0 + njobs) (those of consecutive positions from pos0) into fbuf; enpos > 0 (requires
  * trpdrv_oz_fused_energy_supported(nvir)): the same launch's energy warps also compute the energies
- * of positions epos0 .. epos0 + enpos - 1, whose f an earlier launch stored at efbuf.  npos = 0 gives an
+ * of positions epos0 .. epos0 + enpos - 1, whose f an earlier launch stored at efbuf.  njobs = 0 gives an
  * energies-only launch. */
 int trpdrv_launch_oz_gemm(const trpdrv_dev_system *h_sys, const trpdrv_oz_system *oz, const void *maps,
-                          int64_t pos0, int npos, double *fbuf, int64_t epos0, int enpos, const double *efbuf,
-                          int *status, int grid, void *stream);
+                          int64_t pos0, int64_t job0, int njobs, double *fbuf, int64_t epos0, int enpos,
+                          const double *efbuf, int *status, int grid, void *stream);
 int trpdrv_oz_fused_energy_supported(int nvir);
-/* threads: 128 (what the plans launch) or 256.  Emulated plans launch the energies of one batch on a
- * second stream, ordered only after that batch's products.  Even nvir: the tiles
- * arrive by TMA (fbuf 16-byte aligned), with a bounded wait that sets *status bit 1 when it runs out;
- * odd nvir (or TRPDRV_OZ_TENGY_TMA=0): cp.async copies. */
+/* The energies as a launch of their own (odd nvir, or TRPDRV_OZ_FUSED_ENERGY=0).  threads: 128 (what the plans launch) or 256.
+ * The plans launch the energies of one batch on a second stream, ordered only after that batch's products.  The
+ * tiles arrive by TMA (fbuf 16-byte aligned), with a bounded wait that sets *status bit 1 when it runs out;
+ * with TRPDRV_OZ_TENGY_TMA=0 by cp.async. */
 int trpdrv_launch_oz_tengy(const trpdrv_dev_system *h_sys, int64_t pos0, int npos, const double *fbuf,
                            int threads, int *status, void *stream);
 int trpdrv_oz_init(void);

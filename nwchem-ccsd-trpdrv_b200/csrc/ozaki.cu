@@ -85,13 +85,14 @@ struct GemmParams {
     trpdrv_dev_system sys;   // fused energies: vectors, triples and energy slots of the system
     const double *ea, *eb;   // power-of-two scales per A row / B column
     const int32_t *triples, *order;
+    const int32_t *jobs;     // this batch's (position, group) products: position << 1 | group
     long long pos0, ntriples, nt;  // ntriples records = n_a * nt triples per a
-    double *fbuf;            // [batch][8][V][V]
+    double *fbuf;            // [batch][8][V][ldf]
     // fused energies: the energies of positions epos0 .. epos0 + enpos - 1, whose f an earlier launch
     // stored (at the fmap's base); unit u = tile pair u % np of position epos0 + u / np
     long long epos0;
     int enpos, np;
-    int V, O, nks, mtiles, ntiles, tiles;  // tiles = 2 * npos * mtiles * ntiles
+    int V, O, ldf, nks, mtiles, ntiles, tiles;  // tiles = jobs * mtiles * ntiles
     int *status;
 };
 
@@ -473,19 +474,20 @@ __device__ __forceinline__ void fused_energies(const GemmParams &P, double *park
 // contraction kernel (persistent: CTA b takes tiles b, b + grid, ...)
 // ------------------------------------------------------------------------------------------------
 struct Tile {
-    int ok, y, grp, planeA, planeB, m0, n0;
+    int ok, y, grp, same, planeA, planeB, m0, n0;  // y: batch position; same: i == k (the t group is the n group)
 };
 
 __device__ __forceinline__ Tile decode_tile(const GemmParams &P, int t)
 {
     Tile d;
     const int per = P.mtiles * P.ntiles;
-    d.y = t / per;
-    const int rem = t - d.y * per;
+    const int job = t / per, rem = t - job * per;
     d.m0 = (rem % P.mtiles) * BM;
     d.n0 = (rem / P.mtiles) * BN;
-    d.grp = d.y & 1;
-    const long long pos = P.pos0 + (d.y >> 1);  // a position over the records ([a][triple])
+    const int jb = P.jobs[job];
+    d.grp = jb & 1;
+    const long long pos = jb >> 1;  // a position over the records ([a][triple])
+    d.y = (int)(pos - P.pos0);
     // records < 2^31 (the host checks): 32-bit division, none for a single a
     const unsigned ai = (P.nt > 0 && pos >= P.nt) ? (unsigned)pos / (unsigned)P.nt : 0u;
     const long long tpos = pos - (long long)ai * P.nt;
@@ -493,6 +495,7 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams &P, int t)
     const int packed = (tt >= 0 && tt < P.nt) ? P.triples[tt] : -1;
     const int i = packed & 1023, j = (packed >> 10) & 1023, k = (packed >> 20) & 1023;
     d.ok = packed >= 0 && i < P.O && j < P.O && k < P.O;
+    d.same = i == k;
     d.planeA = (int)ai * P.O + (d.grp ? k : i);  // the A operands carry the a index
     d.planeB = j * P.O + (d.grp ? i : k);
     return d;
@@ -510,7 +513,9 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
     __shared__ __align__(8) unsigned long long full[C::STAGES], empty[C::STAGES], tfull[1], tempty[1], done[1], ubar[1];
     __shared__ unsigned tmem_sh;
     __shared__ double red[4 * NENG];
-    char *stages = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    // aligned by an offset, not by integer arithmetic on the pointer: the compiler then still knows that the park
+    // is shared memory
+    char *stages = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
     double *park = reinterpret_cast<double *>(stages + (size_t)C::STAGES * C::STAGE);  // 1024-byte aligned
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -628,7 +633,7 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
         const int qd = warp & 3, half = (warp - REC0) >> 2;
         constexpr int WC = BN / 2;  // columns per recombination warp
         const int V = P.V;
-        const size_t vv = (size_t)V * V;
+        const size_t vv = (size_t)V * P.ldf;
         int it = 0;
         for (int t = blockIdx.x; t < P.tiles; t += gridDim.x, ++it) {
             const Tile d = decode_tile(P, t);
@@ -673,16 +678,17 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
             if (d.ok && r < 2 * V) {
                 const double sa = P.ea[(size_t)d.planeA * 2 * V + r];
                 const int rh = r >= V ? 1 : 0, b = r - rh * V;
-                double *fj = P.fbuf + (size_t)(d.y >> 1) * 8 * vv + (size_t)d.grp * 4 * vv;
+                double *fj = P.fbuf + (size_t)d.y * 8 * vv + (size_t)d.grp * 4 * vv;
                 const double *eb = P.eb + (size_t)d.planeB * 2 * V;
 #pragma unroll
                 for (int c = 0; c < WC; ++c) {
                     const int col = d.n0 + half * WC + c;
                     if (col < 2 * V) {
                         const int ch = col >= V ? 1 : 0, cc = col - ch * V;
-                        double *dst = fj + (size_t)(rh + 2 * ch) * vv + b + (size_t)cc * V;
+                        double *dst = fj + (size_t)(rh + 2 * ch) * vv + b + (size_t)cc * P.ldf;
                         const double val = acc[c] * sa * __ldg(eb + col);
                         __stcs(dst, val);  // evict-first: read once, by a later launch; keeps the digits in L2
+                        if (d.same) __stcs(dst + 4 * vv, val);
                     }
                 }
             }
@@ -823,8 +829,8 @@ template <int TNTHREAD>
 __device__ __forceinline__ void tengy_park_cpasync(const TengyParams &P, const TengyItem &it, double *park)
 {
     constexpr int TP = TW + 1, TILE = TW * TP;
-    const int nvir = P.sys.nvir;
-    const size_t lnvv = (size_t)nvir * nvir;
+    const int nvir = P.sys.nvir, ldf = trpdrv_oz_ldf(nvir);
+    const size_t lnvv = (size_t)nvir * ldf;
     const double *f = P.fbuf + (size_t)it.y * 8 * lnvv;
     const int ntiles = it.diag ? 8 : 16;
     for (int idx = threadIdx.x; idx < ntiles * TW * TW; idx += TNTHREAD) {
@@ -832,7 +838,7 @@ __device__ __forceinline__ void tengy_park_cpasync(const TengyParams &P, const T
         const int o = tile >> 3, xf = tile & 7;
         const int row = (o ? it.c0 : it.b0) + r, col = (o ? it.b0 : it.c0) + q;
         const bool ok = row < nvir && col < nvir;
-        cp_async_8(park + tile * TILE + r * TP + q, ok ? f + (size_t)xf * lnvv + row + (size_t)col * nvir : f, ok);
+        cp_async_8(park + tile * TILE + r * TP + q, ok ? f + (size_t)xf * lnvv + row + (size_t)col * ldf : f, ok);
     }
     cp_async_commit();
     cp_async_wait<0>();
@@ -866,8 +872,7 @@ oz_tengy_kernel(const __grid_constant__ TengyParams P, int np, int npos)
     extern __shared__ __align__(16) double tsmem[];
     __shared__ double red[4 * (TNTHREAD / 32)];
     __shared__ __align__(8) unsigned long long tbar[1];
-    double *park = TMA ? reinterpret_cast<double *>((reinterpret_cast<uintptr_t>(tsmem) + 1023) & ~(uintptr_t)1023)
-                       : tsmem;
+    double *park = TMA ? tsmem + ((1024u - (saddr(tsmem) & 1023u)) & 1023u) / sizeof(double) : tsmem;
     if (TMA) {
         if (threadIdx.x == 0) {
             mbar_init(tbar, 1);
@@ -957,13 +962,14 @@ static int make_map_i8(CUtensorMap *m, const signed char *base, unsigned long lo
 
 // 3-D map over the f of a batch for the TMA form of the energies: dims {nvir rows (contiguous), nvir
 // columns, planes}, box {16, 16, 8} (the eight f of one triple), 128-byte swizzle, zero fill past nvir.
-// Needs even nvir (row pitch a multiple of 16 bytes) and a 16-byte aligned base.
+// Columns are trpdrv_oz_ldf(nvir) doubles apart (a multiple of 16 bytes); needs a 16-byte aligned base.
 static int make_map_f64(CUtensorMap *m, const double *base, int nvir, unsigned long long planes)
 {
     PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
-    if (!fn || nvir < 2 || (nvir & 1) || (reinterpret_cast<uintptr_t>(base) & 15)) return 1;
+    if (!fn || (reinterpret_cast<uintptr_t>(base) & 15)) return 1;
     const cuuint64_t dims[3] = {(cuuint64_t)nvir, (cuuint64_t)nvir, planes};
-    const cuuint64_t strides[2] = {(cuuint64_t)nvir * sizeof(double), (cuuint64_t)nvir * nvir * sizeof(double)};
+    const cuuint64_t ldf = (cuuint64_t)trpdrv_oz_ldf(nvir);
+    const cuuint64_t strides[2] = {ldf * sizeof(double), ldf * nvir * sizeof(double)};
     const cuuint32_t box[3] = {(cuuint32_t)TW, (cuuint32_t)TW, 8};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(base), dims, strides, box, estr,
@@ -1010,7 +1016,7 @@ extern "C" int trpdrv_oz_slices_supported(int slices) { return slices >= TRPDRV_
 
 extern "C" int trpdrv_oz_dp(int nocc, int nvir) { return ((nvir + nocc) + 31) / 32 * 32; }
 
-// Energies inside the contraction launch (the default for even nvir: the f tiles are read by TMA): the
+// Energies inside the contraction launch (the default for even nvir; the f tiles are read by TMA): the
 // kernel's energy warps compute the previous batch's energies while the tensor cores run this batch's
 // products; 1.3 % faster than the separate energy launch at (40, 300), 3.4 % at (30, 400), 7 slices.
 // TRPDRV_OZ_FUSED_ENERGY=0 (read at each call) selects the separate launch for every nvir.
@@ -1061,10 +1067,10 @@ extern "C" int trpdrv_launch_oz_slices(const trpdrv_dev_system *h_sys, const trp
 }
 
 extern "C" int trpdrv_launch_oz_gemm(const trpdrv_dev_system *h_sys, const trpdrv_oz_system *oz, const void *maps,
-                                     int64_t pos0, int npos, double *fbuf, int64_t epos0, int enpos,
+                                     int64_t pos0, int64_t job0, int njobs, double *fbuf, int64_t epos0, int enpos,
                                      const double *efbuf, int *status, int grid, void *stream)
 {
-    if (npos < 0 || enpos < 0 || (npos == 0 && enpos == 0)) return 0;
+    if (njobs < 0 || enpos < 0 || (njobs == 0 && enpos == 0)) return 0;
     oz::GemmParams P;
     memset(&P, 0, sizeof(P));
     if (enpos > 0) {  // energies of an earlier launch's positions, fused into this one
@@ -1083,16 +1089,18 @@ extern "C" int trpdrv_launch_oz_gemm(const trpdrv_dev_system *h_sys, const trpdr
     P.eb = oz->eb;
     P.triples = h_sys->triples;
     P.order = h_sys->order;
+    P.jobs = oz->jobs + job0;
     P.pos0 = pos0;
     P.ntriples = h_sys->ntriples;
     P.nt = h_sys->nt;
     P.fbuf = fbuf;
     P.V = oz->nvir;
     P.O = oz->nocc;
+    P.ldf = trpdrv_oz_ldf(oz->nvir);
     P.nks = oz->dp / oz::KSTEP;
     P.mtiles = (2 * oz->nvir + oz::BM - 1) / oz::BM;
     P.ntiles = (2 * oz->nvir + oz::BN - 1) / oz::BN;
-    P.tiles = 2 * npos * P.mtiles * P.ntiles;
+    P.tiles = njobs * P.mtiles * P.ntiles;
     P.status = status;
     const long long work = P.tiles > 0 ? P.tiles : (long long)P.np * enpos;  // an energies-only launch
     if (grid < 1) grid = 1;
