@@ -558,16 +558,8 @@ __device__ __forceinline__ void prefetch_epilogue(const ItemCtx &cx, int lane)
 {
     if (lane >= 28) return;
     const int v = lane >> 2, r = (lane >> 1) & 1, l = lane & 1;
-    const double *base;
-    switch (v) {
-    case 0: base = cx.eorb + cx.ncor + cx.nocc; break;
-    case 1: base = cx.t1v1; break;
-    case 2: base = cx.t1v2; break;
-    case 3: base = cx.dintx1; break;
-    case 4: base = cx.dintx2; break;
-    case 5: base = cx.dintc1; break;
-    default: base = cx.dintc2; break;
-    }
+    // the seven pointers at the head of the context (a switch over them would run as seven divergent branches)
+    const double *base = (&cx.eorb)[v] + (v == 0 ? cx.ncor + cx.nocc : 0);
     const int idx = (r ? cx.c0 : cx.b0) + 16 * l;
     if (idx < cx.nvir) asm volatile("prefetch.global.L1 [%0];" ::"l"(base + idx));
 }
@@ -641,7 +633,10 @@ struct Item {
     __device__ __forceinline__ int zb(int fam) const { return fam ? zb1 : zb0; }
 };
 
-__device__ __forceinline__ Item decode_item(const trpdrv_dev_system *__restrict__ sys, int nsys, long long item)
+// pair_major: a system's items run pair by pair, those of two tiles (twice the products) before the diagonal ones, each
+// over all triples: small launches then end with the small items on every SM.
+__device__ __forceinline__ Item decode_item(const trpdrv_dev_system *__restrict__ sys, int nsys, long long item,
+                                            int pair_major)
 {
     Item it;
     int s = 0;
@@ -650,19 +645,31 @@ __device__ __forceinline__ Item decode_item(const trpdrv_dev_system *__restrict_
     it.S = &S;
     it.s = s;
     const long long local = item - S.item_begin;
-    const long long qpos = local / S.npairs;  // processing position over the system's records
-    const int p = (int)(local - qpos * S.npairs);
+    long long qpos;  // processing position over the system's records
+    int B = 0, C;
+    if (pair_major && S.ntriples > 0) {
+        int rem = (int)(local / S.ntriples);
+        qpos = local - (long long)rem * S.ntriples;
+        const int noff = S.npairs - S.nb;
+        if (rem >= noff) {
+            B = C = rem - noff;
+        } else {
+            while (B < S.nb && rem >= S.nb - 1 - B) rem -= S.nb - 1 - B++;
+            C = B + 1 + rem;
+        }
+    } else {
+        qpos = local / S.npairs;
+        int rem = (int)(local - qpos * S.npairs);
+        while (B < S.nb && rem >= S.nb - B) rem -= S.nb - B++;
+        C = B + rem;
+    }
+    const int p = B * S.nb - B * (B - 1) / 2 + C - B;  // the pair's slot within the record
     // a index (records are [a][triple], fewer than 2^31: the host checks); no division for a single a
     const long long ai = (S.nt > 0 && qpos >= S.nt) ? (long long)((unsigned)qpos / (unsigned)S.nt) : 0;
     const long long tpos = qpos - ai * S.nt;
     const long long tt = (S.order && local >= 0 && qpos < S.ntriples) ? (long long)S.order[tpos] : tpos;
     it.own = (ai * S.nt + tt) * S.npairs + p;  // energies go to the record's own items
-    int B = 0, rem = p;
-    while (B < S.nb && rem >= S.nb - B) {
-        rem -= S.nb - B;
-        ++B;
-    }
-    const int C = B + rem, O = S.nocc;
+    const int O = S.nocc;
     it.B = B;
     it.C = C;
     it.ai = (int)ai;
@@ -889,7 +896,7 @@ struct CpStage {
 };
 
 template <class Stage>
-__device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ sys, int nsys, long long total,
+__device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ sys, int nsys, long long total, int pair_major,
                                          unsigned long long *counter, int *status, Stage &sg, char *stages,
                                          unsigned long long *full, unsigned long long *empty, ItemCtx *ring,
                                          long long *tickets, unsigned long long *tbar, int pw, int lane)
@@ -914,7 +921,7 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
                 if (item >= total) break;
                 if (lane == 0) next = (long long)atomicAdd(counter, 1ULL);  // the following ticket, early
                 next = __shfl_sync(FULL, next, 0);
-                it = decode_item(sys, nsys, item);
+                it = decode_item(sys, nsys, item, pair_major);
                 if (!it.skip) break;
             }
             if (lane == 0) {
@@ -924,7 +931,7 @@ __device__ __forceinline__ void producer(const trpdrv_dev_system *__restrict__ s
         } else {
             if (!mbar_wait(&tbar[tq], (unsigned)((n / TICKETS) & 1), status)) return;
             item = tickets[tq];
-            if (item < total) it = decode_item(sys, nsys, item);
+            if (item < total) it = decode_item(sys, nsys, item, pair_major);
         }
         ItemCtx &cx = ring[n % RING];
         if (item >= total || !it.ok) {
@@ -1018,8 +1025,8 @@ template <> struct StageParam<2> : NoParam {};
 // STG: operand staging, 0 = TMA, 1 / 2 = cp.async with 8 / 16-byte copies.  KS: FP64 MMA shape.
 template <int KS, int STG>
 __global__ void __launch_bounds__(NTHREAD, 1)
-fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long total, unsigned long long *counter,
-             int *status, const __grid_constant__ StageParam<STG> param)
+fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long total, int pair_major,
+             unsigned long long *counter, int *status, const __grid_constant__ StageParam<STG> param)
 {
     extern __shared__ char smem_raw[];
     __shared__ __align__(8) unsigned long long full[STAGES], empty[STAGES], tbar[TICKETS];
@@ -1047,11 +1054,11 @@ fused_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, long long tota
         if constexpr (STG == 0) {
             TmaStage sg;
             sg.maps = &param.maps;
-            producer(sys, nsys, total, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
+            producer(sys, nsys, total, pair_major, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
                             lane);
         } else {
             CpStage<STG> sg;
-            producer(sys, nsys, total, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
+            producer(sys, nsys, total, pair_major, counter, status, sg, stages, full, empty, ring, tickets, tbar, warp - NCW,
                             lane);
             asm volatile("cp.async.wait_all;" ::: "memory");
         }
@@ -1260,16 +1267,16 @@ extern "C" int trpdrv_tma_prepare(const trpdrv_dev_system *h_sys, int nsys, void
 }
 
 template <int KS, int STG>
-static int launch_kernel(const trpdrv_dev_system *d_sys, int nsys, int64_t total, unsigned long long *counter,
-                         int *status, int grid, const tma::StageParam<STG> &param, void *stream)
+static int launch_kernel(const trpdrv_dev_system *d_sys, int nsys, int64_t total, int pair_major,
+                         unsigned long long *counter, int *status, int grid, const tma::StageParam<STG> &param, void *stream)
 {
     tma::fused_kernel<KS, STG><<<grid, tma::NTHREAD, tma::SMEM_BYTES, (cudaStream_t)stream>>>(
-        d_sys, nsys, total, counter, status, param);
+        d_sys, nsys, total, pair_major, counter, status, param);
     return (int)cudaGetLastError();
 }
 
 extern "C" int trpdrv_launch_fused_tma(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items,
-                                       unsigned long long *counter, int *status, int grid, const void *maps,
+                                       int pair_major, unsigned long long *counter, int *status, int grid, const void *maps,
                                        int mma_k, void *stream)
 {
     if (grid <= 0 || total_items <= 0) return 0;
@@ -1277,14 +1284,14 @@ extern "C" int trpdrv_launch_fused_tma(const trpdrv_dev_system *d_sys, int nsys,
     if (nsys > TRPDRV_TMA_MAX_SYSTEMS) return (int)cudaErrorInvalidValue;
     const tma::StageParam<0> &m = *static_cast<const tma::StageParam<0> *>(maps);
     if (mma_k == 16)
-        return launch_kernel<16, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
+        return launch_kernel<16, 0>(d_sys, nsys, total_items, pair_major, counter, status, grid, m, stream);
     if (mma_k == 8)
-        return launch_kernel<8, 0>(d_sys, nsys, total_items, counter, status, grid, m, stream);
+        return launch_kernel<8, 0>(d_sys, nsys, total_items, pair_major, counter, status, grid, m, stream);
     return (int)cudaErrorInvalidValue;
 }
 
 extern "C" int trpdrv_launch_fused(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items,
-                                   unsigned long long *counter, int *status, int grid, int vec2, int mma_k,
+                                   int pair_major, unsigned long long *counter, int *status, int grid, int vec2, int mma_k,
                                    void *stream)
 {
     if (grid <= 0 || total_items <= 0) return 0;
@@ -1292,10 +1299,10 @@ extern "C" int trpdrv_launch_fused(const trpdrv_dev_system *d_sys, int nsys, int
     const tma::StageParam<1> p1 = {};
     const tma::StageParam<2> p2 = {};
     if (mma_k == 4)
-        return vec2 ? launch_kernel<4, 2>(d_sys, nsys, total_items, counter, status, grid, p2, stream)
-                    : launch_kernel<4, 1>(d_sys, nsys, total_items, counter, status, grid, p1, stream);
-    return vec2 ? launch_kernel<8, 2>(d_sys, nsys, total_items, counter, status, grid, p2, stream)
-                : launch_kernel<8, 1>(d_sys, nsys, total_items, counter, status, grid, p1, stream);
+        return vec2 ? launch_kernel<4, 2>(d_sys, nsys, total_items, pair_major, counter, status, grid, p2, stream)
+                    : launch_kernel<4, 1>(d_sys, nsys, total_items, pair_major, counter, status, grid, p1, stream);
+    return vec2 ? launch_kernel<8, 2>(d_sys, nsys, total_items, pair_major, counter, status, grid, p2, stream)
+                : launch_kernel<8, 1>(d_sys, nsys, total_items, pair_major, counter, status, grid, p1, stream);
 }
 
 extern "C" int trpdrv_launch_wait_selftest(unsigned long long limit_ns, int *status, unsigned long long *elapsed_ns,

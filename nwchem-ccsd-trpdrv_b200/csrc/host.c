@@ -196,9 +196,11 @@ struct trpdrv_plan {
     cudaStream_t stream;
     sysbuf *s;
     trpdrv_dev_system *h_dev, *d_dev;
-    unsigned long long *d_counter;
+    unsigned long long *d_counter; /* work tickets and, 8 bytes on, the status word: cleared together */
     int *d_status;
-    double *d_tot;
+    double *d_bsum;   /* block sums of the totals */
+    unsigned *d_done; /* finished blocks per system */
+    double *h_res;    /* pinned: totals per system (emp4 hi, lo, emp5 hi, lo), then the status word */
     int64_t total_items;
     double *d_f, *d_bpart; /* plain form: f and energy partials of one batch of triples */
     unsigned *d_tcount;
@@ -277,8 +279,9 @@ static void plan_free(trpdrv_plan *p)
     free(p->tma_maps);
     if (p->d_dev) cudaFree(p->d_dev);
     if (p->d_counter) cudaFree(p->d_counter);
-    if (p->d_status) cudaFree(p->d_status);
-    if (p->d_tot) cudaFree(p->d_tot);
+    if (p->d_bsum) cudaFree(p->d_bsum);
+    if (p->d_done) cudaFree(p->d_done);
+    if (p->h_res) cudaFreeHost(p->h_res);
     if (p->d_f) cudaFree(p->d_f);
     if (p->d_fbuf) cudaFree(p->d_fbuf);
     for (int h = 0; h < 2; ++h) {
@@ -442,11 +445,14 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
     p->total_items = item;
     p->vec2 = even;
     CUDA_TRY(cudaMalloc((void **)&p->d_dev, sizeof(trpdrv_dev_system) * (size_t)p->nsys));
-    CUDA_TRY(cudaMalloc((void **)&p->d_counter, sizeof(unsigned long long)));
-    CUDA_TRY(cudaMalloc((void **)&p->d_status, sizeof(int)));
-    CUDA_TRY(cudaMemset(p->d_status, 0, sizeof(int)));
-    CUDA_TRY(cudaMalloc((void **)&p->d_tot, sizeof(double) * 4 * (size_t)p->nsys));
-    CUDA_TRY(cudaMemset(p->d_tot, 0, sizeof(double) * 4 * (size_t)p->nsys));
+    CUDA_TRY(cudaMalloc((void **)&p->d_counter, 2 * sizeof(unsigned long long)));
+    CUDA_TRY(cudaMemset(p->d_counter, 0, 2 * sizeof(unsigned long long)));
+    p->d_status = (int *)(p->d_counter + 1);
+    CUDA_TRY(cudaMalloc((void **)&p->d_bsum, sizeof(double) * 4 * TRPDRV_FINISH_BLOCKS * (size_t)p->nsys));
+    CUDA_TRY(cudaMalloc((void **)&p->d_done, sizeof(unsigned) * (size_t)p->nsys));
+    CUDA_TRY(cudaMemset(p->d_done, 0, sizeof(unsigned) * (size_t)p->nsys));
+    CUDA_TRY(cudaMallocHost((void **)&p->h_res, sizeof(double) * (4 * (size_t)p->nsys + 1)));
+    memset(p->h_res, 0, sizeof(double) * (4 * (size_t)p->nsys + 1));
     if (o->mode == TRPDRV_MODE_EMULATED) {
         p->fbuf_batch = o->batch > TUNE_MAX_BATCH ? o->batch : TUNE_MAX_BATCH;
         p->fbuf_half = 8 * (size_t)p->fbuf_batch * maxv * trpdrv_oz_ldf(maxv);
@@ -796,31 +802,39 @@ int trpdrv_plan_bind_device(trpdrv_plan *p, const trpdrv_system *dev)
     return plan_publish(p);
 }
 
+/* The records and totals of everything enqueued before on `st`, the totals straight into p->h_res. */
+static int enqueue_finish(trpdrv_plan *p, cudaStream_t st, int64_t *launches)
+{
+    if (p->opt.mode != TRPDRV_MODE_PLAIN) {
+        LAUNCH_TRY(trpdrv_launch_records(p->h_dev, p->d_dev, p->nsys, st));
+        if (launches) ++*launches;
+    }
+    LAUNCH_TRY(trpdrv_launch_totals(p->h_dev, p->d_dev, p->nsys, p->d_bsum, p->d_done, p->d_status, p->h_res, st));
+    if (launches) ++*launches;
+    return TRPDRV_OK;
+}
+
 static int enqueue_fused(trpdrv_plan *p, cudaStream_t st, int capturing)
 {
     int64_t launches = 0;
-    CUDA_TRY(cudaMemsetAsync(p->d_counter, 0, sizeof(unsigned long long), st));
-    CUDA_TRY(cudaMemsetAsync(p->d_status, 0, sizeof(int), st));
-    CUDA_TRY(cudaMemsetAsync(p->d_tot, 0, sizeof(double) * 4 * (size_t)p->nsys, st));
+    CUDA_TRY(cudaMemsetAsync(p->d_counter, 0, 2 * sizeof(unsigned long long), st)); /* and the status word */
     CUDA_TRY(cudaEventRecordWithFlags(p->ev0, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
+    /* few items per SM: the large ones first.  Inputs this small stay in L2 whatever the order.  (10, 60), 11 items
+     * an SM: 133 -> 125 us; (4, 300), 15 an SM: 511 -> 490 us; at 64 and more the two orders time the same */
+    const int pair_major = p->total_items <= 64 * (int64_t)p->nsm;
     if (p->total_items > 0) {
         for (int q = 0; q < p->nsys; ++q)
             if (p->h_dev[q].ntriples > 0) TRY(pad_refill(p, q, 1, 0, p->s[q].shape.nocc, st, &launches));
         if (p->use_tma)
-            LAUNCH_TRY(trpdrv_launch_fused_tma(p->d_dev, p->nsys, p->total_items, p->d_counter, p->d_status,
-                                               p->grid_tma, p->tma_maps, p->tma_mma_k, st));
+            LAUNCH_TRY(trpdrv_launch_fused_tma(p->d_dev, p->nsys, p->total_items, pair_major, p->d_counter,
+                                               p->d_status, p->grid_tma, p->tma_maps, p->tma_mma_k, st));
         else
-            LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, p->total_items, p->d_counter, p->d_status, p->grid,
+            LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, p->total_items, pair_major, p->d_counter, p->d_status, p->grid,
                                            p->vec2 || p->padded, p->opt.mma_k, st));
         ++launches;
     }
     CUDA_TRY(cudaEventRecordWithFlags(p->ev1, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
-    for (int q = 0; q < p->nsys; ++q) {
-        if (p->h_dev[q].ntriples <= 0) continue;
-        LAUNCH_TRY(trpdrv_launch_item_reduce(&p->h_dev[q], st));
-        LAUNCH_TRY(trpdrv_launch_system_reduce(p->s[q].rec, p->s[q].d_triples, p->s[q].ntriples, p->s[q].nt, p->d_tot + 4 * q, st));
-        launches += 2;
-    }
+    TRY(enqueue_finish(p, st, &launches));
     p->last_launches = launches;
     return TRPDRV_OK;
 }
@@ -890,7 +904,6 @@ static int enqueue_emulated(trpdrv_plan *p, cudaStream_t st, int capturing)
 {
     int64_t launches = 0, bi = 0;
     CUDA_TRY(cudaMemsetAsync(p->d_status, 0, sizeof(int), st));
-    CUDA_TRY(cudaMemsetAsync(p->d_tot, 0, sizeof(double) * 4 * (size_t)p->nsys, st));
     CUDA_TRY(cudaEventRecordWithFlags(p->ev0, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
     for (int q = 0; q < p->nsys; ++q) {
         const trpdrv_dev_system *d = &p->h_dev[q];
@@ -902,12 +915,7 @@ static int enqueue_emulated(trpdrv_plan *p, cudaStream_t st, int capturing)
     }
     TRY(emulated_join(p, st, bi));
     CUDA_TRY(cudaEventRecordWithFlags(p->ev1, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
-    for (int q = 0; q < p->nsys; ++q) {
-        if (p->h_dev[q].ntriples <= 0) continue;
-        LAUNCH_TRY(trpdrv_launch_item_reduce(&p->h_dev[q], st));
-        LAUNCH_TRY(trpdrv_launch_system_reduce(p->s[q].rec, p->s[q].d_triples, p->s[q].ntriples, p->s[q].nt, p->d_tot + 4 * q, st));
-        launches += 2;
-    }
+    TRY(enqueue_finish(p, st, &launches));
     p->last_launches = launches;
     return TRPDRV_OK;
 }
@@ -920,7 +928,6 @@ static int enqueue_device(trpdrv_plan *p, cudaStream_t st, int capturing)
 static int enqueue_plain(trpdrv_plan *p, cudaStream_t st)
 {
     int64_t launches = 0;
-    CUDA_TRY(cudaMemsetAsync(p->d_tot, 0, sizeof(double) * 4 * (size_t)p->nsys, st));
     CUDA_TRY(cudaEventRecord(p->ev0, st));
     for (int q = 0; q < p->nsys; ++q) {
         const sysbuf *b = &p->s[q];
@@ -932,11 +939,7 @@ static int enqueue_plain(trpdrv_plan *p, cudaStream_t st)
         }
     }
     CUDA_TRY(cudaEventRecord(p->ev1, st));
-    for (int q = 0; q < p->nsys; ++q) {
-        if (p->s[q].ntriples <= 0) continue;
-        LAUNCH_TRY(trpdrv_launch_system_reduce(p->s[q].rec, p->s[q].d_triples, p->s[q].ntriples, p->s[q].nt, p->d_tot + 4 * q, st));
-        ++launches;
-    }
+    TRY(enqueue_finish(p, st, &launches));
     p->last_launches = launches;
     return TRPDRV_OK;
 }
@@ -1164,7 +1167,6 @@ int trpdrv_plan_upload_execute(trpdrv_plan *p, const trpdrv_system *host, int ch
     if (rc == TRPDRV_OK)
         for (int c = 0; c < nsp; ++c) p->h_chunk_first[c] = (unsigned long long)sp[c].first;
     STEP_CUDA(cudaMemsetAsync(p->d_status, 0, sizeof(int), p->stream));
-    STEP_CUDA(cudaMemsetAsync(p->d_tot, 0, sizeof(double) * 4 * (size_t)p->nsys, p->stream));
     if (nsp > 0)
         STEP_CUDA(cudaMemcpyAsync(p->d_chunk_first, p->h_chunk_first, sizeof(unsigned long long) * (size_t)nsp,
                                   cudaMemcpyHostToDevice, p->stream));
@@ -1193,23 +1195,15 @@ int trpdrv_plan_upload_execute(trpdrv_plan *p, const trpdrv_system *host, int ch
         const int cap = p->use_tma ? p->grid_tma : p->grid;
         const int grid = (int64_t)cap < n ? cap : (int)n;
         if (n <= 0 || rc != TRPDRV_OK) continue;
-        int e = p->use_tma ? trpdrv_launch_fused_tma(p->d_dev, p->nsys, sp[c].end, p->d_chunk_first + c, p->d_status,
+        int e = p->use_tma ? trpdrv_launch_fused_tma(p->d_dev, p->nsys, sp[c].end, 0, p->d_chunk_first + c, p->d_status,
                                                      grid, p->tma_maps, p->tma_mma_k, p->stream)
-                           : trpdrv_launch_fused(p->d_dev, p->nsys, sp[c].end, p->d_chunk_first + c, p->d_status,
+                           : trpdrv_launch_fused(p->d_dev, p->nsys, sp[c].end, 0, p->d_chunk_first + c, p->d_status,
                                                  grid, p->vec2 || p->padded, p->opt.mma_k, p->stream);
         if (e) rc = fail(TRPDRV_ERR_CUDA, "fused launch of span %d: %s", c, cudaGetErrorString((cudaError_t)e));
         ++launches;
     }
     STEP_CUDA(cudaEventRecord(p->ev1, p->stream));
-    for (int q = 0; q < p->nsys && rc == TRPDRV_OK; ++q) {
-        if (p->h_dev[q].ntriples <= 0) continue;
-        int e = trpdrv_launch_item_reduce(&p->h_dev[q], p->stream);
-        if (!e)
-            e = trpdrv_launch_system_reduce(p->s[q].rec, p->s[q].d_triples, p->s[q].ntriples, p->s[q].nt,
-                                            p->d_tot + 4 * q, p->stream);
-        if (e) rc = fail(TRPDRV_ERR_CUDA, "reduction launch: %s", cudaGetErrorString((cudaError_t)e));
-        launches += 2;
-    }
+    STEP(enqueue_finish(p, p->stream, &launches));
     if (user) {
         STEP_CUDA(cudaEventRecord(p->ev_out, p->stream));
         STEP_CUDA(cudaStreamWaitEvent(user, p->ev_out, 0));
@@ -1230,8 +1224,7 @@ static int plan_wait(trpdrv_plan *p)
     CUDA_TRY(cudaSetDevice(p->device));
     CUDA_TRY(cudaStreamSynchronize(p->last_stream ? p->last_stream : p->stream));
     p->last_stream = NULL; /* the job is done: the caller may now destroy its stream */
-    int status = 0;
-    CUDA_TRY(cudaMemcpy(&status, p->d_status, sizeof(int), cudaMemcpyDeviceToHost));
+    const int status = (int)p->h_res[4 * p->nsys];
     if (status & 2) return fail(TRPDRV_ERR_DEVICE, "a fused-kernel pipeline wait ran out of time");
     if (status) return fail(TRPDRV_ERR_DEVICE, "a device kernel rejected a malformed work-queue entry");
     return TRPDRV_OK;
@@ -1241,18 +1234,11 @@ int trpdrv_plan_energies(trpdrv_plan *p, double *emp4, double *emp5)
 {
     if (!p) return fail(TRPDRV_ERR_ARG, "NULL plan");
     TRY(plan_wait(p));
-    double *tot = (double *)malloc(sizeof(double) * 4 * (size_t)p->nsys);
-    if (!tot) return fail(TRPDRV_ERR_NOMEM, "host allocation failed");
-    cudaError_t e = cudaMemcpy(tot, p->d_tot, sizeof(double) * 4 * (size_t)p->nsys, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) {
-        free(tot);
-        return fail(TRPDRV_ERR_CUDA, "energy copy: %s", cudaGetErrorString(e));
-    }
     for (int q = 0; q < p->nsys; ++q) {
-        if (emp4) emp4[q] = tot[4 * q + 0] + tot[4 * q + 1];
-        if (emp5) emp5[q] = tot[4 * q + 2] + tot[4 * q + 3];
+        const double *tot = p->h_res + 4 * q;
+        if (emp4) emp4[q] = tot[0] + tot[1];
+        if (emp5) emp5[q] = tot[2] + tot[3];
     }
-    free(tot);
     return TRPDRV_OK;
 }
 
@@ -1491,10 +1477,10 @@ static int tune_time(trpdrv_plan *p, const trpdrv_tune_candidate *c, double *est
                 CUDA_TRY(cudaStreamSynchronize(st)); /* `first` is a host stack value */
                 CUDA_TRY(cudaEventRecord(p->ev0, st));
                 if (c->staging == 2)
-                    LAUNCH_TRY(trpdrv_launch_fused_tma(p->d_dev, p->nsys, d->item_begin + sample, p->d_counter,
+                    LAUNCH_TRY(trpdrv_launch_fused_tma(p->d_dev, p->nsys, d->item_begin + sample, 0, p->d_counter,
                                                        p->d_status, grid, p->tma_maps, c->mma_k, st));
                 else
-                    LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, d->item_begin + sample, p->d_counter,
+                    LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, d->item_begin + sample, 0, p->d_counter,
                                                    p->d_status, grid, p->vec2 || p->padded, c->mma_k, st));
                 CUDA_TRY(cudaEventRecord(p->ev1, st));
                 TRY(tune_elapsed(p, &ms));
@@ -1556,9 +1542,12 @@ static int tune_sample_records(trpdrv_plan *p, double **host)
         int64_t bi = 0;
         TRY(emulated_batches(p, d, b, 0, n, p->opt.batch, st, &bi, NULL));
         TRY(emulated_join(p, st, bi));
-        LAUNCH_TRY(trpdrv_launch_item_reduce(d, st));
-        CUDA_TRY(cudaMemcpyAsync(host[q], b->rec, sizeof(double) * 4 * (size_t)b->ntriples, cudaMemcpyDeviceToHost, st));
     }
+    TRY(enqueue_finish(p, st, NULL));
+    for (int q = 0; q < p->nsys; ++q)
+        if (p->s[q].ntriples > 0)
+            CUDA_TRY(cudaMemcpyAsync(host[q], p->s[q].rec, sizeof(double) * 4 * (size_t)p->s[q].ntriples,
+                                     cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     return TRPDRV_OK;
 }

@@ -47,7 +47,8 @@ typedef struct trpdrv_dev_system {
 
 /* Fused persistent kernel (fused_tma.cu): grid CTAs (one per SM) pull (triple, tile pair) items from
  * *counter (must be 0 at launch) and write per-item energies.  *status bit 0: malformed queue entry; bit 1: a
- * pipeline wait ran out.  Two stagings of the operands feed the same MMA loop:
+ * pipeline wait ran out.  pair_major = 1: a system's items run pair by pair over all its triples instead of triple
+ * by triple (whole systems only: item ranges no longer follow the processing order).  Two stagings of the operands feed the same MMA loop:
  *   trpdrv_launch_fused: cp.async; any sizes, any number of systems.  vec2 = 1 (16-byte copies) requires
  *     even nvir and nocc and 16-byte aligned tensors for every system; mma_k selects the FP64 MMA shape
  *     m16n8k4 (4) or m16n8k8 (8).
@@ -55,7 +56,7 @@ typedef struct trpdrv_dev_system {
  *     TRPDRV_TMA_MAX_SYSTEMS systems (trpdrv_tma_supported); mma_k 8 or 16.  trpdrv_tma_prepare encodes the
  *     tensor maps of every system into a host blob of trpdrv_tma_maps_bytes() bytes (64-byte aligned)
  *     that each launch passes by value. */
-int trpdrv_launch_fused(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items,
+int trpdrv_launch_fused(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items, int pair_major,
                         unsigned long long *counter, int *status, int grid, int vec2, int mma_k,
                         void *stream);
 #define TRPDRV_TMA_MAX_SYSTEMS 8
@@ -64,7 +65,7 @@ int trpdrv_tma_supported(const trpdrv_dev_system *h_sys, int nsys);
 int trpdrv_tma_pack_edge(int nvir);
 size_t trpdrv_tma_maps_bytes(void);
 int trpdrv_tma_prepare(const trpdrv_dev_system *h_sys, int nsys, void *maps_out);
-int trpdrv_launch_fused_tma(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items,
+int trpdrv_launch_fused_tma(const trpdrv_dev_system *d_sys, int nsys, int64_t total_items, int pair_major,
                             unsigned long long *counter, int *status, int grid, const void *maps,
                             int mma_k, void *stream);
 int trpdrv_fused_tma_init(void);
@@ -82,7 +83,7 @@ int trpdrv_launch_wait_selftest(unsigned long long limit_ns, int *status, unsign
  * system's processing order starting at pos0: the contraction kernel writes their f into
  * fbuf [npos][8][nvir][trpdrv_oz_ldf(nvir)] and the tengy kernel writes the sums of each 16-wide tile pair into
  * one slot of the triple's items in `partial` (the other slots must be zero), for
- * trpdrv_launch_item_reduce.  *status as the fused kernels (bit 0 malformed entry, bit 1 a wait
+ * trpdrv_launch_records.  *status as the fused kernels (bit 0 malformed entry, bit 1 a wait
  * ran out).  The contraction kernel is persistent: grid = CTAs (one per SM). */
 #define TRPDRV_OZ_MIN_SLICES 4
 #define TRPDRV_OZ_MAX_SLICES 8
@@ -119,13 +120,16 @@ int trpdrv_launch_oz_tengy(const trpdrv_dev_system *h_sys, int64_t pos0, int npo
                            int threads, int *status, void *stream);
 int trpdrv_oz_init(void);
 
-/* Per-triple sum of the per-item energies of one system (partial -> rec). */
-int trpdrv_launch_item_reduce(const trpdrv_dev_system *h_sys, void *stream);
+/* Per-triple sums of the per-item energies of nsys systems (descriptors on host and device): partial -> rec. */
+int trpdrv_launch_records(const trpdrv_dev_system *h_sys, const trpdrv_dev_system *d_sys, int nsys, void *stream);
 
-/* Compensated per-system total over rec: out[0..3] = emp4 hi, emp4 lo, emp5 hi, emp5 lo, where the
- * total is emp4i + [i != k] emp4k summed over the triples. */
-int trpdrv_launch_system_reduce(const double *rec, const int32_t *triples, int64_t ntriples, int64_t nt,
-                                double *out, void *stream);
+/* Each system's compensated total over rec, of emp4i + [i != k] emp4k summed over the triples:
+ * res[4 s ..] = emp4 hi, emp4 lo, emp5 hi, emp5 lo; res[4 nsys] = the value of *status.  res is pinned host memory
+ * (device-accessible).  bsum: nsys * TRPDRV_FINISH_BLOCKS * 4 doubles; done: nsys zeros (left at zero).  Systems
+ * without records are not written. */
+#define TRPDRV_FINISH_BLOCKS 1024
+int trpdrv_launch_totals(const trpdrv_dev_system *h_sys, const trpdrv_dev_system *d_sys, int nsys, double *bsum,
+                         unsigned *done, const int *status, double *res, void *stream);
 
 /* dst[i] = -src[i]. */
 int trpdrv_launch_negate(const double *src, double *dst, size_t n, void *stream);

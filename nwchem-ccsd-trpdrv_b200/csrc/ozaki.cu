@@ -813,7 +813,7 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(const SliceParams P)
 // batched tengy over the f of a batch: one CTA per (16-wide tile pair, triple), six or more CTAs per
 // SM.  A CTA's four sums go to its own slot of the triple's items (slot index = tile-pair index; the
 // 16-wide pairs fit in the 8 slots of each 32-wide item, and the slots no CTA writes are zero from
-// plan creation), so item_reduce sums them in a fixed order.
+// plan creation), so records_kernel sums them in a fixed order.
 struct TengyParams {
     CUtensorMap fmap;  // TMA form: fbuf as {nvir rows (contiguous), nvir columns, 8 * npos planes}
     trpdrv_dev_system sys;

@@ -1,10 +1,10 @@
 // Deterministic energy reductions and small device utilities.
 //
-//  item_reduce_kernel:   per triple, the compensated sum of its tile-pair items (fixed order) -> rec[t][4]
-//  system_reduce_kernel: per system, the compensated total of emp4i + [i != k] emp4k and of
+//  records_kernel:       per triple, the compensated sum of its tile-pair items (fixed order) -> rec[t][4]
+//  totals_kernel:        per system, the compensated total of emp4i + [i != k] emp4k and of
 //                        emp5i + [i != k] emp5k over the triples (the accumulation of
-//                        omp/ccsd_trpdrv_omp_cbody.c:133-142), as a double-double (hi, lo) pair,
-//                        built with error-free TwoSum in a fixed order.
+//                        omp/ccsd_trpdrv_omp_cbody.c:133-142), as a double-double (hi, lo) pair, built with
+//                        error-free TwoSum in a fixed order.
 //  negate_kernel:        dst = -src (the occupied A operands are stored negated).
 //  pack_rows_kernel:     rows of odd length copied to an even pitch (operands of the cp.async staging).
 
@@ -12,32 +12,6 @@
 #include "launch.h"
 
 namespace trpdrv {
-
-__global__ void item_reduce_kernel(const double *__restrict__ partial, int npairs, long long ntriples,
-                                   double *__restrict__ rec)
-{
-    const long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (t >= ntriples) return;
-    const int nslot = npairs * TRPDRV_FUSED_SLOTS;
-    const double *p = partial + 4 * t * (long long)nslot;
-    // compensated per lane (error-free TwoSum, errors carried in lo), then the lanes' hi and lo sums
-    double hi[4] = {0.0, 0.0, 0.0, 0.0}, lo[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int q = lane; q < nslot; q += 32) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            double s, e;
-            two_sum(hi[c], p[4 * q + c], s, e);
-            hi[c] = s;
-            lo[c] += e;
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const double h = warp_sum(hi[c]), l = warp_sum(lo[c]);
-        if (lane == 0) rec[4 * t + c] = h + l;
-    }
-}
 
 __device__ __forceinline__ void dd_add(double &hi, double &lo, double x)
 {
@@ -47,50 +21,137 @@ __device__ __forceinline__ void dd_add(double &hi, double &lo, double x)
     lo += e;
 }
 
-constexpr int RED_THREADS = 1024;
-
-__global__ void __launch_bounds__(RED_THREADS)
-system_reduce_kernel(const double *__restrict__ rec, const int32_t *__restrict__ triples, long long n, long long nt,
-                     double *__restrict__ out)
-{
-    __shared__ double sh[4][RED_THREADS];
-    double h4 = 0.0, l4 = 0.0, h5 = 0.0, l5 = 0.0;
-    for (long long t = threadIdx.x; t < n; t += RED_THREADS) {
-        const int packed = triples[t % nt];  // records are [a][triple]
-        const int i = packed & 1023, k = (packed >> 20) & 1023;
-        dd_add(h4, l4, rec[4 * t + 0]);
-        dd_add(h5, l5, rec[4 * t + 1]);
-        if (i != k) {
-            dd_add(h4, l4, rec[4 * t + 2]);
-            dd_add(h5, l5, rec[4 * t + 3]);
+struct DdPair {
+    double h4, l4, h5, l5;
+    __device__ __forceinline__ void add_record(const double (&rec)[4], int packed)
+    {
+        dd_add(h4, l4, rec[0]);
+        dd_add(h5, l5, rec[1]);
+        if ((packed & 1023) != ((packed >> 20) & 1023)) {  // i != k
+            dd_add(h4, l4, rec[2]);
+            dd_add(h5, l5, rec[3]);
         }
     }
-    sh[0][threadIdx.x] = h4;
-    sh[1][threadIdx.x] = l4;
-    sh[2][threadIdx.x] = h5;
-    sh[3][threadIdx.x] = l5;
+};
+
+constexpr int REC_WARPS = 8;       // records per block of records_kernel
+constexpr int FIN_THREADS = 512;   // totals_kernel
+
+// The block's sum of every thread's pair in thread 0 (a fixed tree).
+__device__ __forceinline__ DdPair block_dd(DdPair v, double (&sh)[4][FIN_THREADS])
+{
+    const int t = threadIdx.x;
+    sh[0][t] = v.h4;
+    sh[1][t] = v.l4;
+    sh[2][t] = v.h5;
+    sh[3][t] = v.l5;
     __syncthreads();
-    for (int w = RED_THREADS / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            const int o = threadIdx.x + w;
+    for (int w = FIN_THREADS / 2; w > 0; w >>= 1) {
+        if (t < w) {
             double s, e;
-            two_sum(sh[0][threadIdx.x], sh[0][o], s, e);
-            sh[0][threadIdx.x] = s;
-            sh[1][threadIdx.x] += sh[1][o] + e;
-            two_sum(sh[2][threadIdx.x], sh[2][o], s, e);
-            sh[2][threadIdx.x] = s;
-            sh[3][threadIdx.x] += sh[3][o] + e;
+            two_sum(sh[0][t], sh[0][t + w], s, e);
+            sh[0][t] = s;
+            sh[1][t] += sh[1][t + w] + e;
+            two_sum(sh[2][t], sh[2][t + w], s, e);
+            sh[2][t] = s;
+            sh[3][t] += sh[3][t + w] + e;
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        double s, e;
-        two_sum(sh[0][0], sh[1][0], s, e);  // renormalise
+    const DdPair r = {sh[0][0], sh[1][0], sh[2][0], sh[3][0]};
+    __syncthreads();
+    return r;
+}
+
+__host__ __device__ inline int total_blocks(long long ntriples)
+{
+    const long long n = (ntriples + FIN_THREADS - 1) / FIN_THREADS;
+    return n < TRPDRV_FINISH_BLOCKS ? (int)n : TRPDRV_FINISH_BLOCKS;
+}
+
+// One row of the grid per system, one warp per record.
+__global__ void __launch_bounds__(REC_WARPS * 32) records_kernel(const trpdrv_dev_system *__restrict__ sys)
+{
+    const trpdrv_dev_system &S = sys[blockIdx.y];
+    const int lane = threadIdx.x & 31, nslot = S.npairs * TRPDRV_FUSED_SLOTS;
+    for (long long t = (long long)blockIdx.x * REC_WARPS + (threadIdx.x >> 5); t < S.ntriples;
+         t += (long long)gridDim.x * REC_WARPS) {
+        const double *p = S.partial + 4 * t * (long long)nslot;
+        // compensated per lane (error-free TwoSum, errors carried in lo), then the lanes' hi and lo sums
+        double hi[4] = {0.0, 0.0, 0.0, 0.0}, lo[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int q = lane; q < nslot; q += 32) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                double s, e;
+                two_sum(hi[c], p[4 * q + c], s, e);
+                hi[c] = s;
+                lo[c] += e;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double h = warp_sum(hi[c]), l = warp_sum(lo[c]);
+            if (lane == 0) S.rec[4 * t + c] = h + l;
+        }
+    }
+}
+
+// One row of the grid per system.  Each block leaves its records' double-double sum; the system's last block adds
+// those in block order and writes the totals and the execution's status word to pinned host memory, so that
+// reading the energies needs no copy.
+__global__ void __launch_bounds__(FIN_THREADS)
+totals_kernel(const trpdrv_dev_system *__restrict__ sys, double *__restrict__ bsum, unsigned *__restrict__ done,
+              const int *__restrict__ status, double *__restrict__ res)
+{
+    __shared__ double sh[4][FIN_THREADS];
+    __shared__ int last;
+    const trpdrv_dev_system &S = sys[blockIdx.y];
+    const long long n = S.ntriples;
+    const int nblk = total_blocks(n), tid = threadIdx.x;
+    if ((int)blockIdx.x >= nblk) return;
+    DdPair v = {0.0, 0.0, 0.0, 0.0};
+    for (long long t = (long long)blockIdx.x * FIN_THREADS + tid; t < n; t += (long long)nblk * FIN_THREADS) {
+        const double rec[4] = {S.rec[4 * t], S.rec[4 * t + 1], S.rec[4 * t + 2], S.rec[4 * t + 3]};
+        v.add_record(rec, S.triples[t % S.nt]);  // records are [a][triple]
+    }
+    v = block_dd(v, sh);
+    if (nblk > 1) {
+        double *bs = bsum + 4 * (size_t)blockIdx.y * TRPDRV_FINISH_BLOCKS;
+        if (tid == 0) {
+            double *b = bs + 4 * blockIdx.x;
+            b[0] = v.h4;
+            b[1] = v.l4;
+            b[2] = v.h5;
+            b[3] = v.l5;
+            __threadfence();
+            last = atomicAdd(&done[blockIdx.y], 1u) == (unsigned)nblk - 1;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        v = {0.0, 0.0, 0.0, 0.0};
+        for (int q = tid; q < nblk; q += FIN_THREADS) {
+            const double *b = bs + 4 * q;
+            double s, e;
+            two_sum(v.h4, __ldcg(b), s, e);
+            v.h4 = s;
+            v.l4 += __ldcg(b + 1) + e;
+            two_sum(v.h5, __ldcg(b + 2), s, e);
+            v.h5 = s;
+            v.l5 += __ldcg(b + 3) + e;
+        }
+        v = block_dd(v, sh);
+        if (tid == 0) done[blockIdx.y] = 0u;
+    }
+    if (tid == 0) {
+        double *out = res + 4 * blockIdx.y, s, e;
+        two_sum(v.h4, v.l4, s, e);  // renormalise
         out[0] = s;
         out[1] = e;
-        two_sum(sh[2][0], sh[3][0], s, e);
+        two_sum(v.h5, v.l5, s, e);
         out[2] = s;
         out[3] = e;
+        res[4 * gridDim.y] = (double)*status;
     }
 }
 
@@ -138,22 +199,31 @@ extern "C" int trpdrv_launch_pack_rows(const trpdrv_pack_list *list, void *strea
     return (int)cudaGetLastError();
 }
 
-extern "C" int trpdrv_launch_item_reduce(const trpdrv_dev_system *h_sys, void *stream)
+extern "C" int trpdrv_launch_records(const trpdrv_dev_system *h_sys, const trpdrv_dev_system *d_sys, int nsys,
+                                     void *stream)
 {
-    if (h_sys->ntriples <= 0) return 0;
-    const int warps = 8;
-    const long long blocks = (h_sys->ntriples + warps - 1) / warps;
-    item_reduce_kernel<<<(unsigned)blocks, warps * 32, 0, (cudaStream_t)stream>>>(h_sys->partial, h_sys->npairs,
-                                                                                 h_sys->ntriples, h_sys->rec);
+    long long blocks = 0;
+    for (int q = 0; q < nsys; ++q) {
+        const long long n = (h_sys[q].ntriples + REC_WARPS - 1) / REC_WARPS;
+        if (n > blocks) blocks = n;
+    }
+    if (blocks == 0) return 0;
+    if (blocks > 65535) blocks = 65535;
+    records_kernel<<<dim3((unsigned)blocks, (unsigned)nsys), REC_WARPS * 32, 0, (cudaStream_t)stream>>>(d_sys);
     return (int)cudaGetLastError();
 }
 
-extern "C" int trpdrv_launch_system_reduce(const double *rec, const int32_t *triples, int64_t ntriples, int64_t nt,
-                                           double *out, void *stream)
+extern "C" int trpdrv_launch_totals(const trpdrv_dev_system *h_sys, const trpdrv_dev_system *d_sys, int nsys,
+                                    double *bsum, unsigned *done, const int *status, double *res, void *stream)
 {
-    if (nt <= 0) return 0;
-    system_reduce_kernel<<<1, RED_THREADS, 0, (cudaStream_t)stream>>>(rec, triples, (long long)ntriples, (long long)nt,
-                                                                     out);
+    int blocks = 0;
+    for (int q = 0; q < nsys; ++q) {
+        const int n = total_blocks(h_sys[q].ntriples);
+        if (n > blocks) blocks = n;
+    }
+    if (blocks == 0) return 0;
+    totals_kernel<<<dim3((unsigned)blocks, (unsigned)nsys), FIN_THREADS, 0, (cudaStream_t)stream>>>(d_sys, bsum, done,
+                                                                                                    status, res);
     return (int)cudaGetLastError();
 }
 
