@@ -199,6 +199,17 @@ __device__ __forceinline__ unsigned long long sdesc_sw64(const void *p)
            (1ull << 46) | (4ull << 61);
 }
 
+// True in one lane of the converged warp.  The branch it guards is compiled with warp-uniform operands: a
+// tcgen05.mma then takes its descriptors from uniform registers.  Under an ordinary `lane == 0` the compiler
+// moves every operand there instruction by instruction, and one thread issues an MMA every 44.7 cycles whatever
+// its N (16 to 80); under elect, every 22.6 (N = 32) and, at N = 64, every 35.1 against 32 of the tensor pipe.
+__device__ __forceinline__ bool elect_one()
+{
+    unsigned r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r != 0;
+}
+
 // A-operand collector buffer use of one MMA: the first MMA of a run that shares its A tile fills the
 // buffer, the following ones read A from it instead of shared memory, the last one releases it.
 enum { COL_DISCARD = 0, COL_FILL = 1, COL_USE = 2, COL_LASTUSE = 3 };
@@ -579,7 +590,8 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {  // MMA issuer: level L = p + q (0-based) accumulates at columns L*BN..
+        const unsigned long long dA0 = sdesc_sw64(stages), dB0 = sdesc_sw64(stages + S * SLICE_A);
+        {  // MMA issuer: level L = p + q (0-based) accumulates at columns L*BN..
             int stage = 0;
             unsigned phase = 0;
             bool alive = true;
@@ -596,8 +608,9 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
                             break;
                         }
                         tc_fence_after();
-                        const char *sA = stages + (size_t)stage * C::STAGE, *sB = sA + S * SLICE_A;
-                        const unsigned long long dA = sdesc_sw64(sA), dB = sdesc_sw64(sB);
+                        const unsigned long long so = (unsigned long long)(stage * (int)(C::STAGE >> 4));
+                        const unsigned long long dA = dA0 + so, dB = dB0 + so;
+                        if (elect_one()) {
 #pragma unroll
                         for (int ks = 0; ks < KC / KSTEP; ++ks) {
                             const int kg = kc * (KC / KSTEP) + ks;
@@ -613,16 +626,18 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
                             }
                         }
                         mma_commit(&empty[stage]);  // the stage is free once these MMAs have read it
+                        }
+                        __syncwarp();
                         if (++stage == C::STAGES) {
                             stage = 0;
                             phase ^= 1;
                         }
                     }
                 }
-                mma_commit(tfull);  // this tile's sums are complete (or the tile was skipped)
+                if (elect_one()) mma_commit(tfull);  // this tile's sums are complete (or the tile was skipped)
             }
             if (it > 0) {  // a CTA with no tiles (an energies-only launch) issued nothing to wait for
-                mma_commit(done);  // every MMA issued by this thread has completed when `done` flips
+                if (elect_one()) mma_commit(done);  // every MMA issued by this thread has completed when `done` flips
                 mbar_wait(done, 0, P.status);
             }
         }
