@@ -104,7 +104,7 @@ struct TengySums {
     double e4i, e5i, e4k, e5k;
 };
 
-// The terms of a position (b,c) and its mirror (c,b) together (BOTH = false: of (b,c) alone).  They share the
+// The terms of a position (b,c) and its mirror (c,b) together.  They share the
 // denominator, and the sums t2 + t3, t1 + t4, n2 + n3, n1 + n4 of each position enter both positions' forms, so a
 // pair costs about 135 FP64 instructions; the forms written out twice cost 200 (FP64 arithmetic
 // is issued at half a warp instruction per clock per scheduler, on the same pipe as the MMAs).  vb, vc: the
@@ -135,15 +135,15 @@ __device__ __forceinline__ void tengy_forms(const TengyPos &p, const TengyPos &q
     g5k = p.ut + q.n1 - 2 * (p.st + q.n2);
 }
 
-template <bool BOTH>
-__device__ __forceinline__ void tengy_pair(const double (&bc)[8], const double (&cb)[8], double denom,
+// both (of a whole warp): false for the term of (b,c) alone.
+__device__ __forceinline__ void tengy_pair(bool both, const double (&bc)[8], const double (&cb)[8], double denom,
                                            const TengyIdx &vb, const TengyIdx &vc, TengySums &s)
 {
     const TengyPos p(bc), q(cb);
     double a4i, a4k, f5i, g5i, f5k, g5k;
     tengy_forms(p, q, a4i, a4k, f5i, g5i, f5k, g5k);
     double e5i = vb.t1v1 * (vc.dx1 * f5i + vc.dc1 * g5i), e5k = vb.t1v2 * (vc.dx2 * f5k + vc.dc2 * g5k);
-    if (BOTH) {
+    if (both) {
         double b4i, b4k;
         tengy_forms(q, p, b4i, b4k, f5i, g5i, f5k, g5k);
         a4i += b4i;
@@ -155,6 +155,13 @@ __device__ __forceinline__ void tengy_pair(const double (&bc)[8], const double (
     s.e4k += denom * a4k;
     s.e5i += denom * e5i;
     s.e5k += denom * e5k;
+}
+
+template <bool BOTH>
+__device__ __forceinline__ void tengy_pair(const double (&bc)[8], const double (&cb)[8], double denom,
+                                           const TengyIdx &vb, const TengyIdx &vc, TengySums &s)
+{
+    tengy_pair(BOTH, bc, cb, denom, vb, vc, s);
 }
 
 // Block-wide sum of the four partial energies; returns the totals in thread 0.  `scratch` must

@@ -13,8 +13,8 @@
 //    (tcgen05.mma kind::i8, int32 accumulators in TMEM).  Pairs with equal p + q carry the same
 //    weight and share one accumulator; |sum| <= S * dp * 64 * 64 < 2^31, so the integer sums are exact;
 //  * the S level sums are recombined in FP64: f = 2^(eA + eB) * sum_L 2^(-7L) C_L.
-// f of a batch of triples go to a device buffer (L2-sized) and the batched tengy kernel reduces
-// them in FP64 exactly like the plain path (omp/ccsd_tengy_c99.c:5-119).
+// f of a batch of triples go to a device buffer and become energies in FP64 (omp/ccsd_tengy_c99.c:5-119): for even nvir
+// beside the next batch's products, in their launch, else in a launch of their own.
 //
 // Operand slices (int8, contraction index d contiguous, zero-padded to dp, a multiple of 32):
 //   SA[x][p][r][d]:      r < V: [J(x) | -TOV(x)] row r;       r >= V: [K(x) | -XOV(x)] row r - V
@@ -23,13 +23,24 @@
 // product [A1; A2] [B1 | B3] holds the four f of the group in its quadrants:
 //   f1n = A1 B1, f2n = A2 B1, f3n = A1 B3, f4n = A2 B3 (and f1t..f4t likewise).
 //
-// Contraction kernel: persistent, one CTA per SM walking 128 x 64 output tiles of the batch's
-// (triple, group) products.  Warp 0 issues TMA loads (64-byte swizzle) of all S digit slices of A and
-// B for 64 contraction indices per stage and runs ahead across tiles; warp 1 allocates tensor memory
-// and one of its threads issues every MMA (M=128, N=64, K=32) into S level accumulators (S*64
-// columns); warps 2-9 wait for a tile's last MMA, drain the accumulators with tcgen05.ld, release
-// them to the next tile and then scale and store in FP64 while its MMAs run.  Every wait is bounded
-// (globaltimer) and reports through *status; tensor memory is released on every path.
+// Contraction kernel: persistent, one CTA per SM walking 128 x 64 output tiles of the batch's products.
+//   warp 0       TMA loads (64-byte swizzle) of all S digit slices of A and B, 64 contraction indices a stage; runs ahead
+//                across tiles
+//   warp 1       allocates tensor memory and issues every MMA (M=128, N=64, K=32) into S level accumulators (S*64
+//                columns)
+//   warp 2       the energies' operands: triples, per-index vectors, f by TMA
+//   warps 4-11   wait for a tile's last MMA, join its levels, release the accumulators to the next tile, then
+//                scale and store in FP64 while that tile's MMAs run
+//   warps 12-15  energies
+// Every wait is bounded (globaltimer) and reports through *status; tensor memory is released on every path.
+//
+// What bounds it: the int8 products take 32 cycles each at best and 35 as issued, 9.8 kclk of a tile of 7 slices and
+// 320 contraction indices; a tile takes 15.6 (13.9 without the energies, 12 without the operands' loads as well).
+// The accumulators fill tensor memory, so nothing overlaps their drain (1.7 kclk), and shared memory is nearly
+// saturated: 84 KB read by the 28 products of a K step and 42 KB written, in 980 cycles.  7 slices, all
+// triples, ms at (nocc, nvir) = (12, 300), (10, 400), (20, 200): 7.79, 9.17, 15.8 with each MMA issued under `lane == 0`;
+// 7.28, 8.45, 14.4 under elect.sync; 6.55, 8.06, 13.0 with scales added to exponents and shorter code; 6.5, 7.9, 12.7 with
+// the levels joined in integers; 5.8, 7.5, 11.8 with the energies' operands prepared by a warp of its own.
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -47,7 +58,7 @@ constexpr int KC = 64;          // contraction bytes (= int8 indices) per stage
 constexpr int KSTEP = 32;       // contraction indices per MMA
 constexpr int NREC = 8;         // recombination warps: two per TMEM lane quadrant, 32 columns each
 constexpr int NENG = 4;         // energy warps (energies fused into the launch)
-// Warpgroup 0: warp 0 TMA, warp 1 MMA + TMEM (warps 2, 3 idle); warpgroups 1, 2 (warps 4 .. 11)
+// Warpgroup 0: warp 0 TMA, warp 1 MMA + TMEM, warp 2 the energies' operands (warp 3 idle); warpgroups 1, 2 (warps 4 .. 11)
 // recombination; warpgroup 3 (warps 12 .. 15) energies.
 constexpr int REC0 = 4, ENG0 = REC0 + NREC;
 constexpr int NTHREAD = 32 * (ENG0 + NENG);
@@ -57,18 +68,22 @@ constexpr int REG_LAUNCH = 128, REG_CTRL = 72, REG_REC = 168, REG_ENG = 104;
 static_assert(128 * REG_CTRL + 256 * REG_REC + 128 * REG_ENG <= NTHREAD * REG_LAUNCH, "register split exceeds the launch");
 constexpr unsigned SLICE_A = BM * KC;
 constexpr unsigned SLICE_B = BN * KC;
-constexpr int SMEM_AVAIL = 227 * 1024 - 2048;
+constexpr int SMEM_AVAIL = 227 * 1024 - 1024;  // less the alignment of the stages
 constexpr unsigned long long WAIT_LIMIT_NS = 4000000000ull;
 
-// fused energies: the f tiles of one tile pair (both orientations, 8 planes of 16 x 16 doubles each)
-constexpr unsigned PARK_BYTES = 2u * 8u * 16u * 16u * 8u;
+// fused energies: the f of half a tile pair (16 b x 8 c), both orientations of the eight f, 8 KB each
+constexpr unsigned HALF_BYTES = 2u * 8u * 16u * 8u * 8u;
 
 template <int S>
 struct Cfg {
     static constexpr unsigned STAGE = S * (SLICE_A + SLICE_B);
-    static constexpr int FIT = (SMEM_AVAIL - (int)PARK_BYTES) / (int)STAGE;
-    static constexpr int STAGES = FIT > 4 ? 4 : FIT;
-    static constexpr size_t SMEM = (size_t)STAGES * STAGE + PARK_BYTES + 1024;  // stages, then the park
+    // two stages or more beside three half-pair buffers of the energies (and 4 KB of static variables), else, for 8
+    // slices, beside two (and 2 KB)
+    static constexpr int FIT3 = (SMEM_AVAIL - 4096 - 3 * (int)HALF_BYTES) / (int)STAGE;
+    static constexpr int FIT2 = (SMEM_AVAIL - 2048 - 2 * (int)HALF_BYTES) / (int)STAGE;
+    static constexpr int HALVES = FIT3 >= 2 ? 3 : 2;
+    static constexpr int STAGES = FIT3 >= 2 ? (FIT3 > 4 ? 4 : FIT3) : FIT2;
+    static constexpr size_t SMEM = (size_t)STAGES * STAGE + (size_t)HALVES * HALF_BYTES + 1024;
     static constexpr unsigned TMEM_COLS = S * BN <= 256 ? 256u : 512u;
     static_assert(STAGES >= 2, "fewer than two stages fit");
     static_assert(S * BN <= 512, "level accumulators exceed tensor memory");
@@ -81,7 +96,8 @@ constexpr unsigned IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >
 
 struct GemmParams {
     CUtensorMap mapA, mapB;  // 64-byte aligned members first
-    CUtensorMap fmap;        // fused energies: efbuf as {V rows (contiguous), V columns, 8 * enpos planes}
+    CUtensorMap fbc, fcb;    // fused energies: efbuf as {V rows (contiguous), V columns, 8 * enpos planes}, in
+                             // boxes of 16 rows x 8 columns (at (b,c)) and 8 rows x 16 columns (at (c,b))
     trpdrv_dev_system sys;   // fused energies: vectors, triples and energy slots of the system
     const double *ea, *eb;   // power-of-two scales per A row / B column
     const int32_t *triples, *order;
@@ -89,7 +105,7 @@ struct GemmParams {
     long long pos0, ntriples, nt;  // ntriples records = n_a * nt triples per a
     double *fbuf;            // [batch][8][V][ldf]
     // fused energies: the energies of positions epos0 .. epos0 + enpos - 1, whose f an earlier launch
-    // stored (at the fmap's base); unit u = tile pair u % np of position epos0 + u / np
+    // stored (at the maps' base); unit u = tile pair u % np of position epos0 + u / np
     long long epos0;
     int enpos, np;
     int V, O, ldf, nks, mtiles, ntiles, tiles;  // tiles = jobs * mtiles * ntiles
@@ -393,9 +409,8 @@ __host__ __device__ inline int tengy_pairs(int nvir)
 
 
 // ------------------------------------------------------------------------------------------------
-// energies fused into the contraction kernel: once every tile of a position has stored its f, the
-// recombination warps of any CTA take that position's tile pairs (units) in order and compute their
-// energies from f that is still in L2, in the time the next tile's products run on the tensor cores
+// energies fused into the contraction kernel: those of the positions whose f the launch before stored, beside
+// this launch's products
 // ------------------------------------------------------------------------------------------------
 constexpr int NENG_THREADS = 32 * NENG;
 
@@ -413,72 +428,194 @@ __device__ __forceinline__ bool eng_bar_or(bool p)
     return r != 0;
 }
 
-// One unit's energies, by the energy threads (te = 0 .. NENG_THREADS - 1); false if the wait for its
-// tiles ran out (status bit 1 set).
-__device__ __forceinline__ bool fused_unit(const GemmParams &P, int u, double *park, double *vsh,
-                                           unsigned long long *ubar, unsigned &uphase, double *red, int te)
+// The fused energies of a CTA: the contiguous range u0 .. u1 of the tile pairs B <= C (16-wide) of the positions
+// whose f an earlier launch stored.  Warp 2 looks up each pair's triple, loads its per-index vectors and copies its f in
+// two halves of 16 b x 8 c into a ring of NBUF buffers; the energy warps find everything in shared memory.
+// Done by the energy warps themselves, the lookups (dependent loads) took 2.8 of the 9 kclk of a pair, and
+// with one buffer of 32 KB nothing of the next pair could be in flight meanwhile.
+struct EnergyUnit {  // of one tile pair
+    double vec[TVROWS * TW];  // as tengy_stage_vecs
+    double eaijk;
+    double *slot;  // the pair's four energies; null: a malformed queue entry
+    int b0, c0;
+};
+
+template <int NBUF>
+struct EnergyRing {
+    static constexpr int NUNIT = NBUF >= 3 ? 2 : 1;  // tables
+    unsigned long long full[NBUF], empty[NBUF];
+    EnergyUnit unit[NUNIT];
+    double red[NUNIT][4 * (NENG - 1)];  // the sums of the energy warps but the first
+    __device__ __forceinline__ void init()
+    {
+        for (int q = 0; q < NBUF; ++q) {
+            mbar_init(&full[q], 32);     // every lane of warp 2, and the bytes
+            mbar_init(&empty[q], NENG);  // one arrival per energy warp
+        }
+    }
+};
+
+__device__ __forceinline__ void energy_range(const GemmParams &P, unsigned &u0, unsigned &u1)
 {
-    TengyItem it;
-    if (!tengy_geom(P.sys, P.epos0, u % P.np, u / P.np, it)) return true;  // same outcome in every thread
-    // the tiles' coordinates need no loads: copies first, the triple and the vectors while they land
-    if (te == 0) {
-        // this park's previous reads (generic proxy) before the tensor-copy writes
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive_expect_tx(ubar, (it.diag ? 1u : 2u) * (PARK_BYTES / 2u));
-        const unsigned long long pol = policy_evict_first();
-        tma_load_3d_hint(park, &P.fmap, ubar, it.b0, it.c0, it.y * 8, pol);
-        if (!it.diag) tma_load_3d_hint(park + PARK_BYTES / 16u, &P.fmap, ubar, it.c0, it.b0, it.y * 8, pol);
-    }
-    const bool valid = tengy_triple(P.sys, P.epos0, it);  // the same in every thread
-    TengyVecs v;
-    if (valid) {
-        v = tengy_vecs(P.sys, it);
-        tengy_stage_vecs(v, it, vsh, te, NENG_THREADS);
-    }
-    const bool ok = mbar_wait(ubar, uphase, P.status);
-    uphase ^= 1u;
-    if (eng_bar_or(!ok)) return false;  // also: the vector table is complete
-    if (!valid) {
-        eng_bar();  // the park and the table are free again
-        return true;
-    }
-    TengySums su = {0.0, 0.0, 0.0, 0.0};
-    tengy_tile_pair_swz16_sv<NENG_THREADS>(park, vsh, it.b0, it.c0, it.diag, v.nvir, v.eaijk, te, su);
-    su.e4i = warp_sum(su.e4i);
-    su.e5i = warp_sum(su.e5i);
-    su.e4k = warp_sum(su.e4k);
-    su.e5k = warp_sum(su.e5k);
-    const int we = te >> 5;
-    if ((te & 31) == 0) {
-        red[4 * we + 0] = su.e4i;
-        red[4 * we + 1] = su.e5i;
-        red[4 * we + 2] = su.e4k;
-        red[4 * we + 3] = su.e5k;
-    }
-    eng_bar();  // also: every read of the park is done before the next unit's copies
-    if (te == 0) {
-        double t[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int w = 0; w < NENG; ++w)  // fixed order: the sums do not depend on which CTA ran the unit
-            for (int e = 0; e < 4; ++e) t[e] += red[4 * w + e];
-        double *out = tengy_slot(P.sys, it);
-        out[0] = t[0];
-        out[1] = t[1];
-        out[2] = t[2];
-        out[3] = t[3];
-    }
-    return true;
+    const unsigned total = (unsigned)P.enpos * (unsigned)P.np, per = (total + gridDim.x - 1) / gridDim.x;
+    u0 = min(total, blockIdx.x * per);
+    u1 = min(total, u0 + per);
 }
 
-// The energy warps' loop: CTA b takes units b, b + grid, ... of the positions whose f an earlier
-// launch stored, while this launch's tiles run on the tensor cores.
-__device__ __forceinline__ void fused_energies(const GemmParams &P, double *park, unsigned long long *ubar,
-                                               double *red, int te)
+// Warp 2, all lanes.
+template <int NBUF>
+__device__ __forceinline__ void energy_operands(const GemmParams &P, char *bufs, EnergyRing<NBUF> &R, int lane)
 {
-    const unsigned total = (unsigned)P.enpos * (unsigned)P.np;
-    __shared__ double vsh[TVROWS * TW];
-    unsigned uphase = 0;
-    for (unsigned u = blockIdx.x; u < total; u += gridDim.x)
-        if (!fused_unit(P, (int)u, park, vsh, ubar, uphase, red, te)) return;
+    constexpr int PER = TVROWS * TW / 32;  // vector entries per lane
+    static_assert(TVROWS * TW % 32 == 0, "vector entries per lane");
+    const trpdrv_dev_system &S = P.sys;
+    unsigned u0, u1;
+    energy_range(P, u0, u1);
+    if (u0 >= u1) return;
+    const int nb = (S.nvir + TW - 1) / TW;
+    const unsigned long long pol = policy_evict_first();
+    TengyItem it;
+    it.y = (int)(u0 / (unsigned)P.np);
+    it.pairi = (int)(u0 % (unsigned)P.np);
+    int B = 0, C = it.pairi;
+    while (B < nb - 1 && C >= nb - B) C -= nb - B++;
+    C += B;
+    bool valid = false, fresh = true;  // of the triple; fresh: a position not looked up yet
+    TengyVecs v;
+    int q = 0;
+    unsigned phase = 1;
+    for (unsigned u = u0; u < u1; ++u) {
+        if (fresh) {
+            valid = P.epos0 + it.y < S.ntriples && S.nt > 0 && tengy_triple(S, P.epos0, it);
+            if (valid) v = tengy_vecs(S, it);
+            fresh = false;
+        }
+        const int b0 = B * TW, c0 = C * TW;
+        double x[PER];
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            const int idx = lane + 32 * e, row = idx / TW, side = row / 7, kind = row % 7, n = (side ? c0 : b0) + idx % TW;
+            const double *src = kind == 0 ? v.t1v1 : kind == 1 ? v.t1v2 : kind == 2 ? v.dintx1 : kind == 3 ? v.dintx2
+                              : kind == 4 ? v.dintc1 : kind == 5 ? v.dintc2 : v.eorb + v.voff;
+            x[e] = valid && n < S.nvir ? __ldg(src + n) : 0.0;
+        }
+#pragma unroll 1
+        for (int hf = 0; hf < 2; ++hf) {
+            if (!mbar_wait(&R.empty[q], phase, P.status)) return;
+            if (hf == 0) {
+                // The table's last readers are done: with three buffers, since this one was freed by the pair before
+                // the last (both of whose halves lie before it); with two, once the pair before has freed the other.
+                if (NBUF == 2 && !mbar_wait(&R.empty[1], phase, P.status)) return;
+                EnergyUnit &t = R.unit[R.NUNIT == 2 ? (u - u0) & 1 : 0];
+#pragma unroll
+                for (int e = 0; e < PER; ++e) t.vec[lane + 32 * e] = x[e];
+                if (lane == 0) {
+                    t.eaijk = valid ? v.eaijk : 0.0;
+                    t.slot = valid ? tengy_slot(S, it) : nullptr;
+                    t.b0 = b0;
+                    t.c0 = c0;
+                }
+            }
+            if (lane == 0) {
+                char *dst = bufs + (size_t)q * HALF_BYTES;
+                // this buffer's previous reads (generic proxy) before the tensor-copy writes
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                mbar_arrive_expect_tx(&R.full[q], HALF_BYTES);
+                tma_load_3d_hint(dst, &P.fbc, &R.full[q], b0, c0 + 8 * hf, it.y * 8, pol);
+                tma_load_3d_hint(dst + HALF_BYTES / 2, &P.fcb, &R.full[q], c0 + 8 * hf, b0, it.y * 8, pol);
+            } else
+                mbar_arrive(&R.full[q]);
+            if (++q == NBUF) {
+                q = 0;
+                phase ^= 1u;
+            }
+        }
+        ++it.pairi;
+        if (++C == nb) {
+            if (++B == nb) {
+                B = 0;
+                ++it.y;
+                it.pairi = 0;
+                fresh = true;
+            }
+            C = B;
+        }
+    }
+}
+
+// The four sums of a warp, each as warp_sum adds it up; lane 8 e (e = 0 .. 3) returns the e-th.
+__device__ __forceinline__ double warp_sum4(const TengySums &s, int lane)
+{
+    const bool h = lane & 16, g = lane & 8;
+    double a = h ? s.e4k : s.e4i, b = h ? s.e5k : s.e5i;  // kept
+    a += __shfl_xor_sync(0xffffffffu, h ? s.e4i : s.e4k, 16);
+    b += __shfl_xor_sync(0xffffffffu, h ? s.e5i : s.e5k, 16);
+    double c = g ? b : a;
+    c += __shfl_xor_sync(0xffffffffu, g ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    return c;  // lanes 0-7: e4i, 8-15: e5i, 16-23: e4k, 24-31: e5k
+}
+
+// The energy warps (te = 0 .. NENG_THREADS - 1), one (b, c) of a half a thread.  Every wait is bounded; one that runs
+// out ends the loop in all threads.
+template <int NBUF>
+__device__ __forceinline__ void fused_energies(const GemmParams &P, const char *bufs, EnergyRing<NBUF> &R, int te)
+{
+    unsigned u0, u1;
+    energy_range(P, u0, u1);
+    const int V = P.sys.nvir, lane = te & 31, we = te >> 5;
+    // (r, c) of this thread within a half: c = cc ^ (r >> 3) keeps the half-warp's reads of both boxes free of bank
+    // conflicts (16 rows of 128 bytes, 128-byte swizzle; lines of 64 bytes, 64-byte swizzle)
+    const int r = te & 15, c = (te >> 4) ^ (r >> 3);
+    const int o1 = c * 128 + (((r >> 1) ^ c) << 4) + ((r & 1) << 3);
+    const int o2 = (int)(HALF_BYTES / 2) + r * 64 + (((c >> 1) ^ ((r >> 1) & 3)) << 4) + ((c & 1) << 3);
+    int q = 0;
+    unsigned phase = 0;
+    bool ok = true;
+    for (unsigned u = u0; u < u1; ++u) {
+        const EnergyUnit &t = R.unit[R.NUNIT == 2 ? (u - u0) & 1 : 0];
+        TengySums su = {0.0, 0.0, 0.0, 0.0};
+        double *slot = nullptr;
+#pragma unroll 1
+        for (int hf = 0; hf < 2; ++hf) {
+            ok = ok && mbar_wait(&R.full[q], phase, P.status);
+            if (ok) {
+                slot = t.slot;
+                const int cc = 8 * hf + c;
+                if (slot && t.b0 + r < V && t.c0 + cc < V) {
+                    const char *p = bufs + (size_t)q * HALF_BYTES;
+                    double fbc[8], fcb[8];
+#pragma unroll
+                    for (int x = 0; x < 8; ++x) {
+                        fbc[x] = *reinterpret_cast<const double *>(p + o1 + x * 1024);
+                        fcb[x] = *reinterpret_cast<const double *>(p + o2 + x * 1024);
+                    }
+                    const double *vb = t.vec + r, *vc = t.vec + 7 * TW + cc;
+                    const TengyIdx ib = {vb[0], vb[TW], vb[2 * TW], vb[3 * TW], vb[4 * TW], vb[5 * TW]};
+                    const TengyIdx ic = {vc[0], vc[TW], vc[2 * TW], vc[3 * TW], vc[4 * TW], vc[5 * TW]};
+                    const double denom = -1.0 / (vb[6 * TW] + vc[6 * TW] + t.eaijk);
+                    tengy_pair(t.b0 != t.c0, fbc, fcb, denom, ib, ic, su);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&R.empty[q]);
+            if (++q == NBUF) {
+                q = 0;
+                phase ^= 1u;
+            }
+        }
+        double *red = R.red[R.NUNIT == 2 ? (u - u0) & 1 : 0];
+        const double s = warp_sum4(su, lane), s0 = __shfl_sync(0xffffffffu, s, 8 * (lane & 3));
+        if (we > 0 && (lane & 7) == 0) red[4 * (we - 1) + (lane >> 3)] = s;
+        if (eng_bar_or(!ok)) return;  // also: the sums are in place
+        if (te < 4 && slot) {  // fixed order: the sums do not depend on which CTA ran the pair
+            double e = s0;
+            for (int w = 0; w < NENG - 1; ++w) e += red[4 * w + te];
+            slot[te] = e;
+        }
+        if (R.NUNIT == 1) eng_bar();  // else the next pair's sums go to the other half of red
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -512,22 +649,93 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams &P, int t)
     return d;
 }
 
-// level accumulators are drained in groups of up to 4: X = sum_l C_l 128^(last - l) is exact in
-// int64 and below 2^53 (|C_l| < 2^24), so one exact conversion and one FMA cover the group
-constexpr int LGROUP = 4;
+// Draining.  The next tile's products wait until the accumulators have been read, so as little as possible happens
+// before they are released; and the roles' code together must stay within the instruction caches, beside
+// which everything but the products ran at half its speed or less.  Three forms, by the width dp of the contraction:
+//   SUM64: all levels joined in integers, two adjacent ones in int32 (128 C_l + C_{l+1}), the pairs in
+//          int64, converted after the release (|C_l| <= (l + 1) dp 64^2; dp <= sum64_limit(S): 503 for S = 7)
+//   PAIRS: pairs of levels joined in int32 and added in FP64 (dp <= pair_limit(S): 811 for S = 7)
+//   LEVELS: level by level in FP64
+// Every one rounds once, so they give the same bits: integer sums are exact, and so is every FP64 addition
+// but the last, from the last levels up.
+enum DrainForm { SUM64, PAIRS, LEVELS };
+
+__host__ __device__ constexpr int pair_limit(int S)
+{
+    const int l = (S - 1) & ~1;               // first level of the last pair (or the last level alone)
+    const int first = l + 1 < S ? l : l - 2;  // first level of the last complete pair
+    return (int)((0x7fffffffLL - 1) / ((long long)(first + 1) * 4096 * 128 + (long long)(first + 2) * 4096));
+}
+
+__host__ __device__ constexpr int sum64_limit(int S)
+{
+    unsigned long long unit = 0;  // the largest |sum| of dp = 1
+    for (int l = 0; l < S; ++l) unit = unit * 128 + (unsigned long long)(l + 1) * 4096;
+    const unsigned long long lim = 0x7fffffffffffffffull / unit;
+    return lim < (unsigned long long)pair_limit(S) ? (int)lim : pair_limit(S);
+}
+
+// 16 columns at TMEM address base: sum_L C_L 2^(-7 (L + 2)); SUM64: the bits of the integer 2^(7 (S + 1)) times that.
+template <int S, DrainForm FORM>
+__device__ __forceinline__ void drain16(unsigned base, double (&val)[16])
+{
+    constexpr int STEP = FORM == LEVELS ? 1 : 2, NP = (S + STEP - 1) / STEP;  // pairs
+#pragma unroll
+    for (int u = 0; u < 16; ++u) val[u] = 0.0;
+#pragma unroll
+    for (int g = 0; g < NP; g += 2) {  // two pairs in flight; FP64: from the last ones up
+        const int k0 = FORM == SUM64 ? g : (NP - g >= 2 ? NP - g - 2 : 0);
+        const int k1 = FORM == SUM64 ? (g + 2 < NP ? g + 2 : NP) : NP - g;
+        unsigned v[2 * STEP][16];
+#pragma unroll
+        for (int l = 0; l < 2 * STEP; ++l)
+            if (k0 * STEP + l < k1 * STEP && k0 * STEP + l < S)
+                tmem_ld16_nowait(base + (unsigned)((k0 * STEP + l) * BN), v[l]);
+        tmem_wait_ld();
+#pragma unroll
+        for (int l = 0; l < 2 * STEP; ++l)
+            if (k0 * STEP + l < k1 * STEP && k0 * STEP + l < S) reg_fence16(v[l]);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const int k = FORM == SUM64 ? k0 + n : k1 - 1 - n;
+            if (k < k0 || k >= k1) continue;
+            const int l = (k - k0) * STEP, lev = k * STEP;
+            const bool two = STEP == 2 && lev + 1 < S;
+            const double w = level_weight(two ? lev + 1 : lev);
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                const int x = two ? (int)v[l][u] * 128 + (int)v[two ? l + 1 : l][u] : (int)v[l][u];
+                if (FORM == SUM64)
+                    val[u] = __longlong_as_double(k == 0 ? (long long)x
+                                                         : __double_as_longlong(val[u]) * (two ? 16384 : 128) + x);
+                else
+                    val[u] = fma((double)x, w, val[u]);
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ int scale_exp(double s) { return (__double2hiint(s) >> 20) - 1023; }  // s = 2^e, normal
+
+// x 2^e by the exponent bits: x zero or normal, and so the result
+__device__ __forceinline__ double scale_by_exp(double x, int e)
+{
+    const int hi = __double2hiint(x);
+    return __hiloint2double((hi & 0x7ff00000) ? hi + (e << 20) : hi, __double2loint(x));
+}
 
 template <int S>
 __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_constant__ GemmParams P)
 {
     using C = Cfg<S>;
     extern __shared__ char smem_raw[];
-    __shared__ __align__(8) unsigned long long full[C::STAGES], empty[C::STAGES], tfull[1], tempty[1], done[1], ubar[1];
+    __shared__ __align__(8) unsigned long long full[C::STAGES], empty[C::STAGES], tfull[1], tempty[1], done[1];
+    __shared__ EnergyRing<C::HALVES> ering;
     __shared__ unsigned tmem_sh;
-    __shared__ double red[4 * NENG];
-    // aligned by an offset, not by integer arithmetic on the pointer: the compiler then still knows that the park
-    // is shared memory
+    // aligned by an offset, not by integer arithmetic on the pointer: the compiler then still knows that they
+    // are shared memory
     char *stages = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
-    double *park = reinterpret_cast<double *>(stages + (size_t)C::STAGES * C::STAGE);  // 1024-byte aligned
+    char *halves = stages + (size_t)C::STAGES * C::STAGE;  // 1024-byte aligned
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nchunks = (P.nks * KSTEP + KC - 1) / KC;
@@ -540,7 +748,7 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
         mbar_init(tfull, 1);
         mbar_init(tempty, NREC);  // one arrival per recombination warp
         mbar_init(done, 1);
-        mbar_init(ubar, 1);
+        ering.init();
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -611,7 +819,7 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
                         const unsigned long long so = (unsigned long long)(stage * (int)(C::STAGE >> 4));
                         const unsigned long long dA = dA0 + so, dB = dB0 + so;
                         if (elect_one()) {
-#pragma unroll
+#pragma unroll 1
                         for (int ks = 0; ks < KC / KSTEP; ++ks) {
                             const int kg = kc * (KC / KSTEP) + ks;
                             if (kg < P.nks) {
@@ -642,7 +850,8 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
             }
         }
         __syncwarp();
-      }
+      } else if (warp == 2 && P.enpos > 0)
+        energy_operands<C::HALVES>(P, halves, ering, lane);
     } else if (warp < ENG0) {  // recombination: TMEM lanes 32*(warp%4).., columns 32*half..
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REG_REC));
         const int qd = warp & 3, half = (warp - REC0) >> 2;
@@ -652,65 +861,73 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
         int it = 0;
         for (int t = blockIdx.x; t < P.tiles; t += gridDim.x, ++it) {
             const Tile d = decode_tile(P, t);
+            // the exponents of the tile's scales, before its products are complete: this lane's row, and this lane's
+            // column of the 32
+            const int r = d.m0 + qd * 32 + lane, lcol = d.n0 + half * WC + lane;
+            int esa = d.ok && r < 2 * V ? scale_exp(P.ea[(size_t)d.planeA * 2 * V + r]) : 0;
+            int esb = d.ok && lcol < 2 * V ? scale_exp(P.eb[(size_t)d.planeB * 2 * V + lcol]) : 0;
             if (!mbar_wait(tfull, it & 1, P.status)) break;
             tc_fence_after();
-            double acc[WC];
+            const int rh = r >= V ? 1 : 0, b = r - rh * V;
+            double *fj = P.fbuf + (size_t)d.y * 8 * vv + (size_t)d.grp * 4 * vv + (size_t)rh * vv + b;
+            const bool row_ok = d.ok && r < 2 * V;
+            const unsigned base = tmem + ((unsigned)(qd * 32) << 16) + (unsigned)(half * WC);
+            double val[WC / 16][16];
+            const int dp = P.nks * KSTEP;
+            if (dp <= sum64_limit(S)) {
 #pragma unroll
-            for (int c = 0; c < WC; ++c) acc[c] = 0.0;
-            if (d.ok) {
-                const unsigned base = tmem + ((unsigned)(qd * 32) << 16) + (unsigned)(half * WC);
+                for (int cb = 0; cb < WC / 16; ++cb) drain16<S, SUM64>(base + (unsigned)(cb * 16), val[cb]);
+            } else if (dp <= pair_limit(S)) {
 #pragma unroll
-                for (int cb = 0; cb < WC / 16; ++cb) {
+                for (int cb = 0; cb < WC / 16; ++cb) drain16<S, PAIRS>(base + (unsigned)(cb * 16), val[cb]);
+            } else {
 #pragma unroll
-                    for (int g0 = 0; g0 < S; g0 += LGROUP) {
-                        const int g1 = (g0 + LGROUP < S) ? g0 + LGROUP : S;  // levels g0..g1-1
-                        unsigned v[LGROUP][16];
-#pragma unroll
-                        for (int l = 0; l < LGROUP; ++l)
-                            if (g0 + l < g1) tmem_ld16_nowait(base + (unsigned)((g0 + l) * BN + cb * 16), v[l]);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int l = 0; l < LGROUP; ++l)
-                            if (g0 + l < g1) reg_fence16(v[l]);
-                        // weight of the group's last level: 2^(-7 (g1 - 1 + 2))
-                        const double w = level_weight(g1 - 1);
-#pragma unroll
-                        for (int u = 0; u < 16; ++u) {
-                            long long x = 0;
-#pragma unroll
-                            for (int l = 0; l < LGROUP; ++l)
-                                if (g0 + l < g1) x = x * 128 + (long long)(int)v[l][u];
-                            acc[cb * 16 + u] = fma((double)x, w, acc[cb * 16 + u]);
-                        }
-                    }
-                }
+                for (int cb = 0; cb < WC / 16; ++cb) drain16<S, LEVELS>(base + (unsigned)(cb * 16), val[cb]);
             }
             // the accumulators may be overwritten by the next tile from here on
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty);
-            const int r = d.m0 + qd * 32 + lane;
-            if (d.ok && r < 2 * V) {
-                const double sa = P.ea[(size_t)d.planeA * 2 * V + r];
-                const int rh = r >= V ? 1 : 0, b = r - rh * V;
-                double *fj = P.fbuf + (size_t)d.y * 8 * vv + (size_t)d.grp * 4 * vv;
-                const double *eb = P.eb + (size_t)d.planeB * 2 * V;
+            if (!d.ok) continue;
+            int e0 = 0;
+            if (dp <= sum64_limit(S)) {
+                e0 = -7 * (S + 1);
+#pragma unroll
+                for (int cb = 0; cb < WC / 16; ++cb)
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) val[cb][u] = (double)__double_as_longlong(val[cb][u]);
+            }
+            // the scales as integer additions to the exponent: exact while every result is a normal number
+            if (!__all_sync(0xffffffffu, esa >= -450 && esa <= 450 && esb >= -450 && esb <= 450)) {
+                const double sa = row_ok ? P.ea[(size_t)d.planeA * 2 * V + r] : 0.0, w0 = e0 ? level_weight(S - 1) : 1.0;
 #pragma unroll
                 for (int c = 0; c < WC; ++c) {
                     const int col = d.n0 + half * WC + c;
-                    if (col < 2 * V) {
-                        const int ch = col >= V ? 1 : 0, cc = col - ch * V;
-                        double *dst = fj + (size_t)(rh + 2 * ch) * vv + b + (size_t)cc * P.ldf;
-                        const double val = acc[c] * sa * __ldg(eb + col);
-                        __stcs(dst, val);  // evict-first: read once, by a later launch; keeps the digits in L2
-                        if (d.same) __stcs(dst + 4 * vv, val);
-                    }
+                    val[c / 16][c % 16] = val[c / 16][c % 16] * w0 * sa;
+                    if (col < 2 * V) val[c / 16][c % 16] *= P.eb[(size_t)d.planeB * 2 * V + col];
                 }
+                esa = esb = e0 = 0;
             }
+            e0 += esa;
+            double *dst = fj + (size_t)(d.n0 + half * WC) * P.ldf;
+#pragma unroll
+            for (int cb = 0; cb < WC / 16; ++cb)
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    const int c = cb * 16 + u, col = d.n0 + half * WC + c;
+                    const double x = scale_by_exp(val[cb][u], e0 + __shfl_sync(0xffffffffu, esb, c));
+                    if (row_ok && col < 2 * V) {
+                        // column col - V of f3, f4 (two planes further) from column V on
+                        double *q = dst + (col >= V ? 2 * vv - (size_t)V * P.ldf : 0);
+                        __stcs(q, x);  // evict-first: read once, by a later launch; keeps the digits in L2
+                        if (d.same) __stcs(q + 4 * vv, x);
+                    }
+                    dst += P.ldf;
+                }
         }
     } else {  // energy warps: the units of the positions an earlier launch stored
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REG_ENG));
-        if (P.enpos > 0) fused_energies(P, park, ubar, red, tid - 32 * ENG0);
+        if (P.enpos > 0) fused_energies<C::HALVES>(P, halves, ering, tid - 32 * ENG0);
     }
     tc_fence_before();
     __syncthreads();
@@ -978,17 +1195,19 @@ static int make_map_i8(CUtensorMap *m, const signed char *base, unsigned long lo
 // 3-D map over the f of a batch for the TMA form of the energies: dims {nvir rows (contiguous), nvir
 // columns, planes}, box {16, 16, 8} (the eight f of one triple), 128-byte swizzle, zero fill past nvir.
 // Columns are trpdrv_oz_ldf(nvir) doubles apart (a multiple of 16 bytes); needs a 16-byte aligned base.
-static int make_map_f64(CUtensorMap *m, const double *base, int nvir, unsigned long long planes)
+static int make_map_f64(CUtensorMap *m, const double *base, int nvir, unsigned long long planes, unsigned rows = TW,
+                        unsigned cols = TW)
 {
     PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
     if (!fn || (reinterpret_cast<uintptr_t>(base) & 15)) return 1;
     const cuuint64_t dims[3] = {(cuuint64_t)nvir, (cuuint64_t)nvir, planes};
     const cuuint64_t ldf = (cuuint64_t)trpdrv_oz_ldf(nvir);
     const cuuint64_t strides[2] = {ldf * sizeof(double), ldf * nvir * sizeof(double)};
-    const cuuint32_t box[3] = {(cuuint32_t)TW, (cuuint32_t)TW, 8};
+    const cuuint32_t box[3] = {(cuuint32_t)rows, (cuuint32_t)cols, 8};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(base), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          rows * sizeof(double) == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : 2;
 }
@@ -1093,7 +1312,9 @@ extern "C" int trpdrv_launch_oz_gemm(const trpdrv_dev_system *h_sys, const trpdr
         P.np = oz::tengy_pairs(h_sys->nvir);
         if (P.np > h_sys->npairs * TRPDRV_FUSED_SLOTS) return (int)cudaErrorInvalidValue;
         if ((long long)P.np * enpos > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
-        if (oz::make_map_f64(&P.fmap, efbuf, h_sys->nvir, 8ull * enpos) != 0) return (int)cudaErrorInvalidValue;
+        if (oz::make_map_f64(&P.fbc, efbuf, h_sys->nvir, 8ull * enpos, 16, 8) != 0 ||
+            oz::make_map_f64(&P.fcb, efbuf, h_sys->nvir, 8ull * enpos, 8, 16) != 0)
+            return (int)cudaErrorInvalidValue;
         P.sys = *h_sys;
         P.epos0 = epos0;
         P.enpos = enpos;
