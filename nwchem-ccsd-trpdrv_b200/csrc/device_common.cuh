@@ -135,26 +135,39 @@ __device__ __forceinline__ void tengy_forms(const TengyPos &p, const TengyPos &q
     g5k = p.ut + q.n1 - 2 * (p.st + q.n2);
 }
 
-// both (of a whole warp): false for the term of (b,c) alone.
-__device__ __forceinline__ void tengy_pair(bool both, const double (&bc)[8], const double (&cb)[8], double denom,
-                                           const TengyIdx &vb, const TengyIdx &vc, TengySums &s)
+// The four terms but for the factor denom; both (of a whole warp): false for those of (b,c) alone.
+struct TengyTerms {
+    double a4i, a4k, e5i, e5k;
+};
+
+__device__ __forceinline__ TengyTerms tengy_terms(bool both, const double (&bc)[8], const double (&cb)[8],
+                                                  const TengyIdx &vb, const TengyIdx &vc)
 {
     const TengyPos p(bc), q(cb);
-    double a4i, a4k, f5i, g5i, f5k, g5k;
-    tengy_forms(p, q, a4i, a4k, f5i, g5i, f5k, g5k);
-    double e5i = vb.t1v1 * (vc.dx1 * f5i + vc.dc1 * g5i), e5k = vb.t1v2 * (vc.dx2 * f5k + vc.dc2 * g5k);
+    TengyTerms r;
+    double f5i, g5i, f5k, g5k;
+    tengy_forms(p, q, r.a4i, r.a4k, f5i, g5i, f5k, g5k);
+    r.e5i = vb.t1v1 * (vc.dx1 * f5i + vc.dc1 * g5i);
+    r.e5k = vb.t1v2 * (vc.dx2 * f5k + vc.dc2 * g5k);
     if (both) {
         double b4i, b4k;
         tengy_forms(q, p, b4i, b4k, f5i, g5i, f5k, g5k);
-        a4i += b4i;
-        a4k += b4k;
-        e5i += vc.t1v1 * (vb.dx1 * f5i + vb.dc1 * g5i);
-        e5k += vc.t1v2 * (vb.dx2 * f5k + vb.dc2 * g5k);
+        r.a4i += b4i;
+        r.a4k += b4k;
+        r.e5i += vc.t1v1 * (vb.dx1 * f5i + vb.dc1 * g5i);
+        r.e5k += vc.t1v2 * (vb.dx2 * f5k + vb.dc2 * g5k);
     }
-    s.e4i += denom * a4i;
-    s.e4k += denom * a4k;
-    s.e5i += denom * e5i;
-    s.e5k += denom * e5k;
+    return r;
+}
+
+__device__ __forceinline__ void tengy_pair(bool both, const double (&bc)[8], const double (&cb)[8], double denom,
+                                           const TengyIdx &vb, const TengyIdx &vc, TengySums &s)
+{
+    const TengyTerms t = tengy_terms(both, bc, cb, vb, vc);
+    s.e4i += denom * t.a4i;
+    s.e4k += denom * t.a4k;
+    s.e5i += denom * t.e5i;
+    s.e5k += denom * t.e5k;
 }
 
 template <bool BOTH>
@@ -164,21 +177,28 @@ __device__ __forceinline__ void tengy_pair(const double (&bc)[8], const double (
     tengy_pair(BOTH, bc, cb, denom, vb, vc, s);
 }
 
+// The four sums of a warp, each as warp_sum adds it up; lanes 8 e .. 8 e + 7 return the e-th (e4i, e5i, e4k, e5k).  Two
+// thirds of the shuffles of four warp_sums.
+__device__ __forceinline__ double warp_sum4(const TengySums &s, int lane)
+{
+    const bool h = lane & 16, g = lane & 8;
+    double a = h ? s.e4k : s.e4i, b = h ? s.e5k : s.e5i;  // kept
+    a += __shfl_xor_sync(0xffffffffu, h ? s.e4i : s.e4k, 16);
+    b += __shfl_xor_sync(0xffffffffu, h ? s.e5i : s.e5k, 16);
+    double c = g ? b : a;
+    c += __shfl_xor_sync(0xffffffffu, g ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    return c;
+}
+
 // Block-wide sum of the four partial energies; returns the totals in thread 0.  `scratch` must
 // hold 4 * (blockDim.x / 32) doubles.  The summation order is fixed (deterministic).
 __device__ __forceinline__ TengySums block_sum4(TengySums s, double *scratch)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    s.e4i = warp_sum(s.e4i);
-    s.e5i = warp_sum(s.e5i);
-    s.e4k = warp_sum(s.e4k);
-    s.e5k = warp_sum(s.e5k);
-    if (lane == 0) {
-        scratch[4 * warp + 0] = s.e4i;
-        scratch[4 * warp + 1] = s.e5i;
-        scratch[4 * warp + 2] = s.e4k;
-        scratch[4 * warp + 3] = s.e5k;
-    }
+    const double sum = warp_sum4(s, lane);
+    if ((lane & 7) == 0) scratch[4 * warp + (lane >> 3)] = sum;
     __syncthreads();
     TengySums r = {0.0, 0.0, 0.0, 0.0};
     if (threadIdx.x == 0) {

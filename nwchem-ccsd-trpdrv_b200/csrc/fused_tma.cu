@@ -574,6 +574,8 @@ __device__ __forceinline__ TengyIdx load_idx(const ItemCtx &cx, int x)
 }
 
 // DIAG: the pair's own mirror block is a block of the same tile (another warp, or this one, adds its terms).
+// No branches: a position past nvir takes the vectors of the last one and adds 0, so that the four positions' chains
+// (a division and some 130 FP64 instructions each) overlap.
 template <bool DIAG>
 __device__ __forceinline__ void warp_epilogue(const ItemCtx &cx, const double (&f)[8][4], const double (&gT)[8][4],
                                               int rb0, int cb0, int g, int t, int lane, double *out)
@@ -583,14 +585,13 @@ __device__ __forceinline__ void warp_epilogue(const ItemCtx &cx, const double (&
     const double *ev = cx.eorb + cx.ncor + cx.nocc;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        const int b = rb0 + perm8(g) + 8 * h;
-        if (b >= V) continue;
-        const TengyIdx vb = load_idx(cx, b);
-        const double eb = __ldg(ev + b);
+        const int b = rb0 + perm8(g) + 8 * h, bi = min(b, V - 1);
+        const TengyIdx vb = load_idx(cx, bi);
+        const double eb = __ldg(ev + bi);
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
-            const int e = 2 * h + w, c = cb0 + perm8(2 * t + w);
-            if (c >= V) continue;
+            const int e = 2 * h + w, c = cb0 + perm8(2 * t + w), ci = min(c, V - 1);
+            const bool valid = b < V && c < V;
             double fbc[8], fcb[8];
 #pragma unroll
             for (int x = 0; x < 8; ++x) {
@@ -598,19 +599,16 @@ __device__ __forceinline__ void warp_epilogue(const ItemCtx &cx, const double (&
                 fcb[x] = gT[x][e];
             }
             // omp/ccsd_tengy_c99.c:65 denominator; e_b + e_c == e_c + e_b, so (b,c) and (c,b) share it
-            tengy_pair<!DIAG>(fbc, fcb, -1.0 / (eb + __ldg(ev + c) + cx.eaijk), vb, load_idx(cx, c), su);
+            const double denom = -1.0 / (valid ? eb + __ldg(ev + ci) + cx.eaijk : 1.0);
+            const TengyTerms p = tengy_terms(!DIAG, fbc, fcb, vb, load_idx(cx, ci));
+            su.e4i += denom * (valid ? p.a4i : 0.0);
+            su.e4k += denom * (valid ? p.a4k : 0.0);
+            su.e5i += denom * (valid ? p.e5i : 0.0);
+            su.e5k += denom * (valid ? p.e5k : 0.0);
         }
     }
-    su.e4i = warp_sum(su.e4i);
-    su.e5i = warp_sum(su.e5i);
-    su.e4k = warp_sum(su.e4k);
-    su.e5k = warp_sum(su.e5k);
-    if (lane == 0 && out) {
-        out[0] = su.e4i;
-        out[1] = su.e5i;
-        out[2] = su.e4k;
-        out[3] = su.e5k;
-    }
+    const double sum = warp_sum4(su, lane);
+    if ((lane & 7) == 0 && out) out[lane >> 3] = sum;
 }
 
 // ------------------------------------------------------------------------------------------------

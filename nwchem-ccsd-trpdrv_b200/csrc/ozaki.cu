@@ -543,20 +543,6 @@ __device__ __forceinline__ void energy_operands(const GemmParams &P, char *bufs,
     }
 }
 
-// The four sums of a warp, each as warp_sum adds it up; lane 8 e (e = 0 .. 3) returns the e-th.
-__device__ __forceinline__ double warp_sum4(const TengySums &s, int lane)
-{
-    const bool h = lane & 16, g = lane & 8;
-    double a = h ? s.e4k : s.e4i, b = h ? s.e5k : s.e5i;  // kept
-    a += __shfl_xor_sync(0xffffffffu, h ? s.e4i : s.e4k, 16);
-    b += __shfl_xor_sync(0xffffffffu, h ? s.e5i : s.e5k, 16);
-    double c = g ? b : a;
-    c += __shfl_xor_sync(0xffffffffu, g ? a : b, 8);
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    return c;  // lanes 0-7: e4i, 8-15: e5i, 16-23: e4k, 24-31: e5k
-}
-
 // The energy warps (te = 0 .. NENG_THREADS - 1), one (b, c) of a half a thread.  Every wait is bounded; one that runs
 // out ends the loop in all threads.
 template <int NBUF>
