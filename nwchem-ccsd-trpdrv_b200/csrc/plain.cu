@@ -9,6 +9,8 @@
 // One triple is 8 (nvir/64)^2 tiles, less than one wave of the chip up to nvir = 300, so the plans run a batch
 // of triples per launch; single-triple callers get 32-wide tiles where the 64-wide ones would leave SMs idle.
 
+#include <type_traits>
+
 #include "device_common.cuh"
 #include "launch.h"
 
@@ -80,6 +82,43 @@ __device__ __forceinline__ void load_stage(double *stage, const Src &s, int r0, 
             cp_async_8(w, p, ok);
     }
 }
+
+// A thread's copies of one panel over the chunks with DK valid contraction indices: the sources advance by a constant.
+// Addresses and bounds worked out per copy were most of the loop's instructions beside the products (tensor pipe active
+// 72 % of the time, L2 19 %, so neither traffic nor arithmetic bounds the loop).
+template <int BM, int VEC>
+struct Copies {
+    static constexpr int U = BM * DK / VEC / NTHREAD;
+    const double *p;  // the first copy's source; the others are `next` apart
+    size_t next, advance;
+    int dst, dnext, n;  // n: copies inside the tensor
+    Copies() = default;
+    // x0: first row (column) of the panel; there is at least one such chunk
+    __device__ __forceinline__ Copies(const double *src, int ld, bool kmajor, int x0, int nvir, int tid)
+    {
+        const int W = kmajor ? BM / VEC : DK / VEC, lo = (tid % W) * VEC, hi = tid / W, step = NTHREAD / W;
+        // K-major: lo a row, hi a contraction index; X-major: lo a contraction index, hi a column
+        const int x = x0 + (kmajor ? lo : hi);
+        n = kmajor ? (x < nvir ? U : 0) : (x < nvir ? min(U, (nvir - x + step - 1) / step) : 0);
+        p = n > 0 ? src + (kmajor ? x + (size_t)hi * ld : lo + (size_t)x * ld) : src;
+        next = (size_t)step * ld;
+        advance = kmajor ? (size_t)DK * ld : DK;
+        dst = kmajor ? hi * Tile<BM>::PK + lo : hi * DK + (((lo >> 1) ^ (hi & 7)) << 1) + (lo & 1);
+        dnext = step * (kmajor ? Tile<BM>::PK : DK);  // X-major: columns a multiple of 8 apart, the same swizzle
+    }
+    __device__ __forceinline__ void issue(double *panel)
+    {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const double *s = u < n ? p + u * next : p;
+            if (VEC == 2)
+                cp_async_16(panel + dst + u * dnext, s, u < n);
+            else
+                cp_async_8(panel + dst + u * dnext, s, u < n);
+        }
+        if (n > 0) p += advance;
+    }
+};
 
 // One chunk's products.  FULL: every m16 and n8 tile of the warp has valid outputs; else only the first mi_n, ni_n.
 template <int BM, bool BK, bool FULL>
@@ -189,7 +228,7 @@ __device__ __forceinline__ bool one_sources(const trpdrv_plain_args &P, int x, S
     return true;
 }
 
-template <int BM, int VEC, int STAGES, bool BATCH>
+template <int BM, int VEC, int STAGES, bool BATCH, bool FAST>
 __device__ __forceinline__ void gemm_body(const trpdrv_plain_args *one, const BatchArgs *batch, int nvir, int nocc,
                                           double *fbase, bool neg)
 {
@@ -207,9 +246,17 @@ __device__ __forceinline__ void gemm_body(const trpdrv_plain_args *one, const Ba
     ph[1].klim = nocc;
     ph[1].bk = 0;
     const int nV = (nvir + DK - 1) / DK, nO = (nocc + DK - 1) / DK, nch = nV + nO;
-    auto load = [&](int ch) {
-        if (ch < nch) {
-            double *st = smem + (ch % STAGES) * L::STAGE;
+    const int nfull = FAST ? nvir / DK : 0;  // chunks copied by running pointers, their products without branches
+    Copies<BM, VEC> ca, cb;
+    if (FAST) {
+        ca = Copies<BM, VEC>(ph[0].a, ph[0].lda, true, r0, nvir, tid);
+        cb = Copies<BM, VEC>(ph[0].b, ph[0].ldb, ph[0].bk, c0, nvir, tid);
+    }
+    auto load = [&](int ch, double *st) {
+        if (FAST && ch < nfull) {
+            ca.issue(st);
+            cb.issue(st + L::APANEL);
+        } else if (ch < nch) {
             if (ch < nV)
                 load_stage<BM, VEC>(st, ph[0], r0, c0, ch * DK, nvir, tid);
             else
@@ -230,28 +277,50 @@ __device__ __forceinline__ void gemm_body(const trpdrv_plain_args *one, const Ba
     int mi_n = mr <= 0 ? 0 : (mr + 15) >> 4, ni_n = nc <= 0 ? 0 : (nc + 7) >> 3;
     if (mi_n > L::MI) mi_n = L::MI;
     if (ni_n > L::NI) ni_n = L::NI;
-    const bool whole = mi_n == L::MI && ni_n == L::NI;
+    const bool whole = !FAST && mi_n == L::MI && ni_n == L::NI;
 
+    double *ring = smem, *fill = smem;  // the stage to multiply and the stage to fill
+    auto next = [&](double *st) { return st == smem + (STAGES - 1) * L::STAGE ? smem : st + L::STAGE; };
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) load(s);
-    for (int ch = 0; ch < nch; ++ch) {
+    for (int s = 0; s < STAGES - 1; ++s) {
+        load(s, fill);
+        fill = next(fill);
+    }
+    int ch = 0;
+    auto step = [&](auto products) {
         cp_async_wait<STAGES - 2>();
         __syncthreads();
-        load(ch + STAGES - 1);
-        const double *As = smem + (ch % STAGES) * L::STAGE, *Bs = As + L::APANEL;
+        load(ch + STAGES - 1, fill);
+        fill = next(fill);
+        products(ring, ring + L::APANEL);
+        ring = next(ring);
+        ++ch;
+    };
+    // the chunks of the K = nvir product without a branch among their products
+    auto fast = [&](auto bk, auto full) {
+#pragma unroll 1
+        while (ch < nfull)
+            step([&](const double *As, const double *Bs) {
+                chunk<BM, decltype(bk)::value, decltype(full)::value>(As, Bs, wm, wn, g, t, 2, false, mi_n, ni_n, acc);
+            });
+    };
+    if (FAST && r0 + BM <= nvir && c0 + BM <= nvir)  // the whole CTA: its warps take the same loop
+        ph[0].bk ? fast(std::true_type{}, std::true_type{}) : fast(std::false_type{}, std::true_type{});
+#pragma unroll 1
+    while (ch < nch) {
         const bool virt = ch < nV;
         const int steps = (virt ? nvir - ch * DK : nocc - (ch - nV) * DK) > 8 ? 2 : 1;
-        if (whole) {
-            if (virt && ph[0].bk)
+        step([&](const double *As, const double *Bs) {
+            if (mi_n <= 0 || ni_n <= 0) return;
+            if (whole && virt && ph[0].bk)
                 chunk<BM, true, true>(As, Bs, wm, wn, g, t, steps, false, 0, 0, acc);
-            else
+            else if (whole)
                 chunk<BM, false, true>(As, Bs, wm, wn, g, t, steps, neg && !virt, 0, 0, acc);
-        } else if (mi_n > 0 && ni_n > 0) {
-            if (virt && ph[0].bk)
+            else if (virt && ph[0].bk)
                 chunk<BM, true, false>(As, Bs, wm, wn, g, t, steps, false, mi_n, ni_n, acc);
             else
                 chunk<BM, false, false>(As, Bs, wm, wn, g, t, steps, neg && !virt, mi_n, ni_n, acc);
-        }
+        });
     }
     cp_async_wait<0>();
     // a batch's products overlap the energies of the batch before; its f goes to the same buffer only after them
@@ -269,20 +338,20 @@ __device__ __forceinline__ void gemm_body(const trpdrv_plain_args *one, const Ba
             }
 }
 
-template <int BM, int VEC>
+template <int BM, int VEC, bool FAST>
 __global__ void __launch_bounds__(NTHREAD, BM == 64 ? 3 : 6) plain_gemm_kernel(const __grid_constant__ trpdrv_plain_args args)
 {
     // the dependent tengy launch may start its prologue (it waits for this grid before reading f)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (args.counter && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) *args.counter = 0u;
-    gemm_body<BM, VEC, one_stages<BM>(), false>(&args, nullptr, args.nvir, args.nocc, args.f, args.neg2 != 0);
+    gemm_body<BM, VEC, one_stages<BM>(), false, FAST>(&args, nullptr, args.nvir, args.nocc, args.f, args.neg2 != 0);
 }
 
-template <int BM, int VEC>
+template <int BM, int VEC, bool FAST>
 __global__ void __launch_bounds__(NTHREAD, BM == 64 ? 3 : 5) plain_batch_kernel(const __grid_constant__ BatchArgs args)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    gemm_body<BM, VEC, BATCH_STAGES, true>(nullptr, &args, args.S.nvir, args.S.nocc, args.f, false);
+    gemm_body<BM, VEC, BATCH_STAGES, true, FAST>(nullptr, &args, args.S.nvir, args.S.nocc, args.f, false);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -300,19 +369,28 @@ struct TengyIn {
     unsigned *counter;
 };
 
-__device__ __forceinline__ TengyIdx load_idx(const TengyIn &P, int x)
+// The per-index vectors of a tile pair, rows of 16 at b and then at c: loaded together with f.  Loaded by each thread
+// after the exchange instead they cost a second round trip to L2 (20, 200: 30.8 against 30.3 ms for all triples, a
+// single triple 19.8 against 18.7 us).
+constexpr int TVROWS = 14;
+
+__device__ __forceinline__ double vec_entry(const TengyIn &P, int row, int n)
 {
-    return {__ldg(P.t1v1 + x), __ldg(P.t1v2 + x), __ldg(P.dintx1 + x), __ldg(P.dintx2 + x), __ldg(P.dintc1 + x),
-            __ldg(P.dintc2 + x)};
+    const int kind = row >= 7 ? row - 7 : row;
+    const double *src = kind == 0 ? P.t1v1 : kind == 1 ? P.t1v2 : kind == 2 ? P.dintx1 : kind == 3 ? P.dintx2
+                      : kind == 4 ? P.dintc1 : kind == 5 ? P.dintc2 : P.ev;
+    return __ldg(src + n);
 }
 
 // One CTA: the terms of (b, c) and (c, b) over a 16-wide tile pair B <= C, one thread per (b, c).  Both tiles of all
 // eight f are read with 128-byte coalesced loads, 16 independent ones per thread; the (c, b) values cross
 // through shared memory.  A latency-bound kernel (a single triple has 91 CTAs at nvir = 200): 16-wide tiles give
 // four times the CTAs of 32-wide ones and one round of loads each.
+// CHAIN: lets the next batch's products start.
+template <bool CHAIN>
 __device__ __forceinline__ void tengy_body(const TengyIn &P, int nvir)
 {
-    __shared__ double xch[8][TW][TW + 1];
+    __shared__ double xch[8][TW][TW + 1], vsh[TVROWS][TW];
     __shared__ double red[4 * (TNTHREAD / 32)];
     __shared__ int s_last;
     const int nb = (nvir + TW - 1) / TW, tid = threadIdx.x;
@@ -326,6 +404,10 @@ __device__ __forceinline__ void tengy_body(const TengyIn &P, int nvir)
     const int b = B * TW + r, c = C * TW + q;    // this thread's (b, c)
     const int cr = C * TW + r, bq = B * TW + q;  // the mirrored tile's element it loads
     const size_t vv = (size_t)nvir * nvir;
+    const int vrow = tid / TW, vn = (vrow < 7 ? B : C) * TW + r;
+    const double ve = vrow < TVROWS && vn < nvir ? vec_entry(P, vrow, vn) : 0.0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // f (and a single triple's counter) come from the launch before
+    if (CHAIN) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     double fbc[8], fcb[8];
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
@@ -335,16 +417,16 @@ __device__ __forceinline__ void tengy_body(const TengyIn &P, int nvir)
     }
 #pragma unroll
     for (int x = 0; x < 8; ++x) xch[x][q][r] = diag ? fbc[x] : fcb[x];
+    if (vrow < TVROWS) vsh[vrow][r] = ve;
     __syncthreads();
     TengySums su = {0.0, 0.0, 0.0, 0.0};
     if (b < nvir && c < nvir) {
 #pragma unroll
         for (int x = 0; x < 8; ++x) fcb[x] = xch[x][r][q];
-        const double denom = -1.0 / (__ldg(P.ev + b) + __ldg(P.ev + c) + P.eaijk);
-        if (diag)
-            tengy_pair<false>(fbc, fcb, denom, load_idx(P, b), load_idx(P, c), su);
-        else
-            tengy_pair<true>(fbc, fcb, denom, load_idx(P, b), load_idx(P, c), su);
+        const double denom = -1.0 / (vsh[6][r] + vsh[13][q] + P.eaijk);
+        const TengyIdx ib = {vsh[0][r], vsh[1][r], vsh[2][r], vsh[3][r], vsh[4][r], vsh[5][r]};
+        const TengyIdx ic = {vsh[7][q], vsh[8][q], vsh[9][q], vsh[10][q], vsh[11][q], vsh[12][q]};
+        tengy_pair(!diag, fbc, fcb, denom, ib, ic, su);
     }
     const TengySums tot = block_sum4(su, red);
     if (tid == 0) {
@@ -396,11 +478,12 @@ __global__ void __launch_bounds__(TNTHREAD) tengy_kernel(const __grid_constant__
     P.partial = a.block_partial;
     P.out = a.out4;
     P.counter = a.counter;
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // f and the counter come from the launch before
-    tengy_body(P, a.nvir);
+    tengy_body<false>(P, a.nvir);
 }
 
-__global__ void __launch_bounds__(TNTHREAD) tengy_batch_kernel(const __grid_constant__ BatchArgs a)
+// Four CTAs per SM (64 registers): a CTA waits on its 16 loads, a division and the sums more than it computes.  39 triples of
+// nvir = 200 took 47 us with three, all triples of nocc = 20 30.3 against 29.6 ms.
+__global__ void __launch_bounds__(TNTHREAD, 4) tengy_batch_kernel(const __grid_constant__ BatchArgs a)
 {
     const trpdrv_dev_system &S = a.S;
     const int n = blockIdx.y;
@@ -419,9 +502,7 @@ __global__ void __launch_bounds__(TNTHREAD) tengy_batch_kernel(const __grid_cons
     P.partial = a.block_partial + (size_t)n * gridDim.x * 4;
     P.out = S.rec + 4 * (a.pos0 + n);
     P.counter = a.counter + n;
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // f comes from the launch before
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    tengy_body(P, S.nvir);
+    tengy_body<true>(P, S.nvir);
 }
 
 // 64-wide tiles where they fill the chip once over (two CTAs per SM) and cover not much more than 32-wide ones:
@@ -433,22 +514,44 @@ bool wide_tiles(int nvir, long long triples)
     return n64 * n64 * 8 * triples >= 2 * 148 && 100 * 4 * n64 * n64 <= 115 * n32 * n32;
 }
 
-template <int BM, int VEC>
+// Running pointers where their set-up pays, from eight copies a thread and panel of 32 rows on: nvir >= 64, or 32 if the
+// copies are of 8 bytes.
+// All triples, ms without and with: (20, 200) 29.63, 28.2; (8, 300) 5.15, 4.91; (17, 111) 4.40, 4.15; (30, 33) 3.67, 3.37;
+// (12, 100) 1.21, 1.18, but (10, 60) 0.155, 0.161 and (16, 16) 0.100, 0.107.
+bool fast_copies(int nvir, int vec2) { return nvir / DK * (vec2 ? 2 : 4) >= 8; }
+
+// f(<BM, VEC, FAST>)
+template <class F>
+int with_variant(bool wide, int vec2, int nvir, F f)
+{
+    using W = std::integral_constant<int, 64>;
+    using N = std::integral_constant<int, 32>;
+    using V1 = std::integral_constant<int, 1>;
+    using V2 = std::integral_constant<int, 2>;
+    using Yes = std::true_type;
+    using No = std::false_type;
+    const bool fast = fast_copies(nvir, vec2);
+    if (wide) return !vec2 ? f(W{}, V1{}, Yes{}) : fast ? f(W{}, V2{}, Yes{}) : f(W{}, V2{}, No{});  // nvir > 32
+    if (fast) return vec2 ? f(N{}, V2{}, Yes{}) : f(N{}, V1{}, Yes{});
+    return vec2 ? f(N{}, V2{}, No{}) : f(N{}, V1{}, No{});
+}
+
+template <int BM, int VEC, bool FAST>
 int set_smem()
 {
-    cudaError_t e = cudaFuncSetAttribute(plain_gemm_kernel<BM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(plain_gemm_kernel<BM, VEC, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)Tile<BM>::smem(one_stages<BM>()));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(plain_batch_kernel<BM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(plain_batch_kernel<BM, VEC, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)Tile<BM>::smem(BATCH_STAGES));
     return (int)e;
 }
 
-template <int BM, int VEC>
+template <int BM, int VEC, bool FAST>
 int launch_one(const trpdrv_plain_args &a, cudaStream_t st)
 {
     const unsigned nbt = (a.nvir + BM - 1) / BM;
-    plain_gemm_kernel<BM, VEC><<<dim3(nbt, nbt, 8), NTHREAD, Tile<BM>::smem(one_stages<BM>()), st>>>(a);
+    plain_gemm_kernel<BM, VEC, FAST><<<dim3(nbt, nbt, 8), NTHREAD, Tile<BM>::smem(one_stages<BM>()), st>>>(a);
     return (int)cudaGetLastError();
 }
 
@@ -469,11 +572,11 @@ int launch(void (*kernel)(const A), dim3 grid, int threads, size_t smem, bool de
     return (int)cudaLaunchKernelEx(&cfg, kernel, args);
 }
 
-template <int BM, int VEC>
+template <int BM, int VEC, bool FAST>
 int launch_batch(const BatchArgs &a, int n, bool dependent, cudaStream_t st)
 {
     const unsigned nbt = (a.S.nvir + BM - 1) / BM;
-    return launch(plain_batch_kernel<BM, VEC>, dim3(nbt, nbt, 8 * n), NTHREAD, Tile<BM>::smem(BATCH_STAGES), dependent, a, st);
+    return launch(plain_batch_kernel<BM, VEC, FAST>, dim3(nbt, nbt, 8 * n), NTHREAD, Tile<BM>::smem(BATCH_STAGES), dependent, a, st);
 }
 
 }  // namespace plain
@@ -484,9 +587,9 @@ using namespace trpdrv;
 extern "C" int trpdrv_launch_plain_gemm(const trpdrv_plain_args *args, int vec2, void *stream)
 {
     cudaStream_t st = (cudaStream_t)stream;
-    if (plain::wide_tiles(args->nvir, 1))
-        return vec2 ? plain::launch_one<64, 2>(*args, st) : plain::launch_one<64, 1>(*args, st);
-    return vec2 ? plain::launch_one<32, 2>(*args, st) : plain::launch_one<32, 1>(*args, st);
+    return plain::with_variant(plain::wide_tiles(args->nvir, 1), vec2, args->nvir, [&](auto bm, auto vec, auto fast) {
+        return plain::launch_one<decltype(bm)::value, decltype(vec)::value, decltype(fast)::value>(*args, st);
+    });
 }
 
 extern "C" int64_t trpdrv_tengy_pairs(int nvir)
@@ -521,11 +624,9 @@ extern "C" int trpdrv_launch_plain_batch(const trpdrv_dev_system *h_sys, int64_t
     a.f = f;
     a.block_partial = block_partial;
     a.counter = counter;
-    int e;
-    if (plain::wide_tiles(h_sys->nvir, n))
-        e = vec2 ? plain::launch_batch<64, 2>(a, n, chained, st) : plain::launch_batch<64, 1>(a, n, chained, st);
-    else
-        e = vec2 ? plain::launch_batch<32, 2>(a, n, chained, st) : plain::launch_batch<32, 1>(a, n, chained, st);
+    const int e = plain::with_variant(plain::wide_tiles(h_sys->nvir, n), vec2, h_sys->nvir, [&](auto bm, auto vec, auto fast) {
+        return plain::launch_batch<decltype(bm)::value, decltype(vec)::value, decltype(fast)::value>(a, n, chained, st);
+    });
     if (e) return e;
     return plain::launch(plain::tengy_batch_kernel, dim3((unsigned)trpdrv_tengy_pairs(h_sys->nvir), (unsigned)n),
                          plain::TNTHREAD, 0, true, a, st);
@@ -533,9 +634,12 @@ extern "C" int trpdrv_launch_plain_batch(const trpdrv_dev_system *h_sys, int64_t
 
 extern "C" int trpdrv_plain_init(void)
 {
-    int e = plain::set_smem<64, 1>();
-    if (!e) e = plain::set_smem<64, 2>();
-    if (!e) e = plain::set_smem<32, 1>();
-    if (!e) e = plain::set_smem<32, 2>();
+    int e = plain::set_smem<64, 1, true>();
+    if (!e) e = plain::set_smem<64, 2, true>();
+    if (!e) e = plain::set_smem<64, 2, false>();
+    if (!e) e = plain::set_smem<32, 1, true>();
+    if (!e) e = plain::set_smem<32, 2, true>();
+    if (!e) e = plain::set_smem<32, 1, false>();
+    if (!e) e = plain::set_smem<32, 2, false>();
     return e;
 }
