@@ -200,7 +200,8 @@ struct trpdrv_plan {
     int *d_status;
     double *d_bsum;   /* block sums of the totals */
     unsigned *d_done; /* finished blocks per system */
-    double *h_res;    /* pinned: totals per system (emp4 hi, lo, emp5 hi, lo), then the status word */
+    double *h_res;    /* registered: totals per system (emp4 hi, lo, emp5 hi, lo), then the status word */
+    double *d_res;    /* its device address */
     int64_t total_items;
     double *d_f, *d_bpart; /* plain form: f and energy partials of one batch of triples */
     unsigned *d_tcount;
@@ -281,7 +282,8 @@ static void plan_free(trpdrv_plan *p)
     if (p->d_counter) cudaFree(p->d_counter);
     if (p->d_bsum) cudaFree(p->d_bsum);
     if (p->d_done) cudaFree(p->d_done);
-    if (p->h_res) cudaFreeHost(p->h_res);
+    if (p->d_res) cudaHostUnregister(p->h_res);
+    free(p->h_res);
     if (p->d_f) cudaFree(p->d_f);
     if (p->d_fbuf) cudaFree(p->d_fbuf);
     for (int h = 0; h < 2; ++h) {
@@ -451,8 +453,18 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
     CUDA_TRY(cudaMalloc((void **)&p->d_bsum, sizeof(double) * 4 * TRPDRV_FINISH_BLOCKS * (size_t)p->nsys));
     CUDA_TRY(cudaMalloc((void **)&p->d_done, sizeof(unsigned) * (size_t)p->nsys));
     CUDA_TRY(cudaMemset(p->d_done, 0, sizeof(unsigned) * (size_t)p->nsys));
-    CUDA_TRY(cudaMallocHost((void **)&p->h_res, sizeof(double) * (4 * (size_t)p->nsys + 1)));
-    memset(p->h_res, 0, sizeof(double) * (4 * (size_t)p->nsys + 1));
+    /* whole pages of our own, registered: 0.3 ms, where cudaMallocHost takes 1 to 2.7 */
+    const size_t res_bytes = (sizeof(double) * (4 * (size_t)p->nsys + 1) + 4095) / 4096 * 4096;
+    void *res = aligned_alloc(4096, res_bytes);
+    if (!res) return fail(TRPDRV_ERR_NOMEM, "out of host memory");
+    p->h_res = (double *)res;
+    memset(res, 0, res_bytes);
+    CUDA_TRY(cudaHostRegister(res, res_bytes, cudaHostRegisterPortable | cudaHostRegisterMapped));
+    {
+        const cudaError_t re = cudaHostGetDevicePointer((void **)&p->d_res, res, 0);
+        if (re != cudaSuccess) cudaHostUnregister(res);
+        CUDA_TRY(re);
+    }
     if (o->mode == TRPDRV_MODE_EMULATED) {
         p->fbuf_batch = o->batch > TUNE_MAX_BATCH ? o->batch : TUNE_MAX_BATCH;
         p->fbuf_half = 8 * (size_t)p->fbuf_batch * maxv * trpdrv_oz_ldf(maxv);
@@ -809,7 +821,7 @@ static int enqueue_finish(trpdrv_plan *p, cudaStream_t st, int64_t *launches)
         LAUNCH_TRY(trpdrv_launch_records(p->h_dev, p->d_dev, p->nsys, st));
         if (launches) ++*launches;
     }
-    LAUNCH_TRY(trpdrv_launch_totals(p->h_dev, p->d_dev, p->nsys, p->d_bsum, p->d_done, p->d_status, p->h_res, st));
+    LAUNCH_TRY(trpdrv_launch_totals(p->h_dev, p->d_dev, p->nsys, p->d_bsum, p->d_done, p->d_status, p->d_res, st));
     if (launches) ++*launches;
     return TRPDRV_OK;
 }
