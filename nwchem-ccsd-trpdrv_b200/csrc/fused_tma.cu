@@ -1,15 +1,18 @@
-// Fused persistent triples kernel, TMA + mbarrier pipeline (sm_100a, FP64 DMMA).
+// Fused persistent triples kernel (sm_100a, FP64 DMMA), operands staged by TMA or cp.async.
 //
-// Same work decomposition and register-resident energy epilogue as fused.cu (a work item is
-// (triple, tile pair {B,C}); each consumer warp owns a 16(b) x 8(c) sub-block and computes all eight
-// f of omp/ccsd_trpdrv_omp_cbody.c:70-117 at (b,c) and, through the operand-swapped MMA, at (c,b)),
-// but the operand panels are staged by the Tensor Memory Accelerator:
+// A work item is (triple, tile pair {B,C}); each consumer warp owns a 16(b) x 8(c) sub-block and computes all eight
+// f of omp/ccsd_trpdrv_omp_cbody.c:70-117 at (b,c) and, through the operand-swapped MMA, at (c,b), so that the
+// energies are evaluated from registers.
 //
-//  * one producer thread takes work tickets, writes each item's context to a ring in shared memory
-//    and issues, per chunk of DK contraction indices, one or two cp.async.bulk.tensor loads per
-//    panel (each CTA loads its own copy) that complete on the stage's "full" mbarrier;
-//  * eight consumer warps wait on "full", run the m16n8k8 DMMAs straight from the staged panels and
+//  * four producer warps: the first takes work tickets and writes each item's context to a ring in shared memory; all
+//    of them fill, per chunk of DK contraction indices, the stage's panels, by cp.async.bulk.tensor loads or (odd or
+//    unaligned tensors, more than eight systems) by cp.async, that complete on the stage's "full" mbarrier;
+//  * eight consumer warps wait on "full", run the DMMAs straight from the staged panels and
 //    release the stage through its "empty" mbarrier; no CTA-wide barrier in the main loop.
+//
+// What bounds it: the FP64 tensor pipe (37.1 TFLOP/s).  nocc 16, nvir 288: 34.9 TFLOP/s (27.8 with branches among a
+// chunk's MMAs, generic loads and an epilogue with branches); 16, 300: 33.5; 20, 200: 29.9, where 8 of the 208 covered
+// indices are padding and an item's epilogue and start-up are 12 % of it; 10, 60: 18.8; 13, 151 (cp.async): 23.8.
 //
 // Panel layouts in shared memory (4 KB per panel, 16 panels per stage, DK = 16):
 //  * K-major panels (rows contiguous in HBM: Jia/Kia/Jka/Kka, -Tia/-Xia/-Tka/-Xka, T2 as T(c,d)):
@@ -32,7 +35,7 @@
 // ragged tails in nvir and nocc are zero-filled by the TMA unit.
 //
 // Every wait is bounded (globaltimer); a wait that runs out sets bit 1 of *status and the CTA stops
-// issuing work.  Requires even nvir and nocc and 16-byte aligned tensors (host checks).
+// issuing work.  TMA staging requires even nvir and nocc and 16-byte aligned tensors (host checks).
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -47,7 +50,7 @@ constexpr int T = TRPDRV_TILE;  // 32
 constexpr int DK = 16;          // contraction indices per stage (two m16n8k8 steps; 128-byte box rows)
 constexpr int STAGES = 3;
 constexpr int NCW = TRPDRV_FUSED_SLOTS;  // consumer warps (8) = two warpgroups
-constexpr int NTHREAD = (NCW + 4) * 32;  // + one producer warpgroup (one thread issues)
+constexpr int NTHREAD = (NCW + 4) * 32;  // + one producer warpgroup
 // Register split by setmaxnreg: launched at 65536 / 384 = 168 per thread; the producer warpgroup drops to 88 and
 // the two consumer warpgroups rise to 208 (2*128*208 + 128*88 = 384*168): at this split the MMA loops do not
 // spill and the producers least (-Xptxas -v; 216 / 64 and 200 / 96 both spill more).
@@ -518,17 +521,98 @@ __device__ __forceinline__ bool run_packed(int n, const FragOffsets &fo, const P
     return true;
 }
 
+// The last chunk of either contraction, where four of its indices or fewer remain past a multiple of 8: one k4 step
+// instead of a k8 step over zeros.  10, 60: 0.123 to 0.119 ms; 12, 100: 0.802 to 0.778; 16, 300: 29.70 to 29.55; 20, 200:
+// 19.88 to 19.81.
+//
+// Products of family FAM with the four contraction indices 8 ks .. 8 ks + 3 of a chunk, m16n8k4: lane t holds index
+// 8 ks + t (in a k8 step 2t and 2t + 1).
+template <bool PH1, bool DIAG, int FAM>
+__device__ __forceinline__ void quarter_products(const FragOffsets &fo, const char *st, const Panels &pn, int ks, int t,
+                                                 double (&f)[8][4], double (&gT)[8][4])
+{
+    constexpr int x0 = FAM * 4;
+    const int r = fo.xA0 >> 7, c = fo.xB >> 7, kk = ks * 1024, kx = ks * 64;
+    auto ldK = [&](int panel, int x) { return FragOffsets::ld(st, panel + kk + kmajor_off(t, x)); };
+    auto ldX = [&](int panel, int x) {
+        return FragOffsets::ld(st, panel + x * 128 + ((((t >> 1) ^ (x & 7)) << 4) ^ kx) + ((t & 1) << 3));
+    };
+    {
+        const double aj[2] = {ldK(pn.a0[0], r), ldK(pn.a0[0], r + 8)}, ak[2] = {ldK(pn.a1[0], r), ldK(pn.a1[0], r + 8)};
+        const double b1 = PH1 ? ldX(pn.b0[0], c) : ldK(pn.b0[0], c), b3 = ldX(pn.b1[0], c);
+        dmma_16x8x4(f[x0 + 0], aj[0], aj[1], b1);
+        dmma_16x8x4(f[x0 + 1], ak[0], ak[1], b1);
+        dmma_16x8x4(f[x0 + 2], aj[0], aj[1], b3);
+        dmma_16x8x4(f[x0 + 3], ak[0], ak[1], b3);
+    }
+    if (DIAG) return;
+    const double b1[2] = {PH1 ? ldX(pn.a0[1], r) : ldK(pn.a0[1], r), PH1 ? ldX(pn.a0[1], r + 8) : ldK(pn.a0[1], r + 8)};
+    const double b3[2] = {ldX(pn.a1[1], r), ldX(pn.a1[1], r + 8)};
+    const double aj = ldK(pn.b0[1], c), ak = ldK(pn.b1[1], c);
+    dmma_16x8x4(gT[x0 + 0], b1[0], b1[1], aj);
+    dmma_16x8x4(gT[x0 + 1], b1[0], b1[1], ak);
+    dmma_16x8x4(gT[x0 + 2], b3[0], b3[1], aj);
+    dmma_16x8x4(gT[x0 + 3], b3[0], b3[1], ak);
+}
+
+// The last chunk of a phase where its last 8 contraction indices hold 1 to 4 valid ones: kind 1, those alone, or 2, a
+// k8 step before them; 0, no such chunk.
+template <int KS, bool PH1, bool DIAG, bool SAME>
+__device__ __forceinline__ bool run_quarter(int kind, const FragOffsets &fo, const Pipe &pp, RingPos &rp, double (&f)[8][4],
+                                            double (&gT)[8][4])
+{
+    constexpr int LAST = SAME ? 0 : 1;
+    if (kind == 0) return true;
+    if (!pp.wait(rp)) return false;
+    const char *st = pp.stages + (size_t)rp.stage * STAGE_BYTES;
+    Group unused;
+    if (kind == 2) {
+        if (!SAME) family_products<KS, 1, PH1, DIAG, 0, false>(fo, st, item_panels<0>(), f, gT, unused);
+        family_products<KS, 1, PH1, DIAG, LAST, false>(fo, st, item_panels<LAST>(), f, gT, unused);
+    }
+    const int t = pp.lane & 3;
+    if (!SAME) quarter_products<PH1, DIAG, 0>(fo, st, item_panels<0>(), kind - 1, t, f, gT);
+    quarter_products<PH1, DIAG, LAST>(fo, st, item_panels<LAST>(), kind - 1, t, f, gT);
+    pp.release(rp);
+    return true;
+}
+
+template <int KS, bool PH1, bool SAME>
+__device__ __forceinline__ bool run_packed_quarter(int kind, const FragOffsets &fo, const Panels &pn, const Pipe &pp, RingPos &rp,
+                                                   double (&f)[8][4], double (&gT)[8][4])
+{
+    if (kind == 0) return true;
+    const int t = pp.lane & 3;
+    Group unused;
+    if (!pp.wait(rp)) return false;
+    const char *st = pp.stages + (size_t)rp.stage * STAGE_BYTES;
+    if (kind == 2) family_products<KS, 1, PH1, false, 0, false>(fo, st, pn, f, gT, unused);
+    quarter_products<PH1, false, 0>(fo, st, pn, kind - 1, t, f, gT);
+    pp.release(rp);
+    if (SAME) return true;
+    if (!pp.wait(rp)) return false;
+    st = pp.stages + (size_t)rp.stage * STAGE_BYTES;
+    if (kind == 2) family_products<KS, 1, PH1, false, 1, false>(fo, st, pn, f, gT, unused);
+    quarter_products<PH1, false, 1>(fo, st, pn, kind - 1, t, f, gT);
+    pp.release(rp);
+    return true;
+}
+
 // The item's chunks by kind: full and one-k-step chunks of the virtual phase, then of the occupied one (the last
 // chunk of a phase runs one k-step when the second lies entirely in the zero padding).
 struct ChunkCounts {
-    int v2, v1, o2, o1;
+    int v2, v1, vq, o2, o1, oq;
+    __device__ __forceinline__ static void split(int n, int &n2, int &n1, int &nq)
+    {
+        const int chunks = (n + DK - 1) / DK, last = n - (chunks - 1) * DK;  // 1 .. 16 indices in the last one
+        nq = last <= 4 ? 1 : last > 8 && last <= 12 ? 2 : 0;
+        n1 = last > 4 && last <= 8;
+        n2 = chunks - n1 - (nq > 0);
+    }
     __device__ __forceinline__ ChunkCounts(int nvir, int nocc)
     {
-        const int nV = (nvir + DK - 1) / DK, nO = (nocc + DK - 1) / DK;
-        v1 = nvir - (nV - 1) * DK <= 8;
-        o1 = nocc - (nO - 1) * DK <= 8;
-        v2 = nV - v1;
-        o2 = nO - o1;
+        split(nvir, v2, v1, vq);
+        split(nocc, o2, o1, oq);
     }
 };
 
@@ -538,8 +622,10 @@ __device__ __forceinline__ bool run_item(const ChunkCounts &n, const FragOffsets
 {
     return run_chunks<KS, 2, false, DIAG, SAME>(n.v2, fo, pp, rp, f, gT) &&
            run_chunks<KS, 1, false, DIAG, SAME>(n.v1, fo, pp, rp, f, gT) &&
+           run_quarter<KS, false, DIAG, SAME>(n.vq, fo, pp, rp, f, gT) &&
            run_chunks<KS, 2, true, DIAG, SAME>(n.o2, fo, pp, rp, f, gT) &&
-           run_chunks<KS, 1, true, DIAG, SAME>(n.o1, fo, pp, rp, f, gT);
+           run_chunks<KS, 1, true, DIAG, SAME>(n.o1, fo, pp, rp, f, gT) &&
+           run_quarter<KS, true, DIAG, SAME>(n.oq, fo, pp, rp, f, gT);
 }
 
 template <int KS, bool SAME>
@@ -548,8 +634,10 @@ __device__ __forceinline__ bool run_packed_item(const ChunkCounts &n, const Frag
 {
     return run_packed<KS, 2, false, SAME>(n.v2, fo, pn, pp, rp, f, gT) &&
            run_packed<KS, 1, false, SAME>(n.v1, fo, pn, pp, rp, f, gT) &&
+           run_packed_quarter<KS, false, SAME>(n.vq, fo, pn, pp, rp, f, gT) &&
            run_packed<KS, 2, true, SAME>(n.o2, fo, pn, pp, rp, f, gT) &&
-           run_packed<KS, 1, true, SAME>(n.o1, fo, pn, pp, rp, f, gT);
+           run_packed<KS, 1, true, SAME>(n.o1, fo, pn, pp, rp, f, gT) &&
+           run_packed_quarter<KS, true, SAME>(n.oq, fo, pn, pp, rp, f, gT);
 }
 
 // Brings the 128-byte lines of the energy vectors the item's epilogue will read into L1 (lanes 0..27:
@@ -565,7 +653,7 @@ __device__ __forceinline__ void prefetch_epilogue(const ItemCtx &cx, int lane)
 }
 
 // ------------------------------------------------------------------------------------------------
-// energies of one warp's sub-block, in registers (as fused.cu)
+// energies of one warp's sub-block, in registers
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ TengyIdx load_idx(const ItemCtx &cx, int x)
 {
