@@ -25,11 +25,11 @@ nocc=40, nvir=300 (32,800 triples, 16.06 TFLOP per step), seeded synthetic input
 --workload c3: the emulated form at nocc=30, nvir=400 with log-uniform integral magnitudes in
   [1e-6, 1]: `value` = triples/s of the emulated form (7 slices), beside the native FP64 fused kernel
   on the same system and the slice sweep with its errors.
---workload c1: the plain per-triple FP64 path (one grouped 16-GEMM launch and one tengy launch per
-  triple) at nocc=20, nvir=200, every triple per step, beside the reference's CPU body.
+--workload c1: the plain FP64 path (f in memory between a launch of the GEMMs and one of the energies, a
+  batch of triples each) at nocc=20, nvir=200, every triple per step, beside the reference's CPU body.
 --workload c4: six systems of uneven size, (8,80) (12,150) (16,220) (24,310) (32,380) (40,450), in
   one fused FP64 launch: `value` = aggregate triples/s; per-system energies checked against
-  single-system plans; compared with one plain FP64 launch pair per triple, serially per system.
+  single-system plans; compared with the plain FP64 path, serially per system.
 --probe-int8: the tcgen05 int8 issue-probe table (N = 64 / 128 / 256 for one SM, a CTA pair and the
   contraction kernel's stage handshake) as one JSON line; nothing else runs.
 With torchrun (N > 1) every rank runs the whole workload for its own virtual index a (weak scaling: the
@@ -105,7 +105,7 @@ def parse():
 def workload_text(name, nocc, nvir):
     n = nocc * nocc * (nocc + 1) // 2
     if name == "c1":
-        return (f"plain per-triple FP64 path (one grouped 16-GEMM launch + one tengy launch per triple), "
+        return (f"plain FP64 path (a launch of the GEMMs + one of tengy per batch of triples), "
                 f"nocc={nocc} nvir={nvir}, all {n} (i,j,k) triples of one a per step")
     if name == "c3":
         return (f"emulated-FP64 triples body (Ozaki int8 digit slices on tcgen05, {DEFAULT_SLICES} slices, "
@@ -196,6 +196,10 @@ def config_for(args):
 def run_reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    if not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libtrpdrv_ref.so")):
+        print(json.dumps({"impl": "reference", "unavailable": "the compiled reference (oracle/_ref) is not built here: "
+                          "its sources are not present"}), flush=True)
         return
     shapes = workload_shapes(args.workload, args.nocc, args.nvir)
     counts = [o * o * (o + 1) // 2 for o, _, _, _ in shapes]
@@ -543,8 +547,8 @@ def plain_sample(T, R, s, flop_triple, frac=16):
         pms = pe0.elapsed_time(pe1)
         nplain = pp.num_triples(0)
     return {"value": nplain / (pms * 1e-3), "unit": "triples/s",
-            "sample": f"{nplain} triples (1/{frac} of nocc={s.nocc} nvir={s.nvir}, driver order), one grouped "
-                      f"16-GEMM launch + one tengy launch per triple",
+            "sample": f"{nplain} triples (1/{frac} of nocc={s.nocc} nvir={s.nvir}, driver order), batches of "
+                      f"triples, one launch of the GEMMs + one of tengy each",
             "tflops_fp64_equiv": nplain * flop_triple / (pms * 1e-3) / 1e12}
 
 
@@ -604,6 +608,8 @@ def cpu_leg(args, R, workload_name=None):
     try:
         out = subprocess.run(cmd, capture_output=True, text=True, timeout=900, env=env, check=True).stdout
         line = json.loads([ln for ln in out.splitlines() if ln.startswith("{")][-1])
+        if "unavailable" in line:
+            raise RuntimeError(line["unavailable"])
         cb = dict(line["cpu_baseline"])
         cb["sample"] = "a reference-arm process of this script (" + " ".join(cmd[2:]) + "): " + cb["sample"]
         return cb
@@ -842,8 +848,8 @@ def run_b200_arm(args):
             per = [plain_sample(T, R, s, T.triple_flops(s.nocc, s.nvir), frac=32) for s in systems]
             serial_sec = sum(T.count_triples(s.nocc) / pl["value"] for s, pl in zip(systems, per))
             plain = {"value": (n_all / R.mult) / serial_sec, "unit": "triples/s",  # one GPU
-                     "sample": "1/32 of each system's triples, one grouped 16-GEMM launch + one tengy launch per "
-                               "triple, systems one after another; serial time extrapolated by triple counts",
+                     "sample": "1/32 of each system's triples, batches, one launch of the GEMMs + one of tengy "
+                               "each, systems one after another; serial time extrapolated by triple counts",
                      "tflops_fp64_equiv": (flop_all / R.mult) / serial_sec / 1e12, "per_system": per}
         else:
             s = systems[0]

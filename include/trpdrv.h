@@ -5,7 +5,7 @@
  * reference driver (omp/test.c) and Fortran/C callers link against this library unchanged.
  * Part 2 is the batched interface: whole systems (every (i,j,k) triple of one `a`, or of a range of
  * `a` with options.a_count) resident on the device, run by one persistent fused FP64 kernel, by the
- * emulated-FP64 int8 form, or by a plain per-triple path, optionally sharded over ranks.
+ * emulated-FP64 int8 form, or by a plain path (the products and the energies in launches of their own), optionally sharded over ranks.
  *
  * Conventions: all real data is IEEE double; integers are 32-bit unless typed otherwise; orbital
  * indices in the reference entry points are 1-based (Fortran convention, as in the reference).
@@ -32,13 +32,11 @@ extern "C" {
  * omp/test.c:39-52).  All arguments by reference; every pointer is caller-owned HOST memory.
  * tkj, jka, kka are offset by (k-klo)*nvir*nvir and tka, xka, jkj, kkj by (k-klo)*nocc*nvir, as in
  * the reference.  f1n..f4t are scratch: they are written back only when TRPDRV_WRITE_F=1.
- * Device work per call: with even nocc and nvir (and TRPDRV_WRITE_F unset) the slices are staged
- * into a fixed one-triple layout (host slices compared with a pinned mirror and copied where they
- * differ by up to TRPDRV_STAGE_THREADS host threads, default up to 16; the i-role and k-role blocks
- * sent to the device only when changed; slices inside registered arrays gathered on the device) and
- * one launch of the fused FP64 kernel computes the energies without writing f; otherwise (or with
- * TRPDRV_DROPIN_PATH=plain) the plain per-triple path runs (16 GEMMs into f, then the tengy
- * reduction).  The call returns after the energies are back on the host.
+ * Device work per call: the slices are staged into one device block, rows padded to an even pitch (host
+ * slices compared with a pinned mirror and copied where they differ by up to TRPDRV_STAGE_THREADS host
+ * threads, default up to 16; the i-role and k-role regions sent to the device only when changed; slices
+ * inside registered arrays read where they lie), and two launches compute f and the energies, which
+ * the second writes to pinned host memory.  The call returns after that.
  * Errors (bad sizes/indices, CUDA failure) print to stderr and abort, unless TRPDRV_ON_ERROR=return,
  * in which case emp4/emp5 are left unchanged and trpdrv_last_error() reports the status. */
 void ccsd_trpdrv_omp_cbody_(double *f1n, double *f1t, double *f2n, double *f2t,
@@ -182,9 +180,11 @@ typedef struct trpdrv_options {
     int use_graph;    /* capture trpdrv_plan_execute's launch sequence in a CUDA graph; default 1 */
     int mma_k;        /* FP64 MMA shape of the fused kernel: 8 = m16n8k8 (default); 16 = m16n8k16 (TMA
                          staging only; cp.async staging then uses 8); 4 = m16n8k4 (cp.async staging only;
-                         TMA staging then uses 8) */
+                         TMA staging then uses 8).  The last chunk of a contraction ends in a k4 step where
+                         that is enough */
     int staging;      /* fused-kernel operand staging: 0 = TMA where supported (even nvir and nocc,
-                         16-byte aligned tensors, <= 8 systems), else cp.async; 1 = cp.async; 2 = TMA
+                         16-byte aligned tensors, <= 8 systems), else cp.async, odd rows from copies
+                         padded to an even pitch; 1 = cp.async; 2 = TMA
                          or fail with TRPDRV_ERR_UNSUPPORTED */
     int slices;       /* EMULATED: base-128 digits per operand element, 4..8; 0 = default (7) */
     int batch;        /* EMULATED: triples per contraction launch (their f fill one half of a double
@@ -333,7 +333,7 @@ int trpdrv_synth_fill(int tensor, int ncor, int nocc, int nvir, uint64_t seed, i
  * (tkj is the (k,j) block itself, not the k-chunk base; likewise jka, kka, tka, xka, jkj, kkj;
  * dintc2/dintx2/t1v2 are the k vectors) and writes out4[0..3] = emp4i, emp5i, emp4k, emp5k on the
  * device.  Enqueues on `stream` and returns without waiting; allocates nothing: its scratch is one
- * static device array of about 4.7 MB per GPU, kept until the process exits, that limits the size
+ * static device array of about 4.2 MB per GPU, kept until the process exits, that limits the size
  * to nvir <= TRPDRV_NOALLOC_MAX_NVIR and nocc <= TRPDRV_NOALLOC_MAX_NOCC (larger sizes are
  * rejected with TRPDRV_ERR_ARG).  All calls on a device share that array: calls that overlap on
  * the GPU race and must be serialised by the caller.  The first call on each device looks up the
