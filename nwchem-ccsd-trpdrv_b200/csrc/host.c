@@ -1555,7 +1555,8 @@ static int tune_sample_records(trpdrv_plan *p, double **host)
         TRY(emulated_batches(p, d, b, 0, n, p->opt.batch, st, &bi, NULL));
         TRY(emulated_join(p, st, bi));
     }
-    TRY(enqueue_finish(p, st, NULL));
+    /* the records alone: the totals stay those of the last execution */
+    LAUNCH_TRY(trpdrv_launch_records(p->h_dev, p->d_dev, p->nsys, st));
     for (int q = 0; q < p->nsys; ++q)
         if (p->s[q].ntriples > 0)
             CUDA_TRY(cudaMemcpyAsync(host[q], p->s[q].rec, sizeof(double) * 4 * (size_t)p->s[q].ntriples,
