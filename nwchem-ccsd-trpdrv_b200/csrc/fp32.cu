@@ -293,13 +293,18 @@ int fail(int status, const char *msg)
         }                                                                               \
     } while (0)
 
+int dev_alloc(void **p, size_t bytes)
+{
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();  // reported here; the next call's launch check must not find it
+    return (int)e;
+}
+void dev_release(void *p) { cudaFree(p); }
+
+// *cap in bytes
 int grow(float **p, size_t *cap, size_t want)
 {
-    if (want <= *cap) return 0;
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-    F32_TRY(cudaMalloc((void **)p, sizeof(float) * want));
-    *cap = want;
+    F32_TRY((cudaError_t)stage_grow((void **)p, cap, sizeof(float) * want, dev_alloc, dev_release));
     return 0;
 }
 

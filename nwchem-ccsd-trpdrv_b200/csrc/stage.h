@@ -1,5 +1,6 @@
 /*
- * stage.h — host staging of one triple's slices for the drop-in entry points (C and CUDA sources).
+ * stage.h — host staging of one triple's slices for the drop-in entry points (C and CUDA sources), and the growth of
+ * their device buffers.
  *
  * The caller's slices are compared with a pinned mirror and copied where they differ, block by block, so the
  * contents decide what is sent, never a pointer.  Rows may be padded in the mirror (rows of `width` bytes,
@@ -133,6 +134,24 @@ static inline int stage_send(const stage_piece *pc, int npc, int threads, size_t
         }
     }
     return 0;
+}
+
+/* A buffer of at least `want` bytes: kept while its capacity suffices, else released and allocated anew.  A failed
+ * allocation leaves neither a buffer nor a capacity, so that the next call, of whatever size, allocates again.
+ * Returns the allocator's result. */
+static inline int stage_grow(void **p, size_t *cap, size_t want, int (*alloc)(void **p, size_t bytes),
+                             void (*release)(void *p))
+{
+    if (want <= *cap) return 0;
+    if (*p) release(*p);
+    *p = NULL;
+    *cap = 0;
+    const int e = alloc(p, want);
+    if (e)
+        *p = NULL;
+    else
+        *cap = want;
+    return e;
 }
 
 #endif /* TRPDRV_STAGE_H */
