@@ -218,6 +218,8 @@ struct trpdrv_plan {
     size_t fbuf_half;   /* doubles in one of the two halves */
     cudaStream_t aux_stream;          /* emulated form: energies of batch n, ordered after its products only */
     cudaEvent_t ev_gemm[2], ev_tengy[2];
+    int tengy_sent[2];  /* ev_tengy was recorded by the job being enqueued: what an earlier one recorded, or a
+                           capture, is not waited for */
     int fbuf_batch;     /* triples d_fbuf holds (>= opt.batch, and room for the autotuner's batches) */
     int tuned_staging;  /* FUSED staging chosen by the autotuner (1 cp.async, 2 TMA), 0 = none */
     void *tma_maps;     /* tensor maps of every system, passed by value to each launch */
@@ -862,6 +864,7 @@ static int enqueue_fused(trpdrv_plan *p, cudaStream_t st, int capturing)
 static int emulated_batches(trpdrv_plan *p, const trpdrv_dev_system *d, const sysbuf *b, int64_t pos0, int64_t pos1,
                             int batch, cudaStream_t st, int64_t *bi, int64_t *launches)
 {
+    if (*bi == 0) p->tengy_sent[0] = p->tengy_sent[1] = 0;
     if (trpdrv_oz_fused_energy_supported(d->nvir)) {
         int64_t epos = 0;
         int en = 0;
@@ -871,7 +874,7 @@ static int emulated_batches(trpdrv_plan *p, const trpdrv_dev_system *d, const sy
             if (n == 0 && en == 0) break;
             const int h = (int)(*bi & 1);
             double *fb = p->d_fbuf + (size_t)h * p->fbuf_half;
-            if (n > 0 && *bi >= 2) CUDA_TRY(cudaStreamWaitEvent(st, p->ev_tengy[h], 0));  /* separate-launch readers */
+            if (n > 0 && p->tengy_sent[h]) CUDA_TRY(cudaStreamWaitEvent(st, p->ev_tengy[h], 0)); /* its separate readers */
             const int64_t j0 = n > 0 ? b->oz_job0[pos] : 0;
             const int nj = n > 0 ? (int)(b->oz_job0[pos + n] - j0) : 0;
             LAUNCH_TRY(trpdrv_launch_oz_gemm(d, &b->oz, b->oz_maps, pos, j0, nj, fb, epos, en, efb, p->d_status,
@@ -889,7 +892,7 @@ static int emulated_batches(trpdrv_plan *p, const trpdrv_dev_system *d, const sy
         const int n = (int)(pos1 - pos < batch ? pos1 - pos : batch);
         const int h = (int)(*bi & 1);
         double *fb = p->d_fbuf + (size_t)h * p->fbuf_half;
-        if (*bi >= 2) CUDA_TRY(cudaStreamWaitEvent(st, p->ev_tengy[h], 0));
+        if (p->tengy_sent[h]) CUDA_TRY(cudaStreamWaitEvent(st, p->ev_tengy[h], 0));
         LAUNCH_TRY(trpdrv_launch_oz_gemm(d, &b->oz, b->oz_maps, pos, b->oz_job0[pos],
                                          (int)(b->oz_job0[pos + n] - b->oz_job0[pos]), fb, 0, 0, NULL, p->d_status,
                                          p->nsm, st));
@@ -897,6 +900,7 @@ static int emulated_batches(trpdrv_plan *p, const trpdrv_dev_system *d, const sy
         CUDA_TRY(cudaStreamWaitEvent(p->aux_stream, p->ev_gemm[h], 0));
         LAUNCH_TRY(trpdrv_launch_oz_tengy(d, pos, n, fb, 128, p->d_status, p->aux_stream));
         CUDA_TRY(cudaEventRecord(p->ev_tengy[h], p->aux_stream));
+        p->tengy_sent[h] = 1;
         ++*bi;
         if (launches) *launches += 2;
     }
@@ -904,9 +908,10 @@ static int emulated_batches(trpdrv_plan *p, const trpdrv_dev_system *d, const sy
 }
 
 /* the main stream waits for every energy launch of the batches enqueued so far */
-static int emulated_join(trpdrv_plan *p, cudaStream_t st, int64_t bi)
+static int emulated_join(trpdrv_plan *p, cudaStream_t st)
 {
-    for (int h = 0; h < 2 && h < bi; ++h) CUDA_TRY(cudaStreamWaitEvent(st, p->ev_tengy[h], 0));
+    for (int h = 0; h < 2; ++h)
+        if (p->tengy_sent[h]) CUDA_TRY(cudaStreamWaitEvent(st, p->ev_tengy[h], 0));
     return TRPDRV_OK;
 }
 
@@ -915,6 +920,7 @@ static int emulated_join(trpdrv_plan *p, cudaStream_t st, int64_t bi)
 static int enqueue_emulated(trpdrv_plan *p, cudaStream_t st, int capturing)
 {
     int64_t launches = 0, bi = 0;
+    p->tengy_sent[0] = p->tengy_sent[1] = 0;
     CUDA_TRY(cudaMemsetAsync(p->d_status, 0, sizeof(int), st));
     CUDA_TRY(cudaEventRecordWithFlags(p->ev0, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
     for (int q = 0; q < p->nsys; ++q) {
@@ -925,7 +931,7 @@ static int enqueue_emulated(trpdrv_plan *p, cudaStream_t st, int capturing)
         ++launches;
         TRY(emulated_batches(p, d, b, 0, d->ntriples, p->opt.batch, st, &bi, &launches));
     }
-    TRY(emulated_join(p, st, bi));
+    TRY(emulated_join(p, st));
     CUDA_TRY(cudaEventRecordWithFlags(p->ev1, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
     TRY(enqueue_finish(p, st, &launches));
     p->last_launches = launches;
@@ -1510,7 +1516,7 @@ static int tune_time(trpdrv_plan *p, const trpdrv_tune_candidate *c, double *est
                 int64_t bi = 0;
                 CUDA_TRY(cudaEventRecord(p->ev0, st));
                 TRY(emulated_batches(p, d, b, 0, n, c->batch, st, &bi, NULL));
-                TRY(emulated_join(p, st, bi));
+                TRY(emulated_join(p, st));
                 CUDA_TRY(cudaEventRecord(p->ev1, st));
                 TRY(tune_elapsed(p, &ms));
                 if (rep == 0 || ms < best) best = ms;
@@ -1553,7 +1559,7 @@ static int tune_sample_records(trpdrv_plan *p, double **host)
         LAUNCH_TRY(trpdrv_launch_oz_slices(d, &b->oz, st));
         int64_t bi = 0;
         TRY(emulated_batches(p, d, b, 0, n, p->opt.batch, st, &bi, NULL));
-        TRY(emulated_join(p, st, bi));
+        TRY(emulated_join(p, st));
     }
     /* the records alone: the totals stay those of the last execution */
     LAUNCH_TRY(trpdrv_launch_records(p->h_dev, p->d_dev, p->nsys, st));
