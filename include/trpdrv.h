@@ -381,8 +381,9 @@ void trpdrv_finalize(void);
  * TRPDRV_ERR_DEVICE instead of a hung device.  This call runs
  * that same bounded wait on an mbarrier that nothing completes, with the given limit (seconds, in
  * (0, 10]), on the current device: *status receives the kernel's status word (2 = the wait gave
- * up, as it must; 4 = it reported a phase that never completed) and *elapsed_seconds how long the
- * wait lasted.  The device stays usable afterwards.  No counterpart in the reference. */
+ * up, as it must; 4 is added if it reported a phase that never completed, 8 if the lanes of a warp did not
+ * give up together where half of them ran out of time first) and *elapsed_seconds how long the wait
+ * lasted.  The device stays usable afterwards.  No counterpart in the reference. */
 int trpdrv_selftest_bounded_wait(double limit_seconds, int *status, double *elapsed_seconds);
 
 #ifdef __cplusplus

@@ -1936,6 +1936,7 @@ int trpdrv_selftest_bounded_wait(double limit_seconds, int *status, double *elap
     if (e == cudaSuccess) e = cudaMemset(d_status, 0, sizeof(int));
     if (e == cudaSuccess)
         e = (cudaError_t)trpdrv_launch_wait_selftest((unsigned long long)(limit_seconds * 1e9), d_status, d_el, NULL);
+    if (e == cudaSuccess) e = (cudaError_t)trpdrv_launch_warp_wait_selftest(5000000ull, d_status, NULL);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = cudaMemcpy(&h_status, d_status, sizeof(int), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(&el, d_el, sizeof el, cudaMemcpyDeviceToHost);

@@ -75,6 +75,10 @@ int trpdrv_fused_tma_init(void);
 int trpdrv_launch_wait_selftest(unsigned long long limit_ns, int *status, unsigned long long *elapsed_ns,
                                 void *stream);
 
+/* One warp waits as the emulated form's warps do, half of its lanes with a shorter limit than the phase takes: bit 3 of
+ * *status unless all lanes give up together. */
+int trpdrv_launch_warp_wait_selftest(unsigned long long limit_ns, int *status, void *stream);
+
 /* Emulated-FP64 (Ozaki int8) form, ozaki.cu.  Per system: digit slices of the A operands
  * sa [nocc][slices][2 nvir][dp] and of the B operands sb [nocc*nocc][slices][2 nvir][dp] (int8,
  * dp = trpdrv_oz_dp: nvir + nocc rounded up to 32), with power-of-two scales ea [nocc][2 nvir] and

@@ -146,7 +146,8 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long *b, unsigned pa
 }
 
 // Bounded wait; false (and status bit 1) when it runs out.
-__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity, int *status)
+__device__ __forceinline__ bool mbar_wait_for(unsigned long long *b, unsigned parity, int *status,
+                                              unsigned long long limit_ns)
 {
     if (mbar_try_wait(b, parity)) return true;
     const unsigned long long t0 = globaltimer();
@@ -154,11 +155,31 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity
 #pragma unroll 1
         for (int spin = 0; spin < 256; ++spin)
             if (mbar_try_wait(b, parity)) return true;
-        if (globaltimer() - t0 > WAIT_LIMIT_NS) {
+        if (globaltimer() - t0 > limit_ns) {
             atomicOr(status, 2);
             return false;
         }
     }
+}
+
+__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity, int *status)
+{
+    return mbar_wait_for(b, parity, status, WAIT_LIMIT_NS);
+}
+
+// The wait of a whole converged warp that goes on to instructions all of its lanes take part in (elect.sync,
+// tcgen05.ld, __syncwarp): every lane polls by its own clock, so one may give up in the moment in which the phase
+// completes for the others.  The same answer in all lanes, or part of the warp would wait at the CTA's last barrier
+// and the rest, for it, inside the loop.
+__device__ __forceinline__ bool mbar_wait_warp_for(unsigned long long *b, unsigned parity, int *status,
+                                                   unsigned long long limit_ns)
+{
+    return __all_sync(0xffffffffu, mbar_wait_for(b, parity, status, limit_ns));
+}
+
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long *b, unsigned parity, int *status)
+{
+    return mbar_wait_warp_for(b, parity, status, WAIT_LIMIT_NS);
 }
 
 // L2 cache policies for loads and stores: evict_last for data read again soon (the digit planes, reused
@@ -287,6 +308,30 @@ __device__ __forceinline__ void reg_fence16(unsigned (&v)[16])
 __device__ __forceinline__ void mbar_arrive(unsigned long long *b)
 {
     asm volatile("mbarrier.arrive.shared.b64 _, [%0];" ::"r"(saddr(b)) : "memory");
+}
+
+// Self-test of mbar_wait_warp: warp 1 completes the phase after twice the limit that half of warp 0's lanes have; the
+// others would wait on.  All lanes of warp 0 must give up together (status bit 3: they did not).
+__global__ void warp_wait_selftest_kernel(unsigned long long limit_ns, int *status)
+{
+    __shared__ __align__(8) unsigned long long bar;
+    __shared__ int local;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        local = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) {
+        const unsigned long long t0 = globaltimer();
+        while (globaltimer() - t0 < 2 * limit_ns) {
+        }
+        if (lane == 0) mbar_arrive(&bar);
+        return;
+    }
+    const bool done = mbar_wait_warp_for(&bar, 0u, &local, lane < 16 ? limit_ns : 64 * limit_ns);
+    if (done) atomicOr(status, 8);
 }
 
 // weight of level L (0-based, slices p + q = L + 2 in 1-based digits): 2^(-7 (L + 2)), exact
@@ -793,11 +838,11 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
             for (int t = blockIdx.x; alive && t < P.tiles; t += gridDim.x, ++it) {
                 const Tile d = decode_tile(P, t);
                 // the accumulators are free once the previous tile has been drained
-                if (!mbar_wait(tempty, (it & 1) ^ 1, P.status)) break;
+                if (!mbar_wait_warp(tempty, (it & 1) ^ 1, P.status)) break;
                 tc_fence_after();
                 if (d.ok) {
                     for (int kc = 0; kc < nchunks; ++kc) {
-                        if (!mbar_wait(&full[stage], phase, P.status)) {
+                        if (!mbar_wait_warp(&full[stage], phase, P.status)) {
                             alive = false;
                             break;
                         }
@@ -852,7 +897,7 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
             const int r = d.m0 + qd * 32 + lane, lcol = d.n0 + half * WC + lane;
             int esa = d.ok && r < 2 * V ? scale_exp(P.ea[(size_t)d.planeA * 2 * V + r]) : 0;
             int esb = d.ok && lcol < 2 * V ? scale_exp(P.eb[(size_t)d.planeB * 2 * V + lcol]) : 0;
-            if (!mbar_wait(tfull, it & 1, P.status)) break;
+            if (!mbar_wait_warp(tfull, it & 1, P.status)) break;
             tc_fence_after();
             const int rh = r >= V ? 1 : 0, b = r - rh * V;
             double *fj = P.fbuf + (size_t)d.y * 8 * vv + (size_t)d.grp * 4 * vv + (size_t)rh * vv + b;
@@ -1367,6 +1412,12 @@ extern "C" int trpdrv_launch_oz_tengy(const trpdrv_dev_system *h_sys, int64_t po
         oz::oz_tengy_kernel<128, false><<<grid, 128, oz::TSMEM_BYTES, st>>>(P, np, npos);
     else
         oz::oz_tengy_kernel<256, false><<<grid, 256, oz::TSMEM_BYTES, st>>>(P, np, npos);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int trpdrv_launch_warp_wait_selftest(unsigned long long limit_ns, int *status, void *stream)
+{
+    oz::warp_wait_selftest_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(limit_ns, status);
     return (int)cudaGetLastError();
 }
 
