@@ -682,15 +682,16 @@ __device__ __forceinline__ Tile decode_tile(const GemmParams &P, int t)
 
 // Draining.  The next tile's products wait until the accumulators have been read, so as little as possible happens
 // before they are released; and the roles' code together must stay within the instruction caches, beside
-// which everything but the products ran at half its speed or less.  Three forms, by the width dp of the contraction:
-//   SUM64: all levels joined in integers, two adjacent ones in int32 (128 C_l + C_{l+1}), the pairs in
-//          int64, converted after the release (|C_l| <= (l + 1) dp 64^2; dp <= sum64_limit(S): 503 for S = 7)
-//   PAIRS: pairs of levels joined in int32 and added in FP64 (dp <= pair_limit(S): 811 for S = 7)
-//   LEVELS: level by level in FP64
-// Every one rounds once, so they give the same bits: integer sums are exact, and so is every FP64 addition
-// but the last, from the last levels up.
-enum DrainForm { SUM64, PAIRS, LEVELS };
+// which everything but the products ran at half its speed or less.  Two forms, by the width dp of the contraction
+// (|C_l| <= (l + 1) dp 64^2):
+//   SUM64:  all levels joined in int64, two adjacent ones in int32 first (128 C_l + C_{l+1}), converted after the
+//           release (dp <= sum64_limit(S): 504 for 7 slices, no width for 8)
+//   GROUPS: levels 0 .. 3 and 4 .. S - 1 joined in int64, the two sums added in FP64
+// Both round once, so they give the same bits: the integer sums are exact, a group's is below 2^53 (group_max_dp) and so
+// exact in FP64, and only the addition of the second group rounds.
+enum DrainForm { SUM64, GROUPS };
 
+// The widest contraction whose pairs of levels stay below 2^31.
 __host__ __device__ constexpr int pair_limit(int S)
 {
     const int l = (S - 1) & ~1;               // first level of the last pair (or the last level alone)
@@ -706,41 +707,52 @@ __host__ __device__ constexpr int sum64_limit(int S)
     return lim < (unsigned long long)pair_limit(S) ? (int)lim : pair_limit(S);
 }
 
+// The widest contraction whose groups of four levels stay below 2^53.
+__host__ __device__ constexpr long long group_max_dp()
+{
+    return (1LL << 53) / (4096LL * (5LL * 128 * 128 * 128 + 6LL * 128 * 128 + 7LL * 128 + 8LL));  // levels 4 .. 7
+}
+static_assert(TRPDRV_MAX_NOCC + TRPDRV_MAX_NVIR + 32 <= group_max_dp(), "a group of four levels exceeds 53 bits");
+
 // 16 columns at TMEM address base: sum_L C_L 2^(-7 (L + 2)); SUM64: the bits of the integer 2^(7 (S + 1)) times that.
 template <int S, DrainForm FORM>
 __device__ __forceinline__ void drain16(unsigned base, double (&val)[16])
 {
-    constexpr int STEP = FORM == LEVELS ? 1 : 2, NP = (S + STEP - 1) / STEP;  // pairs
+    constexpr int GROUP = 4;
 #pragma unroll
     for (int u = 0; u < 16; ++u) val[u] = 0.0;
 #pragma unroll
-    for (int g = 0; g < NP; g += 2) {  // two pairs in flight; FP64: from the last ones up
-        const int k0 = FORM == SUM64 ? g : (NP - g >= 2 ? NP - g - 2 : 0);
-        const int k1 = FORM == SUM64 ? (g + 2 < NP ? g + 2 : NP) : NP - g;
-        unsigned v[2 * STEP][16];
+    for (int g = 0; g < S; g += GROUP) {
+        const int n = S - g < GROUP ? S - g : GROUP;
+        unsigned v[GROUP][16];
 #pragma unroll
-        for (int l = 0; l < 2 * STEP; ++l)
-            if (k0 * STEP + l < k1 * STEP && k0 * STEP + l < S)
-                tmem_ld16_nowait(base + (unsigned)((k0 * STEP + l) * BN), v[l]);
+        for (int l = 0; l < GROUP; ++l)
+            if (l < n) tmem_ld16_nowait(base + (unsigned)((g + l) * BN), v[l]);
         tmem_wait_ld();
 #pragma unroll
-        for (int l = 0; l < 2 * STEP; ++l)
-            if (k0 * STEP + l < k1 * STEP && k0 * STEP + l < S) reg_fence16(v[l]);
+        for (int l = 0; l < GROUP; ++l)
+            if (l < n) reg_fence16(v[l]);
+        if (FORM == SUM64) {
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const int k = FORM == SUM64 ? k0 + n : k1 - 1 - n;
-            if (k < k0 || k >= k1) continue;
-            const int l = (k - k0) * STEP, lev = k * STEP;
-            const bool two = STEP == 2 && lev + 1 < S;
-            const double w = level_weight(two ? lev + 1 : lev);
+            for (int l = 0; l < GROUP; l += 2) {
+                if (l >= n) break;
+                const bool two = l + 1 < n;
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    const int x = two ? (int)v[l][u] * 128 + (int)v[two ? l + 1 : l][u] : (int)v[l][u];
+                    val[u] = __longlong_as_double(
+                        g + l == 0 ? (long long)x : __double_as_longlong(val[u]) * (two ? 16384 : 128) + x);
+                }
+            }
+        } else {
+            const double w = level_weight(g + n - 1);
 #pragma unroll
             for (int u = 0; u < 16; ++u) {
-                const int x = two ? (int)v[l][u] * 128 + (int)v[two ? l + 1 : l][u] : (int)v[l][u];
-                if (FORM == SUM64)
-                    val[u] = __longlong_as_double(k == 0 ? (long long)x
-                                                         : __double_as_longlong(val[u]) * (two ? 16384 : 128) + x);
-                else
-                    val[u] = fma((double)x, w, val[u]);
+                long long sum = (int)v[0][u];
+#pragma unroll
+                for (int l = 1; l < GROUP; ++l)
+                    if (l < n) sum = sum * 128 + (int)v[l][u];
+                val[u] = fma((double)sum, w, val[u]);
             }
         }
     }
@@ -887,6 +899,7 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REG_REC));
         const int qd = warp & 3, half = (warp - REC0) >> 2;
         constexpr int WC = BN / 2;  // columns per recombination warp
+        constexpr bool SUM64_FITS = sum64_limit(S) >= KSTEP;  // the narrowest contraction; false for 8 slices
         const int V = P.V;
         const size_t vv = (size_t)V * P.ldf;
         int it = 0;
@@ -905,15 +918,13 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
             const unsigned base = tmem + ((unsigned)(qd * 32) << 16) + (unsigned)(half * WC);
             double val[WC / 16][16];
             const int dp = P.nks * KSTEP;
-            if (dp <= sum64_limit(S)) {
+            const bool sum64 = SUM64_FITS && dp <= sum64_limit(S);
+            if (sum64) {
 #pragma unroll
                 for (int cb = 0; cb < WC / 16; ++cb) drain16<S, SUM64>(base + (unsigned)(cb * 16), val[cb]);
-            } else if (dp <= pair_limit(S)) {
-#pragma unroll
-                for (int cb = 0; cb < WC / 16; ++cb) drain16<S, PAIRS>(base + (unsigned)(cb * 16), val[cb]);
             } else {
 #pragma unroll
-                for (int cb = 0; cb < WC / 16; ++cb) drain16<S, LEVELS>(base + (unsigned)(cb * 16), val[cb]);
+                for (int cb = 0; cb < WC / 16; ++cb) drain16<S, GROUPS>(base + (unsigned)(cb * 16), val[cb]);
             }
             // the accumulators may be overwritten by the next tile from here on
             tc_fence_before();
@@ -921,7 +932,7 @@ __global__ void __launch_bounds__(NTHREAD, 1) oz_gemm_kernel(const __grid_consta
             if (lane == 0) mbar_arrive(tempty);
             if (!d.ok) continue;
             int e0 = 0;
-            if (dp <= sum64_limit(S)) {
+            if (sum64) {
                 e0 = -7 * (S + 1);
 #pragma unroll
                 for (int cb = 0; cb < WC / 16; ++cb)
