@@ -452,7 +452,7 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
     CUDA_TRY(cudaMalloc((void **)&p->d_counter, 2 * sizeof(unsigned long long)));
     CUDA_TRY(cudaMemset(p->d_counter, 0, 2 * sizeof(unsigned long long)));
     p->d_status = (int *)(p->d_counter + 1);
-    CUDA_TRY(cudaMalloc((void **)&p->d_bsum, sizeof(double) * 4 * TRPDRV_FINISH_BLOCKS * (size_t)p->nsys));
+    CUDA_TRY(cudaMalloc((void **)&p->d_bsum, sizeof(double) * (trpdrv_totals_doubles(p->h_dev, p->nsys) + 1)));
     CUDA_TRY(cudaMalloc((void **)&p->d_done, sizeof(unsigned) * (size_t)p->nsys));
     CUDA_TRY(cudaMemset(p->d_done, 0, sizeof(unsigned) * (size_t)p->nsys));
     /* whole pages of our own, registered: 0.3 ms, where cudaMallocHost takes 1 to 2.7 */

@@ -129,9 +129,9 @@ int trpdrv_launch_records(const trpdrv_dev_system *h_sys, const trpdrv_dev_syste
 
 /* Each system's compensated total over rec, of emp4i + [i != k] emp4k summed over the triples:
  * res[4 s ..] = emp4 hi, emp4 lo, emp5 hi, emp5 lo; res[4 nsys] = the value of *status.  res is pinned host memory
- * (device-accessible).  bsum: nsys * TRPDRV_FINISH_BLOCKS * 4 doubles; done: nsys zeros (left at zero).  Systems
+ * (device-accessible).  bsum: trpdrv_totals_doubles doubles; done: nsys zeros (left at zero).  Systems
  * without records are not written. */
-#define TRPDRV_FINISH_BLOCKS 1024
+size_t trpdrv_totals_doubles(const trpdrv_dev_system *h_sys, int nsys);
 int trpdrv_launch_totals(const trpdrv_dev_system *h_sys, const trpdrv_dev_system *d_sys, int nsys, double *bsum,
                          unsigned *done, const int *status, double *res, void *stream);
 

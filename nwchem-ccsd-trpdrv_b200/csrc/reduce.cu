@@ -36,6 +36,8 @@ struct DdPair {
 
 constexpr int REC_WARPS = 8;       // records per block of records_kernel
 constexpr int FIN_THREADS = 512;   // totals_kernel
+constexpr int FIN_BLOCKS = 1024;   // its most blocks per system
+constexpr int MAX_GRID_Y = 65535;  // rows of a grid
 
 // The block's sum of every thread's pair in thread 0 (a fixed tree).
 __device__ __forceinline__ DdPair block_dd(DdPair v, double (&sh)[4][FIN_THREADS])
@@ -66,46 +68,47 @@ __device__ __forceinline__ DdPair block_dd(DdPair v, double (&sh)[4][FIN_THREADS
 __host__ __device__ inline int total_blocks(long long ntriples)
 {
     const long long n = (ntriples + FIN_THREADS - 1) / FIN_THREADS;
-    return n < TRPDRV_FINISH_BLOCKS ? (int)n : TRPDRV_FINISH_BLOCKS;
+    return n < FIN_BLOCKS ? (int)n : FIN_BLOCKS;
 }
 
-// One row of the grid per system, one warp per record.
-__global__ void __launch_bounds__(REC_WARPS * 32) records_kernel(const trpdrv_dev_system *__restrict__ sys)
+// Rows of the grid take systems (more systems than MAX_GRID_Y share rows), one warp per record.
+__global__ void __launch_bounds__(REC_WARPS * 32) records_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys)
 {
-    const trpdrv_dev_system &S = sys[blockIdx.y];
-    const int lane = threadIdx.x & 31, nslot = S.npairs * TRPDRV_FUSED_SLOTS;
-    for (long long t = (long long)blockIdx.x * REC_WARPS + (threadIdx.x >> 5); t < S.ntriples;
-         t += (long long)gridDim.x * REC_WARPS) {
-        const double *p = S.partial + 4 * t * (long long)nslot;
-        // compensated per lane (error-free TwoSum, errors carried in lo), then the lanes' hi and lo sums
-        double hi[4] = {0.0, 0.0, 0.0, 0.0}, lo[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int q = lane; q < nslot; q += 32) {
+    const int lane = threadIdx.x & 31;
+    for (int s = blockIdx.y; s < nsys; s += gridDim.y) {
+        const trpdrv_dev_system &S = sys[s];
+        const int nslot = S.npairs * TRPDRV_FUSED_SLOTS;
+        for (long long t = (long long)blockIdx.x * REC_WARPS + (threadIdx.x >> 5); t < S.ntriples;
+             t += (long long)gridDim.x * REC_WARPS) {
+            const double *p = S.partial + 4 * t * (long long)nslot;
+            // compensated per lane (error-free TwoSum, errors carried in lo), then the lanes' hi and lo sums
+            double hi[4] = {0.0, 0.0, 0.0, 0.0}, lo[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int q = lane; q < nslot; q += 32) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    double v, e;
+                    two_sum(hi[c], p[4 * q + c], v, e);
+                    hi[c] = v;
+                    lo[c] += e;
+                }
+            }
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                double s, e;
-                two_sum(hi[c], p[4 * q + c], s, e);
-                hi[c] = s;
-                lo[c] += e;
+                const double h = warp_sum(hi[c]), l = warp_sum(lo[c]);
+                if (lane == 0) S.rec[4 * t + c] = h + l;
             }
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const double h = warp_sum(hi[c]), l = warp_sum(lo[c]);
-            if (lane == 0) S.rec[4 * t + c] = h + l;
         }
     }
 }
 
-// One row of the grid per system.  Each block leaves its records' double-double sum; the system's last block adds
-// those in block order and writes the totals and the execution's status word to pinned host memory, so that
-// reading the energies needs no copy.
-__global__ void __launch_bounds__(FIN_THREADS)
-totals_kernel(const trpdrv_dev_system *__restrict__ sys, double *__restrict__ bsum, unsigned *__restrict__ done,
-              const int *__restrict__ status, double *__restrict__ res)
+// One system: each block leaves its records' double-double sum; the system's last block adds those in block order and
+// writes the totals and the execution's status word to pinned host memory, so that reading the energies needs
+// no copy.
+__device__ __forceinline__ void system_totals(const trpdrv_dev_system &S, double *__restrict__ bs,
+                                              unsigned *__restrict__ done, double *__restrict__ out,
+                                              double *__restrict__ status_out, const int *__restrict__ status,
+                                              double (&sh)[4][FIN_THREADS], int &last)
 {
-    __shared__ double sh[4][FIN_THREADS];
-    __shared__ int last;
-    const trpdrv_dev_system &S = sys[blockIdx.y];
     const long long n = S.ntriples;
     const int nblk = total_blocks(n), tid = threadIdx.x;
     if ((int)blockIdx.x >= nblk) return;
@@ -116,7 +119,6 @@ totals_kernel(const trpdrv_dev_system *__restrict__ sys, double *__restrict__ bs
     }
     v = block_dd(v, sh);
     if (nblk > 1) {
-        double *bs = bsum + 4 * (size_t)blockIdx.y * TRPDRV_FINISH_BLOCKS;
         if (tid == 0) {
             double *b = bs + 4 * blockIdx.x;
             b[0] = v.h4;
@@ -124,7 +126,7 @@ totals_kernel(const trpdrv_dev_system *__restrict__ sys, double *__restrict__ bs
             b[2] = v.h5;
             b[3] = v.l5;
             __threadfence();
-            last = atomicAdd(&done[blockIdx.y], 1u) == (unsigned)nblk - 1;
+            last = atomicAdd(done, 1u) == (unsigned)nblk - 1;
         }
         __syncthreads();
         if (!last) return;
@@ -141,18 +143,30 @@ totals_kernel(const trpdrv_dev_system *__restrict__ sys, double *__restrict__ bs
             v.l5 += __ldcg(b + 3) + e;
         }
         v = block_dd(v, sh);
-        if (tid == 0) done[blockIdx.y] = 0u;
+        if (tid == 0) *done = 0u;
     }
     if (tid == 0) {
-        double *out = res + 4 * blockIdx.y, s, e;
+        double s, e;
         two_sum(v.h4, v.l4, s, e);  // renormalise
         out[0] = s;
         out[1] = e;
         two_sum(v.h5, v.l5, s, e);
         out[2] = s;
         out[3] = e;
-        res[4 * gridDim.y] = (double)*status;
+        *status_out = (double)*status;
     }
+}
+
+// Rows of the grid take systems, as in records_kernel.
+__global__ void __launch_bounds__(FIN_THREADS)
+totals_kernel(const trpdrv_dev_system *__restrict__ sys, int nsys, double *__restrict__ bsum, unsigned *__restrict__ done,
+              const int *__restrict__ status, double *__restrict__ res)
+{
+    __shared__ double sh[4][FIN_THREADS];
+    __shared__ int last;
+    for (int s = blockIdx.y; s < nsys; s += gridDim.y)
+        system_totals(sys[s], bsum + 4 * (size_t)s * gridDim.x, done + s, res + 4 * (size_t)s,
+                      res + 4 * (size_t)nsys, status, sh, last);
 }
 
 __global__ void negate_kernel(const double *__restrict__ src, double *__restrict__ dst, size_t n)
@@ -209,21 +223,33 @@ extern "C" int trpdrv_launch_records(const trpdrv_dev_system *h_sys, const trpdr
     }
     if (blocks == 0) return 0;
     if (blocks > 65535) blocks = 65535;
-    records_kernel<<<dim3((unsigned)blocks, (unsigned)nsys), REC_WARPS * 32, 0, (cudaStream_t)stream>>>(d_sys);
+    records_kernel<<<dim3((unsigned)blocks, (unsigned)(nsys < MAX_GRID_Y ? nsys : MAX_GRID_Y)), REC_WARPS * 32, 0,
+                     (cudaStream_t)stream>>>(d_sys, nsys);
     return (int)cudaGetLastError();
 }
 
-extern "C" int trpdrv_launch_totals(const trpdrv_dev_system *h_sys, const trpdrv_dev_system *d_sys, int nsys,
-                                    double *bsum, unsigned *done, const int *status, double *res, void *stream)
+static int most_total_blocks(const trpdrv_dev_system *h_sys, int nsys)
 {
     int blocks = 0;
     for (int q = 0; q < nsys; ++q) {
         const int n = total_blocks(h_sys[q].ntriples);
         if (n > blocks) blocks = n;
     }
+    return blocks;
+}
+
+extern "C" size_t trpdrv_totals_doubles(const trpdrv_dev_system *h_sys, int nsys)
+{
+    return 4 * (size_t)nsys * (size_t)most_total_blocks(h_sys, nsys);
+}
+
+extern "C" int trpdrv_launch_totals(const trpdrv_dev_system *h_sys, const trpdrv_dev_system *d_sys, int nsys,
+                                    double *bsum, unsigned *done, const int *status, double *res, void *stream)
+{
+    const int blocks = most_total_blocks(h_sys, nsys);
     if (blocks == 0) return 0;
-    totals_kernel<<<dim3((unsigned)blocks, (unsigned)nsys), FIN_THREADS, 0, (cudaStream_t)stream>>>(d_sys, bsum, done,
-                                                                                                    status, res);
+    totals_kernel<<<dim3((unsigned)blocks, (unsigned)(nsys < MAX_GRID_Y ? nsys : MAX_GRID_Y)), FIN_THREADS, 0,
+                    (cudaStream_t)stream>>>(d_sys, nsys, bsum, done, status, res);
     return (int)cudaGetLastError();
 }
 
