@@ -371,8 +371,9 @@ int trpdrv_register_host(const void *ptr, size_t bytes);
 int trpdrv_refresh_host(const void *ptr);
 int trpdrv_unregister_host(const void *ptr);
 
-/* Releases the drop-in entry points' device state (buffers, stream, registered arrays).  Safe to
- * call repeatedly. */
+/* Releases the drop-in entry points' device state (buffers, stream, registered arrays) and the 32 KB of
+ * pinned memory that plans share for their totals (while plans live: when the last one is destroyed).
+ * Safe to call repeatedly. */
 void trpdrv_finalize(void);
 
 /* Failure-detection self-test.  Every mbarrier wait inside the TMA FP64 kernel and the int8

@@ -200,8 +200,9 @@ struct trpdrv_plan {
     int *d_status;
     double *d_bsum;   /* block sums of the totals */
     unsigned *d_done; /* finished blocks per system */
-    double *h_res;    /* registered: totals per system (emp4 hi, lo, emp5 hi, lo), then the status word */
+    double *h_res;    /* pinned (res_take): totals per system (emp4 hi, lo, emp5 hi, lo), then the status word */
     double *d_res;    /* its device address */
+    int res_own;      /* h_res is pages of this plan's own */
     int64_t total_items;
     double *d_f, *d_bpart; /* plain form: f and energy partials of one batch of triples */
     unsigned *d_tcount;
@@ -248,6 +249,94 @@ void trpdrv_options_default(trpdrv_options *opt)
     opt->batch = 64;
 }
 
+/* ------------------------------------------------------------------------------------------ */
+/* pinned memory for the plans' totals                                                          */
+/* ------------------------------------------------------------------------------------------ */
+
+/* One pinned block for the whole process, of which every plan takes a few 64-byte lines for as long as it lives:
+ * pinning memory of its own (0.25 ms, and as much to give it back) doubled the creation of a small plan, which a caller
+ * of trpdrv_run pays on every call.  trpdrv_finalize frees it, or the last plan does that is left then.  Plans of
+ * more systems than there is room for pin pages of their own. */
+enum { RES_LINE = 8, RES_LINES = 512 }; /* doubles per line; 32 KB */
+static pthread_mutex_t g_res_mu = PTHREAD_MUTEX_INITIALIZER;
+static double *g_res;
+static unsigned char g_res_taken[RES_LINES];
+static int g_res_plans, g_res_closing;
+
+/* Room for n doubles, zeroed; *own: pages of this plan alone. */
+static int res_take(size_t n, double **out, int *own)
+{
+    const size_t lines = (n + RES_LINE - 1) / RES_LINE;
+    *out = NULL;
+    *own = 0;
+    pthread_mutex_lock(&g_res_mu);
+    cudaError_t e = cudaSuccess;
+    if (lines <= RES_LINES && !g_res)
+        e = cudaHostAlloc((void **)&g_res, sizeof(double) * RES_LINE * RES_LINES,
+                          cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e == cudaSuccess && lines <= RES_LINES) {
+        size_t run = 0;
+        for (size_t l = 0; l < RES_LINES && run < lines; ++l) {
+            run = g_res_taken[l] ? 0 : run + 1;
+            if (run == lines) {
+                *out = g_res + RES_LINE * (l + 1 - lines);
+                memset(g_res_taken + (l + 1 - lines), 1, lines);
+                ++g_res_plans;
+                g_res_closing = 0;
+            }
+        }
+    }
+    pthread_mutex_unlock(&g_res_mu);
+    CUDA_TRY(e);
+    if (!*out) {
+        const size_t bytes = (sizeof(double) * n + 4095) / 4096 * 4096;
+        void *pages = aligned_alloc(4096, bytes);
+        if (!pages) return fail(TRPDRV_ERR_NOMEM, "out of host memory");
+        e = cudaHostRegister(pages, bytes, cudaHostRegisterPortable | cudaHostRegisterMapped);
+        if (e != cudaSuccess) free(pages);
+        CUDA_TRY(e);
+        *out = (double *)pages;
+        *own = 1;
+    }
+    memset(*out, 0, sizeof(double) * n);
+    return TRPDRV_OK;
+}
+
+/* with g_res_mu held */
+static void res_free_unused(void)
+{
+    if (g_res && g_res_plans == 0) {
+        cudaFreeHost(g_res);
+        g_res = NULL;
+    }
+}
+
+/* No kernel writes there any more. */
+static void res_give(double *res, size_t n, int own)
+{
+    if (!res) return;
+    if (own) {
+        cudaHostUnregister(res);
+        free(res);
+        return;
+    }
+    pthread_mutex_lock(&g_res_mu);
+    memset(g_res_taken + (res - g_res) / RES_LINE, 0, (n + RES_LINE - 1) / RES_LINE);
+    --g_res_plans;
+    if (g_res_closing) res_free_unused();
+    pthread_mutex_unlock(&g_res_mu);
+}
+
+static void res_close(void)
+{
+    pthread_mutex_lock(&g_res_mu);
+    g_res_closing = 1;
+    res_free_unused();
+    pthread_mutex_unlock(&g_res_mu);
+}
+
+static size_t res_doubles(const trpdrv_plan *p) { return 4 * (size_t)p->nsys + 1; }
+
 static void plan_free(trpdrv_plan *p)
 {
     if (!p) return;
@@ -284,8 +373,6 @@ static void plan_free(trpdrv_plan *p)
     if (p->d_counter) cudaFree(p->d_counter);
     if (p->d_bsum) cudaFree(p->d_bsum);
     if (p->d_done) cudaFree(p->d_done);
-    if (p->d_res) cudaHostUnregister(p->h_res);
-    free(p->h_res);
     if (p->d_f) cudaFree(p->d_f);
     if (p->d_fbuf) cudaFree(p->d_fbuf);
     for (int h = 0; h < 2; ++h) {
@@ -305,6 +392,8 @@ static void plan_free(trpdrv_plan *p)
     free(p->h_chunk_first);
     if (p->copy_stream) cudaStreamDestroy(p->copy_stream);
     if (p->stream) cudaStreamDestroy(p->stream);
+    if (p->last_stream) cudaDeviceSynchronize(); /* an execution nobody waited for still writes its totals */
+    res_give(p->h_res, res_doubles(p), p->res_own);
     free(p);
 }
 
@@ -455,18 +544,8 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
     CUDA_TRY(cudaMalloc((void **)&p->d_bsum, sizeof(double) * (trpdrv_totals_doubles(p->h_dev, p->nsys) + 1)));
     CUDA_TRY(cudaMalloc((void **)&p->d_done, sizeof(unsigned) * (size_t)p->nsys));
     CUDA_TRY(cudaMemset(p->d_done, 0, sizeof(unsigned) * (size_t)p->nsys));
-    /* whole pages of our own, registered: 0.3 ms, where cudaMallocHost takes 1 to 2.7 */
-    const size_t res_bytes = (sizeof(double) * (4 * (size_t)p->nsys + 1) + 4095) / 4096 * 4096;
-    void *res = aligned_alloc(4096, res_bytes);
-    if (!res) return fail(TRPDRV_ERR_NOMEM, "out of host memory");
-    p->h_res = (double *)res;
-    memset(res, 0, res_bytes);
-    CUDA_TRY(cudaHostRegister(res, res_bytes, cudaHostRegisterPortable | cudaHostRegisterMapped));
-    {
-        const cudaError_t re = cudaHostGetDevicePointer((void **)&p->d_res, res, 0);
-        if (re != cudaSuccess) cudaHostUnregister(res);
-        CUDA_TRY(re);
-    }
+    TRY(res_take(res_doubles(p), &p->h_res, &p->res_own));
+    CUDA_TRY(cudaHostGetDevicePointer((void **)&p->d_res, p->h_res, 0));
     if (o->mode == TRPDRV_MODE_EMULATED) {
         p->fbuf_batch = o->batch > TUNE_MAX_BATCH ? o->batch : TUNE_MAX_BATCH;
         p->fbuf_half = 8 * (size_t)p->fbuf_batch * maxv * trpdrv_oz_ldf(maxv);
@@ -1953,6 +2032,7 @@ void trpdrv_finalize(void)
     pthread_mutex_lock(&g_di_mu);
     di_release();
     pthread_mutex_unlock(&g_di_mu);
+    res_close();
 }
 
 #define DI_GROW(ptr, cap, count)                                                                    \
