@@ -34,8 +34,8 @@ extern "C" {
  * the reference.  f1n..f4t are scratch: they are written back only when TRPDRV_WRITE_F=1.
  * Device work per call: the slices are staged into one device block, rows padded to an even pitch (host
  * slices compared with a pinned mirror and copied where they differ by up to TRPDRV_STAGE_THREADS host
- * threads, default up to 16; the i-role and k-role regions sent to the device only when changed; slices
- * inside registered arrays read where they lie), and two launches compute f and the energies, which
+ * threads, default up to 16; sent to the device in segments of about 512 KB, those that changed; slices
+ * inside registered arrays read where they lie, neither compared nor sent), and two launches compute f and the energies, which
  * the second writes to pinned host memory.  The call returns after that.
  * Errors (bad sizes/indices, CUDA failure) print to stderr and abort, unless TRPDRV_ON_ERROR=return,
  * in which case emp4/emp5 are left unchanged and trpdrv_last_error() reports the status. */

@@ -36,6 +36,10 @@ static inline int stage_threads(void)
     return n < 1 ? 1 : n;
 }
 
+/* Pads and the rounding of slots between two pieces that follow one another, at most. */
+enum { STAGE_GAP = 512 };
+
+static inline char *stage_end(const stage_piece *p) { return p->dst + (p->rows - 1) * p->pitch + p->width; }
 static inline size_t stage_bytes(const stage_piece *p) { return p->rows * p->width; }
 
 /* Block b of a piece brought up to date; returns 1 if it was written. */
@@ -91,9 +95,10 @@ static inline int stage_update(const stage_piece *pc, int npc, int threads)
     return changed;
 }
 
-/* Cuts the pieces (ascending dst) into segments of about `seg` bytes and calls send(ctx, lo, hi) for each segment
- * of the mirror [lo, hi) in which something changed, as soon as it is up to date: the transfer of one segment
- * runs while the next is compared.  Returns the first non-zero result of send. */
+/* Cuts the pieces (ascending dst) into segments of about `seg` bytes and calls send(ctx, lo, hi) for the range
+ * [lo, hi) of the mirror that a segment in which something changed covers, as soon as it is up to date: the transfer
+ * of one segment runs while the next is compared.  Pieces further apart than the rounding of their slots (what lies
+ * between is read elsewhere) go in ranges of their own.  Returns the first non-zero result of send. */
 static inline int stage_send(const stage_piece *pc, int npc, int threads, size_t seg,
                              int (*send)(void *ctx, char *lo, char *hi), void *ctx)
 {
@@ -123,10 +128,12 @@ static inline int stage_send(const stage_piece *pc, int npc, int threads, size_t
             have += stage_bytes(&t);
             const int done = q == npc - 1 && (p.rows == 0 || p.width == 0);
             if (have >= seg || np == MAX_PARTS || done) {
-                const stage_piece *l = &part[np - 1];
                 if (stage_update(part, np, threads)) {
-                    const int e = send(ctx, part[0].dst, l->dst + (l->rows - 1) * l->pitch + l->width);
-                    if (e) return e;
+                    for (int lo = 0, hi = 1; lo < np; lo = hi++) { /* parts lo .. hi - 1 follow one another */
+                        while (hi < np && part[hi].dst <= stage_end(&part[hi - 1]) + STAGE_GAP) ++hi;
+                        const int e = send(ctx, part[lo].dst, stage_end(&part[hi - 1]));
+                        if (e) return e;
+                    }
                 }
                 np = 0;
                 have = 0;
