@@ -907,14 +907,16 @@ static int enqueue_finish(trpdrv_plan *p, cudaStream_t st, int64_t *launches)
     return TRPDRV_OK;
 }
 
+/* Few items per SM: the large ones first.  Inputs this small stay in L2 whatever the order.  (10, 60), 11 items
+ * an SM: 133 -> 125 us; (4, 300), 15 an SM: 511 -> 490 us; at 64 and more the two orders time the same. */
+static int plan_pair_major(const trpdrv_plan *p) { return p->total_items <= 64 * (int64_t)p->nsm; }
+
 static int enqueue_fused(trpdrv_plan *p, cudaStream_t st, int capturing)
 {
     int64_t launches = 0;
     CUDA_TRY(cudaMemsetAsync(p->d_counter, 0, 2 * sizeof(unsigned long long), st)); /* and the status word */
     CUDA_TRY(cudaEventRecordWithFlags(p->ev0, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
-    /* few items per SM: the large ones first.  Inputs this small stay in L2 whatever the order.  (10, 60), 11 items
-     * an SM: 133 -> 125 us; (4, 300), 15 an SM: 511 -> 490 us; at 64 and more the two orders time the same */
-    const int pair_major = p->total_items <= 64 * (int64_t)p->nsm;
+    const int pair_major = plan_pair_major(p);
     if (p->total_items > 0) {
         for (int q = 0; q < p->nsys; ++q)
             if (p->h_dev[q].ntriples > 0) TRY(pad_refill(p, q, 1, 0, p->s[q].shape.nocc, st, &launches));
@@ -1568,16 +1570,18 @@ static int tune_time(trpdrv_plan *p, const trpdrv_tune_candidate *c, double *est
             int grid = c->staging == 2 ? p->nsm : c->ctas_per_sm * p->nsm;
             if (grid > sample) grid = (int)sample;
             TRY(tune_set_edge_pack(p, c->edge_pack));
+            /* in the order in which the plan runs them; plans that run pair by pair are timed whole */
+            const int pair_major = plan_pair_major(p) && sample == items;
             float best = 0.0f;
             for (int rep = 0; rep < TUNE_REPS; ++rep) {
                 CUDA_TRY(cudaMemcpyAsync(p->d_counter, &first, sizeof first, cudaMemcpyHostToDevice, st));
                 CUDA_TRY(cudaStreamSynchronize(st)); /* `first` is a host stack value */
                 CUDA_TRY(cudaEventRecord(p->ev0, st));
                 if (c->staging == 2)
-                    LAUNCH_TRY(trpdrv_launch_fused_tma(p->d_dev, p->nsys, d->item_begin + sample, 0, p->d_counter,
+                    LAUNCH_TRY(trpdrv_launch_fused_tma(p->d_dev, p->nsys, d->item_begin + sample, pair_major, p->d_counter,
                                                        p->d_status, grid, p->tma_maps, c->mma_k, st));
                 else
-                    LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, d->item_begin + sample, 0, p->d_counter,
+                    LAUNCH_TRY(trpdrv_launch_fused(p->d_dev, p->nsys, d->item_begin + sample, pair_major, p->d_counter,
                                                    p->d_status, grid, p->vec2 || p->padded, c->mma_k, st));
                 CUDA_TRY(cudaEventRecord(p->ev1, st));
                 TRY(tune_elapsed(p, &ms));
