@@ -253,7 +253,7 @@ int trpdrv_plan_destroy(trpdrv_plan *plan);
  * slices (4..8) that meet the accuracy target on the same sample.  The choice is cached per device and set of shapes for
  * the life of the process; a later plan with the same key takes it without timing.  With
  * TRPDRV_TUNE_CACHE naming a file, choices are also appended there (one text line each, keyed by the
- * device model, the library version and the plan's shapes and options) and read back by later
+ * device model, the library version, the revision of its kernels and the plan's shapes and options) and read back by later
  * processes.  result->from_cache: 0 = timed now, 1 = this process's cache, 2 = the file.  No
  * counterpart in the reference (its BLAS call sites have nothing to tune).  `result` may be NULL. */
 typedef struct trpdrv_tune_candidate {

@@ -1394,7 +1394,7 @@ int trpdrv_plan_last_kernel_ms(trpdrv_plan *p, double *ms)
 /* ------------------------------------------------------------------------------------------ */
 
 typedef struct tune_entry {
-    int used, dev, mode, slices, world, rank, nsys, staging;
+    int used, dev, mode, slices, world, rank, nsys, staging, a_count;
     int shape[3 * TRPDRV_TMA_MAX_SYSTEMS];
     trpdrv_tune_candidate best;
 } tune_entry;
@@ -1412,6 +1412,7 @@ static void tune_key(const trpdrv_plan *p, tune_entry *k)
     k->rank = p->opt.rank;
     k->nsys = p->nsys;
     k->staging = p->opt.staging; /* a forced staging limits the candidates */
+    k->a_count = p->opt.a_count;
     for (int q = 0; q < p->nsys && q < TRPDRV_TMA_MAX_SYSTEMS; ++q) {
         k->shape[3 * q] = p->s[q].shape.nocc;
         k->shape[3 * q + 1] = p->s[q].shape.nvir;
@@ -1422,13 +1423,16 @@ static void tune_key(const trpdrv_plan *p, tune_entry *k)
 static int tune_same(const tune_entry *a, const tune_entry *b)
 {
     return a->dev == b->dev && a->mode == b->mode && a->slices == b->slices && a->world == b->world &&
-           a->rank == b->rank && a->nsys == b->nsys && a->staging == b->staging && memcmp(a->shape, b->shape, sizeof a->shape) == 0;
+           a->rank == b->rank && a->nsys == b->nsys && a->staging == b->staging && a->a_count == b->a_count &&
+           memcmp(a->shape, b->shape, sizeof a->shape) == 0;
 }
 
 /* ---- persistent tuning cache (TRPDRV_TUNE_CACHE = path of a text file shared by processes) ----
  * One line per choice: "<key> -> <staging> <mma_k> <ctas_per_sm> <batch> <edge_pack> <ms>", where the key names
- * the device model (name, SM count), the library version and every field of tune_entry.  Lookups
+ * the device model (name, SM count), the library version, the revision of the kernels and every field of tune_entry.  Lookups
  * take the last matching line; stores append under an exclusive lock. */
+/* Raised whenever the kernels that candidates are timed with change: choices made with others are timed again. */
+#define TUNE_KERNELS 2
 static int tune_file_key(const trpdrv_plan *p, const tune_entry *k, char *buf, size_t n)
 {
     struct cudaDeviceProp prop;
@@ -1437,9 +1441,9 @@ static int tune_file_key(const trpdrv_plan *p, const tune_entry *k, char *buf, s
     size_t q = 0;
     for (const char *c = prop.name; *c && q + 1 < sizeof name; ++c) name[q++] = (*c == ' ' || *c == '>') ? '_' : *c;
     name[q] = '\0';
-    int w = snprintf(buf, n, "trpdrv-tune v%d %s sm%d mode=%d slices=%d world=%d rank=%d staging=%d nsys=%d shapes=",
-                     trpdrv_version(), name, prop.multiProcessorCount, k->mode, k->slices, k->world, k->rank,
-                     k->staging, k->nsys);
+    int w = snprintf(buf, n, "trpdrv-tune v%d.%d %s sm%d mode=%d slices=%d world=%d rank=%d staging=%d a=%d nsys=%d shapes=",
+                     trpdrv_version(), TUNE_KERNELS, name, prop.multiProcessorCount, k->mode, k->slices, k->world, k->rank,
+                     k->staging, k->a_count, k->nsys);
     for (int s = 0; s < k->nsys && s < TRPDRV_TMA_MAX_SYSTEMS && w > 0 && (size_t)w < n; ++s)
         w += snprintf(buf + w, n - (size_t)w, "%s%d,%d,%d", s ? ";" : "", k->shape[3 * s], k->shape[3 * s + 1],
                       k->shape[3 * s + 2]);
