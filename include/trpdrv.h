@@ -183,9 +183,13 @@ typedef struct trpdrv_options {
                          TMA staging then uses 8).  The last chunk of a contraction ends in a k4 step where
                          that is enough */
     int staging;      /* fused-kernel operand staging: 0 = TMA where supported (even nvir and nocc,
-                         16-byte aligned tensors, <= 8 systems), else cp.async, odd rows from copies
-                         padded to an even pitch; 1 = cp.async; 2 = TMA
-                         or fail with TRPDRV_ERR_UNSUPPORTED */
+                         16-byte aligned tensors, <= 8 systems), else cp.async; 1 = cp.async; 2 = TMA
+                         or fail with TRPDRV_ERR_UNSUPPORTED.  With cp.async, T2, JVV, KVV, JOV and KOV
+                         with odd rows or off a 16-byte boundary are read through copies with an even
+                         pitch: the plan then holds about the bytes of those tensors once more (odd
+                         nvir: all five), if at upload or bind time that is a quarter of the free
+                         device memory at most (or 16 MB), and else reads the tensors themselves in 8-byte pieces
+                         (13, 151: 4.2 instead of 3.0 ms) */
     int slices;       /* EMULATED: base-128 digits per operand element, 4..8; 0 = default (7) */
     int batch;        /* EMULATED: triples per contraction launch (their f fill one half of a double
                          buffer that the energy stage reads back); 0 = default (64) */

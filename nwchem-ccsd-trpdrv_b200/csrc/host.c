@@ -663,24 +663,45 @@ static int tensor_rows(const sysbuf *b, int w, long long *rows)
 
 static int row_pitch(int width) { return width + (width & 1); }
 
+/* Bytes of the padded copy that tensor w of system b needs for 16-byte copies and does not have yet. */
+static size_t pad_bytes(const sysbuf *b, int w)
+{
+    long long rows;
+    const int width = tensor_rows(b, w, &rows);
+    if (!width || rows == 0 || b->pad[w]) return 0;
+    if (!(width & 1) && !(((uintptr_t)b->t[w]) & 15u)) return 0;
+    return sizeof(double) * (size_t)rows * row_pitch(width);
+}
+
 /* Fused plans that cannot copy 16 bytes at a time from the bound tensors (an odd nvir or nocc, or an
  * unaligned pointer) and do not use TMA: the tensors concerned get copies with rows padded to an even length
  * (zero pads), which every execution refills.  Copying each input once costs little beside the kernel, which
  * reads a block of T2 for every triple: (13, 151) runs 4.2 ms with 8-byte copies from the bound tensors.
- * Without the memory for the copies the kernel reads the bound tensors with 8-byte copies. */
+ * The copies take as much memory as those tensors.  The caller did not ask for them, so they are made only out of
+ * plenty: a quarter of the memory that is free at this moment, at most (asked for above 16 MB: the question takes
+ * 0.1 ms, as long as a small plan's execution).  Else, or where the allocation fails, the kernel reads the bound
+ * tensors with 8-byte copies. */
+#define PAD_FREELY ((size_t)16 << 20)
 static int plan_pad(trpdrv_plan *p, int tma_ok)
 {
     p->padded = 0;
     for (int q = 0; q < p->nsys; ++q) p->h_dev[q].ldv = p->h_dev[q].ldo = 0;
     if (p->opt.mode != TRPDRV_MODE_FUSED || p->vec2 || tma_ok) return TRPDRV_OK;
+    size_t need = 0;
+    for (int q = 0; q < p->nsys; ++q)
+        for (int w = 0; w < TRPDRV_T_COUNT; ++w) need += pad_bytes(&p->s[q], w);
     int ok = 1;
+    if (need > PAD_FREELY) {
+        size_t avail = 0, total = 0;
+        CUDA_TRY(cudaMemGetInfo(&avail, &total));
+        ok = need <= avail / 4;
+    }
     for (int q = 0; q < p->nsys && ok; ++q) {
         sysbuf *b = &p->s[q];
         for (int w = 0; w < TRPDRV_T_COUNT && ok; ++w) {
-            long long rows;
-            const int width = tensor_rows(b, w, &rows);
-            if (!width || rows == 0 || (!(width & 1) && !(((uintptr_t)b->t[w]) & 15u)) || b->pad[w]) continue;
-            if (cudaMalloc((void **)&b->pad[w], sizeof(double) * (size_t)rows * row_pitch(width)) != cudaSuccess) {
+            const size_t bytes = pad_bytes(b, w);
+            if (bytes == 0) continue;
+            if (cudaMalloc((void **)&b->pad[w], bytes) != cudaSuccess) {
                 b->pad[w] = NULL;
                 cudaGetLastError();
                 ok = 0;
