@@ -36,7 +36,8 @@ extern "C" {
  * slices compared with a pinned mirror and copied where they differ by up to TRPDRV_STAGE_THREADS host
  * threads, default up to 16; sent to the device in segments of about 512 KB, those that changed; slices
  * inside registered arrays read where they lie, neither compared nor sent), and two launches compute f and the energies, which
- * the second writes to pinned host memory.  The call returns after that.
+ * the second writes to pinned host memory.  The call returns after that.  TRPDRV_DROPIN_PATH=plain, which
+ * asked for these kernels while there was a choice, is accepted and changes nothing.
  * Errors (bad sizes/indices, CUDA failure) print to stderr and abort, unless TRPDRV_ON_ERROR=return,
  * in which case emp4/emp5 are left unchanged and trpdrv_last_error() reports the status. */
 void ccsd_trpdrv_omp_cbody_(double *f1n, double *f1t, double *f2n, double *f2t,
