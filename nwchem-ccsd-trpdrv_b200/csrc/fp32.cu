@@ -288,17 +288,13 @@ int fail(int status, const char *msg)
         const cudaError_t e_ = (call);                                                  \
         if (e_ != cudaSuccess) {                                                        \
             char m_[200];                                                               \
+            cudaGetLastError(); /* reported here: the next launch's check must not find it */ \
             snprintf(m_, sizeof m_, "%s: %s", #call, cudaGetErrorString(e_));          \
             return fail(e_ == cudaErrorMemoryAllocation ? 3 : 2, m_);                   \
         }                                                                               \
     } while (0)
 
-int dev_alloc(void **p, size_t bytes)
-{
-    const cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) cudaGetLastError();  // reported here; the next call's launch check must not find it
-    return (int)e;
-}
+int dev_alloc(void **p, size_t bytes) { return (int)cudaMalloc(p, bytes); }
 void dev_release(void *p) { cudaFree(p); }
 
 // *cap in bytes

@@ -69,9 +69,11 @@ const char *trpdrv_status_string(int status)
 #define CUDA_TRY(call)                                                                              \
     do {                                                                                            \
         cudaError_t e_ = (call);                                                                    \
-        if (e_ != cudaSuccess)                                                                      \
+        if (e_ != cudaSuccess) {                                                                    \
+            cudaGetLastError(); /* reported here: the next launch's check must not find it again */ \
             return fail(e_ == cudaErrorMemoryAllocation ? TRPDRV_ERR_NOMEM : TRPDRV_ERR_CUDA,       \
                         "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__);       \
+        }                                                                                           \
     } while (0)
 
 #define LAUNCH_TRY(call)                                                                            \
@@ -1260,8 +1262,10 @@ int trpdrv_plan_upload_execute(trpdrv_plan *p, const trpdrv_system *host, int ch
     do {                                                                                            \
         if (rc == TRPDRV_OK) {                                                                      \
             cudaError_t e_ = (call);                                                                \
-            if (e_ != cudaSuccess)                                                                  \
+            if (e_ != cudaSuccess) {                                                                \
+                cudaGetLastError();                                                                 \
                 rc = fail(TRPDRV_ERR_CUDA, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+            }                                                                                       \
         }                                                                                           \
     } while (0)
     /* both streams after the caller's stream and after the previous execution */
@@ -1972,6 +1976,7 @@ int trpdrv_register_host(const void *ptr, size_t bytes)
             cudaError_t e = cudaMalloc((void **)&dev, bytes);
             if (e == cudaSuccess) e = cudaMemcpy(dev, ptr, bytes, cudaMemcpyHostToDevice);
             if (e != cudaSuccess) {
+                cudaGetLastError();
                 if (dev) cudaFree(dev);
                 rc = fail(e == cudaErrorMemoryAllocation ? TRPDRV_ERR_NOMEM : TRPDRV_ERR_CUDA, "register: %s",
                           cudaGetErrorString(e));
@@ -2004,7 +2009,10 @@ int trpdrv_refresh_host(const void *ptr)
     } else {
         cudaSetDevice(g_di.device);
         const cudaError_t e = cudaMemcpy(g_reg[r].dev, g_reg[r].host, g_reg[r].bytes, cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) rc = fail(TRPDRV_ERR_CUDA, "refresh: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            rc = fail(TRPDRV_ERR_CUDA, "refresh: %s", cudaGetErrorString(e));
+        }
     }
     pthread_mutex_unlock(&g_di_mu);
     return rc;
@@ -2050,7 +2058,7 @@ int trpdrv_selftest_bounded_wait(double limit_seconds, int *status, double *elap
     if (e == cudaSuccess) e = cudaMemcpy(&el, d_el, sizeof el, cudaMemcpyDeviceToHost);
     if (d_status) cudaFree(d_status);
     if (d_el) cudaFree(d_el);
-    if (e != cudaSuccess) return fail(TRPDRV_ERR_CUDA, "selftest: %s", cudaGetErrorString(e));
+    CUDA_TRY(e);
     *status = h_status;
     *elapsed_seconds = (double)el * 1e-9;
     return TRPDRV_OK;
