@@ -210,7 +210,8 @@ void trpdrv_options_default(trpdrv_options *opt);
 typedef struct trpdrv_plan trpdrv_plan;
 
 /* Allocates device storage and work queues for nsys systems (only ncor/nocc/nvir/a of `shape` are
- * read).  Returns TRPDRV_OK and sets *plan. */
+ * read).  Plain plans hold the f of a batch of triples: 96 MB at most, a quarter of the free device
+ * memory at most (or 4 MB), but of one triple at least.  Returns TRPDRV_OK and sets *plan. */
 int trpdrv_plan_create(trpdrv_plan **plan, const trpdrv_system *shape, int nsys,
                        const trpdrv_options *opt);
 /* Copies every host tensor of `host` (nsys entries, same shapes) into the plan's device storage

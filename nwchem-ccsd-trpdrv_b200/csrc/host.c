@@ -208,6 +208,7 @@ struct trpdrv_plan {
     int64_t total_items;
     double *d_f, *d_bpart; /* plain form: f and energy partials of one batch of triples */
     unsigned *d_tcount;
+    int plain_cap;         /* the most triples they hold */
     cudaGraph_t graph;
     cudaGraphExec_t gexec;
     int graph_ready;
@@ -399,11 +400,50 @@ static void plan_free(trpdrv_plan *p)
     free(p);
 }
 
-/* Triples per launch of a plain plan's system. */
-static int64_t plain_batch(const sysbuf *b)
+/* Triples per launch of a plain plan's system: at most `cap`. */
+static int64_t plain_batch(const sysbuf *b, int cap)
 {
-    const int64_t n = trpdrv_plain_batch(b->shape.nvir);
+    int64_t n = trpdrv_plain_batch(b->shape.nvir);
+    if (n > cap) n = cap;
     return b->ntriples < n ? (b->ntriples > 0 ? b->ntriples : 1) : n;
+}
+
+/* The buffers of one batch of the largest system, f and energy partials.  f of a full batch is 96 MB.  The plan's own
+ * tensors and whatever the application holds come after it, so f takes a quarter of the free memory at most (asked for
+ * above 4 MB: the question takes 0.1 ms): batches are halved until it does and the allocation succeeds, down to the
+ * single triple that a plan cannot do without. */
+static int plain_buffers(trpdrv_plan *p)
+{
+    size_t limit = (size_t)4 << 20;
+    int asked = 0;
+    for (p->plain_cap = 256;; p->plain_cap /= 2) {
+        size_t nf = 1, nbp = 1, nct = 1;
+        for (int q = 0; q < p->nsys; ++q) {
+            const size_t V = (size_t)p->s[q].shape.nvir, n = (size_t)plain_batch(&p->s[q], p->plain_cap);
+            if (n * 8 * V * V > nf) nf = n * 8 * V * V;
+            if (n * 4 * (size_t)trpdrv_tengy_pairs((int)V) > nbp) nbp = n * 4 * (size_t)trpdrv_tengy_pairs((int)V);
+            if (n > nct) nct = n;
+        }
+        if (sizeof(double) * nf > limit && !asked) {
+            size_t avail = 0, total = 0;
+            CUDA_TRY(cudaMemGetInfo(&avail, &total));
+            if (avail / 4 > limit) limit = avail / 4;
+            asked = 1;
+        }
+        if (sizeof(double) * nf > limit && p->plain_cap > 1) continue;
+        cudaError_t e = cudaMalloc((void **)&p->d_f, sizeof(double) * nf);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&p->d_bpart, sizeof(double) * nbp);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&p->d_tcount, sizeof(unsigned) * nct);
+        if (e == cudaSuccess) e = cudaMemset(p->d_tcount, 0, sizeof(unsigned) * nct);
+        if (e == cudaSuccess) return TRPDRV_OK;
+        if (e != cudaErrorMemoryAllocation || p->plain_cap == 1) CUDA_TRY(e);
+        cudaGetLastError();
+        if (p->d_f) cudaFree(p->d_f);
+        if (p->d_bpart) cudaFree(p->d_bpart);
+        if (p->d_tcount) cudaFree(p->d_tcount);
+        p->d_f = p->d_bpart = NULL;
+        p->d_tcount = NULL;
+    }
 }
 
 static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
@@ -558,19 +598,7 @@ static int plan_build(trpdrv_plan *p, const trpdrv_system *shape)
             CUDA_TRY(cudaEventCreateWithFlags(&p->ev_tengy[h], cudaEventDisableTiming));
         }
     }
-    if (o->mode == TRPDRV_MODE_PLAIN) {
-        size_t nf = 1, nbp = 1, nct = 1; /* one batch of the largest system */
-        for (int q = 0; q < p->nsys; ++q) {
-            const size_t V = (size_t)shape[q].nvir, n = (size_t)plain_batch(&p->s[q]);
-            if (n * 8 * V * V > nf) nf = n * 8 * V * V;
-            if (n * 4 * (size_t)trpdrv_tengy_pairs((int)V) > nbp) nbp = n * 4 * (size_t)trpdrv_tengy_pairs((int)V);
-            if (n > nct) nct = n;
-        }
-        CUDA_TRY(cudaMalloc((void **)&p->d_f, sizeof(double) * nf));
-        CUDA_TRY(cudaMalloc((void **)&p->d_bpart, sizeof(double) * nbp));
-        CUDA_TRY(cudaMalloc((void **)&p->d_tcount, sizeof(unsigned) * nct));
-        CUDA_TRY(cudaMemset(p->d_tcount, 0, sizeof(unsigned) * nct));
-    }
+    if (o->mode == TRPDRV_MODE_PLAIN) TRY(plain_buffers(p));
 
     int per_sm = o->ctas_per_sm;
     if (per_sm <= 0) per_sm = 1; /* the fused kernel's stages fill an SM's shared memory */
@@ -1053,7 +1081,7 @@ static int enqueue_plain(trpdrv_plan *p, cudaStream_t st)
     CUDA_TRY(cudaEventRecord(p->ev0, st));
     for (int q = 0; q < p->nsys; ++q) {
         const sysbuf *b = &p->s[q];
-        const int64_t batch = plain_batch(b);
+        const int64_t batch = plain_batch(b, p->plain_cap);
         for (int64_t r = 0; r < b->ntriples; r += batch) {
             const int n = (int)(b->ntriples - r < batch ? b->ntriples - r : batch);
             LAUNCH_TRY(trpdrv_launch_plain_batch(&p->h_dev[q], r, n, p->d_f, p->d_bpart, p->d_tcount, p->vec2, r > 0, st));
