@@ -12,8 +12,8 @@ nocc=40, nvir=300 (32,800 triples, 16.06 TFLOP per step), seeded synthetic input
   one trpdrv_plan_upload_execute call, which copies T2/JOV/KOV span by span under the fused kernel,
   with the upload-then-execute figure beside it);
   `roofline` = FP64 tensor-pipe fraction of the fused kernel against the FP64 DMMA peak measured live
-  by the library's probe; `plain_gpu` = the plain per-triple GPU path (16 GEMMs + tengy per triple) on a
-  bounded sample; `cpu_baseline` = the reference's own CPU body (oracle/_ref, OpenBLAS) on a bounded
+  by the library's probe; `plain_gpu` = the plain GPU path (f in memory between the products and the energies of a
+  batch of triples) on a bounded sample; `cpu_baseline` = the reference's own CPU body (oracle/_ref, OpenBLAS) on a bounded
   sample with all host threads (rank 0, N = 1 only).
 --impl reference: the reference's CPU path alone (oracle/_ref/libtrpdrv_ref.so: the reference
   omp/ccsd_trpdrv_omp_cbody.c + omp/ccsd_tengy_c99.c compiled unmodified), each step a bounded sample of
@@ -533,7 +533,7 @@ def emulated_sweep(T, R, systems, ref_e4, ref_e5, steps, warmup, slice_list, int
 
 
 def plain_sample(T, R, s, flop_triple, frac=16):
-    """The plain per-triple path (BASELINE config 1's method) on 1/frac of one system's triples."""
+    """The plain path (products and energies in launches of their own) on 1/frac of one system's triples."""
     torch = R.torch
     with T.Plan([s], mode=T.MODE_PLAIN, rank=0, world=frac, device=R.local) as pp:
         pp.upload(stream=R.sp)
@@ -706,7 +706,7 @@ def strong_split(T, R, args, steps, warmup):
 
 
 def run_c1(args, T, R, systems, in_bytes, n_all, flop_all, probe, cublas_dgemm, fp64_probe, peak):
-    """the plain per-triple path on every triple of (20, 200), checked against the fused
+    """The plain path on every triple of nocc = 20, nvir = 200, checked against the fused
     FP64 kernel on the same inputs (both are checked against the reference by the tests)."""
     with T.Plan(systems, mode=T.MODE_PLAIN, **R.shard, device=R.local) as p:
         p.upload(stream=R.sp)
@@ -841,7 +841,7 @@ def run_b200_arm(args):
             p.upload(stream=R.sp)
             emu_e2e_sec = time_e2e(T, R, p, args.steps, args.warmup)
 
-    # plain per-triple GPU path: a bounded sample of each system, serially
+    # plain GPU path: a bounded sample of each system, serially
     plain = None
     if not args.no_plain and R.rank == 0:
         if args.workload == "c4":

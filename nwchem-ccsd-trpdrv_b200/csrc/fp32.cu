@@ -473,7 +473,7 @@ int body(float *f1n, float *f1t, float *f2n, float *f2t, float *f3n, float *f3t,
         G.a2[x] = dev[A + (x & 1 ? DS_XO : DS_TO)];
         G.b2[x] = dev[B + (two ? DS_JO : DS_KO)];
     }
-    // 64-wide tiles once they fill the chip
+    // 64-wide tiles once they fill the chip's 148 SMs
     const unsigned n64 = (unsigned)(nvir + 63) / 64, n32 = (unsigned)(nvir + 31) / 32;
     if (n64 * n64 * 8 >= 148)
         sgemm_group_kernel<64><<<dim3(n64, n64, 8), Tile<64>::THREADS, 0, g.st>>>(G);

@@ -25,9 +25,10 @@
 // Fragment row/column labels are permuted, lane group g owning row (and column) PERM[g] of its 8,
 // PERM = {0,6,1,7,2,4,3,5}: the two rows a quarter-warp reads with one 128-bit load of an X-major
 // panel then differ in bit 2 (disjoint bank sets under the 128-byte swizzle) and the rows of one
-// 64-bit load of a K-major panel differ in bit 1 where they share bit 0, so no fragment read has a
-// bank conflict.  The permutation only relabels which (b, c) a register holds; the epilogue and the
-// diagonal exchange use the permuted coordinates.
+// 64-bit load of a K-major panel differ in bit 1 where they share bit 0, so no fragment read of a k8 or
+// k16 step has a bank conflict.  (The k4 step of a last chunk, whose lanes hold other contraction indices,
+// reads both kinds in two wavefronts.)  The permutation only relabels which (b, c) a register holds; the
+// epilogue and the diagonal exchange use the permuted coordinates.
 // The MMA shape is a template parameter: m16n8k8 (two k-steps per 16-index chunk) or m16n8k16,
 // whose fragments are exactly the two k8 fragments of the chunk side by side (lane t holds logical
 // k = t + 4q at physical index 2t + (q & 1) + 8 (q >> 1)).
@@ -526,7 +527,8 @@ __device__ __forceinline__ bool run_packed(int n, const FragOffsets &fo, const P
 // 19.88 to 19.81.
 //
 // Products of family FAM with the four contraction indices 8 ks .. 8 ks + 3 of a chunk, m16n8k4: lane t holds index
-// 8 ks + t (in a k8 step 2t and 2t + 1).
+// 8 ks + t (in a k8 step 2t and 2t + 1).  Its reads, of both panel kinds, take two wavefronts each; it runs once a
+// contraction at most.
 template <bool PH1, bool DIAG, int FAM>
 __device__ __forceinline__ void quarter_products(const FragOffsets &fo, const char *st, const Panels &pn, int ks, int t,
                                                  double (&f)[8][4], double (&gT)[8][4])

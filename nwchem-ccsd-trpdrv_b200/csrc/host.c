@@ -990,7 +990,7 @@ static int enqueue_fused(trpdrv_plan *p, cudaStream_t st, int capturing)
  * contraction launch writes its batch's f into one half while its energy warps compute the energies of
  * the previous batch from the other half, which the previous launch (on the same stream) filled; an
  * energies-only launch closes the system.  Odd nvir, or TRPDRV_OZ_FUSED_ENERGY=0: each batch's
- * energies run as a separate launch on the auxiliary stream (128-thread CTAs) while the next batch's
+ * energies run as a separate launch on the auxiliary stream while the next batch's
  * products go to the other half; a half is reused only after the energies that read it.  Finish with
  * emulated_join. */
 static int emulated_batches(trpdrv_plan *p, const trpdrv_dev_system *d, const sysbuf *b, int64_t pos0, int64_t pos1,
@@ -1030,7 +1030,7 @@ static int emulated_batches(trpdrv_plan *p, const trpdrv_dev_system *d, const sy
                                          p->nsm, st));
         CUDA_TRY(cudaEventRecord(p->ev_gemm[h], st));
         CUDA_TRY(cudaStreamWaitEvent(p->aux_stream, p->ev_gemm[h], 0));
-        LAUNCH_TRY(trpdrv_launch_oz_tengy(d, pos, n, fb, 128, p->d_status, p->aux_stream));
+        LAUNCH_TRY(trpdrv_launch_oz_tengy(d, pos, n, fb, p->d_status, p->aux_stream));
         CUDA_TRY(cudaEventRecord(p->ev_tengy[h], p->aux_stream));
         p->tengy_sent[h] = 1;
         ++*bi;

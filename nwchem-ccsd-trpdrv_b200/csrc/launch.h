@@ -13,7 +13,7 @@
 extern "C" {
 #endif
 
-/* Width of the (b,c) tiles of the fused kernel and of the standalone tengy kernel. */
+/* Width of the (b,c) tiles of the fused kernel. */
 #define TRPDRV_TILE 32
 /* Energy slots per fused work item (one per warp of the fused CTA). */
 #define TRPDRV_FUSED_SLOTS 8
@@ -116,12 +116,12 @@ int trpdrv_launch_oz_gemm(const trpdrv_dev_system *h_sys, const trpdrv_oz_system
                           int64_t pos0, int64_t job0, int njobs, double *fbuf, int64_t epos0, int enpos,
                           const double *efbuf, int *status, int grid, void *stream);
 int trpdrv_oz_fused_energy_supported(int nvir);
-/* The energies as a launch of their own (odd nvir, or TRPDRV_OZ_FUSED_ENERGY=0).  threads: 128 (what the plans launch) or 256.
+/* The energies as a launch of their own (odd nvir, or TRPDRV_OZ_FUSED_ENERGY=0).
  * The plans launch the energies of one batch on a second stream, ordered only after that batch's products.  The
  * tiles arrive by TMA (fbuf 16-byte aligned), with a bounded wait that sets *status bit 1 when it runs out;
  * with TRPDRV_OZ_TENGY_TMA=0 by cp.async. */
-int trpdrv_launch_oz_tengy(const trpdrv_dev_system *h_sys, int64_t pos0, int npos, const double *fbuf,
-                           int threads, int *status, void *stream);
+int trpdrv_launch_oz_tengy(const trpdrv_dev_system *h_sys, int64_t pos0, int npos, const double *fbuf, int *status,
+                           void *stream);
 int trpdrv_oz_init(void);
 
 /* Per-triple sums of the per-item energies of nsys systems (descriptors on host and device): partial -> rec. */

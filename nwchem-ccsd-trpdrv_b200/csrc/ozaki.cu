@@ -345,15 +345,14 @@ __device__ __forceinline__ double level_weight(int L)
 // ------------------------------------------------------------------------------------------------
 constexpr int TW = 16;
 constexpr size_t TSMEM_BYTES = (size_t)16 * TW * (TW + 1) * sizeof(double);
-// TMA form (even nvir): the eight f tiles of one orientation arrive as one 16 x 16 x 8 box with the
-// 128-byte swizzle; both orientations take 32 KB on a 1024-byte boundary.
+// TMA form: the eight f tiles of one orientation arrive as one 16 x 16 x 8 box with the 128-byte swizzle; both
+// orientations take 32 KB on a 1024-byte boundary.  Odd nvir too: f's columns are padded to an even length.
 constexpr int TBOX = TW * TW * 8;  // doubles of one orientation
 constexpr size_t TSMEM_TMA_BYTES = (size_t)2 * TBOX * sizeof(double) + 1024;
-// The plans launch 128-thread CTAs (at most 96 registers, five per SM); 256 is the other size the
-// launcher accepts.  The energies of one batch are launched on a second stream after its contraction
-// launch; since the contraction kernel holds every register of its SMs (512 threads x 128), they run
-// on the SMs it has left, between its launches.
-
+// Threads of a CTA of the separate energy launch (at most 96 registers, five CTAs per SM).  The energies of one batch
+// are launched on a second stream after its contraction launch; since the contraction kernel holds every
+// register of its SMs (512 threads x 128), they run on the SMs it has left, between its launches.
+constexpr int TNTHREAD = 128;
 
 struct TengyItem {
     int i, j, k, pairi, y, b0, c0;
@@ -1099,7 +1098,6 @@ struct TengyParams {
 // cp.async form: park f(B,C) (o = 0) and f(C,B) (o = 1) tiles of all eight f, W x (W + 1) doubles
 // each; column q of a tile is contiguous in f.  Every copy of a thread is issued before any is
 // waited for (zero fill outside nvir), so that a CTA keeps its whole 32 KB in flight.
-template <int TNTHREAD>
 __device__ __forceinline__ void tengy_park_cpasync(const TengyParams &P, const TengyItem &it, double *park)
 {
     constexpr int TP = TW + 1, TILE = TW * TP;
@@ -1120,7 +1118,6 @@ __device__ __forceinline__ void tengy_park_cpasync(const TengyParams &P, const T
 }
 
 // Energies of one item from its tiles parked by cp.async, summed over the CTA into its slot.
-template <int TNTHREAD>
 __device__ __forceinline__ void tengy_finish(const TengyParams &P, const TengyItem &it, const double *park, double *red)
 {
     const int tid = threadIdx.x;
@@ -1139,9 +1136,8 @@ __device__ __forceinline__ void tengy_finish(const TengyParams &P, const TengyIt
 }
 
 // CTA b takes items b, b + grid, ... (the launches use one CTA per item).
-template <int TNTHREAD, bool TMA>
-__global__ void __launch_bounds__(TNTHREAD, TNTHREAD == 128 ? 5 : 1)
-oz_tengy_kernel(const __grid_constant__ TengyParams P, int np, int npos)
+template <bool TMA>
+__global__ void __launch_bounds__(TNTHREAD, 5) oz_tengy_kernel(const __grid_constant__ TengyParams P, int np, int npos)
 {
     extern __shared__ __align__(16) double tsmem[];
     __shared__ double red[4 * (TNTHREAD / 32)];
@@ -1194,10 +1190,10 @@ oz_tengy_kernel(const __grid_constant__ TengyParams P, int np, int npos)
             __syncthreads();  // the park, the vectors and the reduction scratch are reused by the next item
             continue;
         }
-        // cp.async form (odd nvir)
+        // cp.async form: TRPDRV_OZ_TENGY_TMA=0, or where the tensor map cannot be encoded
         if (!tengy_decode(P.sys, P.pos0, (int)(w % np), (int)(w / np), it)) continue;  // uniform over the CTA
-        tengy_park_cpasync<TNTHREAD>(P, it, park);
-        tengy_finish<TNTHREAD>(P, it, park, red);
+        tengy_park_cpasync(P, it, park);
+        tengy_finish(P, it, park, red);
     }
 }
 
@@ -1294,7 +1290,8 @@ extern "C" int trpdrv_oz_dp(int nocc, int nvir) { return ((nvir + nocc) + 31) / 
 
 // Energies inside the contraction launch (the default for even nvir; the f tiles are read by TMA): the
 // kernel's energy warps compute the previous batch's energies while the tensor cores run this batch's
-// products; 1.3 % faster than the separate energy launch at (40, 300), 3.4 % at (30, 400), 7 slices.
+// products.  Odd nvir, whose f TMA could read here too since its columns are padded, keeps the separate launch, which
+// the tests hold it to.
 // TRPDRV_OZ_FUSED_ENERGY=0 (read at each call) selects the separate launch for every nvir.
 extern "C" int trpdrv_oz_fused_energy_supported(int nvir)
 {
@@ -1396,12 +1393,11 @@ extern "C" int trpdrv_launch_oz_gemm(const trpdrv_dev_system *h_sys, const trpdr
 }
 
 extern "C" int trpdrv_launch_oz_tengy(const trpdrv_dev_system *h_sys, int64_t pos0, int npos, const double *fbuf,
-                                      int threads, int *status, void *stream)
+                                      int *status, void *stream)
 {
     if (npos <= 0) return 0;
     const int np = oz::tengy_pairs(h_sys->nvir);
     if (np > h_sys->npairs * TRPDRV_FUSED_SLOTS) return (int)cudaErrorInvalidValue;
-    if (threads != 128 && threads != 256) return (int)cudaErrorInvalidValue;
     const long long items = (long long)np * npos;
     if (items > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
     oz::TengyParams P;
@@ -1415,14 +1411,10 @@ extern "C" int trpdrv_launch_oz_tengy(const trpdrv_dev_system *h_sys, int64_t po
     // over many items) was measured 30 % slower overall, too little memory parallelism per SM
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned grid = (unsigned)items;
-    if (tma && threads == 128)
-        oz::oz_tengy_kernel<128, true><<<grid, 128, oz::TSMEM_TMA_BYTES, st>>>(P, np, npos);
-    else if (tma)
-        oz::oz_tengy_kernel<256, true><<<grid, 256, oz::TSMEM_TMA_BYTES, st>>>(P, np, npos);
-    else if (threads == 128)
-        oz::oz_tengy_kernel<128, false><<<grid, 128, oz::TSMEM_BYTES, st>>>(P, np, npos);
+    if (tma)
+        oz::oz_tengy_kernel<true><<<grid, oz::TNTHREAD, oz::TSMEM_TMA_BYTES, st>>>(P, np, npos);
     else
-        oz::oz_tengy_kernel<256, false><<<grid, 256, oz::TSMEM_BYTES, st>>>(P, np, npos);
+        oz::oz_tengy_kernel<false><<<grid, oz::TNTHREAD, oz::TSMEM_BYTES, st>>>(P, np, npos);
     return (int)cudaGetLastError();
 }
 
@@ -1455,8 +1447,6 @@ extern "C" int trpdrv_oz_init(void)
     if ((e = oz::set_attr<7>()) != 0) return e;
     if ((e = oz::set_attr<8>()) != 0) return e;
     const cudaFuncAttribute dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if ((e = (int)cudaFuncSetAttribute(oz::oz_tengy_kernel<128, false>, dyn, (int)oz::TSMEM_BYTES)) != 0) return e;
-    if ((e = (int)cudaFuncSetAttribute(oz::oz_tengy_kernel<256, false>, dyn, (int)oz::TSMEM_BYTES)) != 0) return e;
-    if ((e = (int)cudaFuncSetAttribute(oz::oz_tengy_kernel<128, true>, dyn, (int)oz::TSMEM_TMA_BYTES)) != 0) return e;
-    return (int)cudaFuncSetAttribute(oz::oz_tengy_kernel<256, true>, dyn, (int)oz::TSMEM_TMA_BYTES);
+    if ((e = (int)cudaFuncSetAttribute(oz::oz_tengy_kernel<false>, dyn, (int)oz::TSMEM_BYTES)) != 0) return e;
+    return (int)cudaFuncSetAttribute(oz::oz_tengy_kernel<true>, dyn, (int)oz::TSMEM_TMA_BYTES);
 }

@@ -508,10 +508,11 @@ __global__ void __launch_bounds__(TNTHREAD, 4) tengy_batch_kernel(const __grid_c
 // 64-wide tiles where they fill the chip once over (two CTAs per SM) and cover not much more than 32-wide ones:
 // at equal padding they are 4 to 12 % faster (nvir = 300, 250, 111), with 1.31 times the area 13 % slower
 // (nvir = 200: 35.8 against 31.6 ms for all triples of nocc = 20).
+constexpr int SMS = 148;  // of a B200
 bool wide_tiles(int nvir, long long triples)
 {
     const long long n64 = (nvir + 63) / 64, n32 = (nvir + 31) / 32;
-    return n64 * n64 * 8 * triples >= 2 * 148 && 100 * 4 * n64 * n64 <= 115 * n32 * n32;
+    return n64 * n64 * 8 * triples >= 2 * SMS && 100 * 4 * n64 * n64 <= 115 * n32 * n32;
 }
 
 // Running pointers where their set-up pays, from eight copies a thread and panel of 32 rows on: nvir >= 64, or 32 if the
